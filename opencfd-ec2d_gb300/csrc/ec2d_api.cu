@@ -134,10 +134,10 @@ struct ec2d_ctx {
   int last_err = 0;
   // launch accounting and optional per-kernel event timing
   long long launches = 0;
-  int lusgs_cs = 0;  // LU-SGS wavefront shape: 0 four lanes per row where it fits, 1 one CTA per block, >1 a cluster
+  int lusgs_cs = 0;  // LU-SGS wavefront shape: 0 bands of eight (or four) lanes per row where they fit, 1 one CTA per block, >1 a cluster
   bool lusgs_fp32 = false;  // LU-SGS sweeps in FP32 (mixed-precision mode)
   bool concurrent = true;   // i- and j-face flux kernels on two streams
-  // test hook (EC2D_TEST_SILENT_BAND_EDGE): the band edges of the four-lane
+  // test hook (EC2D_TEST_SILENT_BAND_EDGE): the band edges of the banded
   // wavefront send nothing, so the downstream waits run out and report
   // EC2D_ERR_TIMEOUT; failure detection is tested without a GPU fault
   bool silent_band_edge = false;

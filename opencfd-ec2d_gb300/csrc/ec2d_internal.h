@@ -35,6 +35,12 @@ void launch_bc(const Lvl &L, int phases, cudaStream_t s);
 void launch_bc_normals(const Lvl &L, int max_nodes, cudaStream_t s);
 // k_lusgs.cu
 void launch_lusgs(const Lvl &L, double alfa1, cudaStream_t s);
+// k_sweep_push.cu: the eight-lane banded wavefront, its record builder and
+// the doubles of its record per cell and pass
+int push_record(int nv);
+bool push_fits(const Lvl &L, int update, int max_rows, int max_cols, int rmax);
+void launch_push_prep(const Lvl &L, double alfa1, int update, int force, cudaStream_t s);
+void launch_push(const Lvl &L, int update, int max_rows, int max_cols, int rmax, cudaStream_t s);
 // k_sweep.cu
 int lusgs_planes(int nv);
 // mode bits of the wavefront launchers: update U in the sweep, and take

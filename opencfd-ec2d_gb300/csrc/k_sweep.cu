@@ -1,5 +1,6 @@
 // k_sweep.cu -- the LU-SGS operator (du_LU_SGS_2D, sub_LU_SGS.f90:4-108) as a
-// latency-optimised wavefront.
+// latency-optimised wavefront, with one or four lanes per row, and the choice
+// of the wavefront's shape; the eight-lane form is in k_sweep_push.cu.
 //
 // The Gauss-Seidel order of the reference is kept exactly: the forward sweep
 // visits hyperplanes p = i+j = 2..nx+ny-2, the backward sweep p = nx+ny-2..2,
@@ -54,7 +55,7 @@ constexpr int TILE = EC2D_TILE;
 //       normal flux is linear in n, so F_n(W, s) = 0.5 s F_n(W, n) and the
 //       constant half F_n(U_nb) of the difference moves into the record
 //  G1I..GCJ  (gamma - 1) times n1, n2 and cc of face i and j,
-//       the pressure coefficients of the multi-lane sweep, which ships
+//       the pressure coefficients of the four-lane sweep, which ships
 //       p / (gamma - 1)
 template <int NV>
 struct Rec {
@@ -76,7 +77,7 @@ struct Slot {
 };
 
 // at least Rec<NV>::N (26, 30, 32 for NV = 4, 5, 6) and the FP32 record
-int lusgs_planes(int nv) { return 3 * nv + 15; }
+int lusgs_planes(int nv) { return std::max(3 * nv + 15, push_record(nv)); }
 static_assert(Rec<4>::N <= 3 * 4 + 15 && Rec<5>::N <= 3 * 5 + 15 && Rec<6>::N <= 3 * 6 + 15, "record planes");
 
 // normal flux of the Euler part (+ convected turbulence variables), the F(U)
@@ -532,26 +533,24 @@ void launch_lanes(const Lvl &L, int update, int R, cudaStream_t s) {
   else k_lusgs_sweep_lanes<NV, false, LPR><<<L.nblk, th, smem, s>>>(L, R);
 }
 
-// ---- mean flow only (NV = 4): four or eight lanes per row, row bands -------
+// ---- mean flow only (NV = 4): four lanes per row, row bands ----------------
 //
-// Lane q of a row owns variable q.  A neighbour's state is held as
+// The shape a host asks for with four lanes (bands of more than 16 rows by
+// default); eight lanes take the push form of k_sweep_push.cu.  Lane q of a row owns
+// variable q.  A neighbour's state is held as
 // X = (rho, rho u, rho v, H = E + p) with u, v and p' = p / (gamma - 1), so
 // that its flux plus dissipation in variable q is one pair of FMAs,
 // X_q w + p' g_q with w = u n1 + v n2 + cc and g = (gamma - 1) (0, n1, n2,
-// -cc) taken from the record (E w + p un = H w - p cc).  With four lanes per
-// row a lane adds both neighbours: 18 FP64 operations per cell and lane (2 x
-// 4 for the neighbours, one for the update, and rcp(rho), u, v, p', H of the
-// new state, formed by every lane of the row after the four variables are
-// gathered by shuffles).  With eight, lanes 0-3 add the row's own previous
-// cell and lanes 4-7 the neighbouring row on operands selected per lane (one
-// FP64 instruction stream for both halves), and a shuffle-add joins them:
-// 15 operations.  A CTA holds at most 32 rows of four lanes or 16 of eight
-// (up to four warps, one per SM sub-partition); a block with more rows is
-// split into bands of R rows on the CTAs of a cluster.  The band edge does
-// not wait for a barrier: the edge row of the upstream band writes each new
-// state straight into the downstream CTA's inbox (one 64-byte entry and one
-// mbarrier per column, through distributed shared memory), and the
-// downstream edge row waits for that column's entry only, so the bands run
+// -cc) taken from the record (E w + p un = H w - p cc).  A lane adds both
+// neighbours: 18 FP64 operations per cell and lane (2 x 4 for the neighbours,
+// one for the update, and rcp(rho), u, v, p', H of the new state, formed by
+// every lane of the row after the four variables are gathered by shuffles).
+// A CTA holds at most 32 rows (four warps, one per SM sub-partition); a block
+// with more rows is split into bands of R rows on the CTAs of a cluster.  The
+// band edge does not wait for a barrier: the edge row of the upstream band
+// writes each new state straight into the downstream CTA's inbox (one 64-byte
+// entry and one mbarrier per column, through distributed shared memory), and
+// the downstream edge row waits for that column's entry only, so the bands run
 // as a pipeline a few planes apart.  The per-lane pressure coefficient g_q
 // is a record field picked by a per-lane offset and masked or sign-flipped
 // with integer operations, so the lanes of a row need no branches or FP64
@@ -559,74 +558,38 @@ void launch_lanes(const Lvl &L, int update, int R, cudaStream_t s) {
 constexpr int QROWS = 32;        // rows per CTA
 constexpr int QCOLS = 1024;      // cells per row the inboxes hold
 constexpr int QWAIT = 1 << 20;   // polls of an inbox mbarrier before the wait gives up (about 20 ms)
+constexpr int QL = 4;            // lanes per row
+// doubles per row of a slot and per inbox entry: rho, rho u, rho v, H, u, v,
+// p / (gamma - 1), one spare
+constexpr int QS = 8;
 
 struct QRec {
   double a, u, c0, ki, kj;  // ki, kj: the lane's raw coefficient field of face i and j
   double2 c, ia, ni, nj;    // (0.5 Lc + Lv) i / j, 1/alfa, scaled normals of face i and j
-  double at[2], ut[2], c0t[2];  // NV = 5, 6: the turbulence rows' A, U and C0
-  double ia5;                   // NV = 5: 1/(alfa + Lv) of the SA row
 };
-// doubles per row of a slot and per inbox entry: rho, rho u, rho v, H (or E),
-// u, v, p / (gamma - 1), one spare; then U + dU and dU of each turbulence
-// variable (NV = 5: nu~; 6: k, omega)
-template <int NV>
-constexpr int qslot() { return 8 + 2 * (NV - 4); }
 // per-lane record offsets of the pressure coefficient g_q: (gamma - 1) n1
 // (q = 1), n2 (q = 2), cc (q = 3, sign flipped below), any field for q = 0
 // (zeroed)
 struct QLane {
   int offi, offj;
   unsigned keep, sign;
-  // eight lanes per row: the half's own face (i for lanes 0-3, j for 4-7)
-  int offk, offn, offc;
-  bool own;
 };
-template <int NV = 4>
-__device__ __forceinline__ QLane qlane(int q, bool own = true) {
-  using RC = Rec<NV>;
+__device__ __forceinline__ QLane qlane(int q) {
+  using RC = Rec<4>;
   QLane l;
   l.offi = q == 1 ? RC::G1I : q == 2 ? RC::G2I : RC::GCI;
   l.offj = q == 1 ? RC::G1J : q == 2 ? RC::G2J : RC::GCJ;
   l.keep = q == 0 ? 0u : 0xffffffffu;
   l.sign = q == 3 ? 0x80000000u : 0u;
-  l.own = own;
-  l.offk = own ? l.offi : l.offj;
-  l.offn = own ? RC::N1I : RC::N1J;
-  l.offc = own ? RC::CI : RC::CJ;
   return l;
 }
 // g_q from the raw field by integer operations only (zero for q = 0, negated for q = 3)
 __device__ __forceinline__ double qcoef(double x, const QLane &l) {
   return __hiloint2double((__double2hiint(x) & (int)l.keep) ^ (int)l.sign, __double2loint(x) & (int)l.keep);
 }
-// four lanes per row load both faces' fields; eight load their half's face
-// only (into ki, ni, c.x) and the fields their half uses
-template <bool FWD, bool update, int LPR = 4, int NV = 4>
+template <bool FWD, bool update>
 __device__ __forceinline__ void qload(QRec &r, const double *rec, int q, const QLane &l) {
-  using RC = Rec<NV>;
-  if (LPR == 8) {
-    if (!FWD || l.own) r.a = __ldcg(rec + RC::A + q);
-    if (FWD || !update) r.u = __ldcg(rec + RC::U + q);
-    if (!FWD && l.own) r.c0 = __ldcg(rec + RC::C0 + q);
-    r.ki = __ldcg(rec + l.offk);
-    if (NV == 5) {
-      // the normals sit at odd offsets of a 5-variable record: two 8-byte loads
-      r.ni.x = __ldcg(rec + l.offn);
-      r.ni.y = __ldcg(rec + l.offn + 1);
-      r.ia5 = __ldcg(rec + RC::IA5);
-    } else {
-      r.ni = __ldcg(reinterpret_cast<const double2 *>(rec + l.offn));
-    }
-#pragma unroll
-    for (int t = 0; t < NV - 4; t++) {
-      r.at[t] = __ldcg(rec + RC::A + 4 + t);
-      r.ut[t] = __ldcg(rec + RC::U + 4 + t);
-      if (!FWD) r.c0t[t] = __ldcg(rec + RC::C0 + 4 + t);
-    }
-    r.c.x = __ldcg(rec + l.offc);
-    r.ia.x = __ldcg(rec + RC::IA);
-    return;
-  }
+  using RC = Rec<4>;
   r.a = __ldcg(rec + RC::A + q);
   if (FWD || !update) r.u = __ldcg(rec + RC::U + q);
   if (!FWD) r.c0 = __ldcg(rec + RC::C0 + q);
@@ -641,8 +604,7 @@ __device__ __forceinline__ void qload(QRec &r, const double *rec, int q, const Q
 // Inbox entries arrive by st.async, each 16-byte store counting its bytes on
 // the entry's mbarrier in the receiving CTA: no fence on the sending side.
 // The receiver arms every entry's mbarrier at start-up (one arrival expecting
-// the entry's bytes: 64, or 80 / 96 with the SA / SST rows), so phase 0
-// completes when the entry has landed.
+// the entry's 64 bytes), so phase 0 completes when the entry has landed.
 __device__ __forceinline__ void qarm(unsigned long long *mb, unsigned bytes) {
   const unsigned a = (unsigned)__cvta_generic_to_shared(mb);
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(1) : "memory");
@@ -682,20 +644,14 @@ struct QBand {
 // has three planes to arrive, enough for a read that crosses to the other
 // die's L2.  The band-edge state goes to the next band by st.async, its
 // bytes counted on the receiving entry's mbarrier (no fence on this side).
-// NV = 5, 6 (eight lanes only): every lane also carries the turbulence
-// rows, the upstream neighbour of its half adding F_n(X_2) + (0.5 Lc + Lv) dX
-// as the one-lane sweep does; lane q = 0 of the leading half stores them.
-template <bool update, bool FWD, int LPR, int NV = 4>
+template <bool update, bool FWD>
 __device__ __forceinline__ void qpass(const Lvl &L, const BlkDev &bd, const QBand &B, double *slot, double *inbox,
                                       unsigned long long *mbar, unsigned rbox, unsigned rmbar, const double *rsrc,
                                       double *recBw, double gm1) {
-  using RC = Rec<NV>;
-  constexpr int QS = qslot<NV>();
-  static_assert(NV == 4 || LPR == 8, "the turbulence rows ride on the eight-lane form only");
-  constexpr int NT = NV - 4;  // turbulence rows
+  using RC = Rec<4>;
   const int R = B.R, rl = B.rl, q = B.q, j = B.j, rows = B.rows, ni = B.ni;
   const long long F = L.F;
-  const QLane ln = qlane<NV>(q, LPR == 4 || !((threadIdx.x >> 2) & 1));
+  const QLane ln = qlane(q);
   // this row's neighbour across the band edge comes through the inbox; the
   // band's edge row feeds the next band's inbox
   const bool from_box = B.row_ok && (FWD ? (rl == 0 && B.rank > 0) : (rl == R - 1 && (int)B.rank + 1 < B.CS && j < rows));
@@ -714,96 +670,42 @@ __device__ __forceinline__ void qpass(const Lvl &L, const BlkDev &bd, const QBan
     for (int c = 0; c < 3; c++) {
       if (c >= ni) break;
       const int m = (m0 + c) & 3;
-      if (m == 0) qload<FWD, update, LPR, NV>(r0, src(c), q, ln);
-      else if (m == 1) qload<FWD, update, LPR, NV>(r1, src(c), q, ln);
-      else if (m == 2) qload<FWD, update, LPR, NV>(r2, src(c), q, ln);
-      else qload<FWD, update, LPR, NV>(r3, src(c), q, ln);
+      if (m == 0) qload<FWD, update>(r0, src(c), q, ln);
+      else if (m == 1) qload<FWD, update>(r1, src(c), q, ln);
+      else if (m == 2) qload<FWD, update>(r2, src(c), q, ln);
+      else qload<FWD, update>(r3, src(c), q, ln);
     }
   }
   double wx = 0.0, wu = 0.0, wv = 0.0, wp = 0.0;  // the row's previous cell
-  double wt[2] = {0.0, 0.0}, wd[2] = {0.0, 0.0};   // and its turbulence X + dX, dX
   int gave_up = 0;                                 // first column whose inbox wait gave up
-  const int gl = (threadIdx.x & 31) & ~(LPR - 1);  // the row's first lane
-  // eight lanes per row: lanes 0-3 take the row's own previous cell, lanes
-  // 4-7 the neighbouring row; four lanes per row take both
-  const bool own_nb = LPR == 4 || !((threadIdx.x >> 2) & 1), row_nb = LPR == 4 || !own_nb;
-  const bool lead = LPR == 4 || own_nb;  // stores and sends
+  const int gl = (threadIdx.x & 31) & ~(QL - 1);   // the row's first lane
   // cur: this plane's record; ahead: the set three planes on (free since the last plane)
   auto plane = [&](int p, const QRec &cur, QRec &ahead) {
     const int i = p - j, buf = p & 1;
     const bool act = B.row_ok && i >= 1 && i <= ni;
     const int k = FWD ? i - 1 : ni - i;
-    if (act && k + 3 < ni) qload<FWD, update, LPR, NV>(ahead, src(k + 3), q, ln);
-    double acc = 0.0, acct[2] = {0.0, 0.0};
+    if (act && k + 3 < ni) qload<FWD, update>(ahead, src(k + 3), q, ln);
+    double st = 0.0, dn = 0.0;
     if (act) {
-      if (LPR == 4) {
-        acc = FWD ? cur.a : cur.c0;
-        if (FWD ? (i > 1) : (i < ni)) {
-          const double w = fma(wu, cur.ni.x, fma(wv, cur.ni.y, cur.c.x));
-          acc = fma(wx, w, fma(wp, qcoef(cur.ki, ln), acc));
-        }
-        if (FWD ? (j > 1) : (j < rows)) {
-          const double *s;
-          if (from_box) {
-            // after one wait has given up the row no longer waits (its results
-            // are void; the step reports EC2D_ERR_TIMEOUT)
-            if (!gave_up && !qwait(mbar + i - 1)) gave_up = i;
-            s = inbox + (size_t)(i - 1) * QS;
-          } else {
-            s = slot + ((size_t)(buf ^ 1) * R + (FWD ? rl - 1 : rl + 1)) * QS;
-          }
-          const double2 uv = *reinterpret_cast<const double2 *>(s + 4);
-          const double sp = s[6], sx = s[q];
-          const double w = fma(uv.x, cur.nj.x, fma(uv.y, cur.nj.y, cur.c.y));
-          acc = fma(sx, w, fma(sp, qcoef(cur.kj, ln), acc));
-        }
-      } else {
-        // both halves run the same FP64 instructions on their own operands
-        const double *s = slot + ((size_t)(buf ^ 1) * R + min(max(FWD ? rl - 1 : rl + 1, 0), R - 1)) * QS;
-        if (row_nb && from_box) {
+      double acc = FWD ? cur.a : cur.c0;
+      if (FWD ? (i > 1) : (i < ni)) {
+        const double w = fma(wu, cur.ni.x, fma(wv, cur.ni.y, cur.c.x));
+        acc = fma(wx, w, fma(wp, qcoef(cur.ki, ln), acc));
+      }
+      if (FWD ? (j > 1) : (j < rows)) {
+        const double *s;
+        if (from_box) {
+          // after one wait has given up the row no longer waits (its results
+          // are void; the step reports EC2D_ERR_TIMEOUT)
           if (!gave_up && !qwait(mbar + i - 1)) gave_up = i;
           s = inbox + (size_t)(i - 1) * QS;
+        } else {
+          s = slot + ((size_t)(buf ^ 1) * R + (FWD ? rl - 1 : rl + 1)) * QS;
         }
         const double2 uv = *reinterpret_cast<const double2 *>(s + 4);
         const double sp = s[6], sx = s[q];
-        const bool has = own_nb ? (FWD ? (i > 1) : (i < ni)) : (FWD ? (j > 1) : (j < rows));
-        const double X = own_nb ? wx : sx, Uu = own_nb ? wu : uv.x, Vv = own_nb ? wv : uv.y, P = own_nb ? wp : sp;
-        // the record fields of this half's face (loaded per half)
-        acc = own_nb ? (FWD ? cur.a : cur.c0) : 0.0;
-#pragma unroll
-        for (int t = 0; t < NT; t++) acct[t] = own_nb ? (FWD ? cur.at[t] : cur.c0t[t]) : 0.0;
-        if (has) {
-          const double w = fma(Uu, cur.ni.x, fma(Vv, cur.ni.y, cur.c.x));
-          acc = fma(X, w, fma(P, qcoef(cur.ki, ln), acc));
-          if (NT > 0) {
-            // F_n(X_2) + (0.5 Lc + Lv) dX: the dissipation on the increment,
-            // as the one-lane sweep (add_shipped) forms it
-            const double un = fma(Uu, cur.ni.x, Vv * cur.ni.y);
-#pragma unroll
-            for (int t = 0; t < NT; t++) {
-              const double T2 = own_nb ? wt[t] : s[8 + 2 * t], D2 = own_nb ? wd[t] : s[9 + 2 * t];
-              acct[t] = fma(cur.c.x, D2, fma(T2, un, acct[t]));
-            }
-          }
-        }
-      }
-    }
-    // eight lanes: the two halves of the row add their neighbours' terms
-    const double other = LPR == 8 ? __shfl_xor_sync(0xffffffffu, acc, 4) : 0.0;
-    double othert[2] = {0.0, 0.0};
-#pragma unroll
-    for (int t = 0; t < NT; t++) othert[t] = __shfl_xor_sync(0xffffffffu, acct[t], 4);
-    double st = 0.0, dn = 0.0, stt[2] = {0.0, 0.0}, dnt[2] = {0.0, 0.0};
-    if (act) {
-      if (LPR == 8) acc = acc + other;
-#pragma unroll
-      for (int t = 0; t < NT; t++) {
-        // the turbulence rows never take the fused U update (only the mean
-        // flow is carried as U + dU); the SA row has its own 1/alfa
-        const double inv = NV == 5 ? cur.ia5 : cur.ia.x;
-        const double a = acct[t] + othert[t];
-        dnt[t] = FWD ? a * inv : fma(a, inv, cur.at[t]);
-        stt[t] = cur.ut[t] + dnt[t];
+        const double w = fma(uv.x, cur.nj.x, fma(uv.y, cur.nj.y, cur.c.y));
+        acc = fma(sx, w, fma(sp, qcoef(cur.kj, ln), acc));
       }
       if (update) {
         // U + dU* going forward (carried in the backward record), U + dU* + dU** going backward
@@ -821,45 +723,26 @@ __device__ __forceinline__ void qpass(const Lvl &L, const BlkDev &bd, const QBan
       const double pr = fma(-0.5, fma(s2, v, s1 * u), s3);  // p / (gamma - 1)
       const double H = fma(gm1, pr, s3);
       const double x = q == 3 ? H : st;
-      if (to_box && lead && q == 0) {
+      if (to_box && q == 0) {
         const unsigned a = rbox + 8u * QS * (unsigned)(i - 1), m = rmbar + 8u * (unsigned)(i - 1);
         qsend2(a, s0, s1, m);
         qsend2(a + 16u, s2, H, m);
         qsend2(a + 32u, u, v, m);
         qsend2(a + 48u, pr, 0.0, m);
-#pragma unroll
-        for (int t = 0; t < NT; t++) qsend2(a + 64u + 16u * t, stt[t], dnt[t], m);
       }
       double *o = slot + ((size_t)buf * R + rl) * QS;
-      if (lead) o[q] = x;
-      if (lead && q == 0) *reinterpret_cast<double2 *>(o + 4) = make_double2(u, v);
-      if (lead && q == 1) o[6] = pr;
-#pragma unroll
-      for (int t = 0; t < NT; t++) {
-        if (lead && q == 2 + t) *reinterpret_cast<double2 *>(o + 8 + 2 * t) = make_double2(stt[t], dnt[t]);
-        wt[t] = stt[t];
-        wd[t] = dnt[t];
-      }
+      o[q] = x;
+      if (q == 0) *reinterpret_cast<double2 *>(o + 4) = make_double2(u, v);
+      if (q == 1) o[6] = pr;
       wx = x; wu = u; wv = v; wp = pr;
-      if (lead) {
-        if (FWD) {
-          recBw[(size_t)(i - 1) * RC::N + RC::A + q] = update ? st : dn;
-#pragma unroll
-          for (int t = 0; t < NT; t++)
-            if (q == 0) recBw[(size_t)(i - 1) * RC::N + RC::A + 4 + t] = dnt[t];
-        } else {
-          // an updating sweep writes U only (DU is read nowhere but inside
-          // du_LU_SGS_2D and the update that follows it)
-          const long long id = bd.off + (long long)(j + 2) * bd.P + (i + 2);
-          if (update) L.U[q * F + id] = st;
-          else L.du[q * F + id] = dn;
-#pragma unroll
-          for (int t = 0; t < NT; t++)
-            if (q == 0) {
-              if (update) L.U[(4 + t) * F + id] = stt[t];
-              else L.du[(4 + t) * F + id] = dnt[t];
-            }
-        }
+      if (FWD) {
+        recBw[(size_t)(i - 1) * RC::N + RC::A + q] = update ? st : dn;
+      } else {
+        // an updating sweep writes U only (DU is read nowhere but inside
+        // du_LU_SGS_2D and the update that follows it)
+        const long long id = bd.off + (long long)(j + 2) * bd.P + (i + 2);
+        if (update) L.U[q * F + id] = st;
+        else L.du[q * F + id] = dn;
       }
     }
     __syncthreads();
@@ -874,11 +757,10 @@ __device__ __forceinline__ void qpass(const Lvl &L, const BlkDev &bd, const QBan
   if (gave_up) set_status(L.status + 4 * bd.cas, 4, B.bk, gave_up, j);
 }
 
-template <bool update, int LPR, int NV = 4>
-__global__ void __launch_bounds__(4 * QROWS, 1) k_lusgs_sweep_quad(Lvl L, int R, int CS) {
+template <bool update>
+__global__ void __launch_bounds__(QL * QROWS, 1) k_lusgs_sweep_quad(Lvl L, int R, int CS) {
   // [2][R][QS] slots | inbox F [ni][QS] | inbox B | mbarriers F [ni] | B
   extern __shared__ __align__(16) double sh[];
-  constexpr int QS = qslot<NV>();
   QBand B;
   B.rank = CS > 1 ? cluster_rank() : 0u;
   B.bk = blockIdx.x / CS;
@@ -886,7 +768,7 @@ __global__ void __launch_bounds__(4 * QROWS, 1) k_lusgs_sweep_quad(Lvl L, int R,
   B.R = R; B.CS = CS;
   B.rows = bd.ny - 1;
   B.ni = bd.nx - 1;
-  B.rl = threadIdx.x / LPR;
+  B.rl = threadIdx.x / QL;
   B.q = threadIdx.x & 3;
   B.j = (int)B.rank * R + B.rl + 1;
   B.row_ok = B.rl < R && B.j <= B.rows;
@@ -904,107 +786,85 @@ __global__ void __launch_bounds__(4 * QROWS, 1) k_lusgs_sweep_quad(Lvl L, int R,
     cluster_barrier();  // every inbox armed before any CTA writes into one
   }
   const int jr = B.row_ok ? B.j : 1;  // record pointers of idle rows stay in the array
-  const double *recF = L.rec + ((size_t)bd.cell0 + (size_t)(jr - 1) * ni) * Rec<NV>::N;
-  const double *recB = recF + (size_t)L.ncell * Rec<NV>::N;
-  double *recBw = L.rec + ((size_t)L.ncell + bd.cell0 + (size_t)(jr - 1) * ni) * Rec<NV>::N;
-  qpass<update, true, LPR, NV>(L, bd, B, slot, inF, mbF, rboxF, rmbF, recF, recBw, gm1);
-  qpass<update, false, LPR, NV>(L, bd, B, slot, inB, mbB, rboxB, rmbB, recB, recBw, gm1);
+  const double *recF = L.rec + ((size_t)bd.cell0 + (size_t)(jr - 1) * ni) * Rec<4>::N;
+  const double *recB = recF + (size_t)L.ncell * Rec<4>::N;
+  double *recBw = L.rec + ((size_t)L.ncell + bd.cell0 + (size_t)(jr - 1) * ni) * Rec<4>::N;
+  qpass<update, true>(L, bd, B, slot, inF, mbF, rboxF, rmbF, recF, recBw, gm1);
+  qpass<update, false>(L, bd, B, slot, inB, mbB, rboxB, rmbB, recB, recBw, gm1);
   if (CS > 1) cluster_barrier();  // no CTA leaves while a neighbour may still write into it
 }
 
-// the four- and eight-lane kernel serves NV = 4 levels (and NV = 5 with eight
-// lanes) whose blocks have at most 16 bands of rows and QCOLS cells per row, when every CTA of the launch
-// gets an SM of its own (with fewer SMs, one lane per row needs fewer FP64
-// instructions) and the device can hold one of its clusters
-// rmax: most rows per CTA (4..32); lanes: lanes per row (4 or 8; 0: eight up
-// to 16 rows, four above).  Clusters of more than 8 CTAs are non-portable
-// sizes, asked for explicitly.
-int quad_ctas(int max_rows, int rmax) {
-  rmax = std::max(4, std::min(rmax, QROWS));
-  return (max_rows + rmax - 1) / rmax;
-}
-static int quad_lanes(int rmax, int lanes) { return lanes == 4 || lanes == 8 ? lanes : (rmax <= 16 ? 8 : 4); }
-static void (*quad_kernel(int lpr, int update, int nv))(Lvl, int, int) {
-  if (nv == 5) return update ? k_lusgs_sweep_quad<true, 8, 5> : k_lusgs_sweep_quad<false, 8, 5>;
-  if (nv == 6) return update ? k_lusgs_sweep_quad<true, 8, 6> : k_lusgs_sweep_quad<false, 8, 6>;
-  return lpr == 8 ? (update ? k_lusgs_sweep_quad<true, 8> : k_lusgs_sweep_quad<false, 8>)
-                  : (update ? k_lusgs_sweep_quad<true, 4> : k_lusgs_sweep_quad<false, 4>);
-}
+// the four-lane kernel serves NV = 4 levels whose blocks have at most 16 bands
+// of rows and QCOLS cells per row, when every CTA of the launch gets an SM of
+// its own (with fewer SMs, one lane per row needs fewer FP64 instructions) and
+// the device can hold one of its clusters
+// rmax: most rows per CTA (4..32).  Clusters of more than 8 CTAs are
+// non-portable sizes, asked for explicitly.
 struct QuadShape {
-  int CS, R, lpr, th, nv;
+  int CS, R, th;
   size_t smem;
 };
-static QuadShape quad_shape(int max_rows, int max_cols, int rmax, int lanes, int nv) {
+static QuadShape quad_shape(int max_rows, int max_cols, int rmax) {
   QuadShape q;
-  q.CS = quad_ctas(max_rows, rmax);
+  rmax = std::max(4, std::min(rmax, QROWS));
+  q.CS = (max_rows + rmax - 1) / rmax;
   q.R = (max_rows + q.CS - 1) / q.CS;
-  q.lpr = nv > 4 ? 8 : quad_lanes(rmax, lanes);
-  q.nv = nv;
-  q.th = (q.lpr * q.R + 31) / 32 * 32;
-  const size_t qs = 8 + 2 * (nv - 4);  // qslot<NV>()
-  q.smem = (size_t)2 * q.R * qs * sizeof(double) + (q.CS > 1 ? (size_t)max_cols * 2 * (qs * sizeof(double) + 8) : 0);
+  q.th = (QL * q.R + 31) / 32 * 32;
+  q.smem = (size_t)2 * q.R * QS * sizeof(double) + (q.CS > 1 ? (size_t)max_cols * 2 * (QS * sizeof(double) + 8) : 0);
   return q;
 }
 // the kernel's attributes for a launch of this shape (dynamic shared memory
 // beyond 48 KiB, cluster sizes beyond 8)
 static void quad_attributes(const QuadShape &q) {
-  for (int update = 0; update < 2; update++) {
-    auto kern = quad_kernel(q.lpr, update, q.nv);
+  for (auto kern : {k_lusgs_sweep_quad<true>, k_lusgs_sweep_quad<false>}) {
     if (q.smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)q.smem);
     if (q.CS > 8) cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   }
 }
-bool quad_fits(const Lvl &L, int max_rows, int max_cols, int rmax, int lanes) {
-  static int nsm = 0;
-  if (!nsm) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  }
-  const QuadShape q = quad_shape(max_rows, max_cols, rmax, lanes, L.nvar);
-  // NV = 5, 6 ride on eight lanes per row, so at most 16 rows per band
-  const bool nv_ok = L.nvar == 4 || (L.nvar <= 6 && std::max(4, std::min(rmax, QROWS)) <= 16 && lanes != 4);
-  if (!(nv_ok && max_rows >= 1 && q.CS <= 16 && max_cols <= QCOLS && L.nblk * q.CS <= nsm)) return false;
-  if (q.CS <= 8) return true;
-  // a non-portable cluster size: launchable only if the device can place one
-  quad_attributes(q);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(L.nblk * q.CS);
-  cfg.blockDim = dim3(q.th);
-  cfg.dynamicSmemBytes = q.smem;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = q.CS;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  int nclusters = 0;
-  const bool ok = cudaOccupancyMaxActiveClusters(&nclusters, quad_kernel(q.lpr, 1, q.nv), &cfg) == cudaSuccess &&
-                  nclusters >= 1;
-  cudaGetLastError();  // a refused query leaves no error behind
-  return ok;
-}
-
-// eight lanes per row: 15 FP64 operations per cell and lane; four: 18
-void launch_quad(const Lvl &L, int update, int max_rows, int max_cols, int rmax, int lanes, cudaStream_t s) {
-  const QuadShape q = quad_shape(max_rows, max_cols, rmax, lanes, L.nvar);
-  quad_attributes(q);
-  auto kern = quad_kernel(q.lpr, update, q.nv);
+static cudaLaunchConfig_t quad_config(const Lvl &L, const QuadShape &q, cudaLaunchAttribute *attr, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(L.nblk * q.CS);
   cfg.blockDim = dim3(q.th);
   cfg.dynamicSmemBytes = q.smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = q.CS;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kern, L, q.R, q.CS);
+  return cfg;
 }
+static bool quad_fits(const Lvl &L, int max_rows, int max_cols, int rmax) {
+  static const int nsm = [] {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n;
+  }();
+  const QuadShape q = quad_shape(max_rows, max_cols, rmax);
+  if (!(L.nvar == 4 && max_rows >= 1 && q.CS <= 16 && max_cols <= QCOLS && L.nblk * q.CS <= nsm)) return false;
+  if (q.CS <= 8) return true;
+  // a non-portable cluster size: launchable only if the device can place one
+  quad_attributes(q);
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = quad_config(L, q, attr, nullptr);
+  int nclusters = 0;
+  const bool ok = cudaOccupancyMaxActiveClusters(&nclusters, k_lusgs_sweep_quad<true>, &cfg) == cudaSuccess &&
+                  nclusters >= 1;
+  cudaGetLastError();  // a refused query leaves no error behind
+  return ok;
+}
+static void launch_quad(const Lvl &L, int update, int max_rows, int max_cols, int rmax, cudaStream_t s) {
+  const QuadShape q = quad_shape(max_rows, max_cols, rmax);
+  quad_attributes(q);
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = quad_config(L, q, attr, s);
+  if (update) cudaLaunchKernelEx(&cfg, k_lusgs_sweep_quad<true>, L, q.R, q.CS);
+  else cudaLaunchKernelEx(&cfg, k_lusgs_sweep_quad<false>, L, q.R, q.CS);
+}
+// lanes per row of a band of at most rmax rows (lanes 0: eight up to 16 rows)
+static int quad_lanes(int rmax, int lanes) { return lanes == 4 || lanes == 8 ? lanes : (rmax <= 16 ? 8 : 4); }
 
 // CS == 1: one CTA per block, planes separated by __syncthreads.
 // CS > 1: a cluster of CS CTAs per block, CTA r owns rows r*R+1..r*R+R; the
@@ -1045,21 +905,30 @@ size_t smem_bytes(int R, int th) {
 template <int NV>
 void sweep_nv(const Lvl &L, double alfa1, int mode, int max_rows, int max_cols, int cs, int rpw, int lanes,
               cudaStream_t s) {
-  if (!(mode & LUSGS_SWEEP_ONLY)) k_lusgs_prep<NV><<<L.nctiles, TILE, 0, s>>>(L, alfa1, mode & LUSGS_FORCE);
-  if (mode & LUSGS_PREP_ONLY) return;
-  const int update = mode & LUSGS_UPDATE;
+  const int update = mode & LUSGS_UPDATE, force = mode & LUSGS_FORCE;
+  const bool prep = !(mode & LUSGS_SWEEP_ONLY), sweep = !(mode & LUSGS_PREP_ONLY);
   if (cs == 0) {
-    // the requested band height and lanes, else four-lane bands of 24 or 32 rows
-    for (int r : {rpw, 24, 32}) {
-      const int ln = r == rpw ? lanes : 0;
-      if (quad_fits(L, max_rows, max_cols, r, ln)) {
-        launch_quad(L, update, max_rows, max_cols, r, ln, s);
-        return;
-      }
+    // the requested band height and lanes, else other heights: eight lanes
+    // where the shared memory holds the records and inboxes of its warps, four
+    // where it does not (long rows in tall bands)
+    const bool eight = quad_lanes(rpw, NV > 4 ? 8 : lanes) == 8;
+    for (int r : {rpw, 8, 16, 24, 32}) {
+      if (!eight || !push_fits(L, update, max_rows, max_cols, r)) continue;
+      if (prep) launch_push_prep(L, alfa1, update, force, s);
+      if (sweep) launch_push(L, update, max_rows, max_cols, r, s);
+      return;
+    }
+    for (int r : {eight ? 24 : rpw, 24, 32}) {
+      if (!quad_fits(L, max_rows, max_cols, r)) continue;
+      if (prep) k_lusgs_prep<NV><<<L.nctiles, TILE, 0, s>>>(L, alfa1, force);
+      if (sweep) launch_quad(L, update, max_rows, max_cols, r, s);
+      return;
     }
     cs = 1;  // one CTA per block, full warps
     rpw = 32;
   }
+  if (prep) k_lusgs_prep<NV><<<L.nctiles, TILE, 0, s>>>(L, alfa1, force);
+  if (!sweep) return;
   const int lpr = sweep_lanes_per_row(max_rows);
   if (lpr == 4) { launch_lanes<NV, 4>(L, update, max_rows, s); return; }
   int CS = std::max(1, std::min(cs, std::min(8, (max_rows + 7) / 8)));
