@@ -2068,7 +2068,7 @@ int ec2d_mlp_train(ec2d_mlp *m, int steps, int batch, double lr, double *loss_ou
   if (!m || steps < 0 || batch < 256 || batch % 256 || !(lr > 0.0) || m->net.nsamp < 1) return EC2D_ERR_ARG;
   Net &net = m->net;
   cudaSetDevice(net.device);
-  if (net.ensure_batch(batch)) return EC2D_ERR_NOMEM;
+  if (net.fused() ? net.ensure_fused(batch) : net.ensure_batch(batch)) return EC2D_ERR_NOMEM;
   // one training step as a CUDA graph (its minibatch seed and Adam step count
   // live in device memory), re-recorded when batch, rate or GEMM path change
   if (!net.train_graph || net.graph_batch != batch || net.graph_lr != (float)lr || net.graph_kind != net.gemm_kind) {
@@ -2076,10 +2076,7 @@ int ec2d_mlp_train(ec2d_mlp *m, int steps, int batch, double lr, double *loss_ou
     net.train_graph = nullptr;
     CK(cudaStreamSynchronize(net.stream));
     CK(cudaStreamBeginCapture(net.stream, cudaStreamCaptureModeThreadLocal));
-    net.gather(batch);
-    net.forward(batch);
-    net.backward(batch);
-    net.adam((float)lr);
+    net.train_step(batch, (float)lr);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(net.stream, &g);
     if (e == cudaSuccess && g) e = cudaGraphInstantiate(&net.train_graph, g, 0);
@@ -2096,10 +2093,7 @@ int ec2d_mlp_train(ec2d_mlp *m, int steps, int batch, double lr, double *loss_ou
     if (net.train_graph) {
       CK(cudaGraphLaunch(net.train_graph, net.stream));
     } else {
-      net.gather(batch);
-      net.forward(batch);
-      net.backward(batch);
-      net.adam((float)lr);
+      net.train_step(batch, (float)lr);
     }
   }
   float l = 0.0f;
@@ -2212,14 +2206,18 @@ int ec2d_mlp_loss_grad(ec2d_mlp *m, const float *x, const float *y, int B, doubl
   if (!m || !x || !y || B < 256 || B % 256) return EC2D_ERR_ARG;
   Net &net = m->net;
   cudaSetDevice(net.device);
-  if (net.ensure_batch(B)) return EC2D_ERR_NOMEM;
+  if (net.ensure_batch(B) || (net.fused() && net.ensure_fused(B))) return EC2D_ERR_NOMEM;
   std::vector<__nv_bfloat16> xb((size_t)B * NIN_PAD, __float2bfloat16(0.0f));
   for (int r = 0; r < B; r++)
     for (int c = 0; c < NIN; c++) xb[(size_t)r * NIN_PAD + c] = __float2bfloat16(x[(size_t)r * NIN + c]);
   CK(cudaMemcpyAsync(net.X, xb.data(), xb.size() * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice, net.stream));
   CK(cudaMemcpyAsync(net.Y, y, (size_t)B * NOUT * sizeof(float), cudaMemcpyHostToDevice, net.stream));
-  net.forward(B);
-  net.backward(B);
+  if (net.fused()) {
+    net.fused_pass(B, FUSED_STAGED, false, 0.0f);
+  } else {
+    net.forward(B);
+    net.backward(B);
+  }
   float l = 0.0f;
   CK(cudaMemcpyAsync(&l, net.d_loss, sizeof(float), cudaMemcpyDeviceToHost, net.stream));
   CK(cudaStreamSynchronize(net.stream));

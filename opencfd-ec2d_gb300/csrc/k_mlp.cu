@@ -8,6 +8,9 @@
 // BF16, accumulation FP32 (the GEMM kernels), master weights and Adam moments
 // FP32.
 //
+// Width 256 with the tcgen05 path runs in the fused kernels of k_mlp_fused.cu;
+// other widths, and the mma.sync path, as the GEMMs here.
+//
 // Every GEMM is C[M x N] = A[M x K] . B[N x K]^T with both operands K-major
 // (row-major with K contiguous).  Backward passes materialise the transposes
 // they need (dZ^T, H^T, W^T) with a tiled transpose kernel, so one GEMM shape
@@ -272,19 +275,12 @@ __global__ void k_to_bf16(const float *__restrict__ w, int rows, int cols, __nv_
 
 // minibatch gather: rows idx = hash(step, k) mod n; standardised bf16 inputs
 // (32 columns, the 7 features then zeros) and standardised fp32 targets
-__device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
-  z += 0x9E3779B97F4A7C15ull;
-  z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-  z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-  return z ^ (z >> 31);
-}
 __global__ void k_gather(const float *__restrict__ feat, const float *__restrict__ targ, long long n, int B,
                          const int *__restrict__ step, unsigned long long seed, const float *__restrict__ nrm,
                          __nv_bfloat16 *__restrict__ X, float *__restrict__ Y) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= B) return;
-  unsigned long long h = mix64(seed ^ mix64(((unsigned long long)(*step) << 32) | (unsigned)k));
-  long long r = (long long)(h % (unsigned long long)n);
+  const long long r = gather_row(seed, *step, (unsigned)k, n);
   for (int c = 0; c < NIN_PAD; c++) {
     float x = 0.0f;
     if (c < NIN) x = (feat[r * NIN + c] - nrm[c]) / nrm[NIN + c];
@@ -507,6 +503,11 @@ int Net::init(int dev, int hidden, int w, unsigned long long seed_) {
     L[l].gb = dev_alloc<float>(owned, no);
     L[l].wb = dev_alloc<__nv_bfloat16>(owned, hw.size());
     L[l].wt = dev_alloc<__nv_bfloat16>(owned, hw.size());
+    if (w == 256) {
+      L[l].wk = dev_alloc<__nv_bfloat16>(owned, hw.size());
+      L[l].wtk = dev_alloc<__nv_bfloat16>(owned, hw.size());
+      if (!L[l].wk || !L[l].wtk) return 3;
+    }
     if (!L[l].w || !L[l].wt) return 3;
     cudaMemcpy(L[l].w, hw.data(), hw.size() * sizeof(float), cudaMemcpyHostToDevice);
   }
@@ -524,6 +525,10 @@ int Net::init(int dev, int hidden, int w, unsigned long long seed_) {
 }
 
 void Net::refresh_bf16() {
+  if (width == 256) {  // all copies, the packed ones among them
+    launch_mlp_pack(pack_args(), stream);
+    return;
+  }
   for (int l = 0; l < nlin; l++) {
     int ni = layer_in(l), no = layer_out(l);
     int n = ni * no;
@@ -551,6 +556,76 @@ int Net::ensure_batch(int B) {
   cpart = dev_alloc<float>(owned, (size_t)(B / 256 + 1) * W);
   lpart = dev_alloc<float>(owned, (size_t)(B / 256 + 1));
   return part ? 0 : 1;
+}
+
+PackArgs Net::pack_args() const {
+  PackArgs p{};
+  p.nlin = nlin;
+  p.b1 = ADAM_B1; p.b2 = ADAM_B2; p.eps = ADAM_EPS;
+  for (int l = 0; l < nlin; l++) {
+    p.w[l] = L[l].w; p.b[l] = L[l].b; p.mw[l] = L[l].mw; p.vw[l] = L[l].vw; p.mb[l] = L[l].mb; p.vb[l] = L[l].vb;
+    p.gw[l] = L[l].gw; p.gb[l] = L[l].gb; p.wb[l] = L[l].wb; p.wt[l] = L[l].wt; p.wk[l] = L[l].wk; p.wtk[l] = L[l].wtk;
+  }
+  return p;
+}
+
+FusedArgs Net::fused_args(int B, int mode) const {
+  FusedArgs a{};
+  a.nlin = nlin; a.ntiles = (B + 127) / 128; a.mode = mode; a.B = B; a.n = nsamp; a.seed = seed; a.step = d_step;
+  a.feat = feat; a.targ = targ; a.nrm = nrm; a.Y = Y; a.X = X; a.Xt = Xt; a.dO = dOt; a.lrow = lrow; a.err = d_err;
+  for (int l = 0; l < nlin; l++) { a.wk[l] = L[l].wk; a.wtk[l] = L[l].wtk; a.bias[l] = L[l].b; }
+  for (int l = 0; l < nlin - 1; l++) { a.H[l] = Ht[l]; a.dz[l] = dZt[l]; }
+  return a;
+}
+
+// splits of the batch in the weight gradients: whole 64-row steps
+static int weight_splits(int B) {
+  int ks = KSPLIT;
+  while (ks > 1 && (B / ks) % 64) ks >>= 1;
+  return ks;
+}
+
+// buffers of the fused training pass; grown, never shrunk, freed with the net
+int Net::ensure_fused(int B) {
+  if (!side) {
+    if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming) != cudaSuccess)
+      return 1;
+  }
+  if (B > cap_fused) {
+    Xt = dev_alloc<__nv_bfloat16>(owned, (size_t)B * 16);
+    dOt = dev_alloc<__nv_bfloat16>(owned, (size_t)B * 16);
+    for (int l = 0; l < nlin - 1; l++) {
+      Ht[l] = dev_alloc<__nv_bfloat16>(owned, (size_t)B * width);
+      dZt[l] = dev_alloc<__nv_bfloat16>(owned, (size_t)B * width);
+      if (!Ht[l] || !dZt[l]) return 1;
+    }
+    fcpart = dev_alloc<float>(owned, (size_t)(B / 256) * width * nlin);
+    lrow = dev_alloc<float>(owned, B);
+    if (!Xt || !dOt || !fcpart || !lrow) return 1;
+    cap_fused = B;
+  }
+  if (!fpart && !(fpart = dev_alloc<float>(owned, (size_t)2 * nlin * KSPLIT * 128 * width))) return 1;
+  return 0;
+}
+
+// one training pass: the tile kernel, then on two branches the weight
+// gradients with their update, and the bias gradients with theirs and the loss
+void Net::fused_pass(int B, int mode, bool adam, float lr) {
+  const FusedArgs a = fused_args(B, mode);
+  const PackArgs p = pack_args();
+  const int ks = weight_splits(B);
+  const long long unit = (long long)KSPLIT * 128 * width;
+  launch_mlp_train_tile(a, stream);
+  if (adam) k_step_inc<<<1, 32, 0, stream>>>(d_step);
+  cudaEventRecord(ev_fork, stream);
+  cudaStreamWaitEvent(side, ev_fork, 0);
+  launch_mlp_bias(a, p, fcpart, B / 256, d_step, lr, adam, d_loss, side);
+  cudaEventRecord(ev_join, side);
+  launch_mlp_dw(a, fpart, unit, ks, B / ks, stream);
+  launch_mlp_reduce(p, fpart, unit, ks, d_step, lr, adam, stream);
+  cudaStreamWaitEvent(stream, ev_join, 0);
 }
 
 // forward of B rows staged in X; leaves pre-activations in Z, outputs in out
@@ -587,8 +662,7 @@ void Net::backward(int B) {
     transpose(hin, B, ni, l == 0 ? NIN_PAD : width, T1, B, stream);
     Epi e{};
     e.mode = EPI_F32; e.fout = part; e.ldc = ni; e.split_stride = (long long)no * ni;
-    int ks = KSPLIT;
-    while (ks > 1 && (B / ks) % 64) ks >>= 1;
+    const int ks = weight_splits(B);
     gemm(T2, B, T1, B, no, ni, B, ks, e);
     long long n = (long long)no * ni;
     k_split_sum<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(part, ks, n, L[l].gw);
@@ -610,15 +684,26 @@ void Net::adam(float lr) {
   k_step_inc<<<1, 32, 0, stream>>>(d_step);
   for (int l = 0; l < nlin; l++) {
     int ni = layer_in(l), no = layer_out(l), n = ni * no;
-    k_adam<<<(n + 255) / 256, 256, 0, stream>>>(L[l].w, L[l].mw, L[l].vw, L[l].gw, no, ni, ni, d_step, lr, 0.9f,
-                                               0.999f, 1e-8f, L[l].wb, ni, L[l].wt, no);
-    k_adam<<<(no + 255) / 256, 256, 0, stream>>>(L[l].b, L[l].mb, L[l].vb, L[l].gb, 1, no, no, d_step, lr, 0.9f,
-                                                0.999f, 1e-8f, nullptr, 0, nullptr, 0);
+    k_adam<<<(n + 255) / 256, 256, 0, stream>>>(L[l].w, L[l].mw, L[l].vw, L[l].gw, no, ni, ni, d_step, lr, ADAM_B1,
+                                               ADAM_B2, ADAM_EPS, L[l].wb, ni, L[l].wt, no);
+    k_adam<<<(no + 255) / 256, 256, 0, stream>>>(L[l].b, L[l].mb, L[l].vb, L[l].gb, 1, no, no, d_step, lr, ADAM_B1,
+                                                ADAM_B2, ADAM_EPS, nullptr, 0, nullptr, 0);
   }
 }
 
 void Net::gather(int B) {
   k_gather<<<(B + 255) / 256, 256, 0, stream>>>(feat, targ, nsamp, B, d_step, seed, nrm, X, Y);
+}
+
+void Net::train_step(int B, float lr) {
+  if (fused()) {
+    fused_pass(B, FUSED_GATHER, true, lr);
+    return;
+  }
+  gather(B);
+  forward(B);
+  backward(B);
+  adam(lr);
 }
 
 int Net::fit_normalization() {
@@ -666,6 +751,18 @@ int Net::reserve_samples(long long n) {
 
 // predictions for n feature rows (device, n x NIN) into pred (device, n x NOUT)
 int Net::predict(const float *f, long long n, float *pred) {
+  if (fused()) {
+    // 128-row tiles shared out over the SMs, up to 2^30 rows a launch
+    for (long long r0 = 0; r0 < n; r0 += 1ll << 30) {
+      const long long m = n - r0 < 1ll << 30 ? n - r0 : 1ll << 30;
+      FusedArgs a = fused_args((int)m, FUSED_ROWS);
+      a.n = m;
+      a.feat = f + r0 * NIN;
+      a.pred = pred + r0 * NOUT;
+      launch_mlp_forward(a, stream);
+    }
+    return cudaGetLastError() == cudaSuccess ? 0 : 2;
+  }
   const int B = 16384;
   if (ensure_batch(B)) return 1;
   for (long long r0 = 0; r0 < n; r0 += B) {
@@ -692,6 +789,9 @@ void Net::destroy() {
   owned.clear();
   if (feat) cudaFree(feat);
   if (targ) cudaFree(targ);
+  if (side) cudaStreamDestroy(side);
+  if (ev_fork) cudaEventDestroy(ev_fork);
+  if (ev_join) cudaEventDestroy(ev_join);
   if (stream) cudaStreamDestroy(stream);
 }
 
