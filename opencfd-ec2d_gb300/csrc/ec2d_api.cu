@@ -744,7 +744,7 @@ void lusgs_update(ec2d_ctx *ctx, int l, double alfa1, bool force = false) {
   const Lvl &L = lv.L;
   const int mode = LUSGS_UPDATE | (force ? LUSGS_FORCE : 0);
   if (ctx->lusgs_fp32 && lv.fast32) {
-    K(ctx, "k_lusgs32", l, 3, [&] { launch_lusgs_fast32(L, alfa1, mode, lv.max_rows, ctx->stream); });
+    K(ctx, "k_lusgs32", l, 3, [&] { launch_lusgs_fast32(L, alfa1, mode, lv.max_rows, lv.max_cols, ctx->stream); });
   } else if (lv.fast64) {
     auto go = [&](int part) {
       launch_lusgs_fast(L, alfa1, mode | part, lv.max_rows, lv.max_cols, ctx->lusgs_cs, ctx->lusgs_rpw,
@@ -1914,7 +1914,7 @@ int ec2d_du_lusgs(ec2d_ctx *ctx, int mesh, double alfa1) {
   cudaSetDevice(ctx->device);
   const Level &lv = ctx->lv[mesh];
   const Lvl &L = lv.L;
-  if (ctx->lusgs_fp32 && lv.fast32) launch_lusgs_fast32(L, alfa1, 0, lv.max_rows, ctx->stream);
+  if (ctx->lusgs_fp32 && lv.fast32) launch_lusgs_fast32(L, alfa1, 0, lv.max_rows, lv.max_cols, ctx->stream);
   else if (lv.fast64)
     launch_lusgs_fast(L, alfa1, 0, lv.max_rows, lv.max_cols, ctx->lusgs_cs, ctx->lusgs_rpw, ctx->lusgs_lanes,
                       ctx->stream);

@@ -59,7 +59,7 @@ void launch_setup_geometry(const Lvl &L, const Lvl *finer, bool fdm, cudaStream_
 void launch_lusgs_fast(const Lvl &L, double alfa1, int mode, int max_rows, int max_cols, int cs, int rpw, int lanes,
                        cudaStream_t s);
 size_t lusgs_smem(int nv, int rows);  // dynamic shared memory of the one-CTA FP64 sweep
-void launch_lusgs_fast32(const Lvl &L, double alfa1, int mode, int max_rows, cudaStream_t s);
+void launch_lusgs_fast32(const Lvl &L, double alfa1, int mode, int max_rows, int max_cols, cudaStream_t s);
 size_t lusgs32_smem(int nv, int rows);
 // warm-start network <-> solver level (k_mlp.cu)
 void launch_features(const Lvl &L, const double *shape, float *feat, float *targ, cudaStream_t s);

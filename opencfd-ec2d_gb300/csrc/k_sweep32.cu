@@ -3,11 +3,22 @@
 // the residual stays FP64, Res is rounded to float when the records are built,
 // U stays FP64 and receives U += (double)dU in a separate all-cells kernel.
 //
-// Same wavefront as the FP64 sweep (k_sweep.cu): hyperplanes p = i+j in the
-// reference's Gauss-Seidel order, one CTA per block, thread j owns row j, the
-// next three cells' records are in flight by cp.async, the neighbouring row's
-// state comes through a double-buffered shared slot.  One difference in
-// arithmetic, not in the operator: the flux difference of comput_DFn
+// The Gauss-Seidel order is the reference's, one CTA per block, thread j owns
+// row j, the next three cells' records are in flight by cp.async.  Two forms
+// with the same arithmetic, term by term (dU is the same to the bit):
+//   k_push32         a cell, once updated, forms the terms it adds to its two
+//                    downstream neighbours: the next cell's stays in the
+//                    thread, the next row's moves by shuffle, or from a warp's
+//                    last row to the next warp through an inbox whose words are
+//                    their own flags (as in k_sweep_push.cu).  Warps run at
+//                    their own pace, a few cells apart; no CTA barrier.
+//   k_lusgs_sweep32  a cell pulls its neighbours' states through a
+//                    double-buffered shared slot, one CTA barrier per plane;
+//                    where the inboxes do not fit shared memory.
+// What bounds the sweep is the chain of about 20 dependent FP32 operations and
+// one reciprocal per cell (some 150 cycles) and what cannot be put beside it.
+// Flat plate, 2 x 96 x 96 cells: @NEW@.
+// One difference in arithmetic, not in the operator: the flux difference of comput_DFn
 // (sub_LU_SGS.f90:117-138), F_n(U + dU) - F_n(U), is evaluated in the
 // algebraically identical increment form
 //     du = (d(rho u) - u d(rho)) / (rho + d(rho)),  dv likewise,
@@ -40,6 +51,8 @@ constexpr int pad4(int n) { return (n + 3) / 4 * 4; }
 //  B        base state of the cell: rho, rho u, rho v, E + p, U_5.., then u, v
 //  CI, CJ   0.5 Lc_nb (+ Lv_nb when viscous) of the upstream neighbours
 //  N1I..N2J face normals of face i / j times the signed 0.5 s of the reference
+//           (push form: of the terms the cell gives to its downstream
+//           neighbours instead of those it takes from the upstream ones)
 //  IA, IA5  1/alfa and, for the SA row, 1/(alfa + Lvi + Lvj)
 template <int NV>
 struct R32 {
@@ -57,7 +70,7 @@ struct S32 {
   static constexpr int S = pad4(DP + 1);
 };
 
-template <int NV>
+template <int NV, bool PUSH>
 __global__ void __launch_bounds__(TILE) k_lusgs_prep32(Lvl L, double alfa1, int force) {
   using RC = R32<NV>;
   int bk, i, j;
@@ -85,7 +98,6 @@ __global__ void __launch_bounds__(TILE) k_lusgs_prep32(Lvl L, double alfa1, int 
   for (int m = 0; m < NV; m++) U[m] = L.U[m * F + id];
   double r = rcp(U[0]), u = U[1] * r, v = U[2] * r;
   double p = gm1 * (U[3] - 0.5 * (U[1] * u + U[2] * v));
-  double ni1 = g[G_NI1 * F + id], ni2 = g[G_NI2 * F + id], nj1 = g[G_NJ1 * F + id], nj2 = g[G_NJ2 * F + id];
 #pragma unroll
   for (int m = 0; m < NV; m++) {
     rf[RC::A + m] = (float)((force && m < 4) ? L.res[m * F + id] + L.qf[m * F + id] : L.res[m * F + id]);
@@ -109,20 +121,24 @@ __global__ void __launch_bounds__(TILE) k_lusgs_prep32(Lvl L, double alfa1, int 
     for (int dir = 0; dir < 2; dir++) {  // 0: i-neighbour, 1: j-neighbour
       const bool fwd = pass == 0;
       const long long step = dir == 0 ? 1 : P;
-      const long long nb = fwd ? id - step : id + step;
-      const bool has = dir == 0 ? (fwd ? i > 1 : i < b.nx - 1) : (fwd ? j > 1 : j < b.ny - 1);
-      double cc = 0.0, hh = 0.0;
+      // the cell that takes the term, the one that gives it
+      const bool up = fwd != PUSH;  // the other cell has the smaller index
+      const long long other = up ? id - step : id + step, to = PUSH ? other : id, nb = PUSH ? id : other;
+      const bool has = dir == 0 ? (up ? i > 1 : i < b.nx - 1) : (up ? j > 1 : j < b.ny - 1);
+      double cc = 0.0, hh = 0.0, n1 = 0.0, n2 = 0.0;
       if (has) {
         cc = 0.5 * lc[(dir == 0 ? L_CI : L_CJ) * F + nb];
         if (visc) cc += lc[(dir == 0 ? L_VI : L_VJ) * F + nb];
-        // forward: +0.5 s of this cell's face; backward: -0.5 s of the
-        // neighbour's face with this cell's normal (sub_LU_SGS.f90:87-88,95-96)
-        hh = 0.5 * g[(dir == 0 ? G_SI : G_SJ) * F + (fwd ? id : nb)];
+        // forward: +0.5 s of the taking cell's face; backward: -0.5 s of the
+        // giving cell's face with the taking cell's normal (sub_LU_SGS.f90:87-88,95-96)
+        hh = 0.5 * g[(dir == 0 ? G_SI : G_SJ) * F + (fwd ? to : nb)];
         if (!fwd) hh = -hh;
+        n1 = g[(dir == 0 ? G_NI1 : G_NJ1) * F + to];
+        n2 = g[(dir == 0 ? G_NI2 : G_NJ2) * F + to];
       }
       q[dir == 0 ? RC::CI : RC::CJ] = (float)cc;
-      q[dir == 0 ? RC::N1I : RC::N1J] = (float)(hh * (dir == 0 ? ni1 : nj1));
-      q[dir == 0 ? RC::N2I : RC::N2J] = (float)(hh * (dir == 0 ? ni2 : nj2));
+      q[dir == 0 ? RC::N1I : RC::N1J] = (float)(hh * n1);
+      q[dir == 0 ? RC::N2I : RC::N2J] = (float)(hh * n2);
     }
   }
   char *base = reinterpret_cast<char *>(L.rec);
@@ -133,6 +149,42 @@ __global__ void __launch_bounds__(TILE) k_lusgs_prep32(Lvl L, double alfa1, int 
     wf[k] = make_float4(rf[4 * k], rf[4 * k + 1], rf[4 * k + 2], rf[4 * k + 3]);
     wb[k] = make_float4(rb[4 * k], rb[4 * k + 1], rb[4 * k + 2], rb[4 * k + 3]);
   }
+}
+
+// the term a cell gives a downstream neighbour: dF_n(its state, scaled normal) +
+// cc dU
+template <int NV>
+__device__ __forceinline__ void dterm(const float *s, float n1, float n2, float cc, float *x) {
+  using SL = S32<NV>;
+  const float unp = s[SL::UP] * n1 + s[SL::VP] * n2;
+  const float dun = s[SL::DU] * n1 + s[SL::DV] * n2;
+  const float dp = s[SL::DP];
+  x[0] = s[SL::D + 0] * unp + s[SL::B + 0] * dun + cc * s[SL::D + 0];
+  x[1] = s[SL::D + 1] * unp + s[SL::B + 1] * dun + dp * n1 + cc * s[SL::D + 1];
+  x[2] = s[SL::D + 2] * unp + s[SL::B + 2] * dun + dp * n2 + cc * s[SL::D + 2];
+  x[3] = (s[SL::D + 3] + dp) * unp + s[SL::B + 3] * dun + cc * s[SL::D + 3];
+#pragma unroll
+  for (int m = 4; m < NV; m++) x[m] = s[SL::D + m] * unp + s[SL::B + m] * dun + cc * s[SL::D + m];
+}
+// the state of a cell that its terms need, from dU (in st) and the record
+template <int NV>
+__device__ __forceinline__ void shipped_state(float *st, const float *cur, float gm1) {
+  using SL = S32<NV>;
+  using RC = R32<NV>;
+#pragma unroll
+  for (int m = 0; m < NV; m++) st[SL::B + m] = cur[RC::B + m];
+  const float rho = cur[RC::B + 0], m1 = cur[RC::B + 1], m2 = cur[RC::B + 2];
+  const float u = cur[RC::BU], v = cur[RC::BV];
+  const float dr = st[SL::D + 0], dm1 = st[SL::D + 1], dm2 = st[SL::D + 2], dE = st[SL::D + 3];
+  float rr;  // 1 / (rho + d rho): the approximate reciprocal (an FP32 preconditioner)
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rr) : "f"(rho + dr));
+  const float du = (dm1 - u * dr) * rr, dv = (dm2 - v * dr) * rr;
+  const float up = u + du, vp = v + dv;
+  st[SL::UP] = up;
+  st[SL::VP] = vp;
+  st[SL::DU] = du;
+  st[SL::DV] = dv;
+  st[SL::DP] = gm1 * (dE - 0.5f * (dm1 * up + m1 * du + dm2 * vp + m2 * dv));
 }
 
 // acc += dF_n(shipped state, scaled normal) + cc dU_nb
@@ -221,23 +273,7 @@ __device__ __forceinline__ void sweep32_pass(const Lvl &L, float *shf, char *rec
         float inv = (NV == 5 && m == 4) ? ia5 : ia;
         st[SL::D + m] = fwd ? acc[m] * inv : cur[RC::A + m] + acc[m] * inv;
       }
-      // state shipped to the two downstream neighbours
-#pragma unroll
-      for (int m = 0; m < NV; m++) st[SL::B + m] = cur[RC::B + m];
-      {
-        const float rho = cur[RC::B + 0], m1 = cur[RC::B + 1], m2 = cur[RC::B + 2];
-        const float u = cur[RC::BU], v = cur[RC::BV];
-        const float dr = st[SL::D + 0], dm1 = st[SL::D + 1], dm2 = st[SL::D + 2], dE = st[SL::D + 3];
-        float rr;  // 1 / (rho + d rho): the approximate reciprocal (an FP32 preconditioner)
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rr) : "f"(rho + dr));
-        const float du = (dm1 - u * dr) * rr, dv = (dm2 - v * dr) * rr;
-        const float up = u + du, vp = v + dv;
-        st[SL::UP] = up;
-        st[SL::VP] = vp;
-        st[SL::DU] = du;
-        st[SL::DV] = dv;
-        st[SL::DP] = gm1 * (dE - 0.5f * (dm1 * up + m1 * du + dm2 * vp + m2 * dv));
-      }
+      shipped_state<NV>(st, cur, gm1);  // for the two downstream neighbours
       float4 *own = reinterpret_cast<float4 *>(shf + ((size_t)buf * (R + 2) + rl + 1) * S);
 #pragma unroll
       for (int m = 0; m < S / 4; m++) own[m] = make_float4(st[4 * m], st[4 * m + 1], st[4 * m + 2], st[4 * m + 3]);
@@ -283,6 +319,177 @@ __global__ void __launch_bounds__(1024) k_lusgs_sweep32(Lvl L) {
   sweep32_pass<NV, false>(L, shf, rec, recF, recB, recBw, st, bd, R, rl, j, row_ok, gm1);
 }
 
+// ---- push form ----------------------------------------------------------------
+constexpr unsigned FULL = 0xffffffffu;
+constexpr int WAIT32 = 1 << 18;  // polls of an inbox before the wait gives up
+// an inbox word nothing has been written to: a NaN no arithmetic produces
+constexpr unsigned EMPTY32 = 0x7fc9e37bu;
+// records per thread: those of the next PRING32 - 2 cells are in flight (an FP32
+// cell takes a third of the L2 latency); padded so that the 16-byte reads of
+// eight neighbouring threads meet eight different groups of banks
+constexpr int PRING32 = 8;
+template <int NV>
+constexpr int ring_bytes() { return PRING32 * R32<NV>::BYTES + 16; }
+static_assert(ring_bytes<4>() % 32 == 16 && ring_bytes<5>() % 32 == 16 && ring_bytes<6>() % 32 == 16, "odd multiples of 16 bytes");
+__device__ __forceinline__ void cp_wait_push() { asm volatile("cp.async.wait_group %0;" ::"n"(PRING32 - 3) : "memory"); }
+__device__ __forceinline__ float4 box_read4(unsigned a) {
+  float4 v;
+  asm volatile("ld.volatile.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void box_write4(unsigned a, float x, float y, float z, float w) {
+  asm volatile("st.volatile.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
+constexpr int PUSH32_THREADS = 352;  // the rings of as many rows fill the shared memory
+template <int NV>
+constexpr int box_words() { return NV == 4 ? 4 : 8; }
+
+template <int NV, bool FWD>
+__device__ __forceinline__ void push32_pass(const Lvl &L, const BlkDev &bd, int bk, char *rec, unsigned box, unsigned out,
+                                            const char *src_row, char *dst_row, int j0, float gm1) {
+  using SL = S32<NV>;
+  using RC = R32<NV>;
+  constexpr int SB = box_words<NV>();
+  const int lane = threadIdx.x & 31, ni = bd.nx - 1, rows = bd.ny - 1;
+  const int last = min(31, rows - j0);  // the warp's last row
+  const bool row_ok = lane <= last;
+  const int lag = FWD ? lane : last - lane;
+  // the inbox serves the warp's first row in the order of the pass; the last one
+  // feeds the next warp
+  const bool has_box = FWD ? j0 > 1 : j0 + 32 <= rows, has_out = FWD ? j0 + 32 <= rows : j0 > 1;
+  const bool first = lane == (FWD ? 0 : last), sends = has_out && !L.silent_band_edge && lane == (FWD ? last : 0);
+  const int from = FWD ? (lane + 31) & 31 : (lane + 1) & 31;
+  auto src = [&](int k) { return src_row + (size_t)(FWD ? k : ni - 1 - k) * RC::BYTES; };
+  auto fetch = [&](int k) {
+    if (row_ok && k < ni) fetch32<NV>(rec + (k & (PRING32 - 1)) * RC::BYTES, src(k));
+    cp_commit();
+  };
+  auto read = [&](float (&c)[RC::NF], int k) {
+    const float4 *p = reinterpret_cast<const float4 *>(rec + (k & (PRING32 - 1)) * RC::BYTES);
+#pragma unroll
+    for (int q = 0; q < RC::NF / 4; q++) {
+      const float4 v = p[q];
+      c[4 * q] = v.x; c[4 * q + 1] = v.y; c[4 * q + 2] = v.z; c[4 * q + 3] = v.w;
+    }
+  };
+  int gave_up = -1;
+  // the inbox entry of step t; polled in the middle of the step before
+  float in[NV];
+#pragma unroll
+  for (int m = 0; m < NV; m++) in[m] = 0.0f;
+  auto poll = [&](int t) {
+    if (!has_box || t >= ni || gave_up >= 0) return;
+    const unsigned p = box + 4u * SB * (unsigned)t;
+    for (int n = 0;; n++) {
+      const float4 v = box_read4(p);
+      in[0] = v.x; in[1] = v.y; in[2] = v.z; in[3] = v.w;
+      if (NV > 4) {
+        const float4 w = box_read4(p + 16u);
+        in[4 < NV ? 4 : 0] = w.x;
+        if (NV > 5) in[NV - 1] = w.y;
+      }
+      bool empty = false;
+#pragma unroll
+      for (int m = 0; m < NV; m++) empty |= __float_as_uint(in[m]) == EMPTY32;
+      if (!__any_sync(FULL, empty)) break;
+      if (n == WAIT32) { gave_up = t; break; }
+    }
+  };
+  float st[SL::S], own[NV], down[NV];  // the cell's state; the terms for the next cell and the next row
+#pragma unroll
+  for (int m = 0; m < SL::S; m++) st[m] = 0.0f;
+#pragma unroll
+  for (int m = 0; m < NV; m++) own[m] = down[m] = 0.0f;
+  float c0[RC::NF], c1[RC::NF];
+  // records of the row's first visits; visit k + PRING32 - 2 is requested in visit
+  // k, one group a step, so that the record of visit k + 1 has landed at the
+  // end of visit k
+  for (int k = 0; k < PRING32 - 2; k++) fetch(k);
+  cp_wait_push();
+  read(c0, 0);
+  poll(0);
+  auto step = [&](int t, float (&cur)[RC::NF], float (&next)[RC::NF]) {
+    const int k = t - lag;
+    const bool act = row_ok && (unsigned)k < (unsigned)ni;
+    float nb[NV];
+#pragma unroll
+    for (int m = 0; m < NV; m++) nb[m] = __shfl_sync(FULL, down[m], from);
+    if (first)
+#pragma unroll
+      for (int m = 0; m < NV; m++) nb[m] = has_box ? in[m] : 0.0f;
+    if (k >= 0) fetch(k + PRING32 - 2);
+    else cp_commit();
+    cp_wait_push();
+    const float ia = cur[RC::IA], ia5 = cur[RC::IA5];
+    float dn[NV];
+#pragma unroll
+    for (int m = 0; m < NV; m++) {
+      float acc = FWD ? cur[RC::A + m] : 0.0f;
+      acc += own[m];
+      acc += nb[m];
+      const float inv = (NV == 5 && m == 4) ? ia5 : ia;
+      dn[m] = FWD ? acc * inv : cur[RC::A + m] + acc * inv;
+    }
+    if (act) {
+#pragma unroll
+      for (int m = 0; m < NV; m++) st[SL::D + m] = dn[m];
+      shipped_state<NV>(st, cur, gm1);
+      dterm<NV>(st, cur[RC::N1J], cur[RC::N2J], cur[RC::CJ], down);
+      dterm<NV>(st, cur[RC::N1I], cur[RC::N2I], cur[RC::CI], own);
+      if (sends) {
+        const unsigned o = out + 4u * SB * (unsigned)k;
+        box_write4(o, down[0], down[1], down[2], down[3]);
+        if (NV > 4) box_write4(o + 16u, down[4 < NV ? 4 : 0], down[NV - 1], 0.0f, 0.0f);
+      }
+      // forward: the A field of the backward record; backward: the final dU
+      // replaces it there (k_apply32 widens it afterwards)
+      float *w = reinterpret_cast<float *>(dst_row + (size_t)(FWD ? k : ni - 1 - k) * RC::BYTES);
+      *reinterpret_cast<float4 *>(w) = make_float4(dn[0], dn[1], dn[2], dn[3]);
+#pragma unroll
+      for (int m = 4; m < NV; m++) w[m] = dn[m];
+    }
+    read(next, max(k + 1, 0));
+    poll(t + 1);
+  };
+  const int steps = ni + last;
+  for (int t = 0; t < steps; t += 2) {
+    step(t, c0, c1);
+    step(t + 1, c1, c0);
+  }
+  cp_wait0();
+  if (gave_up >= 0 && lane == 0)
+    set_status(L.status + 4 * bd.cas, 4, bk, FWD ? gave_up + 1 : ni - gave_up, j0);
+}
+
+template <int NV>
+__global__ void __launch_bounds__(PUSH32_THREADS, 1) k_push32(Lvl L) {
+  using RC = R32<NV>;
+  extern __shared__ __align__(16) char sh[];  // rings [thread], inboxes [warp][column][SB]
+  const BlkDev bd = L.blk[blockIdx.x];
+  const int rows = bd.ny - 1, ni = bd.nx - 1, w = threadIdx.x >> 5, j0 = 32 * w + 1, j = threadIdx.x + 1;
+  const float gm1 = (float)(L.cs[bd.cas].gamma - 1.0);
+  char *rec = sh + (size_t)threadIdx.x * ring_bytes<NV>();
+  float *boxes = reinterpret_cast<float *>(sh + (size_t)blockDim.x * ring_bytes<NV>());
+  const size_t words = (size_t)ni * box_words<NV>();
+  float *box = boxes + w * words;
+  const unsigned mine = (unsigned)__cvta_generic_to_shared(box), step = 4u * (unsigned)words;
+  auto clear = [&] {
+    for (size_t t = threadIdx.x & 31; t < words; t += 32) box[t] = __uint_as_float(EMPTY32);
+  };
+  const int jr = min(j, rows);  // record pointers of idle rows stay in the array
+  char *recF = reinterpret_cast<char *>(L.rec) + ((size_t)bd.cell0 + (size_t)(jr - 1) * ni) * RC::BYTES;
+  char *recB = recF + (size_t)L.ncell * RC::BYTES;
+  clear();
+  __syncthreads();  // every inbox empty before any warp writes into one
+  if (j0 <= rows) {
+    push32_pass<NV, true>(L, bd, blockIdx.x, rec, mine, mine + step, recF, recB, j0, gm1);
+    __syncwarp();
+    clear();
+  }
+  __syncthreads();  // and again before the backward pass (the others wait for the last warp anyway)
+  if (j0 <= rows) push32_pass<NV, false>(L, bd, blockIdx.x, rec, mine, mine - step, recB, recB, j0, gm1);
+}
+
 // dU (FP32, in the backward records) -> U += dU in FP64, or -> L.du
 // (NS_Time_advance_LU_SGS, sub_NS_singlegrid.f90:203-211)
 template <int NV>
@@ -314,15 +521,28 @@ size_t smem32(int rows) {
   return (size_t)2 * (th + 2) * S32<NV>::S * sizeof(float) + (size_t)th * RING32 * R32<NV>::BYTES;
 }
 
+// shared memory of the push form; it serves blocks whose inboxes fit
 template <int NV>
-void sweep32_nv(const Lvl &L, double alfa1, int mode, int max_rows, cudaStream_t s) {
-  k_lusgs_prep32<NV><<<L.nctiles, TILE, 0, s>>>(L, alfa1, mode & LUSGS_FORCE);
-  const int update = mode & LUSGS_UPDATE;
-  int th = ((max_rows + 31) / 32) * 32;
-  size_t smem = smem32<NV>(max_rows);
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(k_lusgs_sweep32<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_lusgs_sweep32<NV><<<L.nblk, th, smem, s>>>(L);
+size_t push32_smem(int rows, int cols) {
+  const int th = ((rows + 31) / 32) * 32;
+  return (size_t)th * ring_bytes<NV>() + (size_t)(th / 32) * cols * box_words<NV>() * sizeof(float);
+}
+
+template <int NV>
+void sweep32_nv(const Lvl &L, double alfa1, int mode, int max_rows, int max_cols, cudaStream_t s) {
+  const int update = mode & LUSGS_UPDATE, force = mode & LUSGS_FORCE;
+  const int th = ((max_rows + 31) / 32) * 32;
+  const size_t push = push32_smem<NV>(max_rows, max_cols), pull = smem32<NV>(max_rows);
+  if (th <= PUSH32_THREADS && push <= 227 * 1024) {
+    k_lusgs_prep32<NV, true><<<L.nctiles, TILE, 0, s>>>(L, alfa1, force);
+    if (push > 48 * 1024) cudaFuncSetAttribute(k_push32<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)push);
+    k_push32<NV><<<L.nblk, th, push, s>>>(L);
+  } else {
+    k_lusgs_prep32<NV, false><<<L.nctiles, TILE, 0, s>>>(L, alfa1, force);
+    if (pull > 48 * 1024)
+      cudaFuncSetAttribute(k_lusgs_sweep32<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pull);
+    k_lusgs_sweep32<NV><<<L.nblk, th, pull, s>>>(L);
+  }
   k_apply32<NV><<<L.ntiles, TILE, 0, s>>>(L, update);
 }
 
@@ -332,10 +552,10 @@ size_t lusgs32_smem(int nv, int rows) {
   return nv == 4 ? smem32<4>(rows) : nv == 5 ? smem32<5>(rows) : smem32<6>(rows);
 }
 
-void launch_lusgs_fast32(const Lvl &L, double alfa1, int mode, int max_rows, cudaStream_t s) {
-  if (L.nvar == 4) sweep32_nv<4>(L, alfa1, mode, max_rows, s);
-  else if (L.nvar == 5) sweep32_nv<5>(L, alfa1, mode, max_rows, s);
-  else sweep32_nv<6>(L, alfa1, mode, max_rows, s);
+void launch_lusgs_fast32(const Lvl &L, double alfa1, int mode, int max_rows, int max_cols, cudaStream_t s) {
+  if (L.nvar == 4) sweep32_nv<4>(L, alfa1, mode, max_rows, max_cols, s);
+  else if (L.nvar == 5) sweep32_nv<5>(L, alfa1, mode, max_rows, max_cols, s);
+  else sweep32_nv<6>(L, alfa1, mode, max_rows, max_cols, s);
 }
 
 }  // namespace ec2d

@@ -76,3 +76,38 @@ def test_sweep_edges(gpu_lib, monkeypatch, nx, ny, rows, turb):
         scale = np.abs(a).reshape(nv, -1).max(axis=1)[:, None, None]
         assert np.max(np.abs(a - c) / scale) <= 1e-10
     g.close()
+
+
+# rows at the edges of the FP32 sweep's 32-row warps, cells around its ring of
+# eight records, and blocks whose rings and inboxes do not fit shared memory
+# (the form with a barrier per plane)
+SIZES32 = [(3, 3), (8, 33), (9, 34), (10, 32), (17, 65), (40, 66), (70, 98), (18, 340)]
+
+
+@pytest.mark.parametrize("turb", [0, 2, 3])
+@pytest.mark.parametrize("nx,ny", SIZES32)
+def test_fp32_sweep_edges(gpu_lib, nx, ny, turb):
+    p, bl = _case(nx, ny, turb)
+    nv = p.nvar()
+    orc, g = make_oracle(p, bl), make_gpu(p, bl)
+    orc.init_flow(), g.init_flow()
+    perturb_state(orc, amp=0.01, seed=nx + ny)
+    orc.bc(), orc.halo()
+    copy_state(orc, g)
+    g.set_lusgs_precision(32)
+    orc.residual()
+    for b in (1, 2):
+        for f in range(6):
+            g.set_field(1, 1, b, f, orc.field(1, b, f))
+    orc.lusgs(1, 1, 0.0), orc.lusgs(1, 2, 0.0)
+    g.lusgs(1, 0.0)
+    for b in (1, 2):
+        a = orc.field(1, b, 6, (nv, nx, ny))[:, :nx - 1, :ny - 1]
+        c = g.field(1, 1, b, 6, (nv, nx, ny))[:, :nx - 1, :ny - 1]
+        for m in range(nv):
+            # float epsilon (6e-8) times the planes of a sweep, at most
+            assert np.abs(a[m] - c[m]).max() <= 6e-8 * max(nx + ny, 40) * np.abs(a[m]).max(), m
+    g.step(1)
+    g.norms()
+    assert g.status()[0] == 0
+    g.close()
