@@ -237,6 +237,12 @@ CaseDev make_casedev(const ec2d_params &p) {
   c.cosA = 1.0 * std::cos(aoa); c.sinA = 1.0 * std::sin(aoa);
   c.p00 = 1.0 / (p.gamma * p.Ma * p.Ma);
   c.Tsb = 110.4 / p.T_inf;
+  c.gm1 = p.gamma - 1.0; c.rg = 1.0 / p.gamma;
+  c.kpr = c.Cp / p.Pr;
+  c.kprt = c.Cp / PrT;
+  c.mu0 = (1.0 + c.Tsb) / p.Re;
+  c.gpr = p.gamma / p.Pr;
+  c.gprt = p.gamma / PrT;
   c.Twall = p.Twall / p.T_inf;
   c.p_outlet = p.P_outlet; c.vt_inf = p.vt_inf; c.Kt_inf = p.Kt_inf; c.Wt_inf = p.Wt_inf;
   c.CFL = p.CFL; c.dtmax = p.dtmax; c.dtmin = p.dtmin; c.dt_global = p.dt_global; c.T_inf = p.T_inf;

@@ -31,14 +31,16 @@ enum { Turb_NONE = 0, Turb_BL = 1, Turb_SA = 2, Turb_SST = 3 };
 // primitive planes in Lvl::q
 enum { Q_D = 0, Q_U = 1, Q_V = 2, Q_T = 3, Q_P = 4, Q_C = 5, NQ = 6 };
 // geometry planes in Lvl::geo
-// G_VI*, G_VJ*: the face-local inverse Jacobian of the viscous terms of an i-
-// or j-face, (Djy, Diy, Djx, Dix) / (Dix Djy - Djx Diy), formed at set-up
-// (k_face_metrics) from the cell centres; G_SIA..G_NJ2A: the cell's face
+// G_VI*, G_VJ*: the metric coefficients of the viscous terms of an i- or j-face,
+// formed at set-up (k_face_metrics) from the cell centres: with the face-local
+// inverse Jacobian (A, B, C, D) = (Djy, Diy, Djx, Dix) / (Dix Djy - Djx Diy) and
+// the unit normal n, P = A n1 - C n2, Q = D n2 - B n1, R = A n2 + C n1, S = B n2 +
+// D n1 (see viscous_face_m); G_SIA..G_NJ2A: the cell's face
 // length and normal averaged over its two i- (j-) faces, G_VI2 / G_VJ2 their
 // squared length over the cell volume (the metric factors of comput_Lvc)
 enum { G_VOL = 0, G_SI = 1, G_SJ = 2, G_NI1 = 3, G_NI2 = 4, G_NJ1 = 5, G_NJ2 = 6,
        G_X = 7, G_Y = 8, G_X1 = 9, G_Y1 = 10, G_DW = 11,
-       G_VIA = 12, G_VIB = 13, G_VIC = 14, G_VID = 15, G_VJA = 16, G_VJB = 17, G_VJC = 18, G_VJD = 19,
+       G_VIP = 12, G_VIQ = 13, G_VIR = 14, G_VIS = 15, G_VJP = 16, G_VJQ = 17, G_VJR = 18, G_VJS = 19,
        G_SIA = 20, G_NI1A = 21, G_NI2A = 22, G_SJA = 23, G_NJ1A = 24, G_NJ2A = 25, G_VI2 = 26, G_VJ2 = 27,
        NG = 28 };
 // spectral-radius / time-step planes in Lvl::lc
@@ -71,6 +73,10 @@ struct CaseDev {
   double xaxis, yaxis;
   double rPr, rCv, rMa, rRe;  // 1/Pr, 1/Cv, 1/Ma, 1/Re
   double rgm1;                // 1/(gamma - 1)
+  double gm1, rg;             // gamma - 1, 1/gamma
+  double kpr, kprt;           // Cp/Pr, Cp/Pr_t
+  double mu0;                 // (1 + Tsb)/Re
+  double gpr, gprt;           // gamma/Pr, gamma/Pr_t
   double ggm1;                // gamma/(gamma - 1)
   int local_dt, pad;
 };
@@ -135,45 +141,168 @@ __device__ __forceinline__ bool core_ij(const Lvl &L, int &bk, int &i, int &j) {
   return true;
 }
 
-// Reciprocal on the face and wavefront paths.  FP64: the hardware's
-// approximate reciprocal (relative error e below 2^-19.9, measured over 4e7
-// mantissas) refined by one third-order step of the series
-// 1/x = r / (1 - e) = r (1 + e + e^2 + ...), e = 1 - x r taken exactly by an
-// fma; the neglected e^3 is below 2^-59, so the result is within an ulp of
-// the quotient in four dependent FP64 operations, against nine times that
-// for a divide; a / b becomes a * rcp(b).  FP32: the division.
+// FP64 arithmetic on the face, primitive and wavefront paths.  An SM completes
+// one FP64 warp instruction per 16 to 19 cycles, and each holds its sub-partition
+// for 64, while that sub-partition could issue an integer or FP32 instruction
+// every cycle: whatever needs no FP64 pipe is done beside it.
+//   * reciprocals and reciprocal square roots start from 44-bit values formed in
+//     FP32 and integers (rcp_seed, rsqrt_seed) and need one Newton step, two and
+//     three FP64 instructions (a divide takes about nine, the hardware's 20-bit
+//     approximation with a third-order step three and five);
+//   * negation, powers of two and comparisons are integer operations.
+// x 2^K, K in -3..1: exact; zeros, infinities and NaNs stay what they are, and so
+// do values below 2^-1019
+template <int K>
+__device__ __forceinline__ double pow2(double x) {
+  const int h = __double2hiint(x);
+  const unsigned e = (unsigned)h & 0x7ff00000u;
+  return __hiloint2double(e - 0x00400000u < 0x7fa00000u ? h + K * 0x00100000 : h, __double2loint(x));
+}
+template <int K>
+__device__ __forceinline__ float pow2(float x) { return x * (K >= 0 ? (float)(1 << (K & 31)) : 1.0f / (float)(1 << (-K & 31))); }
+template <typename T>
+__device__ __forceinline__ T half(T x) { return pow2<-1>(x); }
+__device__ __forceinline__ double neg(double x) {
+  return __hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x));
+}
+__device__ __forceinline__ float neg(float x) { return -x; }
+// Conversions between double and float, rounded to nearest even: a conversion
+// instruction occupies the FP64 pipe as an FP64 instruction does (64 to 100 cycles), so
+// values within the float's normal range are converted by integer operations.
+template <typename T>
+__device__ __forceinline__ T to(double x);
+template <>
+__device__ __forceinline__ double to<double>(double x) { return x; }
+template <>
+__device__ __forceinline__ float to<float>(double x) {
+  const long long i = __double_as_longlong(x);
+  const unsigned hi = (unsigned)(i >> 32), a = hi & 0x7fffffffu;
+  const long long r = i + 0x0fffffffll + ((i >> 29) & 1);
+  // 2^-126 <= |x| < 2^127, or zero
+  if (a - 0x38100000u < 0x47e00000u - 0x38100000u)
+    return __uint_as_float((((unsigned)(r >> 29) - (896u << 23)) & 0x7fffffffu) | (hi & 0x80000000u));
+  return (i << 1) == 0 ? __uint_as_float(hi) : (float)x;
+}
+__device__ __forceinline__ double to_double(double x) { return x; }
+__device__ __forceinline__ double to_double(float x) {
+  const unsigned i = __float_as_uint(x), a = i & 0x7fffffffu;
+  if (a - 0x00800000u < 0x7f800000u - 0x00800000u)
+    return __hiloint2double((int)(((a >> 3) + (896u << 20)) | (i & 0x80000000u)), (int)(i << 29));
+  return a == 0 ? __hiloint2double((int)i, 0) : (double)x;
+}
+// sign bit clear; x < y, x >= y and x > y for any x and a y of clear sign bit (false
+// for a NaN x)
+__device__ __forceinline__ bool sign_clear(double x) { return __double2hiint(x) >= 0; }
+__device__ __forceinline__ bool sign_clear(float x) { return __float_as_int(x) >= 0; }
+__device__ __forceinline__ bool below(double x, double y) {
+  const long long i = __double_as_longlong(x);
+  return i < __double_as_longlong(y) && (unsigned long long)i <= 0xfff0000000000000ull;
+}
+__device__ __forceinline__ bool below(float x, float y) { return x < y; }
+__device__ __forceinline__ bool at_least(double x, double y) {
+  const long long i = __double_as_longlong(x);
+  return i >= __double_as_longlong(y) && i <= 0x7ff0000000000000ll;
+}
+__device__ __forceinline__ bool above(double x, double y) {
+  const long long i = __double_as_longlong(x);
+  return i > __double_as_longlong(y) && i <= 0x7ff0000000000000ll;
+}
+
+// 1/x to about 44 bits: x's mantissa as a float and the float of its remaining
+// bits, the FP32 approximate reciprocal r of the first, and the correction
+// r (e + e^2), e = 1 - x r, added to r's double as an integer.  NaN for zero,
+// subnormal, infinite or NaN x and from 2^1022.
+__device__ __forceinline__ double rcp_seed(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const float xf = __uint_as_float((__funnelshift_l(lo, hi, 3) & 0x7fffffu) | 0x3f800000u);
+  const float xl = fmaf(__uint_as_float(((lo >> 6) & 0x7fffffu) | 0x3f800000u), 0x1p-23f, -0x1p-23f);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(xf));  // in (0.5, 1]
+  const float e = fmaf(-xl, r, fmaf(-xf, r, 1.0f));
+  // the correction in units of 2^-52 (the double's are 2^-53 below 1)
+  const int q = __float2int_rn(r * 0x1p52f * fmaf(e, e, e));
+  const unsigned rb = __float_as_uint(r), ex = hi & 0x7ff00000u;
+  const unsigned long long y = (((unsigned long long)(rb >> 3) << 32) | (rb << 29)) + (unsigned long long)(2ll * q);
+  const unsigned yh = (unsigned)(y >> 32) + ((1023u - 127u) << 20) + (0x3ff00000u - ex);
+  return __hiloint2double(ex - 0x00100000u < 0x7fc00000u ? (int)(yh | (hi & 0x80000000u)) : 0x7ff80000,
+                          (int)(unsigned)y);
+}
+// 1/sqrt(x) to about 44 bits the same way: the exponent made even, r the FP32
+// approximate reciprocal root, the correction r e (1/2 + 3/8 e), e = 1 - x r^2.
+// NaN for negative, infinite or NaN x; for zero (and subnormal x) NaN or, ZERO, 1,
+// so that x times the root is zero.
+template <bool ZERO>
+__device__ __forceinline__ double rsqrt_seed(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned odd = (hi & 0x00100000u) ? 0u : 1u;  // biased exponent even: mantissa in [2, 4)
+  const float xf = __uint_as_float((__funnelshift_l(lo, hi, 3) & 0x7fffffu) | (odd ? 0x40000000u : 0x3f800000u));
+  const float ul = odd ? 0x1p-22f : 0x1p-23f;
+  const float xl = fmaf(__uint_as_float(((lo >> 6) & 0x7fffffu) | 0x3f800000u), ul, -ul);
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(xf));  // in (0.5, 1]
+  const float r2 = r * r, r2l = fmaf(r, r, -r2);
+  const float e = fmaf(-xl, r2, fmaf(-xf, r2l, fmaf(-xf, r2, 1.0f)));
+  const int q = __float2int_rn(r * 0x1p52f * (e * fmaf(0.375f, e, 0.5f)));
+  const unsigned rb = __float_as_uint(r);
+  const unsigned long long y = (((unsigned long long)(rb >> 3) << 32) | (rb << 29)) + (unsigned long long)(2ll * q);
+  // x = m 4^k with k = (exponent - odd) / 2 of the unbiased exponent
+  const int k = ((int)(hi >> 20) - 1023 - (int)odd) >> 1;
+  const unsigned yh = (unsigned)(y >> 32) + ((1023u - 127u) << 20) - ((unsigned)k << 20);
+  const int out = ZERO && (hi & 0x7ff00000u) == 0 ? 0x3ff00000 : 0x7ff80000;
+  return __hiloint2double(hi - 0x00100000u < 0x7fe00000u ? (int)yh : out, (int)(unsigned)y);
+}
+
+// 1/x: FP64 within an ulp of the quotient, FP32 the division
 template <typename T>
 __device__ __forceinline__ T rcp(T x);
 template <>
 __device__ __forceinline__ double rcp<double>(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-x, r, 1.0);
-  return fma(r, fma(e, e, e), r);
+  const double r = rcp_seed(x);
+  return fma(r, fma(-x, r, 1.0), r);
 }
 template <>
 __device__ __forceinline__ float rcp<float>(float x) { return 1.0f / x; }
 
-// 1/sqrt(x), x > 0, FP64: the hardware's approximate reciprocal square root
-// (|x y^2 - 1| below 2^-19, measured over 4e7 samples) refined by one
-// third-order step of the series (1 - e)^(-1/2) = 1 + e/2 + 3e^2/8 + ...,
-// e = 1 - x y^2; within an ulp of 1/sqrt(x), and x times it within two ulps
-// of sqrt(x) (measured), in six dependent FP64 operations.
+// 1/sqrt(x), x > 0, within an ulp
 __device__ __forceinline__ double rsqrt_d(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y * y, 1.0);
-  return fma(y, e * fma(0.375, e, 0.5), y);
+  const double y = rsqrt_seed<false>(x), e = fma(-x, y * y, 1.0);
+  return fma(half(y), e, y);
 }
-// sqrt(x), x > 0, on the face and primitive paths: FP64 x * rsqrt_d(x)
-// (within two ulps of the rounded root, seven FP64 operations against about
-// ten for the correctly rounded one); FP32 the square root
+// sqrt(x) on the face and primitive paths: FP64 within two ulps of the
+// rounded root, FP32 the square root
 template <typename T>
 __device__ __forceinline__ T sqrt_p(T x);
 template <>
-__device__ __forceinline__ double sqrt_p<double>(double x) { return x * rsqrt_d(x); }
+__device__ __forceinline__ double sqrt_p<double>(double x) {
+  const double y = rsqrt_seed<true>(x), g = x * y, e = fma(-x, y * y, 1.0);
+  return fma(half(g), e, g);
+}
 template <>
 __device__ __forceinline__ float sqrt_p<float>(float x) { return sqrtf(x); }
+// the square root function where x is not a positive normal number (T < 0: NaN)
+__device__ __forceinline__ double sqrt_t(double x) {
+  return (unsigned)__double2hiint(x) - 0x00100000u < 0x7fe00000u ? sqrt_p(x) : sqrt(x);
+}
+// sqrt(a / b) = |a| / sqrt(a b): no reciprocal
+template <typename T>
+__device__ __forceinline__ T sqrt_ratio(T a, T b);
+template <>
+__device__ __forceinline__ double sqrt_ratio<double>(double a, double b) {
+  const double w = a * b, y = rsqrt_seed<true>(w), g = fabs(a) * y, e = fma(-w, y * y, 1.0);
+  return fma(half(g), e, g);
+}
+template <>
+__device__ __forceinline__ float sqrt_ratio<float>(float a, float b) { return sqrtf(a / b); }
+
+// the gas constants of a case in the arithmetic of a face
+template <typename T>
+struct Gas {
+  T g, gm1, ggm1, rgm1, rg;  // gamma, gamma - 1, gamma / (gamma - 1), 1 / (gamma - 1), 1 / gamma
+};
+template <typename T>
+__device__ __forceinline__ Gas<T> gas(const CaseDev &c) {
+  return {to<T>(c.gamma), to<T>(c.gm1), to<T>(c.ggm1), to<T>(c.rgm1), to<T>(c.rg)};
+}
 
 // The face physics below is written once for the arithmetic type T: double
 // is the reference's arithmetic (every literal T(x) is then the same double
@@ -181,270 +310,287 @@ __device__ __forceinline__ float sqrt_p<float>(float x) { return sqrtf(x); }
 
 // ---- reconstruction, sub_Residual.f90:477-659 --------------------------------
 template <typename T>
-__device__ __forceinline__ T minmod(T a, T b) {
-  if (a * b <= T(0.0)) return T(0.0);
-  return (fabs(a) <= fabs(b)) ? a : b;
+__device__ __forceinline__ T minmod(T a, T b);
+// zero where a b <= 0, else the one of smaller magnitude, by integer compares
+template <>
+__device__ __forceinline__ double minmod<double>(double a, double b) {
+  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+  const long long ax = x & 0x7fffffffffffffffll, ay = y & 0x7fffffffffffffffll, inf = 0x7ff0000000000000ll;
+  if (ax > inf || ay > inf) return b;  // a NaN: as the comparisons of doubles take it
+  if ((x ^ y) < 0 || ax == 0 || ay == 0) return 0.0;
+  return ax <= ay ? a : b;
+}
+template <>
+__device__ __forceinline__ float minmod<float>(float a, float b) {
+  if (a * b <= 0.0f) return 0.0f;
+  return (fabsf(a) <= fabsf(b)) ? a : b;
 }
 
-// scheme_fP (sub_Residual.f90:591-623): left state at the face between u2 and u3
+// scheme_fP and scheme_fm (sub_Residual.f90:591-659): the left and right state
+// at the face between u2 and u3.  Both sides in one pass over the three
+// differences; every scheme is u2 (u3) plus a correction, in the same formulas as the
+// reference with one reciprocal in place of its divides.
 template <typename T>
-__device__ __forceinline__ T scheme_fp(T u1, T u2, T u3, T u4, int flag) {
+__device__ __forceinline__ void scheme_pair(T u1, T u2, T u3, T u4, int flag, T &l, T &r) {
   const T ep = T(1.0e-6), k3 = T(1.0) / T(3.0);
+  const T d1 = u2 - u1, d2 = u3 - u2, d3 = u4 - u3;
   switch (flag) {
-    case Scheme_UD1: return u2;
-    case Scheme_UD3: return (-u1 + T(5.0) * u2 + T(2.0) * u3) / T(6.0);
-    case Scheme_NND2: return u2 + T(0.5) * minmod(u2 - u1, u3 - u2);
+    case Scheme_UD1: l = u2; r = u3; return;
+    case Scheme_UD3:
+      l = (-u1 + T(5.0) * u2 + T(2.0) * u3) * (T(1.0) / T(6.0));
+      r = (T(2.0) * u2 + T(5.0) * u3 - u4) * (T(1.0) / T(6.0));
+      return;
+    case Scheme_NND2:
+      l = u2 + half(minmod(d1, d2));
+      r = u3 - half(minmod(d2, d3));
+      return;
     case Scheme_WENO3: {
-      T IS1 = (u2 - u1) * (u2 - u1), IS2 = (u3 - u2) * (u3 - u2);
-      T e1 = T(1.0e-6) + IS1, e2 = T(1.0e-6) + IS2;
-      T a1 = T(1.0) / (T(3.0) * (e1 * e1)), a2 = T(2.0) / (T(3.0) * (e2 * e2));
-      T w1 = a1 / (a1 + a2), w2 = a2 / (a1 + a2);
-      return w1 * (-u1 / T(2.0) + T(3.0) * u2 / T(2.0)) + w2 * (u2 / T(2.0) + u3 / T(2.0));
+      // weights a_1 / (a_1 + a_2), a_2 / (a_1 + a_2) with a_1 = 1 / (3 q_1), a_2 = 2 / (3 q_2)
+      // over the common denominator q_2 + 2 q_1, q_k = (ep + d_k^2)^2 >= 1e-12
+      const T e1 = fma(d1, d1, ep), e2 = fma(d2, d2, ep), e3 = fma(d3, d3, ep);
+      const T q1 = pow2<1>(e1 * e1), q2 = e2 * e2, q3 = pow2<1>(e3 * e3);
+      l = fma(half(fma(q1, d2, q2 * d1)), rcp(q1 + q2), u2);
+      r = fma(-(half(fma(q3, d2, q2 * d3))), rcp(q3 + q2), u3);
+      return;
     }
-    case Scheme_MUSCL2:  // k=1, b=2
-      return u2 + T(0.25) * ((T(1.0) - T(1.0)) * minmod(u2 - u1, T(2.0) * (u3 - u2)) + (T(1.0) + T(1.0)) * minmod(u3 - u2, T(2.0) * (u2 - u1)));
-    case Scheme_MUSCL3: {
-      T up = u3 - u2, um = u2 - u1;
-      T s = (T(2.0) * up * um + ep) * rcp(up * up + um * um + ep);
-      return u2 + T(0.25) * s * ((T(1.0) - k3 * s) * um + (T(1.0) + k3 * s) * up);
-    }
-    case Scheme_OMUSCL2: {
-      T r1 = (u2 - u1 + ep) / (u3 - u2 + ep), r2 = (u3 - u2 + ep) / (u4 - u3 + ep);
-      T f1 = T(0.8) - T(0.175) / r2 + T(0.375) * r1;
-      T f = fmax(T(0.0), fmin(fmin(T(2.0), f1), T(2.0) * r1));
-      return u2 + T(0.5) * f * (u3 - u2);
-    }
-  }
-  return T(0.0);
-}
-// scheme_fm (sub_Residual.f90:626-659): right state at the face between u2 and u3
-template <typename T>
-__device__ __forceinline__ T scheme_fm(T u1, T u2, T u3, T u4, int flag) {
-  const T ep = T(1.0e-6), k3 = T(1.0) / T(3.0);
-  switch (flag) {
-    case Scheme_UD1: return u3;
-    case Scheme_UD3: return (T(2.0) * u2 + T(5.0) * u3 - u4) / T(6.0);
-    case Scheme_NND2: return u3 - T(0.5) * minmod(u3 - u2, u4 - u3);
-    case Scheme_WENO3: {
-      T IS1 = (u3 - u4) * (u3 - u4), IS2 = (u2 - u3) * (u2 - u3);
-      T e1 = T(1.0e-6) + IS1, e2 = T(1.0e-6) + IS2;
-      T a1 = T(1.0) / (T(3.0) * (e1 * e1)), a2 = T(2.0) / (T(3.0) * (e2 * e2));
-      T w1 = a1 / (a1 + a2), w2 = a2 / (a1 + a2);
-      return w1 * (-u4 / T(2.0) + T(3.0) * u3 / T(2.0)) + w2 * (u3 / T(2.0) + u2 / T(2.0));
-    }
-    case Scheme_MUSCL2: {  // k=1/3, b=1
-      const T k = T(1.0) / T(3.0);
-      return u3 - T(0.25) * ((T(1.0) - k) * minmod(u4 - u3, (u3 - u2)) + (T(1.0) + k) * minmod(u3 - u2, (u4 - u3)));
+    case Scheme_MUSCL2: {  // left: k = 1, b = 2; right: k = 1/3, b = 1
+      l = u2 + half(minmod(d2, pow2<1>(d1)));
+      const T k = T(1.0) / T(3.0), m = minmod(d3, d2);
+      r = u3 - pow2<-2>((T(1.0) - k) * m + (T(1.0) + k) * minmod(d2, d3));
+      return;
     }
     case Scheme_MUSCL3: {
-      T up = u4 - u3, um = u3 - u2;
-      T s = (T(2.0) * up * um + ep) * rcp(up * up + um * um + ep);
-      return u3 - T(0.25) * s * ((T(1.0) - k3 * s) * up + (T(1.0) + k3 * s) * um);
+      // s ((1 - k s) um + (1 + k s) up) / 4 = s ((um + up) + k s (up - um)) / 4, van
+      // Albada's s = (2 up um + ep) / (up^2 + um^2 + ep); on the right up and um change
+      // places
+      const T e2 = fma(d2, d2, ep), t2 = pow2<1>(d2);
+      T s = fma(t2, d1, ep) * rcp(fma(d1, d1, e2));
+      l = fma(pow2<-2>(s), fma(k3 * s, d2 - d1, u3 - u1), u2);
+      s = fma(t2, d3, ep) * rcp(fma(d3, d3, e2));
+      r = fma(-(pow2<-2>(s)), fma(k3 * s, d2 - d3, u4 - u2), u3);
+      return;
     }
     case Scheme_OMUSCL2: {
-      T r1 = (u4 - u3 + ep) / (u3 - u2 + ep), r2 = (u3 - u2 + ep) / (u2 - u1 + ep);
+      T r1 = (d1 + ep) / (d2 + ep), r2 = (d2 + ep) / (d3 + ep);
       T f1 = T(0.8) - T(0.175) / r2 + T(0.375) * r1;
       T f = fmax(T(0.0), fmin(fmin(T(2.0), f1), T(2.0) * r1));
-      return u3 - T(0.5) * f * (u3 - u2);
+      l = u2 + T(0.5) * f * d2;
+      r1 = (d3 + ep) / (d2 + ep);
+      r2 = (d2 + ep) / (d1 + ep);
+      f1 = T(0.8) - T(0.175) / r2 + T(0.375) * r1;
+      f = fmax(T(0.0), fmin(fmin(T(2.0), f1), T(2.0) * r1));
+      r = u3 - T(0.5) * f * d2;
+      return;
     }
   }
-  return T(0.0);
+  l = r = T(0.0);
 }
 
 // conservative (rho, rho u, rho v, E) -> primitive (rho, u, v, p), as at the
 // end of Reconstuction_conservative/Characteristic (sub_Residual.f90:526-527)
 template <typename T>
 __device__ __forceinline__ void cons_to_prim(const T Q[4], T W[4], T gm1) {
+  const T r = rcp(Q[0]);
   W[0] = Q[0];
-  W[1] = Q[1] / W[0];
-  W[2] = Q[2] / W[0];
-  W[3] = (Q[3] - (W[1] * Q[1] + W[2] * Q[2]) * T(0.5)) * gm1;
+  W[1] = Q[1] * r;
+  W[2] = Q[2] * r;
+  W[3] = (Q[3] - half(fma(W[2], Q[2], W[1] * Q[1]))) * gm1;
 }
 
 // S0[k][m]: stencil points k = i-2..i+1 (or j-2..j+1), variable m.
 // Reconstuction_original/conservative/Characteristic (sub_Residual.f90:505-586)
 template <typename T>
-__device__ __forceinline__ void reconstruct(int recon, int scheme, T S0[4][4], T gamma,
-                                            T UL[4], T UR[4]) {
+__device__ __forceinline__ void reconstruct(int recon, int scheme, T S0[4][4], const Gas<T> &G, T UL[4], T UR[4]) {
   if (recon == Recon_Original) {
 #pragma unroll
-    for (int m = 0; m < 4; m++) {
-      UL[m] = scheme_fp(S0[0][m], S0[1][m], S0[2][m], S0[3][m], scheme);
-      UR[m] = scheme_fm(S0[0][m], S0[1][m], S0[2][m], S0[3][m], scheme);
-    }
+    for (int m = 0; m < 4; m++) scheme_pair(S0[0][m], S0[1][m], S0[2][m], S0[3][m], scheme, UL[m], UR[m]);
     return;
   }
-  T gm1 = gamma - T(1.0);
+  T QL[4], QR[4];
   if (recon == Recon_Conservative) {
-    T QL[4], QR[4];
 #pragma unroll
-    for (int m = 0; m < 4; m++) {
-      QL[m] = scheme_fp(S0[0][m], S0[1][m], S0[2][m], S0[3][m], scheme);
-      QR[m] = scheme_fm(S0[0][m], S0[1][m], S0[2][m], S0[3][m], scheme);
-    }
-    cons_to_prim(QL, UL, gm1);
-    cons_to_prim(QR, UR, gm1);
+    for (int m = 0; m < 4; m++) scheme_pair(S0[0][m], S0[1][m], S0[2][m], S0[3][m], scheme, QL[m], QR[m]);
+    cons_to_prim(QL, UL, G.gm1);
+    cons_to_prim(QR, UR, G.gm1);
     return;
   }
   // characteristic: project on the left eigenvectors at the arithmetic
   // mid-state, limit each characteristic variable, project back
   T Uh[4];
 #pragma unroll
-  for (int m = 0; m < 4; m++) Uh[m] = T(0.5) * (S0[1][m] + S0[2][m]);
-  T d1 = Uh[0], u1 = Uh[1] / d1, v1 = Uh[2] / d1;
-  T p1 = (Uh[3] - (Uh[1] * u1 + Uh[2] * v1) * T(0.5)) * gm1;
-  T c1 = sqrt(gamma * p1 / d1);
-  T V2 = (u1 * u1 + v1 * v1) * T(0.5);
-  T tmp1 = gm1 / c1, tmp3 = gm1 / (c1 * c1), tmp5 = T(1.0) / (T(2.0) * c1), tmp0 = T(1.0) / tmp3;
-  const T Sm[4][4] = {{V2 - tmp0, -u1, -v1, T(1.0)},
-                           {-v1, T(0.0), T(1.0), T(0.0)},
-                           {-u1 - V2 * tmp1, T(1.0) + tmp1 * u1, tmp1 * v1, -tmp1},
-                           {-u1 + V2 * tmp1, T(1.0) - tmp1 * u1, -tmp1 * v1, tmp1}};
+  for (int m = 0; m < 4; m++) Uh[m] = half(S0[1][m] + S0[2][m]);
+  const T rd = rcp(Uh[0]), u1 = Uh[1] * rd, v1 = Uh[2] * rd;
+  const T p1 = (Uh[3] - half(fma(Uh[2], v1, Uh[1] * u1))) * G.gm1;
+  // sound speed c1 and its inverse from c^2 = gamma p / rho
+  const T c2 = G.g * p1 * rd;
+  const T c1 = sqrt_p(c2), ic = c1 * rcp(c2);
+  const T V2 = half(fma(v1, v1, u1 * u1));
+  const T tmp1 = G.gm1 * ic, tmp3 = tmp1 * ic, tmp5 = half(ic), tmp0 = c2 * G.rgm1;
+  const T a0 = V2 - tmp0, vt = V2 * tmp1, ut = tmp1 * u1, wt = tmp1 * v1;
   T V0[4][4];
 #pragma unroll
-  for (int k = 0; k < 4; k++)
-#pragma unroll
-    for (int m = 0; m < 4; m++)
-      V0[k][m] = Sm[m][0] * S0[k][0] + Sm[m][1] * S0[k][1] + Sm[m][2] * S0[k][2] + Sm[m][3] * S0[k][3];
+  for (int k = 0; k < 4; k++) {
+    const T *S = S0[k];
+    V0[k][0] = fma(a0, S[0], fma(-u1, S[1], fma(-v1, S[2], S[3])));
+    V0[k][1] = fma(-v1, S[0], S[2]);
+    // the two acoustic rows share everything but a sign
+    const T e = fma(vt, S[0], fma(-ut, S[1], fma(-wt, S[2], tmp1 * S[3])));
+    const T o = fma(-u1, S[0], S[1]);
+    V0[k][2] = o - e;
+    V0[k][3] = o + e;
+  }
   T VL[4], VR[4];
 #pragma unroll
-  for (int m = 0; m < 4; m++) {
-    VL[m] = scheme_fp(V0[0][m], V0[1][m], V0[2][m], V0[3][m], scheme);
-    VR[m] = scheme_fm(V0[0][m], V0[1][m], V0[2][m], V0[3][m], scheme);
-  }
-  const T S1[4][4] = {{-tmp3, T(0.0), -tmp5, tmp5},
-                           {-tmp3 * u1, T(0.0), T(0.5) - u1 * tmp5, T(0.5) + u1 * tmp5},
-                           {-tmp3 * v1, T(1.0), -v1 * tmp5, v1 * tmp5},
-                           {-tmp3 * V2, v1, (c1 * u1 - V2 - tmp0) * tmp5, (c1 * u1 + V2 + tmp0) * tmp5}};
-  T QL[4], QR[4];
+  for (int m = 0; m < 4; m++) scheme_pair(V0[0][m], V0[1][m], V0[2][m], V0[3][m], scheme, VL[m], VR[m]);
 #pragma unroll
-  for (int m = 0; m < 4; m++) {
-    QL[m] = S1[m][0] * VL[0] + S1[m][1] * VL[1] + S1[m][2] * VL[2] + S1[m][3] * VL[3];
-    QR[m] = S1[m][0] * VR[0] + S1[m][1] * VR[1] + S1[m][2] * VR[2] + S1[m][3] * VR[3];
+  for (int side = 0; side < 2; side++) {
+    const T *V = side ? VR : VL;
+    T *Q = side ? QR : QL;
+    // back: with e = -tmp3 V0 (entropy), s = V2 + V3, d = (V3 - V2) tmp5
+    const T e = -(tmp3 * V[0]), sum = V[2] + V[3], dif = (V[3] - V[2]) * tmp5, r0 = e + dif;
+    Q[0] = r0;
+    Q[1] = fma(u1, r0, half(sum));
+    Q[2] = fma(v1, r0, V[1]);
+    Q[3] = fma(V2, r0, fma(v1, V[1], fma(u1, half(sum), tmp0 * dif)));
   }
-  cons_to_prim(QL, UL, gm1);
-  cons_to_prim(QR, UR, gm1);
+  cons_to_prim(QL, UL, G.gm1);
+  cons_to_prim(QR, UR, G.gm1);
 }
 
-// ---- 1-D face fluxes on rotated primitive states (rho, u_n, u_t, p) ----------
+// ---- face fluxes -------------------------------------------------------------
+// Roe and AUSM+ take the primitive states (rho, u, v, p) as they are and give
+// F = -s (flux through the face with unit normal n and length s): the reference
+// turns the states into the face's frame and the flux back, which multiplies
+// out to the same sums (16 FP64 instructions less).
 // Flux_Roe_1D, sub_flux_split.f90:265-324 (Harten entropy fix, delta = 0.1)
 template <typename T>
-__device__ __forceinline__ void flux_roe(const T *QL, const T *QR, T *F, T gamma, T ggm1) {
-  const T delt = T(0.1);
-  T dl = QL[0], uul = QL[1], vvl = QL[2], pl = QL[3];
-  T dr = QR[0], uur = QR[1], vvr = QR[2], pr = QR[3];
-  T gm1 = gamma - T(1.0);
-  const T rdl = rcp(dl), rdr = rcp(dr);
-  T hl = ggm1 * pl * rdl + T(0.5) * (uul * uul + vvl * vvl);
-  T hr = ggm1 * pr * rdr + T(0.5) * (uur * uur + vvr * vvr);
-  T Fl0 = dl * uul, Fl1 = dl * uul * uul + pl, Fl2 = dl * uul * vvl, Fl3 = uul * dl * hl;
-  T Fr0 = dr * uur, Fr1 = dr * uur * uur + pr, Fr2 = dr * uur * vvr, Fr3 = uur * dr * hr;
-  T tmpp = sqrt_p(dr * rdl);
-  T inv = rcp(T(1.0) + tmpp);
-  T avd = T(0.25) * dl * (T(1.0) + tmpp) * (T(1.0) + tmpp);
-  T avu = (uul + tmpp * uur) * inv;
-  T avv = (vvl + tmpp * vvr) * inv;
-  T avh = (hl + tmpp * hr) * inv;
-  T ava = sqrt_p(gm1 * (avh - T(0.5) * (avu * avu + avv * avv)));
-  T l0 = fabs(avu - ava), l1 = fabs(avu), l3 = fabs(avu + ava);
-  const T i2d = T(1.0) / (T(2.0) * delt);
-  if (l0 < delt) l0 = (l0 * l0 + delt * delt) * i2d;
-  if (l1 < delt) l1 = (l1 * l1 + delt * delt) * i2d;
-  T l2 = l1;
-  if (l3 < delt) l3 = (l3 * l3 + delt * delt) * i2d;
-  T ia = rcp(ava);
-  T i2aa = T(0.5) * ia * ia;
-  T dp = pr - pl;
-  T a0 = (avd * ava * (-uur + uul) + dp) * i2aa;
-  T a1 = dr - dl - dp * (ia * ia);
-  T a2 = avd * (vvr - vvl) * ia;
-  T a3 = (avd * ava * (uur - uul) + dp) * i2aa;
-  F[0] = T(0.5) * (Fl0 + Fr0) - T(0.5) * (l0 * a0 + l1 * a1 + l3 * a3);
-  F[1] = T(0.5) * (Fl1 + Fr1) - T(0.5) * (l0 * a0 * (avu - ava) + l1 * a1 * avu + l3 * a3 * (avu + ava));
-  F[2] = T(0.5) * (Fl2 + Fr2) - T(0.5) * (l0 * a0 * avv + l1 * a1 * avv + l2 * a2 + l3 * a3 * avv);
-  F[3] = T(0.5) * (Fl3 + Fr3) - T(0.5) * (l0 * a0 * (avh - avu * ava) + l1 * a1 * T(0.5) * (avu * avu + avv * avv) +
-                                    l2 * a2 * avv + l3 * a3 * (avh + avu * ava));
+__device__ __forceinline__ T harten(T l) {
+  const T delt = T(0.1), i2d = T(1.0) / (T(2.0) * delt);
+  if (below(l, delt)) l = fma(l, l, delt * delt) * i2d;
+  return l;
 }
-
-// Flux_Ausm_1Da (AUSM+), sub_flux_split.f90:195-261
 template <typename T>
-__device__ __forceinline__ void flux_ausm(const T *QL, const T *QR, T *F, T gamma, T ggm1) {
-  T dl = QL[0], uul = QL[1], vvl = QL[2], pl = QL[3];
-  T dr = QR[0], uur = QR[1], vvr = QR[2], pr = QR[3];
-  const T rdl = rcp(dl), rdr = rcp(dr);
-  const T prl = pl * rdl, prr = pr * rdr;  // p / rho
-  T hl = ggm1 * prl + T(0.5) * (uul * uul + vvl * vvl);
-  T hr = ggm1 * prr + T(0.5) * (uur * uur + vvr * vvr);
-  T al = sqrt_p(gamma * prl), ar = sqrt_p(gamma * prr);
-  T a = T(0.5) * (al + ar);
-  T ia = rcp(a);
-  T Ml = uul * ia, Mr = uur * ia;
-  T Mp4, Mm4, Pp5, Pm5;
-  T ml2 = Ml * Ml - T(1.0), mr2 = Mr * Mr - T(1.0);
-  if (fabs(Ml) >= T(1.0)) { Mp4 = T(0.5) * (Ml + fabs(Ml)); Pp5 = T(0.5) * (Ml + fabs(Ml)) / Ml; }
-  else { Mp4 = T(0.25) * (Ml + T(1.0)) * (Ml + T(1.0)) + T(0.125) * ml2 * ml2;
-         Pp5 = T(0.25) * (Ml + T(1.0)) * (Ml + T(1.0)) * (T(2.0) - Ml) + T(3.0) * Ml * ml2 * ml2 / T(16.0); }
-  if (fabs(Mr) >= T(1.0)) { Mm4 = T(0.5) * (Mr - fabs(Mr)); Pm5 = T(0.5) * (Mr - fabs(Mr)) / Mr; }
-  else { Mm4 = -T(0.25) * (Mr - T(1.0)) * (Mr - T(1.0)) - T(0.125) * mr2 * mr2;
-         Pm5 = T(0.25) * (Mr - T(1.0)) * (Mr - T(1.0)) * (T(2.0) + Mr) - T(3.0) * Mr * mr2 * mr2 / T(16.0); }
-  T M = Mp4 + Mm4;
-  T xm = dl * a * fmax(T(0.0), M) + dr * a * fmin(T(0.0), M);
-  T dm = (M >= T(0.0)) ? a * fabs(M) * dl : a * fabs(M) * dr;
-  T p = pl * Pp5 + pr * Pm5;
-  F[0] = xm;  // 0.5 xm (1 + 1) - 0.5 dm (1 - 1): the same value for finite xm, dm
-  F[1] = T(0.5) * xm * (uul + uur) - T(0.5) * dm * (uur - uul) + p;
-  F[2] = T(0.5) * xm * (vvl + vvr) - T(0.5) * dm * (vvr - vvl);
-  F[3] = T(0.5) * xm * (hl + hr) - T(0.5) * dm * (hr - hl);
+__device__ __forceinline__ void flux_roe(const T *L, const T *R, T n1, T n2, T s, T *F, const Gas<T> &G) {
+  const T dl = L[0], ul = L[1], vl = L[2], pl = L[3], dr = R[0], ur = R[1], vr = R[2], pr = R[3];
+  const T unl = fma(vl, n2, ul * n1), unr = fma(vr, n2, ur * n1);
+  const T hl = fma(G.ggm1 * pl, rcp(dl), half(fma(vl, vl, ul * ul)));
+  const T hr = fma(G.ggm1 * pr, rcp(dr), half(fma(vr, vr, ur * ur)));
+  // Roe averages: t = sqrt(rho_r / rho_l)
+  const T t = sqrt_ratio(dr, dl), t1 = t + T(1.0), inv = rcp(t1);
+  const T ad = pow2<-2>(dl * (t1 * t1));
+  const T au = fma(t, ur, ul) * inv, av = fma(t, vr, vl) * inv, ah = fma(t, hr, hl) * inv;
+  const T an = fma(av, n2, au * n1), at = fma(av, n1, -(au * n2));  // normal and tangential
+  const T k2 = half(fma(av, av, au * au));
+  const T c2 = G.gm1 * (ah - k2);
+  const T c = sqrt_p(c2), ic2 = rcp(c2), ic = c * ic2;
+  const T l0 = harten(fabs(an - c)), l1 = harten(fabs(an)), l3 = harten(fabs(an + c));
+  const T dp = pr - pl, du = ur - ul, dv = vr - vl;
+  const T x = (ad * c) * (unr - unl), i2 = half(ic2);
+  const T w0 = l0 * ((dp - x) * i2), w3 = l3 * ((dp + x) * i2), w1 = l1 * fma(-dp, ic2, dr - dl);
+  const T w2 = l1 * (ad * fma(dv, n1, -(du * n2)) * ic);
+  // with S = w0 + w1 + w3 and q = (w3 - w0) c the dissipation is (S, S u + q n1 - w2 n2,
+  // S v + q n2 + w2 n1, (w0 + w3) h + q u_n + w1 |u|^2 / 2 + w2 u_t)
+  const T w03 = w0 + w3, S = w03 + w1, q = (w3 - w0) * c;
+  const T ml = dl * unl, mr = dr * unr, pp = (pl + pr) - q, hs = neg(half(s));
+  F[0] = ((ml + mr) - S) * hs;
+  F[1] = fma(ml, ul, fma(mr, ur, fma(-S, au, fma(pp, n1, w2 * n2)))) * hs;
+  F[2] = fma(ml, vl, fma(mr, vr, fma(-S, av, fma(pp, n2, -(w2 * n1))))) * hs;
+  F[3] = (fma(ml, hl, mr * hr) - fma(w03, ah, fma(q, an, fma(w1, k2, w2 * at)))) * hs;
 }
 
+// Flux_Ausm_1Da (AUSM+), sub_flux_split.f90:195-261.  Its sums 0.5 xm (f_l + f_r) -
+// 0.5 dm (f_r - f_l) with dm = a |M| rho of the upwind side are xm times f of the
+// upwind side, so only that side's enthalpy is formed.
+template <typename T>
+__device__ __forceinline__ bool supersonic(T m);
+template <>
+__device__ __forceinline__ bool supersonic<double>(double m) {  // 1 <= |m| < infinity
+  return ((unsigned)__double2hiint(m) & 0x7fffffffu) - 0x3ff00000u < 0x40000000u;
+}
+template <>
+__device__ __forceinline__ bool supersonic<float>(float m) { return fabsf(m) >= 1.0f; }
+// split Mach number and pressure of the left state; the right state's are -m4(-M)
+// and p5(-M)
+template <typename T>
+__device__ __forceinline__ void ausm_split(T m, T &m4, T &p5) {
+  if (supersonic(m)) {
+    m4 = sign_clear(m) ? m : T(0.0);
+    p5 = sign_clear(m) ? T(1.0) : T(0.0);
+    return;
+  }
+  const T a = m + T(1.0), q = pow2<-2>(a * a), r = fma(m, m, T(-1.0)), w = r * r;
+  m4 = fma(T(0.125), w, q);
+  p5 = fma(T(0.1875) * m, w, q * (T(2.0) - m));
+}
+template <typename T>
+__device__ __forceinline__ void flux_ausm(const T *L, const T *R, T n1, T n2, T s, T *F, const Gas<T> &G) {
+  const T unl = fma(L[2], n2, L[1] * n1), unr = fma(R[2], n2, R[1] * n1);
+  const T al = sqrt_ratio(G.g * L[3], L[0]), ar = sqrt_ratio(G.g * R[3], R[0]);
+  const T a = half(al + ar), ia = rcp(a);
+  T m4, p5, n4, q5;
+  ausm_split(unl * ia, m4, p5);
+  ausm_split(-(unr * ia), n4, q5);
+  const T M = m4 - n4;
+  const bool left = sign_clear(M);
+  const T d = left ? L[0] : R[0], u = left ? L[1] : R[1], v = left ? L[2] : R[2], c = left ? al : ar;
+  const T ns = neg(s), xm = (a * M) * (d * ns), p = fma(L[3], p5, R[3] * q5) * ns;
+  const T h = fma(c * c, G.rgm1, half(fma(v, v, u * u)));
+  F[0] = xm;
+  F[1] = fma(xm, u, p * n1);
+  F[2] = fma(xm, v, p * n2);
+  F[3] = xm * h;
+}
+
+// The other fluxes in the face's frame: rotated primitive states (rho, u_n, u_t, p).
 // Flux_Van_Leer_1Da, sub_flux_split.f90:139-189
 template <typename T>
-__device__ __forceinline__ void flux_vanleer(const T *QL, const T *QR, T *F, T gamma) {
+__device__ __forceinline__ void flux_vanleer(const T *QL, const T *QR, T *F, const Gas<T> &G) {
   T dl = QL[0], uul = QL[1], vvl = QL[2], pl = QL[3];
   T dr = QR[0], uur = QR[1], vvr = QR[2], pr = QR[3];
-  T gm1 = gamma - T(1.0);
-  T al = sqrt(gamma * pl / dl), ar = sqrt(gamma * pr / dr);
-  T Ml = uul / al, Mr = uur / ar;
+  const T gamma = G.g, gm1 = G.gm1, rg = G.rg, rgg = rcp(gamma * gamma - T(1.0));
+  T al = sqrt_ratio(gamma * pl, dl), ar = sqrt_ratio(gamma * pr, dr);
   T fp0 = 0, fp1 = 0, fp2 = 0, fp3 = 0, fm0 = 0, fm1 = 0, fm2 = 0, fm3 = 0;
-  if (Ml >= T(1.0)) {
+  if (uul >= al) {
     fp0 = dl * uul; fp1 = dl * uul * uul + pl; fp2 = dl * uul * vvl;
-    fp3 = uul * (gamma * pl / gm1 + T(0.5) * dl * (uul * uul + vvl * vvl));
-  } else if (fabs(Ml) < T(1.0)) {
+    fp3 = uul * (G.ggm1 * pl + T(0.5) * dl * (uul * uul + vvl * vvl));
+  } else if (fabs(uul) < al) {
+    const T Ml = uul * rcp(al);
     T tmp0 = dl * al * (T(0.25) * (T(1.0) + Ml) * (T(1.0) + Ml));
     T w = gm1 * uul + T(2.0) * al;
-    fp0 = tmp0; fp1 = tmp0 * w / gamma; fp2 = tmp0 * vvl;
-    fp3 = tmp0 * (w * w * T(0.5) / (gamma * gamma - T(1.0)) + T(0.5) * (vvl * vvl));
+    fp0 = tmp0; fp1 = tmp0 * w * rg; fp2 = tmp0 * vvl;
+    fp3 = tmp0 * T(0.5) * (w * w * rgg + vvl * vvl);
   }
-  if (Mr >= T(1.0)) {
-  } else if (fabs(Mr) < T(1.0)) {
+  if (uur >= ar) {
+  } else if (fabs(uur) < ar) {
+    const T Mr = uur * rcp(ar);
     T tmp0 = dr * ar * (-T(0.25) * (Mr - T(1.0)) * (Mr - T(1.0)));
     T w = gm1 * uur - T(2.0) * ar;
-    fm0 = tmp0; fm1 = tmp0 * w / gamma; fm2 = tmp0 * vvr;
-    fm3 = tmp0 * (w * w * T(0.5) / (gamma * gamma - T(1.0)) + T(0.5) * (vvr * vvr));
-  } else if (Mr <= -T(1.0)) {
+    fm0 = tmp0; fm1 = tmp0 * w * rg; fm2 = tmp0 * vvr;
+    fm3 = tmp0 * T(0.5) * (w * w * rgg + vvr * vvr);
+  } else if (uur <= -ar) {
     fm0 = dr * uur; fm1 = dr * uur * uur + pr; fm2 = dr * uur * vvr;
-    fm3 = uur * (gamma * pr / gm1 + T(0.5) * dr * (uur * uur + vvr * vvr));
+    fm3 = uur * (G.ggm1 * pr + T(0.5) * dr * (uur * uur + vvr * vvr));
   }
   F[0] = fp0 + fm0; F[1] = fp1 + fm1; F[2] = fp2 + fm2; F[3] = fp3 + fm3;
 }
 
 // Flux_steger_warming_1Da, sub_flux_split.f90:99-136
 template <typename T>
-__device__ __forceinline__ void flux_sw(const T *QL, const T *QR, T *F, T gamma) {
+__device__ __forceinline__ void flux_sw(const T *QL, const T *QR, T *F, const Gas<T> &G) {
   T dl = QL[0], uul = QL[1], vvl = QL[2], pl = QL[3];
   T dr = QR[0], uur = QR[1], vvr = QR[2], pr = QR[3];
-  T al = sqrt(gamma * pl / dl), ar = sqrt(gamma * pr / dr);
-  T gm1 = gamma - T(1.0);
-  T tmp1 = T(2.0) * gm1, tmp3 = (T(3.0) - gamma) / (T(2.0) * gm1);
+  const T gamma = G.g, gm1 = G.gm1;
+  T al = sqrt_ratio(gamma * pl, dl), ar = sqrt_ratio(gamma * pr, dr);
+  T tmp1 = T(2.0) * gm1, tmp3 = T(0.5) * (T(3.0) - gamma) * G.rgm1;
   T E1P = (uul + fabs(uul)) * T(0.5), E2P = (uul - al + fabs(uul - al)) * T(0.5), E3P = (uul + al + fabs(uul + al)) * T(0.5);
-  T t0 = dl / (T(2.0) * gamma);
+  T t0 = dl * T(0.5) * G.rg;
   T p0 = t0 * (tmp1 * E1P + E2P + E3P);
   T p1 = t0 * (tmp1 * E1P * uul + E2P * (uul - al) + E3P * (uul + al));
   T p2 = t0 * (tmp1 * E1P * vvl + E2P * vvl + E3P * vvl);
   T p3 = t0 * (E1P * gm1 * (uul * uul + vvl * vvl) + E2P * ((uul - al) * (uul - al) + vvl * vvl) * T(0.5) +
                     E3P * ((uul + al) * (uul + al) + vvl * vvl) * T(0.5) + tmp3 * al * al * (E2P + E3P));
   T E1M = (uur - fabs(uur)) * T(0.5), E2M = (uur - ar - fabs(uur - ar)) * T(0.5), E3M = (uur + ar - fabs(uur + ar)) * T(0.5);
-  t0 = dr / (T(2.0) * gamma);
+  t0 = dr * T(0.5) * G.rg;
   T m0 = t0 * (tmp1 * E1M + E2M + E3M);
   T m1 = t0 * (tmp1 * E1M * uur + E2M * (uur - ar) + E3M * (uur + ar));
   T m2 = t0 * (tmp1 * E1M * vvr + E2M * vvr + E3M * vvr);
@@ -455,59 +601,66 @@ __device__ __forceinline__ void flux_sw(const T *QL, const T *QR, T *F, T gamma)
 
 // Flux_HLL_HLLC_1D, sub_flux_split.f90:16-93
 template <typename T>
-__device__ __forceinline__ void flux_hll(const T *QL, const T *QR, T *F, T gamma, bool hllc) {
+__device__ __forceinline__ void flux_hll(const T *QL, const T *QR, T *F, const Gas<T> &G, bool hllc) {
   T dl = QL[0], uul = QL[1], vvl = QL[2], pl = QL[3];
   T dr = QR[0], uur = QR[1], vvr = QR[2], pr = QR[3];
-  T gm1 = gamma - T(1.0);
-  T UL[4] = {dl, dl * uul, dl * vvl, pl / gm1 + dl * (uul * uul + vvl * vvl) * T(0.5)};
-  T UR[4] = {dr, dr * uur, dr * vvr, pr / gm1 + dr * (uur * uur + vvr * vvr) * T(0.5)};
-  T al = sqrt(gamma * pl / dl), ar = sqrt(gamma * pr / dr);
-  T p_pvrs = T(0.5) * (pl + pr) - (uur - uul) * (dl + dr) * (al + ar) * T(0.125);
+  T UL[4] = {dl, dl * uul, dl * vvl, pl * G.rgm1 + dl * half(uul * uul + vvl * vvl)};
+  T UR[4] = {dr, dr * uur, dr * vvr, pr * G.rgm1 + dr * half(uur * uur + vvr * vvr)};
+  T al = sqrt_ratio(G.g * pl, dl), ar = sqrt_ratio(G.g * pr, dr);
+  T p_pvrs = half(pl + pr) - (uur - uul) * (dl + dr) * pow2<-3>(al + ar);
   T p_star = fmax(T(0.0), p_pvrs);
-  T g2 = (gamma + T(1.0)) / (T(2.0) * gamma);
-  T qql = (p_star <= pl) ? T(1.0) : sqrt(T(1.0) + g2 * (p_star / pl - T(1.0)));
-  T qqr = (p_star <= pr) ? T(1.0) : sqrt(T(1.0) + g2 * (p_star / pr - T(1.0)));
+  const T g2 = half((G.g + T(1.0)) * G.rg);
+  T qql = (p_star <= pl) ? T(1.0) : sqrt_p(fma(g2, p_star * rcp(pl) - T(1.0), T(1.0)));
+  T qqr = (p_star <= pr) ? T(1.0) : sqrt_p(fma(g2, p_star * rcp(pr) - T(1.0), T(1.0)));
   T Sl = uul - al * qql, Sr = uur + ar * qqr;
   T Fl[4] = {UL[1], UL[1] * uul + pl, UL[2] * uul, uul * (UL[3] + pl)};
   T Fr[4] = {UR[1], UR[1] * uur + pr, UR[2] * uur, uur * (UR[3] + pr)};
   if (!hllc) {
     if (Sl >= 0) { for (int m = 0; m < 4; m++) F[m] = Fl[m]; }
     else if (Sr <= 0) { for (int m = 0; m < 4; m++) F[m] = Fr[m]; }
-    else { T inv = T(1.0) / (Sr - Sl);
+    else { T inv = rcp(Sr - Sl);
       for (int m = 0; m < 4; m++) F[m] = (Sr * Fl[m] - Sl * Fr[m] + Sl * Sr * (UR[m] - UL[m])) * inv; }
     return;
   }
-  T S_star = (pr - pl + dl * uul * (Sl - uul) - dr * uur * (Sr - uur)) / (dl * (Sl - uul) - dr * (Sr - uur));
+  const T bl = dl * (Sl - uul), br = dr * (Sr - uur);
+  T S_star = (pr - pl + bl * uul - br * uur) * rcp(bl - br);
   if (Sl >= 0) { for (int m = 0; m < 4; m++) F[m] = Fl[m]; return; }
   if (Sr <= 0) { for (int m = 0; m < 4; m++) F[m] = Fr[m]; return; }
-  if (S_star >= 0) {
-    T tmpl = dl * (Sl - uul) / (Sl - S_star);
-    T tmp = UL[3] / dl + (S_star - uul) * (S_star + pl / (dl * (Sl - uul)));
-    F[0] = Fl[0] + Sl * (tmpl - UL[0]);
-    F[1] = Fl[1] + Sl * (tmpl * S_star - UL[1]);
-    F[2] = Fl[2] + Sl * (tmpl * vvl - UL[2]);
-    F[3] = Fl[3] + Sl * (tmpl * tmp - UL[3]);
-  } else {
-    T tmpr = dr * (Sr - uur) / (Sr - S_star);
-    T tmp = UR[3] / dr + (S_star - uur) * (S_star + pr / (dr * (Sr - uur)));
-    F[0] = Fr[0] + Sr * (tmpr - UR[0]);
-    F[1] = Fr[1] + Sr * (tmpr * S_star - UR[1]);
-    F[2] = Fr[2] + Sr * (tmpr * vvr - UR[2]);
-    F[3] = Fr[3] + Sr * (tmpr * tmp - UR[3]);
-  }
+  // the star state of the side the face lies in
+  const bool left = S_star >= 0;
+  T U[4], Fs[4];
+#pragma unroll
+  for (int m = 0; m < 4; m++) { U[m] = left ? UL[m] : UR[m]; Fs[m] = left ? Fl[m] : Fr[m]; }
+  const T u = left ? uul : uur, v = left ? vvl : vvr, p = left ? pl : pr, b = left ? bl : br, S = left ? Sl : Sr;
+  // E / rho + (S* - u) (S* + p / b) over one reciprocal of rho b
+  const T d = U[0], rdb = rcp(d * b);
+  const T ts = b * rcp(S - S_star);
+  const T e = U[3] * (b * rdb) + (S_star - u) * (S_star + p * (d * rdb));
+  F[0] = Fs[0] + S * (ts - d);
+  F[1] = Fs[1] + S * (ts * S_star - U[1]);
+  F[2] = Fs[2] + S * (ts * v - U[2]);
+  F[3] = Fs[3] + S * (ts * e - U[3]);
 }
 
+// F = -s (flux through the face with unit normal n and length s)
 template <typename T>
-__device__ __forceinline__ void face_flux(int iflux, const T *QL, const T *QR, T *F, T gamma, T ggm1) {
+__device__ __forceinline__ void face_flux(int iflux, const T *L, const T *R, T n1, T n2, T s, T *F, const Gas<T> &G) {
+  if (iflux == Flux_Roe) { flux_roe(L, R, n1, n2, s, F, G); return; }
+  if (iflux == Flux_Ausm) { flux_ausm(L, R, n1, n2, s, F, G); return; }
+  const T QL[4] = {L[0], L[1] * n1 + L[2] * n2, -L[1] * n2 + L[2] * n1, L[3]};
+  const T QR[4] = {R[0], R[1] * n1 + R[2] * n2, -R[1] * n2 + R[2] * n1, R[3]};
+  T f[4] = {T(0.0), T(0.0), T(0.0), T(0.0)};
   switch (iflux) {
-    case Flux_Roe: flux_roe(QL, QR, F, gamma, ggm1); return;
-    case Flux_Ausm: flux_ausm(QL, QR, F, gamma, ggm1); return;
-    case Flux_VanLeer: flux_vanleer(QL, QR, F, gamma); return;
-    case Flux_SW: flux_sw(QL, QR, F, gamma); return;
-    case Flux_HLL: flux_hll(QL, QR, F, gamma, false); return;
-    case Flux_HLLC: flux_hll(QL, QR, F, gamma, true); return;
+    case Flux_VanLeer: flux_vanleer(QL, QR, f, G); break;
+    case Flux_SW: flux_sw(QL, QR, f, G); break;
+    case Flux_HLL: flux_hll(QL, QR, f, G, false); break;
+    case Flux_HLLC: flux_hll(QL, QR, f, G, true); break;
   }
-  F[0] = F[1] = F[2] = F[3] = T(0.0);
+  const T ns = neg(s);
+  F[0] = f[0] * ns;
+  F[1] = (f[1] * n1 - f[2] * n2) * ns;
+  F[2] = (f[1] * n2 + f[2] * n1) * ns;
+  F[3] = f[3] * ns;
 }
 
 // viscous stress and heat flux through a face from the face-local 2x2
@@ -529,21 +682,27 @@ __device__ __forceinline__ void viscous_face(T Dix, T Diy, T Djx, T Djy, T Diu, 
   F4 += (E1 * n1 + E2 * n2) * s;
 }
 
-// the same from the face's precomputed inverse Jacobian (A, B, C, D) =
-// (Djy, Diy, Djx, Dix) / (Dix Djy - Djx Diy): u_x = Diu A - Dju B,
-// u_y = Dju D - Diu C
+// The same from the face's four metric coefficients formed at set-up
+// (G_VIP..G_VIS, k_face_metrics), which give the derivatives of a quantity q
+// across the face and along it from its differences: d_n q = Diq P + Djq Q,
+// d_t q = Djq S - Diq R (a factor 1/4 of the averaged differences is in the
+// coefficients).  In the frame of the face the stress on it is
+//   F_x = mu (d_n u - d_t v + n1 div / 3),  F_y = mu (d_n v + d_t u + n2 div / 3),
+//   div = n1 (d_n u + d_t v) + n2 (d_n v - d_t u),
+// the same sums as (t11 n1 + t12 n2, t12 n1 + t22 n2), and the work and heat
+// u F_x + v F_y + k d_n T.  us, vs: the sums of the velocities of both sides; mu
+// and k already hold the face length.
 template <typename T>
-__device__ __forceinline__ void viscous_face_m(T A, T B, T C, T D, T Diu, T Div, T DiT, T Dju, T Djv, T DjT,
-                                               T Amu1, T Amk1, T u1, T v1, T n1, T n2, T s, T &F2, T &F3, T &F4) {
-  T ux = fma(Diu, A, -Dju * B), vx = fma(Div, A, -Djv * B), Tx = fma(DiT, A, -DjT * B);
-  T uy = fma(Dju, D, -Diu * C), vy = fma(Djv, D, -Div * C), Ty = fma(DjT, D, -DiT * C);
-  T t11 = ((T(4.0) / T(3.0)) * ux - (T(2.0) / T(3.0)) * vy) * Amu1;
-  T t22 = ((T(4.0) / T(3.0)) * vy - (T(2.0) / T(3.0)) * ux) * Amu1;
-  T t12 = (uy + vx) * Amu1;
-  T E1 = u1 * t11 + v1 * t12 + Amk1 * Tx, E2 = u1 * t12 + v1 * t22 + Amk1 * Ty;
-  F2 += (t11 * n1 + t12 * n2) * s;
-  F3 += (t12 * n1 + t22 * n2) * s;
-  F4 += (E1 * n1 + E2 * n2) * s;
+__device__ __forceinline__ void viscous_face_m(T P, T Q, T R, T S, T Diu, T Div, T DiT, T Dju, T Djv, T DjT, T mu, T k,
+                                               T us, T vs, T n1, T n2, T &F2, T &F3, T &F4) {
+  const T nu = fma(Diu, P, Dju * Q), nv = fma(Div, P, Djv * Q);
+  const T tu = fma(Dju, S, -(Diu * R)), tv = fma(Djv, S, -(Div * R));
+  const T d3 = fma(n1, nu + tv, n2 * (nv - tu)) * (T(1.0) / T(3.0));
+  const T fx = fma(n1, d3, nu - tv), fy = fma(n2, d3, nv + tu);
+  F2 = fma(fx, mu, F2);
+  F3 = fma(fy, mu, F3);
+  F4 = fma(fma(us, fx, vs * fy), half(mu), F4);
+  F4 = fma(fma(DiT, P, DjT * Q), k, F4);
 }
 
 // device-side error record (first error of a case wins)

@@ -220,11 +220,8 @@ __device__ __forceinline__ unsigned long long inbox_read(unsigned a) {
   asm volatile("ld.relaxed.cluster.shared::cta.b64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
   return v;
 }
-// -x and 2 x on the integer pipe (2 x of a normal number below 2^1022;
-// infinities and NaNs are left as they are)
-__device__ __forceinline__ double neg(double x) {
-  return __hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x));
-}
+// 2 x on the integer pipe (of a normal number below 2^1022; infinities and NaNs
+// are left as they are)
 __device__ __forceinline__ double twice(double x) {
   const int h = __double2hiint(x);
   return __hiloint2double((h & 0x7ff00000) < 0x7fe00000 ? h + 0x00100000 : h, __double2loint(x));
@@ -267,26 +264,6 @@ __device__ __forceinline__ void inbox_write_if(bool local, bool remote, unsigned
       "@q st.relaxed.cluster.shared::cluster.b64 [%0], %1;\n\t}" ::"r"(a),
       "l"(__double_as_longlong(x)), "r"((int)local), "r"((int)remote)
       : "memory");
-}
-
-// 1/x to about 44 bits without the FP64 pipe: x's mantissa as a float and the
-// float of its remaining bits, the FP32 approximate reciprocal r of the first,
-// and the correction r (e + e^2), e = 1 - x r, added to r's double as an
-// integer.  Runs in the shadow of FP64 instructions; one FP64 Newton step
-// makes it 1/x to an ulp.
-__device__ __forceinline__ double rcp_seed(double x) {
-  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-  const float xf = __uint_as_float((__funnelshift_l(lo, hi, 3) & 0x7fffffu) | 0x3f800000u);
-  const float xl = fmaf(__uint_as_float(((lo >> 6) & 0x7fffffu) | 0x3f800000u), 0x1p-23f, -0x1p-23f);
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(xf));  // in (0.5, 1]
-  const float e = fmaf(-xl, r, fmaf(-xf, r, 1.0f));
-  // the correction in units of 2^-52 (the double's are 2^-53 below 1)
-  const int q = __float2int_rn(r * 0x1p52f * fmaf(e, e, e));
-  const unsigned rb = __float_as_uint(r);
-  const unsigned long long y = (((unsigned long long)(rb >> 3) << 32) | (rb << 29)) + (unsigned long long)(2ll * q);
-  const unsigned yh = (unsigned)(y >> 32) + ((1023u - 127u) << 20) + (0x3ff00000u - (hi & 0x7ff00000u));
-  return __hiloint2double((int)(yh | (hi & 0x80000000u)), (int)(unsigned)y);
 }
 
 // what a lane reads for one step, one step ahead

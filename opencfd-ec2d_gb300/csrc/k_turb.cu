@@ -82,12 +82,11 @@ __global__ void k_sa_faces(Lvl L) {
     double vn1 = uu[w] * n1 + vv[w] * n2, vn2 = uu[id] * n1 + vv[id] * n2;
     double vfi = -0.5 * ((vn1 + fabs(vn1)) * vt[w] + (vn2 - fabs(vn2)) * vt[id]) * s0;
     double v0 = c0 * (vt[id] + amu[id] * rcp(d[id]) + vt[w] + amu[w] * rcp(d[w]));
-    // the face's inverse Jacobian, formed at set-up (k_face_metrics)
+    // the normal derivative by the face's coefficients formed at set-up (k_face_metrics)
     const double *gm = L.geo + id;
     double Div = vt[id] - vt[w];
-    double Djv = (vt[nN - 1] + vt[nN] - vt[nS - 1] - vt[nS]) * 0.25;
-    double vtx = fma(Div, gm[G_VIA * F], -Djv * gm[G_VIB * F]), vty = fma(Djv, gm[G_VID * F], -Div * gm[G_VIC * F]);
-    double g = (vtx * n1 + vty * n2) * s0;
+    double Djv = (vt[nN - 1] - vt[nS - 1]) + (vt[nN] - vt[nS]);
+    double g = fma(Div, gm[G_VIP * F], Djv * gm[G_VIQ * F]) * s0;
     L.fi[4 * F + id] = vfi + v0 * g;
     L.fi[5 * F + id] = g;
   }
@@ -98,10 +97,9 @@ __global__ void k_sa_faces(Lvl L) {
     double vfi = -0.5 * ((vn1 + fabs(vn1)) * vt[s] + (vn2 - fabs(vn2)) * vt[id]) * s0;
     double v0 = c0 * (vt[id] + amu[id] * rcp(d[id]) + vt[s] + amu[s] * rcp(d[s]));
     const double *gm = L.geo + id;
-    double Div = (vt[s + 1] + vt[id + 1] - vt[s - 1] - vt[id - 1]) * 0.25;
+    double Div = (vt[s + 1] - vt[s - 1]) + (vt[id + 1] - vt[id - 1]);
     double Djv = vt[id] - vt[s];
-    double vtx = fma(Div, gm[G_VJA * F], -Djv * gm[G_VJB * F]), vty = fma(Djv, gm[G_VJD * F], -Div * gm[G_VJC * F]);
-    double g = (vtx * n1 + vty * n2) * s0;
+    double g = fma(Div, gm[G_VJP * F], Djv * gm[G_VJQ * F]) * s0;
     L.fj[4 * F + id] = vfi + v0 * g;
     L.fj[5 * F + id] = g;
   }
