@@ -450,7 +450,7 @@ int build_level(ec2d_ctx *ctx, int l) {
   L.un1 = (P.Time_Method == Time_Dual && l == 1) ? dalloc<double>(lv, nv * F) : nullptr;
   L.fi = dalloc<double>(lv, 6 * F);
   L.fj = dalloc<double>(lv, 6 * F);
-  L.tb = (L.turb == Turb_SST) ? dalloc<double>(lv, 5 * F) : (L.turb == Turb_BL) ? dalloc<double>(lv, F) : nullptr;
+  L.tb = (L.turb == Turb_SST) ? dalloc<double>(lv, SST_PLANES * F) : (L.turb == Turb_BL) ? dalloc<double>(lv, F) : nullptr;
   bool anyfdm = false;
   for (auto &B : lv.hb) anyfdm |= B.fdm;
   L.met = anyfdm ? dalloc<double>(lv, 5 * F) : nullptr;

@@ -19,6 +19,7 @@ namespace ec2d {
 constexpr int LAP = 2;
 constexpr int LFDM = 4;
 constexpr double PrT = 0.9;
+constexpr int SST_PLANES = 7;  // scratch planes of the SST model
 
 enum { Scheme_UD1 = 0, Scheme_NND2 = 1, Scheme_UD3 = 2, Scheme_WENO3 = 3,
        Scheme_MUSCL2 = 4, Scheme_MUSCL3 = 5, Scheme_OMUSCL2 = 6 };
@@ -252,7 +253,7 @@ __device__ __forceinline__ double rsqrt_seed(double x) {
   return __hiloint2double(hi - 0x00100000u < 0x7fe00000u ? (int)yh : out, (int)(unsigned)y);
 }
 
-// 1/x: FP64 within an ulp of the quotient, FP32 the division
+// 1/x: FP64 the rounded quotient in all of 8e8 samples, FP32 the division
 template <typename T>
 __device__ __forceinline__ T rcp(T x);
 template <>
@@ -263,13 +264,21 @@ __device__ __forceinline__ double rcp<double>(double x) {
 template <>
 __device__ __forceinline__ float rcp<float>(float x) { return 1.0f / x; }
 
-// 1/sqrt(x), x > 0, within an ulp
+// 1/x where x may be zero or infinite: by the divide there
+__device__ __forceinline__ double rcp_any(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7ff00000u) - 0x00100000u < 0x7fc00000u ? rcp(x) : 1.0 / x;
+}
+// max(x, 0) and min(x, 0) by the sign (a NaN goes to one of them)
+__device__ __forceinline__ double pos_part(double x) { return __double2hiint(x) >= 0 ? x : 0.0; }
+__device__ __forceinline__ double neg_part(double x) { return __double2hiint(x) < 0 ? x : 0.0; }
+
+// 1/sqrt(x), x > 0, to two ulps
 __device__ __forceinline__ double rsqrt_d(double x) {
   const double y = rsqrt_seed<false>(x), e = fma(-x, y * y, 1.0);
   return fma(half(y), e, y);
 }
-// sqrt(x) on the face and primitive paths: FP64 within two ulps of the
-// rounded root, FP32 the square root
+// sqrt(x) on the face and primitive paths: FP64 within an ulp of the rounded
+// root, FP32 the square root
 template <typename T>
 __device__ __forceinline__ T sqrt_p(T x);
 template <>
