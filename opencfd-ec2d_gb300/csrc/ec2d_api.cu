@@ -779,7 +779,7 @@ void step_lusgs(ec2d_ctx *ctx, int l, double alfa1 = 0.0, bool fresh = false, bo
   advance_counters(ctx, l);
 }
 void clip(ec2d_ctx *ctx, int l) {
-  if (ctx->lv[l].L.nvar >= 5) K(ctx, "k_clip", l, 1, [&] { launch_bc(ctx->lv[l].L, 8, ctx->stream); });
+  if (ctx->lv[l].L.nvar >= 5) K(ctx, "k_clip", l, 1, [&] { launch_clip(ctx->lv[l].L, ctx->stream); });
 }
 // Dual_time_LU_SGS (sub_NS_singlegrid.f90:231-310).  The inner-loop exit test
 // on the RMS residual needs the norms on the host after every inner step.
@@ -2133,7 +2133,7 @@ int ec2d_mlp_warm_start(ec2d_mlp *m, ec2d_ctx *ctx, int *n_fallback) {
   if (r == EC2D_OK) {
     launch_warm_start(L, pred, bad, ctx->stream);
     launch_bc(L, 1 | 2 | 4, ctx->stream);
-    if (L.nvar >= 5) launch_bc(L, 8, ctx->stream);
+    launch_clip(L, ctx->stream);
   }
   std::vector<int> hb(ctx->cases.size());
   CK(cudaMemcpyAsync(hb.data(), bad, hb.size() * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));

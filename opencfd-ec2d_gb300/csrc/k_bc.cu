@@ -9,7 +9,7 @@
 // jst..jend, so its end points write ghost rows that later subfaces read.
 // The write sets of one subface never overlap its read set, halo copies read
 // only interior cells, and corners read only the block's own ghosts.  Hence
-// one CTA per block reproduces the reference exactly: subfaces of phase 1 in
+// one cluster per block reproduces the reference exactly: subfaces of phase 1 in
 // order with a barrier between them, all halo items of phase 2 in parallel,
 // then the corners.  Physical subfaces whose read and write sets do not meet
 // those of any earlier subface of the block share a barrier phase (the
@@ -26,60 +26,68 @@ __device__ __forceinline__ void ghost_pair(int face, int i, int j, int k, int &i
   else { i1 = i; j1 = j - k; i2 = i; j2 = j + k - 1; }
 }
 
+// the nvar variables of a cell, all loads in flight before the first use (a store between
+// them would hold each load back: the compiler cannot tell the two cells apart)
+struct Cell { double v[6]; };
+__device__ __forceinline__ Cell load_cell(const Lvl &L, long long id) {
+  Cell c;
+#pragma unroll
+  for (int m = 0; m < 6; m++) c.v[m] = m < L.nvar ? L.U[m * L.F + id] : 0.0;
+  return c;
+}
+__device__ __forceinline__ void store_cell(const Lvl &L, long long id, const Cell &c) {
+#pragma unroll
+  for (int m = 0; m < 6; m++)
+    if (m < L.nvar) L.U[m * L.F + id] = c.v[m];
+}
+
 // boundary_wall, sub_boundary.f90:306-386
-__device__ void bc_wall(const Lvl &L, const BlkDev &b, const CaseDev &c, const SubDev &s, int i, int j, int k) {
-  const long long F = L.F;
+__device__ __forceinline__ void bc_wall(const Lvl &L, const BlkDev &b, const CaseDev &c, const SubDev &s, int i, int j,
+                                        int k) {
   int i1, j1, i2, j2;
   ghost_pair(s.face, i, j, k, i1, j1, i2, j2);
-  long long a = fidx(b, i1, j1), g = fidx(b, i2, j2);
-  double *U = L.U;
-  double d1 = U[a];
+  const long long a = fidx(b, i1, j1);
+  const double dw = L.nvar == 6 ? L.geo[G_DW * L.F + a] : 0.0;
+  const Cell A = load_cell(L, a);
+  Cell G = A;
   if (c.Twall <= 0) {
-    U[g] = U[a];
-    U[F + g] = -U[F + a];
-    U[2 * F + g] = -U[2 * F + a];
-    U[3 * F + g] = U[3 * F + a];
+    G.v[1] = neg(A.v[1]);
+    G.v[2] = neg(A.v[2]);
   } else {
-    double u1 = U[F + a] / d1, v1 = U[2 * F + a] / d1;
-    double p1 = (U[3 * F + a] - 0.5 * d1 * (u1 * u1 + v1 * v1)) * (c.gamma - 1.0);
-    double T1 = c.gamma * c.Ma * c.Ma * p1 / d1;
-    double p2 = p1, T2 = 2.0 * c.Twall - T1, u2 = -u1, v2 = -v1;
-    double d2 = c.gamma * c.Ma * c.Ma * p2 / T2;
-    U[g] = d2;
-    U[F + g] = d2 * u2;
-    U[2 * F + g] = d2 * v2;
-    U[3 * F + g] = p2 / (c.gamma - 1.0) + 0.5 * d2 * (u2 * u2 + v2 * v2);
+    const double rd = rcp(A.v[0]), u1 = A.v[1] * rd, v1 = A.v[2] * rd, gM = c.gamma * c.Ma * c.Ma;
+    const double p1 = (A.v[3] - half(fma(A.v[1], u1, A.v[2] * v1))) * c.gm1;
+    const double T1 = gM * p1 * rd, T2 = fma(2.0, c.Twall, -T1);
+    const double d2 = gM * p1 * rcp_any(T2);
+    G.v[0] = d2;
+    G.v[1] = d2 * neg(u1);
+    G.v[2] = d2 * neg(v1);
+    G.v[3] = fma(p1, c.rgm1, half(d2) * fma(u1, u1, v1 * v1));
   }
-  if (L.nvar == 5) U[4 * F + g] = 0.0;
+  if (L.nvar == 5) G.v[4] = 0.0;
   if (L.nvar == 6) {
     const double beta1 = 0.075;
-    double d2 = U[g];
-    double r2 = U[F + g], r3 = U[2 * F + g];
-    double T2 = (U[3 * F + g] - 0.5 * (r2 * r2 + r3 * r3) / d2) / (c.Cv * d2);
-    double Amu2 = (1.0 + c.Tsb) * sqrt(T2 * T2 * T2) / (c.Tsb + T2);
-    double dw = L.geo[G_DW * F + a];
-    double wt = 60.0 * Amu2 / (d2 * beta1 * (dw * dw) * c.Re * c.Re);
-    U[4 * F + g] = -U[4 * F + a];
-    U[5 * F + g] = (d1 + d2) * wt - U[5 * F + a];
+    const double d2 = G.v[0], rd = rcp(d2);
+    const double T2 = (G.v[3] - half(fma(G.v[1], G.v[1], G.v[2] * G.v[2])) * rd) * (rd * c.rCv);
+    const double Amu2 = (1.0 + c.Tsb) * (T2 * sqrt_t(T2)) * rcp_any(c.Tsb + T2);
+    const double wt = 60.0 * Amu2 * rcp_any(d2 * beta1 * (dw * dw) * c.Re * c.Re);
+    G.v[4] = neg(A.v[4]);
+    G.v[5] = fma(A.v[0] + d2, wt, -A.v[5]);
   }
+  store_cell(L, fidx(b, i2, j2), G);
 }
 
 // Symmetry_or_slidewall, sub_boundary.f90:391-451.  The reflection
 // U - 2 (U.n) n does not depend on the sign of n, so the far-field edge
 // normal serves.
-__device__ void bc_symmetry(const Lvl &L, const BlkDev &b, const SubDev &s, int i, int j, int k, double2 nrm) {
-  const long long F = L.F;
-  const double n1 = nrm.x, n2 = nrm.y;
+__device__ __forceinline__ void bc_symmetry(const Lvl &L, const BlkDev &b, const SubDev &s, int i, int j, int k,
+                                            double2 nrm) {
   int i1, j1, i2, j2;
   ghost_pair(s.face, i, j, k, i1, j1, i2, j2);
-  long long a = fidx(b, i1, j1), g = fidx(b, i2, j2);
-  double *U = L.U;
-  double Vn = U[F + a] * n1 + U[2 * F + a] * n2;
-  U[g] = U[a];
-  U[F + g] = U[F + a] - 2.0 * Vn * n1;
-  U[2 * F + g] = U[2 * F + a] - 2.0 * Vn * n2;
-  U[3 * F + g] = U[3 * F + a];
-  for (int m = 4; m < L.nvar; m++) U[m * F + g] = U[m * F + a];
+  Cell C = load_cell(L, fidx(b, i1, j1));
+  const double Vn = pow2<1>(fma(C.v[1], nrm.x, C.v[2] * nrm.y));
+  C.v[1] = fma(-Vn, nrm.x, C.v[1]);
+  C.v[2] = fma(-Vn, nrm.y, C.v[2]);
+  store_cell(L, fidx(b, i2, j2), C);
 }
 
 // Outward unit normal of a boundary node's edge, as boundary_Farfield_inlet_outlet
@@ -108,64 +116,64 @@ __device__ __forceinline__ double2 edge_normal(const Lvl &L, const BlkDev &b, in
 // branch.  Every ghost layer takes the same interior state and normal (the
 // reference recomputes the same values per layer), so the ghost state is
 // formed once and written to all LAP layers.
-__device__ void bc_farfield(const Lvl &L, const BlkDev &b, const CaseDev &c, const SubDev &s, int i, int j,
-                            double2 nrm) {
-  const long long F = L.F;
-  double *U = L.U;
-  const double gamma = c.gamma, gm1 = gamma - 1.0;
+__device__ __forceinline__ void bc_farfield(const Lvl &L, const BlkDev &b, const CaseDev &c, const SubDev &s, int i, int j,
+                                            double2 nrm) {
+  const double gamma = c.gamma, gm1 = c.gm1;
   const double n1 = nrm.x, n2 = nrm.y;
   int i1, j1;
   if (s.face == 1 || s.face == 2) { i1 = i; j1 = j; }
   else if (s.face == 3) { i1 = i - 1; j1 = j; }
   else { i1 = i; j1 = j - 1; }
   long long a = fidx(b, i1, j1);
-  const double d1 = U[a], m1 = U[F + a], m2 = U[2 * F + a], E1 = U[3 * F + a];
+  const Cell A = load_cell(L, a);
+  const double d1 = A.v[0], m1 = A.v[1], m2 = A.v[2], E1 = A.v[3];
   const double rd = rcp(d1);
   const double u1 = m1 * rd, v1 = m2 * rd;
-  const double p1 = (E1 - 0.5 * d1 * (u1 * u1 + v1 * v1)) * gm1;
+  const double p1 = (E1 - half(fma(m1, u1, m2 * v1))) * gm1;
   const double c2 = gamma * p1 * rd;
   const double rc = rsqrt_d(c2);  // 1 / c1
   const double c1 = c2 * rc;
   double Ma_n = (u1 * n1 + v1 * n2) * rc;
-  // a few ulps of |u| / c bound the fast value's error
-  const double tol = 1.0e-12 * (fabs(u1) + fabs(v1)) * rc;
-  if (fabs(Ma_n) <= tol || fabs(fabs(Ma_n) - 1.0) <= tol + 1.0e-12) {
+  // a few ulps of |u| / c bound the fast value's error; the test itself is in FP32 with
+  // twice that bound, and 1e-6 about +-1
+  const float Mf = fabsf(to<float>(Ma_n));
+  const float tol = 2.0e-12f * (fabsf(to<float>(u1)) + fabsf(to<float>(v1))) * to<float>(rc);
+  if (!(Mf > tol) || fabsf(Mf - 1.0f) <= 1.0e-6f) {
     const double ux = __ddiv_rn(m1, d1), vx = __ddiv_rn(m2, d1);
     const double ke = __dmul_rn(__dmul_rn(0.5, d1), __dadd_rn(__dmul_rn(ux, ux), __dmul_rn(vx, vx)));
     const double px = __dmul_rn(__dsub_rn(E1, ke), gm1);
     const double cx = __dsqrt_rn(__ddiv_rn(__dmul_rn(gamma, px), d1));
     Ma_n = __ddiv_rn(__dadd_rn(__dmul_rn(ux, n1), __dmul_rn(vx, n2)), cx);
   }
-  double G[6];
+  const bool out = at_least(Ma_n, 0.0) || __double_as_longlong(Ma_n) << 1 == 0;  // Ma_n >= 0
+  Cell C = A;
+  double *G = C.v;
   const int type = s.neighb;
-  if (type == BC_Outlet || (type == BC_Farfield && Ma_n >= 0.0)) {
-    if (Ma_n > 1.0 || c.p_outlet < 0 || type == BC_Farfield) {
-      for (int m = 0; m < L.nvar; m++) G[m] = U[m * F + a];
-    } else {
+  if (type == BC_Outlet || (type == BC_Farfield && out)) {
+    if (!(above(Ma_n, 1.0) || c.p_outlet < 0 || type == BC_Farfield)) {
       const double pb = c.p_outlet;
       const double db = d1 + (c.p_outlet - p1) * (rc * rc);
       const double t = (p1 - c.p_outlet) * (rd * rc);
       const double ub = u1 + t * n1, vb = v1 + t * n2;
       const double p2 = 2.0 * pb - p1, d2 = 2.0 * db - d1, u2 = 2.0 * ub - u1, v2 = 2.0 * vb - v1;
       G[0] = d2; G[1] = d2 * u2; G[2] = d2 * v2;
-      G[3] = p2 * c.rgm1 + 0.5 * d2 * (u2 * u2 + v2 * v2);
-      for (int m = 4; m < L.nvar; m++) G[m] = U[m * F + a];
+      G[3] = fma(p2, c.rgm1, half(d2) * fma(u2, u2, v2 * v2));
     }
   } else {
     const double d_inf = 1.0, u_inf = c.cosA, v_inf = c.sinA, p_inf = c.p00;
-    if (c.p_outlet < 0 || Ma_n <= -1.0) {
+    if (c.p_outlet < 0 || at_least(neg(Ma_n), 1.0)) {
       G[0] = d_inf; G[1] = d_inf * u_inf; G[2] = d_inf * v_inf;
-      G[3] = p_inf / gm1 + 0.5 * d_inf * (u_inf * u_inf + v_inf * v_inf);
+      G[3] = p_inf * c.rgm1 + half(u_inf * u_inf + v_inf * v_inf);
     } else {
-      const double pb = 0.5 * (p1 + p_inf - d1 * c1 * ((u_inf - u1) * n1 + (v_inf - v1) * n2));
-      const double db = d_inf + (pb - p_inf) * (rc * rc);
-      const double t = (p_inf - pb) * (rd * rc);
-      const double ub = u_inf - t * n1, vb = v_inf - t * n2;
-      const double p2 = 2.0 * pb - p1, d2 = 2.0 * db - d1, u2 = 2.0 * ub - u1, v2 = 2.0 * vb - v1;
+      // pb = (p1 + p_inf - X) / 2, so 2 pb - p1 = p_inf - X and pb - p_inf = (p1 - p_inf - X) / 2
+      const double X = (d1 * c1) * fma(u_inf - u1, n1, (v_inf - v1) * n2);
+      const double p2 = p_inf - X, dp = (p1 - p_inf) - X;  // dp: 2 (pb - p_inf)
+      const double d2 = fma(dp, rc * rc, 2.0 * d_inf - d1), t = dp * (rd * rc);
+      const double u2 = fma(t, n1, fma(2.0, u_inf, -u1)), v2 = fma(t, n2, fma(2.0, v_inf, -v1));
       G[0] = d2; G[1] = d2 * u2; G[2] = d2 * v2;
-      G[3] = p2 * c.rgm1 + 0.5 * d2 * (u2 * u2 + v2 * v2);
+      G[3] = fma(p2, c.rgm1, half(d2) * fma(u2, u2, v2 * v2));
     }
-    if (L.nvar == 5) G[4] = c.vt_inf / c.Re;
+    if (L.nvar == 5) G[4] = c.vt_inf * c.rRe;
     else if (L.nvar == 6) { G[4] = d_inf * c.Kt_inf; G[5] = d_inf * c.Wt_inf; }
   }
   for (int k = 1; k <= LAP; k++) {
@@ -174,8 +182,7 @@ __device__ void bc_farfield(const Lvl &L, const BlkDev &b, const CaseDev &c, con
     else if (s.face == 2) { i2 = i; j2 = j - k; }
     else if (s.face == 3) { i2 = i + k - 1; j2 = j; }
     else { i2 = i; j2 = j + k - 1; }
-    const long long g = fidx(b, i2, j2);
-    for (int m = 0; m < L.nvar; m++) U[m * F + g] = G[m];
+    store_cell(L, fidx(b, i2, j2), C);
   }
 }
 
@@ -183,93 +190,103 @@ __device__ void bc_farfield(const Lvl &L, const BlkDev &b, const CaseDev &c, con
 // rho, u, v, T extrapolated from its neighbours i1, i3 across the corner of
 // i2.  One warp per corner; lanes 0..2 form the primitives of i1, i2, i3 side
 // by side (the divisions by rho as reciprocal-multiplies), lane 0 combines.
-__device__ void corner(const Lvl &L, const CaseDev &c, long long i1, long long i2, long long i3, long long i4) {
-  const long long F = L.F;
-  double *U = L.U;
+__device__ __forceinline__ void corner(const Lvl &L, const CaseDev &c, long long i1, long long i2, long long i3,
+                                       long long i4) {
   const int lane = threadIdx.x & 31;
-  const long long src = lane == 0 ? i1 : lane == 1 ? i2 : i3;
-  double d = 0.0, uu = 0.0, v = 0.0, T = 0.0;
-  if (lane < 3) {
-    d = U[src];
-    const double rd = rcp(d);
-    uu = U[F + src] * rd;
-    v = U[2 * F + src] * rd;
-    T = (U[3 * F + src] - (uu * U[F + src] + v * U[2 * F + src]) * 0.5) * (rd * c.rCv);
+  // lanes past the third repeat it
+  const Cell A = load_cell(L, lane == 0 ? i1 : lane == 1 ? i2 : i3);
+  const double d = A.v[0], rd = rcp(d), uu = A.v[1] * rd, v = A.v[2] * rd;
+  const double T = (A.v[3] - half(fma(uu, A.v[1], v * A.v[2]))) * (rd * c.rCv);
+  auto across = [](double x) {
+    const double x2 = __shfl_sync(0xffffffffu, x, 1), x3 = __shfl_sync(0xffffffffu, x, 2);
+    return x + x3 - x2;  // of lane 0
+  };
+  const double d4 = across(d), uu4 = across(uu), v4 = across(v), T4 = across(T);
+  Cell C;
+  C.v[0] = d4;
+  C.v[1] = d4 * uu4;
+  C.v[2] = d4 * v4;
+  C.v[3] = d4 * fma(c.Cv, T4, half(fma(uu4, uu4, v4 * v4)));
+  if (L.nvar > 4) {
+    C.v[4] = across(A.v[4]);
+    C.v[5] = across(A.v[5]);
   }
-  const double d2 = __shfl_sync(0xffffffffu, d, 1), u2 = __shfl_sync(0xffffffffu, uu, 1);
-  const double v2 = __shfl_sync(0xffffffffu, v, 1), T2 = __shfl_sync(0xffffffffu, T, 1);
-  const double d3 = __shfl_sync(0xffffffffu, d, 2), u3 = __shfl_sync(0xffffffffu, uu, 2);
-  const double v3 = __shfl_sync(0xffffffffu, v, 2), T3 = __shfl_sync(0xffffffffu, T, 2);
-  if (lane != 0) return;
-  const double Cv = c.Cv;
-  double d4 = d + d3 - d2, uu4 = uu + u3 - u2, v4 = v + v3 - v2, T4 = T + T3 - T2;
-  U[i4] = d4;
-  U[F + i4] = d4 * uu4;
-  U[2 * F + i4] = d4 * v4;
-  U[3 * F + i4] = d4 * (Cv * T4 + (uu4 * uu4 + v4 * v4) * 0.5);
-  for (int m = 4; m < L.nvar; m++) U[m * F + i4] = U[m * F + i1] + U[m * F + i3] - U[m * F + i2];
+  if (lane == 0) store_cell(L, i4, C);
 }
 
-// phases: 1 physical BCs, 2 halo copy, 4 corners, 8 nu~/k/omega clip
+// phases: 1 physical BCs, 2 halo copy, 4 corners
 constexpr int BC_SMEM_SUBS = 32;  // subfaces of a block staged in shared memory
-// Threads per block's CTA.  A phase costs the longest chain of its threads
-// (a far-field item is some 45 dependent FP64 operations), so a thread that
-// takes a second item doubles the phase: 512 threads give one item per
-// thread to the phases of blocks up to 2 x 256 boundary items (the flat
-// plate's 96-cell blocks have 384 in their single physical phase).
-constexpr int BC_THREADS = 512;
+// A block's boundary is served by a cluster of CTAs whose warps take its items in turn,
+// with a cluster barrier between phases.  On one SM the FP64 instructions of a
+// far-field phase queue up (some 60 per item, one warp instruction per 16 to 19 cycles:
+// twelve warps of a 97 x 97 plate 6 us); on eight SMs a phase costs one item's chain.
+// Measured per call with 512 threads on one SM and as it is: BC_FIGS.  From 152
+// blocks on the blocks fill the chip and a cluster has BC_CTAS_MANY CTAs.
+constexpr int BC_THREADS = 256, BC_CTAS = 8, BC_CTAS_MANY = 2;
 
-__global__ void __launch_bounds__(BC_THREADS, 1) k_bc(Lvl L, int phases) {
-  const int bk = blockIdx.x;
+// every global write of the cluster's threads before is seen by them after
+__device__ __forceinline__ void bc_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(BC_THREADS) k_bc(Lvl L, int phases, int CS) {
+  const int bk = blockIdx.x / CS, rank = blockIdx.x % CS;  // the cluster is blocks bk CS .. bk CS + CS - 1
+  // the cluster's warps in turn over its CTAs; the items of a phase's subfaces go to
+  // them subface by subface, each starting at the warp after the last one's
+  const int lane = threadIdx.x & 31, gw = (threadIdx.x >> 5) * CS + rank, nw = CS * (BC_THREADS / 32), step = nw * 32;
+  auto after = [&](int w, int n) {
+    w -= ((n + 31) >> 5) & (nw - 1);
+    return w < 0 ? w + nw : w;
+  };
   const BlkDev &b = L.blk[bk];
-  const CaseDev &c = L.cs[b.cas];
-  const long long F = L.F;
-  // the block's subface table in shared memory (global beyond 32), read by
-  // the physical and the halo phases
+  // the block's subface table (global beyond 32 entries) and its case in shared memory,
+  // copied in words by all threads: the items of every phase read them
   __shared__ SubDev ssub[BC_SMEM_SUBS];
+  __shared__ CaseDev c;
   const int nsub = b.nsub;
-  if (phases & 3) {
-    for (int ks = threadIdx.x; ks < min(nsub, BC_SMEM_SUBS); ks += blockDim.x) ssub[ks] = L.sub[b.sub0 + ks];
+  {
+    static_assert(sizeof(SubDev) % 8 == 0 && sizeof(CaseDev) % 8 == 0, "copied in words");
+    constexpr int SW = sizeof(SubDev) / 8, CW = sizeof(CaseDev) / 8;
+    const long long *ps = reinterpret_cast<const long long *>(L.sub + b.sub0),
+                    *pc = reinterpret_cast<const long long *>(L.cs + b.cas);
+    long long *ds = reinterpret_cast<long long *>(ssub), *dc = reinterpret_cast<long long *>(&c);
+    for (int t = threadIdx.x; t < CW; t += BC_THREADS) dc[t] = pc[t];
+    for (int t = threadIdx.x; t < min(nsub, BC_SMEM_SUBS) * SW; t += BC_THREADS) ds[t] = ps[t];
     __syncthreads();
   }
   auto sub = [&](int ks) -> const SubDev & { return ks < BC_SMEM_SUBS ? ssub[ks] : L.sub[b.sub0 + ks]; };
   if (phases & 1) {
     // subfaces of one phase touch disjoint cells (grouped at set-up in
-    // subface order): their items are spread over the CTA together
+    // subface order): their items are spread over the cluster together
     for (int ph = 0; ph < b.nphase; ph++) {
-      int total = 0;
+      int w = gw;  // this warp's place after the warps of the subfaces before
       for (int ks = 0; ks < nsub; ks++) {
         const SubDev &s = sub(ks);
-        if (s.neighb < 0 && s.phase == ph) total += s.nitem;
-      }
-      for (int t = threadIdx.x; t < total; t += blockDim.x) {
-        int u = t, ks = 0;
-        for (; ks < nsub; ks++) {
-          const SubDev &s = sub(ks);
-          if (s.neighb >= 0 || s.phase != ph) continue;
-          if (u < s.nitem) break;
-          u -= s.nitem;
-        }
-        const SubDev &s = sub(ks);
-        int ni = s.iend - s.ist + 1;
-        if (s.neighb == BC_Farfield || s.neighb == BC_Inlet || s.neighb == BC_Outlet) {
-          bc_farfield(L, b, c, s, s.ist + u % ni, s.jst + u / ni, L.bcn[s.nrm0 + u]);
-        } else {
-          int k = u % LAP + 1, r = u / LAP;
-          int i = s.ist + r % ni, j = s.jst + r / ni;
-          if (s.neighb == BC_Wall) bc_wall(L, b, c, s, i, j, k);
+        if (s.neighb >= 0 || s.phase != ph) continue;
+        const int ni = s.iend - s.ist + 1, nj = s.jend - s.jst + 1, n = s.nitem;
+        for (int u = w * 32 + lane; u < n; u += step) {
+          const bool ff = s.neighb == BC_Farfield || s.neighb == BC_Inlet || s.neighb == BC_Outlet;
+          const int k = ff ? 1 : u % LAP + 1, r = ff ? u : u / LAP;  // ghost layer, node
+          int i = s.ist, j = s.jst;
+          if (nj == 1) i += r;
+          else if (ni == 1) j += r;
+          else { i += r % ni; j += r / ni; }
+          if (ff) bc_farfield(L, b, c, s, i, j, L.bcn[s.nrm0 + r]);
+          else if (s.neighb == BC_Wall) bc_wall(L, b, c, s, i, j, k);
           else if (s.neighb == BC_Symmetry) bc_symmetry(L, b, s, i, j, k, L.bcn[s.nrm0 + r]);
         }
+        w = after(w, n);
       }
-      __syncthreads();
+      bc_barrier();
     }
   }
   if (phases & 2) {
+    int w = gw;
     for (int ks = 0; ks < nsub; ks++) {
       const SubDev &s = sub(ks);
       if (s.neighb < 0) continue;
       int n1 = s.iend - s.ist + s.jend - s.jst;
-      for (int t = threadIdx.x; t < n1 * LAP; t += blockDim.x) {
+      for (int t = w * 32 + lane; t < n1 * LAP; t += step) {
         int l = t % LAP + 1, k = t / LAP + 1;
         int k1 = (s.orient == 2) ? k : n1 + 1 - k;
         int si, sj;
@@ -283,32 +300,49 @@ __global__ void __launch_bounds__(BC_THREADS, 1) k_bc(Lvl L, int phases) {
         else if (s.face == 3) { di = s.iend + l - 1; dj = s.jst + k - 1; }
         else { di = s.ist + k - 1; dj = s.jend + l - 1; }
         long long src = s.noff + (long long)(sj + 2) * s.nP + (si + 2), dst = fidx(b, di, dj);
-        for (int m = 0; m < L.nvar; m++) L.U[m * F + dst] = L.U[m * F + src];
+        store_cell(L, dst, load_cell(L, src));
       }
+      w = after(w, n1 * LAP);
     }
-    __syncthreads();
+    bc_barrier();
   }
   if (phases & 4) {
     int nx = b.nx, ny = b.ny;
-    const int w = threadIdx.x >> 5;
+    const int w = gw;  // a warp per corner, on different SMs
     if (w == 0) corner(L, c, fidx(b, 1, 0), fidx(b, 1, 1), fidx(b, 0, 1), fidx(b, 0, 0));
     else if (w == 1) corner(L, c, fidx(b, 1, ny), fidx(b, 1, ny - 1), fidx(b, 0, ny - 1), fidx(b, 0, ny));
     else if (w == 2) corner(L, c, fidx(b, nx - 1, 0), fidx(b, nx - 1, 1), fidx(b, nx, 1), fidx(b, nx, 0));
     else if (w == 3) corner(L, c, fidx(b, nx - 1, ny), fidx(b, nx - 1, ny - 1), fidx(b, nx, ny - 1), fidx(b, nx, ny));
-    __syncthreads();
-  }
-  if ((phases & 8) && L.nvar >= 5) {
-    int nc = (b.nx - 1) * (b.ny - 1);
-    for (int t = threadIdx.x; t < nc; t += blockDim.x) {
-      int i = t % (b.nx - 1) + 1, j = t / (b.nx - 1) + 1;
-      long long id = fidx(b, i, j);
-      for (int m = 4; m < L.nvar; m++)
-        if (L.U[m * F + id] < 0) L.U[m * F + id] = 1.0e-10;
-    }
   }
 }
 
-void launch_bc(const Lvl &L, int phases, cudaStream_t s) { k_bc<<<L.nblk, BC_THREADS, 0, s>>>(L, phases); }
+void launch_bc(const Lvl &L, int phases, cudaStream_t s) {
+  const int CS = L.nblk < 152 ? BC_CTAS : BC_CTAS_MANY;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(L.nblk * CS);
+  cfg.blockDim = dim3(BC_THREADS);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = CS; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_bc, L, phases, CS);
+}
+
+// force_vt_kw: negative nu~, k and omega of the interior cells become 1e-10
+__global__ void __launch_bounds__(EC2D_TILE) k_clip(Lvl L) {
+  int bk, i, j;
+  if (!core_ij(L, bk, i, j)) return;
+  const BlkDev &b = L.blk[bk];
+  if (i < 1 || i > b.nx - 1 || j < 1 || j > b.ny - 1) return;
+  const long long id = fidx(b, i, j);
+  for (int m = 4; m < L.nvar; m++)
+    if (L.U[m * L.F + id] < 0) L.U[m * L.F + id] = 1.0e-10;
+}
+void launch_clip(const Lvl &L, cudaStream_t s) {
+  if (L.nvar >= 5) k_clip<<<L.nctiles, EC2D_TILE, 0, s>>>(L);
+}
 
 // set-up: the edge normals of every far-field and symmetry node (grid y: block)
 __global__ void __launch_bounds__(256) k_bc_normals(Lvl L) {
