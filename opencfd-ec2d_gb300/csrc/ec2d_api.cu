@@ -621,6 +621,17 @@ static void apply_mg_amut(ec2d_ctx *ctx) {
   const bool on = ctx->mg_amut && ctx->P.If_viscous == 1 && ctx->P.Iflag_turbulence_model != Turb_NONE;
   for (int l = 2; l <= ctx->num_mesh; l++) ctx->lv[l].L.keep_amut = on ? 1 : 0;
 }
+// a context with FP32 parts keeps the order of operations of the formulas written out
+// (ec2d_mixed.cuh); the viscous metric coefficients of its faces are other ones
+static void apply_mixed(ec2d_ctx *ctx) {
+  const int mixed = ctx->lusgs_fp32 || ctx->coarse_fp32;
+  for (int l = 1; l <= ctx->num_mesh; l++) {
+    Lvl &L = ctx->lv[l].L;
+    if (L.mixed == mixed) continue;
+    L.mixed = mixed;
+    launch_face_metrics(L, ctx->stream);
+  }
+}
 // the stream that issues the next write of level l's Res waits for the norms
 // of its previous evaluation
 void join_norms(ec2d_ctx *ctx, int l) {
@@ -1231,6 +1242,7 @@ int ec2d_setup(ec2d_ctx *ctx) {
   CK(cudaDeviceSynchronize());
   ctx->setup_done = true;
   apply_mg_amut(ctx);
+  apply_mixed(ctx);
   return EC2D_OK;
 }
 
@@ -1696,7 +1708,10 @@ int ec2d_set_coarse_precision(ec2d_ctx *ctx, int bits) {
   bool fp32 = bits == 32;
   if (fp32 != ctx->coarse_fp32) drop_graph(ctx);
   ctx->coarse_fp32 = fp32;
-  return EC2D_OK;
+  if (!ctx->setup_done) return EC2D_OK;
+  cudaSetDevice(ctx->device);
+  apply_mixed(ctx);
+  return check_launch(ctx);
 }
 
 int ec2d_set_lusgs_precision(ec2d_ctx *ctx, int bits) {
@@ -1709,7 +1724,10 @@ int ec2d_set_lusgs_precision(ec2d_ctx *ctx, int bits) {
     ctx->step_graph = nullptr;
   }
   ctx->lusgs_fp32 = fp32;
-  return EC2D_OK;
+  if (!ctx->setup_done) return EC2D_OK;
+  cudaSetDevice(ctx->device);
+  apply_mixed(ctx);
+  return check_launch(ctx);
 }
 
 int ec2d_residual(ec2d_ctx *ctx, int case_id, int mesh, double res_max[6], double res_rms[6], int *kstep,

@@ -108,6 +108,7 @@ struct Lvl {
   unsigned *nctr;           // tiles of k_res done (the last one reduces the partials)
   int *status;              // per case: code, block, i, j
   int silent_band_edge;     // test hook: band edges of the four-lane wavefront send nothing
+  int mixed;                // a context with FP32 parts: arithmetic of ec2d_mixed.cuh
   int keep_amut;            // coarse level: amut is restricted from the finer level, not zeroed
 };
 
@@ -142,13 +143,53 @@ __device__ __forceinline__ bool core_ij(const Lvl &L, int &bk, int &i, int &j) {
   return true;
 }
 
-// FP64 arithmetic on the face, primitive and wavefront paths.  An SM completes
+// Reciprocal on the face and wavefront paths.  FP64: the hardware's
+// approximate reciprocal (relative error e below 2^-19.9, measured over 4e7
+// mantissas) refined by one third-order step of the series
+// 1/x = r / (1 - e) = r (1 + e + e^2 + ...), e = 1 - x r taken exactly by an
+// fma; the neglected e^3 is below 2^-59, so the result is within an ulp of
+// the quotient in four dependent FP64 operations, against nine times that
+// for a divide; a / b becomes a * rcp(b).  FP32: the division.
+template <typename T>
+__device__ __forceinline__ T rcp(T x);
+template <>
+__device__ __forceinline__ double rcp<double>(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+template <>
+__device__ __forceinline__ float rcp<float>(float x) { return 1.0f / x; }
+
+// 1/sqrt(x), x > 0, FP64: the hardware's approximate reciprocal square root
+// (|x y^2 - 1| below 2^-19, measured over 4e7 samples) refined by one
+// third-order step of the series (1 - e)^(-1/2) = 1 + e/2 + 3e^2/8 + ...,
+// e = 1 - x y^2; within an ulp of 1/sqrt(x), and x times it within two ulps
+// of sqrt(x) (measured), in six dependent FP64 operations.
+__device__ __forceinline__ double rsqrt_d(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y * y, 1.0);
+  return fma(y, e * fma(0.375, e, 0.5), y);
+}
+// sqrt(x), x > 0, on the face and primitive paths: FP64 x * rsqrt_d(x)
+// (within two ulps of the rounded root, seven FP64 operations against about
+// ten for the correctly rounded one); FP32 the square root
+template <typename T>
+__device__ __forceinline__ T sqrt_p(T x);
+template <>
+__device__ __forceinline__ double sqrt_p<double>(double x) { return x * rsqrt_d(x); }
+template <>
+__device__ __forceinline__ float sqrt_p<float>(float x) { return sqrtf(x); }
+
+// FP64 arithmetic of the face, primitive and turbulence kernels.  An SM completes
 // one FP64 warp instruction per 16 to 19 cycles, and each holds its sub-partition
 // for 64, while that sub-partition could issue an integer or FP32 instruction
 // every cycle: whatever needs no FP64 pipe is done beside it.
 //   * reciprocals and reciprocal square roots start from 44-bit values formed in
-//     FP32 and integers (rcp_seed, rsqrt_seed) and need one Newton step, two and
-//     three FP64 instructions (a divide takes about nine, the hardware's 20-bit
+//     FP32 and integers (rcp_seed, rsqrt_seed) and need one step, two and three FP64
+//     instructions (a divide takes about nine, the hardware's 20-bit
 //     approximation with a third-order step three and five);
 //   * negation, powers of two and comparisons are integer operations.
 // x 2^K, K in -3..1: exact; zeros, infinities and NaNs stay what they are, and so
@@ -159,14 +200,10 @@ __device__ __forceinline__ double pow2(double x) {
   const unsigned e = (unsigned)h & 0x7ff00000u;
   return __hiloint2double(e - 0x00400000u < 0x7fa00000u ? h + K * 0x00100000 : h, __double2loint(x));
 }
-template <int K>
-__device__ __forceinline__ float pow2(float x) { return x * (K >= 0 ? (float)(1 << (K & 31)) : 1.0f / (float)(1 << (-K & 31))); }
-template <typename T>
-__device__ __forceinline__ T half(T x) { return pow2<-1>(x); }
+__device__ __forceinline__ double half(double x) { return pow2<-1>(x); }
 __device__ __forceinline__ double neg(double x) {
   return __hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x));
 }
-__device__ __forceinline__ float neg(float x) { return -x; }
 // Conversions between double and float, rounded to nearest even: a conversion
 // instruction occupies the FP64 pipe as an FP64 instruction does (64 to 100 cycles), so
 // values within the float's normal range are converted by integer operations.
@@ -194,12 +231,10 @@ __device__ __forceinline__ double to_double(float x) {
 // sign bit clear; x < y, x >= y and x > y for any x and a y of clear sign bit (false
 // for a NaN x)
 __device__ __forceinline__ bool sign_clear(double x) { return __double2hiint(x) >= 0; }
-__device__ __forceinline__ bool sign_clear(float x) { return __float_as_int(x) >= 0; }
 __device__ __forceinline__ bool below(double x, double y) {
   const long long i = __double_as_longlong(x);
   return i < __double_as_longlong(y) && (unsigned long long)i <= 0xfff0000000000000ull;
 }
-__device__ __forceinline__ bool below(float x, float y) { return x < y; }
 __device__ __forceinline__ bool at_least(double x, double y) {
   const long long i = __double_as_longlong(x);
   return i >= __double_as_longlong(y) && i <= 0x7ff0000000000000ll;
@@ -253,101 +288,72 @@ __device__ __forceinline__ double rsqrt_seed(double x) {
   return __hiloint2double(hi - 0x00100000u < 0x7fe00000u ? (int)yh : out, (int)(unsigned)y);
 }
 
-// 1/x: FP64 the rounded quotient in all of 8e8 samples, FP32 the division
-template <typename T>
-__device__ __forceinline__ T rcp(T x);
-template <>
-__device__ __forceinline__ double rcp<double>(double x) {
+// 1/x: the rounded quotient in all of 8e8 samples
+__device__ __forceinline__ double recip(double x) {
   const double r = rcp_seed(x);
   return fma(r, fma(-x, r, 1.0), r);
 }
-template <>
-__device__ __forceinline__ float rcp<float>(float x) { return 1.0f / x; }
-
 // 1/x where x may be zero or infinite: by the divide there
-__device__ __forceinline__ double rcp_any(double x) {
-  return ((unsigned)__double2hiint(x) & 0x7ff00000u) - 0x00100000u < 0x7fc00000u ? rcp(x) : 1.0 / x;
+__device__ __forceinline__ double recip_any(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7ff00000u) - 0x00100000u < 0x7fc00000u ? recip(x) : 1.0 / x;
 }
 // max(x, 0) and min(x, 0) by the sign (a NaN goes to one of them)
 __device__ __forceinline__ double pos_part(double x) { return __double2hiint(x) >= 0 ? x : 0.0; }
 __device__ __forceinline__ double neg_part(double x) { return __double2hiint(x) < 0 ? x : 0.0; }
 
 // 1/sqrt(x), x > 0, to two ulps
-__device__ __forceinline__ double rsqrt_d(double x) {
+__device__ __forceinline__ double rroot(double x) {
   const double y = rsqrt_seed<false>(x), e = fma(-x, y * y, 1.0);
   return fma(half(y), e, y);
 }
-// sqrt(x) on the face and primitive paths: FP64 within an ulp of the rounded
-// root, FP32 the square root
-template <typename T>
-__device__ __forceinline__ T sqrt_p(T x);
-template <>
-__device__ __forceinline__ double sqrt_p<double>(double x) {
-  const double y = rsqrt_seed<true>(x), g = x * y, e = fma(-x, y * y, 1.0);
-  return fma(half(g), e, g);
+// sqrt(x): from g = x y the remainder x - g^2, exact by an fma, gives the root's last bits
+// (the rounded root in all of 8e8 samples)
+__device__ __forceinline__ double root(double x) {
+  const double y = rsqrt_seed<true>(x), g = x * y;
+  return fma(half(y), fma(-g, g, x), g);
 }
-template <>
-__device__ __forceinline__ float sqrt_p<float>(float x) { return sqrtf(x); }
 // the square root function where x is not a positive normal number (T < 0: NaN)
-__device__ __forceinline__ double sqrt_t(double x) {
-  return (unsigned)__double2hiint(x) - 0x00100000u < 0x7fe00000u ? sqrt_p(x) : sqrt(x);
+__device__ __forceinline__ double root_t(double x) {
+  return (unsigned)__double2hiint(x) - 0x00100000u < 0x7fe00000u ? root(x) : sqrt(x);
 }
-// sqrt(a / b) = |a| / sqrt(a b): no reciprocal
-template <typename T>
-__device__ __forceinline__ T sqrt_ratio(T a, T b);
-template <>
-__device__ __forceinline__ double sqrt_ratio<double>(double a, double b) {
-  const double w = a * b, y = rsqrt_seed<true>(w), g = fabs(a) * y, e = fma(-w, y * y, 1.0);
-  return fma(half(g), e, g);
+// sqrt(a / b) = |a| / sqrt(a b): no reciprocal; the same remainder, a - g^2 b; to two ulps
+__device__ __forceinline__ double root_ratio(double a, double b) {
+  const double w = a * b, y = rsqrt_seed<true>(w), g = fabs(a) * y;
+  return fma(half(y), fma(-(g * fabs(b)), g, fabs(a)), g);
 }
-template <>
-__device__ __forceinline__ float sqrt_ratio<float>(float a, float b) { return sqrtf(a / b); }
 
 // the gas constants of a case in the arithmetic of a face
-template <typename T>
 struct Gas {
-  T g, gm1, ggm1, rgm1, rg;  // gamma, gamma - 1, gamma / (gamma - 1), 1 / (gamma - 1), 1 / gamma
+  double g, gm1, ggm1, rgm1, rg;  // gamma, gamma - 1, gamma / (gamma - 1), 1 / (gamma - 1), 1 / gamma
 };
-template <typename T>
-__device__ __forceinline__ Gas<T> gas(const CaseDev &c) {
-  return {to<T>(c.gamma), to<T>(c.gm1), to<T>(c.ggm1), to<T>(c.rgm1), to<T>(c.rg)};
+__device__ __forceinline__ Gas gas(const CaseDev &c) {
+  return {c.gamma, c.gm1, c.ggm1, c.rgm1, c.rg};
 }
 
-// The face physics below is written once for the arithmetic type T: double
-// is the reference's arithmetic (every literal T(x) is then the same double
-// constant), float serves the FP32 coarse multigrid levels.
+// The face physics of FP64 contexts (ec2d_mixed.cuh: of contexts with FP32 parts).
 
 // ---- reconstruction, sub_Residual.f90:477-659 --------------------------------
-template <typename T>
-__device__ __forceinline__ T minmod(T a, T b);
 // zero where a b <= 0, else the one of smaller magnitude, by integer compares
-template <>
-__device__ __forceinline__ double minmod<double>(double a, double b) {
+__device__ __forceinline__ double minmod(double a, double b) {
   const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
   const long long ax = x & 0x7fffffffffffffffll, ay = y & 0x7fffffffffffffffll, inf = 0x7ff0000000000000ll;
   if (ax > inf || ay > inf) return b;  // a NaN: as the comparisons of doubles take it
   if ((x ^ y) < 0 || ax == 0 || ay == 0) return 0.0;
   return ax <= ay ? a : b;
 }
-template <>
-__device__ __forceinline__ float minmod<float>(float a, float b) {
-  if (a * b <= 0.0f) return 0.0f;
-  return (fabsf(a) <= fabsf(b)) ? a : b;
-}
 
 // scheme_fP and scheme_fm (sub_Residual.f90:591-659): the left and right state
 // at the face between u2 and u3.  Both sides in one pass over the three
 // differences; every scheme is u2 (u3) plus a correction, in the same formulas as the
 // reference with one reciprocal in place of its divides.
-template <typename T>
-__device__ __forceinline__ void scheme_pair(T u1, T u2, T u3, T u4, int flag, T &l, T &r) {
-  const T ep = T(1.0e-6), k3 = T(1.0) / T(3.0);
-  const T d1 = u2 - u1, d2 = u3 - u2, d3 = u4 - u3;
+__device__ __forceinline__ void scheme_pair(double u1, double u2, double u3, double u4, int flag, double &l, double &r) {
+  const double ep = 1.0e-6, k3 = 1.0 / 3.0;
+  const double d1 = u2 - u1, d2 = u3 - u2, d3 = u4 - u3;
   switch (flag) {
     case Scheme_UD1: l = u2; r = u3; return;
     case Scheme_UD3:
-      l = (-u1 + T(5.0) * u2 + T(2.0) * u3) * (T(1.0) / T(6.0));
-      r = (T(2.0) * u2 + T(5.0) * u3 - u4) * (T(1.0) / T(6.0));
+      l = (-u1 + 5.0 * u2 + 2.0 * u3) * (1.0 / 6.0);
+      r = (2.0 * u2 + 5.0 * u3 - u4) * (1.0 / 6.0);
       return;
     case Scheme_NND2:
       l = u2 + half(minmod(d1, d2));
@@ -356,50 +362,49 @@ __device__ __forceinline__ void scheme_pair(T u1, T u2, T u3, T u4, int flag, T 
     case Scheme_WENO3: {
       // weights a_1 / (a_1 + a_2), a_2 / (a_1 + a_2) with a_1 = 1 / (3 q_1), a_2 = 2 / (3 q_2)
       // over the common denominator q_2 + 2 q_1, q_k = (ep + d_k^2)^2 >= 1e-12
-      const T e1 = fma(d1, d1, ep), e2 = fma(d2, d2, ep), e3 = fma(d3, d3, ep);
-      const T q1 = pow2<1>(e1 * e1), q2 = e2 * e2, q3 = pow2<1>(e3 * e3);
-      l = fma(half(fma(q1, d2, q2 * d1)), rcp(q1 + q2), u2);
-      r = fma(-(half(fma(q3, d2, q2 * d3))), rcp(q3 + q2), u3);
+      const double e1 = fma(d1, d1, ep), e2 = fma(d2, d2, ep), e3 = fma(d3, d3, ep);
+      const double q1 = pow2<1>(e1 * e1), q2 = e2 * e2, q3 = pow2<1>(e3 * e3);
+      l = fma(half(fma(q1, d2, q2 * d1)), recip(q1 + q2), u2);
+      r = fma(-(half(fma(q3, d2, q2 * d3))), recip(q3 + q2), u3);
       return;
     }
     case Scheme_MUSCL2: {  // left: k = 1, b = 2; right: k = 1/3, b = 1
       l = u2 + half(minmod(d2, pow2<1>(d1)));
-      const T k = T(1.0) / T(3.0), m = minmod(d3, d2);
-      r = u3 - pow2<-2>((T(1.0) - k) * m + (T(1.0) + k) * minmod(d2, d3));
+      const double k = 1.0 / 3.0, m = minmod(d3, d2);
+      r = u3 - pow2<-2>((1.0 - k) * m + (1.0 + k) * minmod(d2, d3));
       return;
     }
     case Scheme_MUSCL3: {
       // s ((1 - k s) um + (1 + k s) up) / 4 = s ((um + up) + k s (up - um)) / 4, van
       // Albada's s = (2 up um + ep) / (up^2 + um^2 + ep); on the right up and um change
       // places
-      const T e2 = fma(d2, d2, ep), t2 = pow2<1>(d2);
-      T s = fma(t2, d1, ep) * rcp(fma(d1, d1, e2));
+      const double e2 = fma(d2, d2, ep), t2 = pow2<1>(d2);
+      double s = fma(t2, d1, ep) * recip(fma(d1, d1, e2));
       l = fma(pow2<-2>(s), fma(k3 * s, d2 - d1, u3 - u1), u2);
-      s = fma(t2, d3, ep) * rcp(fma(d3, d3, e2));
+      s = fma(t2, d3, ep) * recip(fma(d3, d3, e2));
       r = fma(-(pow2<-2>(s)), fma(k3 * s, d2 - d3, u4 - u2), u3);
       return;
     }
     case Scheme_OMUSCL2: {
-      T r1 = (d1 + ep) / (d2 + ep), r2 = (d2 + ep) / (d3 + ep);
-      T f1 = T(0.8) - T(0.175) / r2 + T(0.375) * r1;
-      T f = fmax(T(0.0), fmin(fmin(T(2.0), f1), T(2.0) * r1));
-      l = u2 + T(0.5) * f * d2;
+      double r1 = (d1 + ep) / (d2 + ep), r2 = (d2 + ep) / (d3 + ep);
+      double f1 = 0.8 - 0.175 / r2 + 0.375 * r1;
+      double f = fmax(0.0, fmin(fmin(2.0, f1), 2.0 * r1));
+      l = u2 + 0.5 * f * d2;
       r1 = (d3 + ep) / (d2 + ep);
       r2 = (d2 + ep) / (d1 + ep);
-      f1 = T(0.8) - T(0.175) / r2 + T(0.375) * r1;
-      f = fmax(T(0.0), fmin(fmin(T(2.0), f1), T(2.0) * r1));
-      r = u3 - T(0.5) * f * d2;
+      f1 = 0.8 - 0.175 / r2 + 0.375 * r1;
+      f = fmax(0.0, fmin(fmin(2.0, f1), 2.0 * r1));
+      r = u3 - 0.5 * f * d2;
       return;
     }
   }
-  l = r = T(0.0);
+  l = r = 0.0;
 }
 
 // conservative (rho, rho u, rho v, E) -> primitive (rho, u, v, p), as at the
 // end of Reconstuction_conservative/Characteristic (sub_Residual.f90:526-527)
-template <typename T>
-__device__ __forceinline__ void cons_to_prim(const T Q[4], T W[4], T gm1) {
-  const T r = rcp(Q[0]);
+__device__ __forceinline__ void cons_to_prim(const double Q[4], double W[4], double gm1) {
+  const double r = recip(Q[0]);
   W[0] = Q[0];
   W[1] = Q[1] * r;
   W[2] = Q[2] * r;
@@ -408,14 +413,13 @@ __device__ __forceinline__ void cons_to_prim(const T Q[4], T W[4], T gm1) {
 
 // S0[k][m]: stencil points k = i-2..i+1 (or j-2..j+1), variable m.
 // Reconstuction_original/conservative/Characteristic (sub_Residual.f90:505-586)
-template <typename T>
-__device__ __forceinline__ void reconstruct(int recon, int scheme, T S0[4][4], const Gas<T> &G, T UL[4], T UR[4]) {
+__device__ __forceinline__ void reconstruct(int recon, int scheme, double S0[4][4], const Gas &G, double UL[4], double UR[4]) {
   if (recon == Recon_Original) {
 #pragma unroll
     for (int m = 0; m < 4; m++) scheme_pair(S0[0][m], S0[1][m], S0[2][m], S0[3][m], scheme, UL[m], UR[m]);
     return;
   }
-  T QL[4], QR[4];
+  double QL[4], QR[4];
   if (recon == Recon_Conservative) {
 #pragma unroll
     for (int m = 0; m < 4; m++) scheme_pair(S0[0][m], S0[1][m], S0[2][m], S0[3][m], scheme, QL[m], QR[m]);
@@ -425,38 +429,38 @@ __device__ __forceinline__ void reconstruct(int recon, int scheme, T S0[4][4], c
   }
   // characteristic: project on the left eigenvectors at the arithmetic
   // mid-state, limit each characteristic variable, project back
-  T Uh[4];
+  double Uh[4];
 #pragma unroll
   for (int m = 0; m < 4; m++) Uh[m] = half(S0[1][m] + S0[2][m]);
-  const T rd = rcp(Uh[0]), u1 = Uh[1] * rd, v1 = Uh[2] * rd;
-  const T p1 = (Uh[3] - half(fma(Uh[2], v1, Uh[1] * u1))) * G.gm1;
+  const double rd = recip(Uh[0]), u1 = Uh[1] * rd, v1 = Uh[2] * rd;
+  const double p1 = (Uh[3] - half(fma(Uh[2], v1, Uh[1] * u1))) * G.gm1;
   // sound speed c1 and its inverse from c^2 = gamma p / rho
-  const T c2 = G.g * p1 * rd;
-  const T c1 = sqrt_p(c2), ic = c1 * rcp(c2);
-  const T V2 = half(fma(v1, v1, u1 * u1));
-  const T tmp1 = G.gm1 * ic, tmp3 = tmp1 * ic, tmp5 = half(ic), tmp0 = c2 * G.rgm1;
-  const T a0 = V2 - tmp0, vt = V2 * tmp1, ut = tmp1 * u1, wt = tmp1 * v1;
-  T V0[4][4];
+  const double c2 = G.g * p1 * rd;
+  const double c1 = root(c2), ic = c1 * recip(c2);
+  const double V2 = half(fma(v1, v1, u1 * u1));
+  const double tmp1 = G.gm1 * ic, tmp3 = tmp1 * ic, tmp5 = half(ic), tmp0 = c2 * G.rgm1;
+  const double a0 = V2 - tmp0, vt = V2 * tmp1, ut = tmp1 * u1, wt = tmp1 * v1;
+  double V0[4][4];
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    const T *S = S0[k];
+    const double *S = S0[k];
     V0[k][0] = fma(a0, S[0], fma(-u1, S[1], fma(-v1, S[2], S[3])));
     V0[k][1] = fma(-v1, S[0], S[2]);
     // the two acoustic rows share everything but a sign
-    const T e = fma(vt, S[0], fma(-ut, S[1], fma(-wt, S[2], tmp1 * S[3])));
-    const T o = fma(-u1, S[0], S[1]);
+    const double e = fma(vt, S[0], fma(-ut, S[1], fma(-wt, S[2], tmp1 * S[3])));
+    const double o = fma(-u1, S[0], S[1]);
     V0[k][2] = o - e;
     V0[k][3] = o + e;
   }
-  T VL[4], VR[4];
+  double VL[4], VR[4];
 #pragma unroll
   for (int m = 0; m < 4; m++) scheme_pair(V0[0][m], V0[1][m], V0[2][m], V0[3][m], scheme, VL[m], VR[m]);
 #pragma unroll
   for (int side = 0; side < 2; side++) {
-    const T *V = side ? VR : VL;
-    T *Q = side ? QR : QL;
+    const double *V = side ? VR : VL;
+    double *Q = side ? QR : QL;
     // back: with e = -tmp3 V0 (entropy), s = V2 + V3, d = (V3 - V2) tmp5
-    const T e = -(tmp3 * V[0]), sum = V[2] + V[3], dif = (V[3] - V[2]) * tmp5, r0 = e + dif;
+    const double e = -(tmp3 * V[0]), sum = V[2] + V[3], dif = (V[3] - V[2]) * tmp5, r0 = e + dif;
     Q[0] = r0;
     Q[1] = fma(u1, r0, half(sum));
     Q[2] = fma(v1, r0, V[1]);
@@ -472,35 +476,33 @@ __device__ __forceinline__ void reconstruct(int recon, int scheme, T S0[4][4], c
 // turns the states into the face's frame and the flux back, which multiplies
 // out to the same sums (16 FP64 instructions less).
 // Flux_Roe_1D, sub_flux_split.f90:265-324 (Harten entropy fix, delta = 0.1)
-template <typename T>
-__device__ __forceinline__ T harten(T l) {
-  const T delt = T(0.1), i2d = T(1.0) / (T(2.0) * delt);
+__device__ __forceinline__ double harten(double l) {
+  const double delt = 0.1, i2d = 1.0 / (2.0 * delt);
   if (below(l, delt)) l = fma(l, l, delt * delt) * i2d;
   return l;
 }
-template <typename T>
-__device__ __forceinline__ void flux_roe(const T *L, const T *R, T n1, T n2, T s, T *F, const Gas<T> &G) {
-  const T dl = L[0], ul = L[1], vl = L[2], pl = L[3], dr = R[0], ur = R[1], vr = R[2], pr = R[3];
-  const T unl = fma(vl, n2, ul * n1), unr = fma(vr, n2, ur * n1);
-  const T hl = fma(G.ggm1 * pl, rcp(dl), half(fma(vl, vl, ul * ul)));
-  const T hr = fma(G.ggm1 * pr, rcp(dr), half(fma(vr, vr, ur * ur)));
+__device__ __forceinline__ void flux_roe(const double *L, const double *R, double n1, double n2, double s, double *F, const Gas &G) {
+  const double dl = L[0], ul = L[1], vl = L[2], pl = L[3], dr = R[0], ur = R[1], vr = R[2], pr = R[3];
+  const double unl = fma(vl, n2, ul * n1), unr = fma(vr, n2, ur * n1);
+  const double hl = fma(G.ggm1 * pl, recip(dl), half(fma(vl, vl, ul * ul)));
+  const double hr = fma(G.ggm1 * pr, recip(dr), half(fma(vr, vr, ur * ur)));
   // Roe averages: t = sqrt(rho_r / rho_l)
-  const T t = sqrt_ratio(dr, dl), t1 = t + T(1.0), inv = rcp(t1);
-  const T ad = pow2<-2>(dl * (t1 * t1));
-  const T au = fma(t, ur, ul) * inv, av = fma(t, vr, vl) * inv, ah = fma(t, hr, hl) * inv;
-  const T an = fma(av, n2, au * n1), at = fma(av, n1, -(au * n2));  // normal and tangential
-  const T k2 = half(fma(av, av, au * au));
-  const T c2 = G.gm1 * (ah - k2);
-  const T c = sqrt_p(c2), ic2 = rcp(c2), ic = c * ic2;
-  const T l0 = harten(fabs(an - c)), l1 = harten(fabs(an)), l3 = harten(fabs(an + c));
-  const T dp = pr - pl, du = ur - ul, dv = vr - vl;
-  const T x = (ad * c) * (unr - unl), i2 = half(ic2);
-  const T w0 = l0 * ((dp - x) * i2), w3 = l3 * ((dp + x) * i2), w1 = l1 * fma(-dp, ic2, dr - dl);
-  const T w2 = l1 * (ad * fma(dv, n1, -(du * n2)) * ic);
+  const double t = root_ratio(dr, dl), t1 = t + 1.0, inv = recip(t1);
+  const double ad = pow2<-2>(dl * (t1 * t1));
+  const double au = fma(t, ur, ul) * inv, av = fma(t, vr, vl) * inv, ah = fma(t, hr, hl) * inv;
+  const double an = fma(av, n2, au * n1), at = fma(av, n1, -(au * n2));  // normal and tangential
+  const double k2 = half(fma(av, av, au * au));
+  const double c2 = G.gm1 * (ah - k2);
+  const double c = root(c2), ic2 = recip(c2), ic = c * ic2;
+  const double l0 = harten(fabs(an - c)), l1 = harten(fabs(an)), l3 = harten(fabs(an + c));
+  const double dp = pr - pl, du = ur - ul, dv = vr - vl;
+  const double x = (ad * c) * (unr - unl), i2 = half(ic2);
+  const double w0 = l0 * ((dp - x) * i2), w3 = l3 * ((dp + x) * i2), w1 = l1 * fma(-dp, ic2, dr - dl);
+  const double w2 = l1 * (ad * fma(dv, n1, -(du * n2)) * ic);
   // with S = w0 + w1 + w3 and q = (w3 - w0) c the dissipation is (S, S u + q n1 - w2 n2,
   // S v + q n2 + w2 n1, (w0 + w3) h + q u_n + w1 |u|^2 / 2 + w2 u_t)
-  const T w03 = w0 + w3, S = w03 + w1, q = (w3 - w0) * c;
-  const T ml = dl * unl, mr = dr * unr, pp = (pl + pr) - q, hs = neg(half(s));
+  const double w03 = w0 + w3, S = w03 + w1, q = (w3 - w0) * c;
+  const double ml = dl * unl, mr = dr * unr, pp = (pl + pr) - q, hs = neg(half(s));
   F[0] = ((ml + mr) - S) * hs;
   F[1] = fma(ml, ul, fma(mr, ur, fma(-S, au, fma(pp, n1, w2 * n2)))) * hs;
   F[2] = fma(ml, vl, fma(mr, vr, fma(-S, av, fma(pp, n2, -(w2 * n1))))) * hs;
@@ -510,40 +512,33 @@ __device__ __forceinline__ void flux_roe(const T *L, const T *R, T n1, T n2, T s
 // Flux_Ausm_1Da (AUSM+), sub_flux_split.f90:195-261.  Its sums 0.5 xm (f_l + f_r) -
 // 0.5 dm (f_r - f_l) with dm = a |M| rho of the upwind side are xm times f of the
 // upwind side, so only that side's enthalpy is formed.
-template <typename T>
-__device__ __forceinline__ bool supersonic(T m);
-template <>
-__device__ __forceinline__ bool supersonic<double>(double m) {  // 1 <= |m| < infinity
+__device__ __forceinline__ bool supersonic(double m) {  // 1 <= |m| < infinity
   return ((unsigned)__double2hiint(m) & 0x7fffffffu) - 0x3ff00000u < 0x40000000u;
 }
-template <>
-__device__ __forceinline__ bool supersonic<float>(float m) { return fabsf(m) >= 1.0f; }
 // split Mach number and pressure of the left state; the right state's are -m4(-M)
 // and p5(-M)
-template <typename T>
-__device__ __forceinline__ void ausm_split(T m, T &m4, T &p5) {
+__device__ __forceinline__ void ausm_split(double m, double &m4, double &p5) {
   if (supersonic(m)) {
-    m4 = sign_clear(m) ? m : T(0.0);
-    p5 = sign_clear(m) ? T(1.0) : T(0.0);
+    m4 = sign_clear(m) ? m : 0.0;
+    p5 = sign_clear(m) ? 1.0 : 0.0;
     return;
   }
-  const T a = m + T(1.0), q = pow2<-2>(a * a), r = fma(m, m, T(-1.0)), w = r * r;
-  m4 = fma(T(0.125), w, q);
-  p5 = fma(T(0.1875) * m, w, q * (T(2.0) - m));
+  const double a = m + 1.0, q = pow2<-2>(a * a), r = fma(m, m, -1.0), w = r * r;
+  m4 = fma(0.125, w, q);
+  p5 = fma(0.1875 * m, w, q * (2.0 - m));
 }
-template <typename T>
-__device__ __forceinline__ void flux_ausm(const T *L, const T *R, T n1, T n2, T s, T *F, const Gas<T> &G) {
-  const T unl = fma(L[2], n2, L[1] * n1), unr = fma(R[2], n2, R[1] * n1);
-  const T al = sqrt_ratio(G.g * L[3], L[0]), ar = sqrt_ratio(G.g * R[3], R[0]);
-  const T a = half(al + ar), ia = rcp(a);
-  T m4, p5, n4, q5;
+__device__ __forceinline__ void flux_ausm(const double *L, const double *R, double n1, double n2, double s, double *F, const Gas &G) {
+  const double unl = fma(L[2], n2, L[1] * n1), unr = fma(R[2], n2, R[1] * n1);
+  const double al = root_ratio(G.g * L[3], L[0]), ar = root_ratio(G.g * R[3], R[0]);
+  const double a = half(al + ar), ia = recip(a);
+  double m4, p5, n4, q5;
   ausm_split(unl * ia, m4, p5);
   ausm_split(-(unr * ia), n4, q5);
-  const T M = m4 - n4;
+  const double M = m4 - n4;
   const bool left = sign_clear(M);
-  const T d = left ? L[0] : R[0], u = left ? L[1] : R[1], v = left ? L[2] : R[2], c = left ? al : ar;
-  const T ns = neg(s), xm = (a * M) * (d * ns), p = fma(L[3], p5, R[3] * q5) * ns;
-  const T h = fma(c * c, G.rgm1, half(fma(v, v, u * u)));
+  const double d = left ? L[0] : R[0], u = left ? L[1] : R[1], v = left ? L[2] : R[2], c = left ? al : ar;
+  const double ns = neg(s), xm = (a * M) * (d * ns), p = fma(L[3], p5, R[3] * q5) * ns;
+  const double h = fma(c * c, G.rgm1, half(fma(v, v, u * u)));
   F[0] = xm;
   F[1] = fma(xm, u, p * n1);
   F[2] = fma(xm, v, p * n2);
@@ -552,99 +547,96 @@ __device__ __forceinline__ void flux_ausm(const T *L, const T *R, T n1, T n2, T 
 
 // The other fluxes in the face's frame: rotated primitive states (rho, u_n, u_t, p).
 // Flux_Van_Leer_1Da, sub_flux_split.f90:139-189
-template <typename T>
-__device__ __forceinline__ void flux_vanleer(const T *QL, const T *QR, T *F, const Gas<T> &G) {
-  T dl = QL[0], uul = QL[1], vvl = QL[2], pl = QL[3];
-  T dr = QR[0], uur = QR[1], vvr = QR[2], pr = QR[3];
-  const T gamma = G.g, gm1 = G.gm1, rg = G.rg, rgg = rcp(gamma * gamma - T(1.0));
-  T al = sqrt_ratio(gamma * pl, dl), ar = sqrt_ratio(gamma * pr, dr);
-  T fp0 = 0, fp1 = 0, fp2 = 0, fp3 = 0, fm0 = 0, fm1 = 0, fm2 = 0, fm3 = 0;
+__device__ __forceinline__ void flux_vanleer(const double *QL, const double *QR, double *F, const Gas &G) {
+  double dl = QL[0], uul = QL[1], vvl = QL[2], pl = QL[3];
+  double dr = QR[0], uur = QR[1], vvr = QR[2], pr = QR[3];
+  const double gamma = G.g, gm1 = G.gm1, rg = G.rg, rgg = recip(gamma * gamma - 1.0);
+  double al = root_ratio(gamma * pl, dl), ar = root_ratio(gamma * pr, dr);
+  double fp0 = 0, fp1 = 0, fp2 = 0, fp3 = 0, fm0 = 0, fm1 = 0, fm2 = 0, fm3 = 0;
   if (uul >= al) {
     fp0 = dl * uul; fp1 = dl * uul * uul + pl; fp2 = dl * uul * vvl;
-    fp3 = uul * (G.ggm1 * pl + T(0.5) * dl * (uul * uul + vvl * vvl));
+    fp3 = uul * (G.ggm1 * pl + 0.5 * dl * (uul * uul + vvl * vvl));
   } else if (fabs(uul) < al) {
-    const T Ml = uul * rcp(al);
-    T tmp0 = dl * al * (T(0.25) * (T(1.0) + Ml) * (T(1.0) + Ml));
-    T w = gm1 * uul + T(2.0) * al;
+    const double Ml = uul * recip(al);
+    double tmp0 = dl * al * (0.25 * (1.0 + Ml) * (1.0 + Ml));
+    double w = gm1 * uul + 2.0 * al;
     fp0 = tmp0; fp1 = tmp0 * w * rg; fp2 = tmp0 * vvl;
-    fp3 = tmp0 * T(0.5) * (w * w * rgg + vvl * vvl);
+    fp3 = tmp0 * 0.5 * (w * w * rgg + vvl * vvl);
   }
   if (uur >= ar) {
   } else if (fabs(uur) < ar) {
-    const T Mr = uur * rcp(ar);
-    T tmp0 = dr * ar * (-T(0.25) * (Mr - T(1.0)) * (Mr - T(1.0)));
-    T w = gm1 * uur - T(2.0) * ar;
+    const double Mr = uur * recip(ar);
+    double tmp0 = dr * ar * (-0.25 * (Mr - 1.0) * (Mr - 1.0));
+    double w = gm1 * uur - 2.0 * ar;
     fm0 = tmp0; fm1 = tmp0 * w * rg; fm2 = tmp0 * vvr;
-    fm3 = tmp0 * T(0.5) * (w * w * rgg + vvr * vvr);
+    fm3 = tmp0 * 0.5 * (w * w * rgg + vvr * vvr);
   } else if (uur <= -ar) {
     fm0 = dr * uur; fm1 = dr * uur * uur + pr; fm2 = dr * uur * vvr;
-    fm3 = uur * (G.ggm1 * pr + T(0.5) * dr * (uur * uur + vvr * vvr));
+    fm3 = uur * (G.ggm1 * pr + 0.5 * dr * (uur * uur + vvr * vvr));
   }
   F[0] = fp0 + fm0; F[1] = fp1 + fm1; F[2] = fp2 + fm2; F[3] = fp3 + fm3;
 }
 
 // Flux_steger_warming_1Da, sub_flux_split.f90:99-136
-template <typename T>
-__device__ __forceinline__ void flux_sw(const T *QL, const T *QR, T *F, const Gas<T> &G) {
-  T dl = QL[0], uul = QL[1], vvl = QL[2], pl = QL[3];
-  T dr = QR[0], uur = QR[1], vvr = QR[2], pr = QR[3];
-  const T gamma = G.g, gm1 = G.gm1;
-  T al = sqrt_ratio(gamma * pl, dl), ar = sqrt_ratio(gamma * pr, dr);
-  T tmp1 = T(2.0) * gm1, tmp3 = T(0.5) * (T(3.0) - gamma) * G.rgm1;
-  T E1P = (uul + fabs(uul)) * T(0.5), E2P = (uul - al + fabs(uul - al)) * T(0.5), E3P = (uul + al + fabs(uul + al)) * T(0.5);
-  T t0 = dl * T(0.5) * G.rg;
-  T p0 = t0 * (tmp1 * E1P + E2P + E3P);
-  T p1 = t0 * (tmp1 * E1P * uul + E2P * (uul - al) + E3P * (uul + al));
-  T p2 = t0 * (tmp1 * E1P * vvl + E2P * vvl + E3P * vvl);
-  T p3 = t0 * (E1P * gm1 * (uul * uul + vvl * vvl) + E2P * ((uul - al) * (uul - al) + vvl * vvl) * T(0.5) +
-                    E3P * ((uul + al) * (uul + al) + vvl * vvl) * T(0.5) + tmp3 * al * al * (E2P + E3P));
-  T E1M = (uur - fabs(uur)) * T(0.5), E2M = (uur - ar - fabs(uur - ar)) * T(0.5), E3M = (uur + ar - fabs(uur + ar)) * T(0.5);
-  t0 = dr * T(0.5) * G.rg;
-  T m0 = t0 * (tmp1 * E1M + E2M + E3M);
-  T m1 = t0 * (tmp1 * E1M * uur + E2M * (uur - ar) + E3M * (uur + ar));
-  T m2 = t0 * (tmp1 * E1M * vvr + E2M * vvr + E3M * vvr);
-  T m3 = t0 * (E1M * gm1 * (uur * uur + vvr * vvr) + E2M * ((uur - ar) * (uur - ar) + vvr * vvr) * T(0.5) +
-                    E3M * ((uur + ar) * (uur + ar) + vvr * vvr) * T(0.5) + tmp3 * ar * ar * (E2M + E3M));
+__device__ __forceinline__ void flux_sw(const double *QL, const double *QR, double *F, const Gas &G) {
+  double dl = QL[0], uul = QL[1], vvl = QL[2], pl = QL[3];
+  double dr = QR[0], uur = QR[1], vvr = QR[2], pr = QR[3];
+  const double gamma = G.g, gm1 = G.gm1;
+  double al = root_ratio(gamma * pl, dl), ar = root_ratio(gamma * pr, dr);
+  double tmp1 = 2.0 * gm1, tmp3 = 0.5 * (3.0 - gamma) * G.rgm1;
+  double E1P = (uul + fabs(uul)) * 0.5, E2P = (uul - al + fabs(uul - al)) * 0.5, E3P = (uul + al + fabs(uul + al)) * 0.5;
+  double t0 = dl * 0.5 * G.rg;
+  double p0 = t0 * (tmp1 * E1P + E2P + E3P);
+  double p1 = t0 * (tmp1 * E1P * uul + E2P * (uul - al) + E3P * (uul + al));
+  double p2 = t0 * (tmp1 * E1P * vvl + E2P * vvl + E3P * vvl);
+  double p3 = t0 * (E1P * gm1 * (uul * uul + vvl * vvl) + E2P * ((uul - al) * (uul - al) + vvl * vvl) * 0.5 +
+                    E3P * ((uul + al) * (uul + al) + vvl * vvl) * 0.5 + tmp3 * al * al * (E2P + E3P));
+  double E1M = (uur - fabs(uur)) * 0.5, E2M = (uur - ar - fabs(uur - ar)) * 0.5, E3M = (uur + ar - fabs(uur + ar)) * 0.5;
+  t0 = dr * 0.5 * G.rg;
+  double m0 = t0 * (tmp1 * E1M + E2M + E3M);
+  double m1 = t0 * (tmp1 * E1M * uur + E2M * (uur - ar) + E3M * (uur + ar));
+  double m2 = t0 * (tmp1 * E1M * vvr + E2M * vvr + E3M * vvr);
+  double m3 = t0 * (E1M * gm1 * (uur * uur + vvr * vvr) + E2M * ((uur - ar) * (uur - ar) + vvr * vvr) * 0.5 +
+                    E3M * ((uur + ar) * (uur + ar) + vvr * vvr) * 0.5 + tmp3 * ar * ar * (E2M + E3M));
   F[0] = p0 + m0; F[1] = p1 + m1; F[2] = p2 + m2; F[3] = p3 + m3;
 }
 
 // Flux_HLL_HLLC_1D, sub_flux_split.f90:16-93
-template <typename T>
-__device__ __forceinline__ void flux_hll(const T *QL, const T *QR, T *F, const Gas<T> &G, bool hllc) {
-  T dl = QL[0], uul = QL[1], vvl = QL[2], pl = QL[3];
-  T dr = QR[0], uur = QR[1], vvr = QR[2], pr = QR[3];
-  T UL[4] = {dl, dl * uul, dl * vvl, pl * G.rgm1 + dl * half(uul * uul + vvl * vvl)};
-  T UR[4] = {dr, dr * uur, dr * vvr, pr * G.rgm1 + dr * half(uur * uur + vvr * vvr)};
-  T al = sqrt_ratio(G.g * pl, dl), ar = sqrt_ratio(G.g * pr, dr);
-  T p_pvrs = half(pl + pr) - (uur - uul) * (dl + dr) * pow2<-3>(al + ar);
-  T p_star = fmax(T(0.0), p_pvrs);
-  const T g2 = half((G.g + T(1.0)) * G.rg);
-  T qql = (p_star <= pl) ? T(1.0) : sqrt_p(fma(g2, p_star * rcp(pl) - T(1.0), T(1.0)));
-  T qqr = (p_star <= pr) ? T(1.0) : sqrt_p(fma(g2, p_star * rcp(pr) - T(1.0), T(1.0)));
-  T Sl = uul - al * qql, Sr = uur + ar * qqr;
-  T Fl[4] = {UL[1], UL[1] * uul + pl, UL[2] * uul, uul * (UL[3] + pl)};
-  T Fr[4] = {UR[1], UR[1] * uur + pr, UR[2] * uur, uur * (UR[3] + pr)};
+__device__ __forceinline__ void flux_hll(const double *QL, const double *QR, double *F, const Gas &G, bool hllc) {
+  double dl = QL[0], uul = QL[1], vvl = QL[2], pl = QL[3];
+  double dr = QR[0], uur = QR[1], vvr = QR[2], pr = QR[3];
+  double UL[4] = {dl, dl * uul, dl * vvl, pl * G.rgm1 + dl * half(uul * uul + vvl * vvl)};
+  double UR[4] = {dr, dr * uur, dr * vvr, pr * G.rgm1 + dr * half(uur * uur + vvr * vvr)};
+  double al = root_ratio(G.g * pl, dl), ar = root_ratio(G.g * pr, dr);
+  double p_pvrs = half(pl + pr) - (uur - uul) * (dl + dr) * pow2<-3>(al + ar);
+  double p_star = fmax(0.0, p_pvrs);
+  const double g2 = half((G.g + 1.0) * G.rg);
+  double qql = (p_star <= pl) ? 1.0 : root(fma(g2, p_star * recip(pl) - 1.0, 1.0));
+  double qqr = (p_star <= pr) ? 1.0 : root(fma(g2, p_star * recip(pr) - 1.0, 1.0));
+  double Sl = uul - al * qql, Sr = uur + ar * qqr;
+  double Fl[4] = {UL[1], UL[1] * uul + pl, UL[2] * uul, uul * (UL[3] + pl)};
+  double Fr[4] = {UR[1], UR[1] * uur + pr, UR[2] * uur, uur * (UR[3] + pr)};
   if (!hllc) {
     if (Sl >= 0) { for (int m = 0; m < 4; m++) F[m] = Fl[m]; }
     else if (Sr <= 0) { for (int m = 0; m < 4; m++) F[m] = Fr[m]; }
-    else { T inv = rcp(Sr - Sl);
+    else { double inv = recip(Sr - Sl);
       for (int m = 0; m < 4; m++) F[m] = (Sr * Fl[m] - Sl * Fr[m] + Sl * Sr * (UR[m] - UL[m])) * inv; }
     return;
   }
-  const T bl = dl * (Sl - uul), br = dr * (Sr - uur);
-  T S_star = (pr - pl + bl * uul - br * uur) * rcp(bl - br);
+  const double bl = dl * (Sl - uul), br = dr * (Sr - uur);
+  double S_star = (pr - pl + bl * uul - br * uur) * recip(bl - br);
   if (Sl >= 0) { for (int m = 0; m < 4; m++) F[m] = Fl[m]; return; }
   if (Sr <= 0) { for (int m = 0; m < 4; m++) F[m] = Fr[m]; return; }
   // the star state of the side the face lies in
   const bool left = S_star >= 0;
-  T U[4], Fs[4];
+  double U[4], Fs[4];
 #pragma unroll
   for (int m = 0; m < 4; m++) { U[m] = left ? UL[m] : UR[m]; Fs[m] = left ? Fl[m] : Fr[m]; }
-  const T u = left ? uul : uur, v = left ? vvl : vvr, p = left ? pl : pr, b = left ? bl : br, S = left ? Sl : Sr;
+  const double u = left ? uul : uur, v = left ? vvl : vvr, p = left ? pl : pr, b = left ? bl : br, S = left ? Sl : Sr;
   // E / rho + (S* - u) (S* + p / b) over one reciprocal of rho b
-  const T d = U[0], rdb = rcp(d * b);
-  const T ts = b * rcp(S - S_star);
-  const T e = U[3] * (b * rdb) + (S_star - u) * (S_star + p * (d * rdb));
+  const double d = U[0], rdb = recip(d * b);
+  const double ts = b * recip(S - S_star);
+  const double e = U[3] * (b * rdb) + (S_star - u) * (S_star + p * (d * rdb));
   F[0] = Fs[0] + S * (ts - d);
   F[1] = Fs[1] + S * (ts * S_star - U[1]);
   F[2] = Fs[2] + S * (ts * v - U[2]);
@@ -652,20 +644,19 @@ __device__ __forceinline__ void flux_hll(const T *QL, const T *QR, T *F, const G
 }
 
 // F = -s (flux through the face with unit normal n and length s)
-template <typename T>
-__device__ __forceinline__ void face_flux(int iflux, const T *L, const T *R, T n1, T n2, T s, T *F, const Gas<T> &G) {
+__device__ __forceinline__ void face_flux(int iflux, const double *L, const double *R, double n1, double n2, double s, double *F, const Gas &G) {
   if (iflux == Flux_Roe) { flux_roe(L, R, n1, n2, s, F, G); return; }
   if (iflux == Flux_Ausm) { flux_ausm(L, R, n1, n2, s, F, G); return; }
-  const T QL[4] = {L[0], L[1] * n1 + L[2] * n2, -L[1] * n2 + L[2] * n1, L[3]};
-  const T QR[4] = {R[0], R[1] * n1 + R[2] * n2, -R[1] * n2 + R[2] * n1, R[3]};
-  T f[4] = {T(0.0), T(0.0), T(0.0), T(0.0)};
+  const double QL[4] = {L[0], L[1] * n1 + L[2] * n2, -L[1] * n2 + L[2] * n1, L[3]};
+  const double QR[4] = {R[0], R[1] * n1 + R[2] * n2, -R[1] * n2 + R[2] * n1, R[3]};
+  double f[4] = {0.0, 0.0, 0.0, 0.0};
   switch (iflux) {
     case Flux_VanLeer: flux_vanleer(QL, QR, f, G); break;
     case Flux_SW: flux_sw(QL, QR, f, G); break;
     case Flux_HLL: flux_hll(QL, QR, f, G, false); break;
     case Flux_HLLC: flux_hll(QL, QR, f, G, true); break;
   }
-  const T ns = neg(s);
+  const double ns = neg(s);
   F[0] = f[0] * ns;
   F[1] = (f[1] * n1 - f[2] * n2) * ns;
   F[2] = (f[1] * n2 + f[2] * n1) * ns;
@@ -674,18 +665,17 @@ __device__ __forceinline__ void face_flux(int iflux, const T *L, const T *R, T n
 
 // viscous stress and heat flux through a face from the face-local 2x2
 // Jacobian of cell centres, sub_Residual.f90:313-343 / 419-450
-template <typename T>
-__device__ __forceinline__ void viscous_face(T Dix, T Diy, T Djx, T Djy, T Diu, T Div,
-                                             T DiT, T Dju, T Djv, T DjT, T Amu1, T Amk1,
-                                             T u1, T v1, T n1, T n2, T s, T &F2,
-                                             T &F3, T &F4) {
-  T Ds = rcp(Dix * Djy - Djx * Diy);
-  T ux = (Diu * Djy - Dju * Diy) * Ds, vx = (Div * Djy - Djv * Diy) * Ds, Tx = (DiT * Djy - DjT * Diy) * Ds;
-  T uy = (-Diu * Djx + Dju * Dix) * Ds, vy = (-Div * Djx + Djv * Dix) * Ds, Ty = (-DiT * Djx + DjT * Dix) * Ds;
-  T t11 = ((T(4.0) / T(3.0)) * ux - (T(2.0) / T(3.0)) * vy) * Amu1;
-  T t22 = ((T(4.0) / T(3.0)) * vy - (T(2.0) / T(3.0)) * ux) * Amu1;
-  T t12 = (uy + vx) * Amu1;
-  T E1 = u1 * t11 + v1 * t12 + Amk1 * Tx, E2 = u1 * t12 + v1 * t22 + Amk1 * Ty;
+__device__ __forceinline__ void viscous_face(double Dix, double Diy, double Djx, double Djy, double Diu, double Div,
+                                             double DiT, double Dju, double Djv, double DjT, double Amu1, double Amk1,
+                                             double u1, double v1, double n1, double n2, double s, double &F2,
+                                             double &F3, double &F4) {
+  double Ds = rcp(Dix * Djy - Djx * Diy);
+  double ux = (Diu * Djy - Dju * Diy) * Ds, vx = (Div * Djy - Djv * Diy) * Ds, Tx = (DiT * Djy - DjT * Diy) * Ds;
+  double uy = (-Diu * Djx + Dju * Dix) * Ds, vy = (-Div * Djx + Djv * Dix) * Ds, Ty = (-DiT * Djx + DjT * Dix) * Ds;
+  double t11 = ((4.0 / 3.0) * ux - (2.0 / 3.0) * vy) * Amu1;
+  double t22 = ((4.0 / 3.0) * vy - (2.0 / 3.0) * ux) * Amu1;
+  double t12 = (uy + vx) * Amu1;
+  double E1 = u1 * t11 + v1 * t12 + Amk1 * Tx, E2 = u1 * t12 + v1 * t22 + Amk1 * Ty;
   F2 += (t11 * n1 + t12 * n2) * s;
   F3 += (t12 * n1 + t22 * n2) * s;
   F4 += (E1 * n1 + E2 * n2) * s;
@@ -701,13 +691,12 @@ __device__ __forceinline__ void viscous_face(T Dix, T Diy, T Djx, T Djy, T Diu, 
 // the same sums as (t11 n1 + t12 n2, t12 n1 + t22 n2), and the work and heat
 // u F_x + v F_y + k d_n T.  us, vs: the sums of the velocities of both sides; mu
 // and k already hold the face length.
-template <typename T>
-__device__ __forceinline__ void viscous_face_m(T P, T Q, T R, T S, T Diu, T Div, T DiT, T Dju, T Djv, T DjT, T mu, T k,
-                                               T us, T vs, T n1, T n2, T &F2, T &F3, T &F4) {
-  const T nu = fma(Diu, P, Dju * Q), nv = fma(Div, P, Djv * Q);
-  const T tu = fma(Dju, S, -(Diu * R)), tv = fma(Djv, S, -(Div * R));
-  const T d3 = fma(n1, nu + tv, n2 * (nv - tu)) * (T(1.0) / T(3.0));
-  const T fx = fma(n1, d3, nu - tv), fy = fma(n2, d3, nv + tu);
+__device__ __forceinline__ void viscous_face_m(double P, double Q, double R, double S, double Diu, double Div, double DiT, double Dju, double Djv, double DjT, double mu, double k,
+                                               double us, double vs, double n1, double n2, double &F2, double &F3, double &F4) {
+  const double nu = fma(Diu, P, Dju * Q), nv = fma(Div, P, Djv * Q);
+  const double tu = fma(Dju, S, -(Diu * R)), tv = fma(Djv, S, -(Div * R));
+  const double d3 = fma(n1, nu + tv, n2 * (nv - tu)) * (1.0 / 3.0);
+  const double fx = fma(n1, d3, nu - tv), fy = fma(n2, d3, nv + tu);
   F2 = fma(fx, mu, F2);
   F3 = fma(fy, mu, F3);
   F4 = fma(fma(us, fx, vs * fy), half(mu), F4);

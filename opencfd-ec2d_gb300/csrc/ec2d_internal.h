@@ -29,6 +29,9 @@ void launch_sst(const Lvl &L, cudaStream_t s);
 void launch_bl(const Lvl &L, cudaStream_t s);
 void launch_amut_boundary(const Lvl &L, cudaStream_t s);
 void launch_fdm(const Lvl &L, cudaStream_t s);
+void launch_sa_rows_mixed(const Lvl &L, cudaStream_t s);
+void launch_sst_rows_mixed(const Lvl &L, cudaStream_t s);
+void launch_fdm_mixed(const Lvl &L, cudaStream_t s);
 void launch_dual_term(const Lvl &L, double sfac, cudaStream_t s);
 // k_bc.cu
 void launch_bc(const Lvl &L, int phases, cudaStream_t s);

@@ -51,27 +51,31 @@ __device__ __forceinline__ void bc_wall(const Lvl &L, const BlkDev &b, const Cas
   const Cell A = load_cell(L, a);
   Cell G = A;
   if (c.Twall <= 0) {
-    G.v[1] = neg(A.v[1]);
-    G.v[2] = neg(A.v[2]);
+    G.v[1] = -A.v[1];
+    G.v[2] = -A.v[2];
   } else {
-    const double rd = rcp(A.v[0]), u1 = A.v[1] * rd, v1 = A.v[2] * rd, gM = c.gamma * c.Ma * c.Ma;
-    const double p1 = (A.v[3] - half(fma(A.v[1], u1, A.v[2] * v1))) * c.gm1;
-    const double T1 = gM * p1 * rd, T2 = fma(2.0, c.Twall, -T1);
-    const double d2 = gM * p1 * rcp_any(T2);
+    const double d1 = A.v[0];
+    double u1 = A.v[1] / d1, v1 = A.v[2] / d1;
+    double p1 = (A.v[3] - 0.5 * d1 * (u1 * u1 + v1 * v1)) * (c.gamma - 1.0);
+    double T1 = c.gamma * c.Ma * c.Ma * p1 / d1;
+    double p2 = p1, T2 = 2.0 * c.Twall - T1, u2 = -u1, v2 = -v1;
+    double d2 = c.gamma * c.Ma * c.Ma * p2 / T2;
     G.v[0] = d2;
-    G.v[1] = d2 * neg(u1);
-    G.v[2] = d2 * neg(v1);
-    G.v[3] = fma(p1, c.rgm1, half(d2) * fma(u1, u1, v1 * v1));
+    G.v[1] = d2 * u2;
+    G.v[2] = d2 * v2;
+    G.v[3] = p2 / (c.gamma - 1.0) + 0.5 * d2 * (u2 * u2 + v2 * v2);
   }
   if (L.nvar == 5) G.v[4] = 0.0;
   if (L.nvar == 6) {
     const double beta1 = 0.075;
-    const double d2 = G.v[0], rd = rcp(d2);
-    const double T2 = (G.v[3] - half(fma(G.v[1], G.v[1], G.v[2] * G.v[2])) * rd) * (rd * c.rCv);
-    const double Amu2 = (1.0 + c.Tsb) * (T2 * sqrt_t(T2)) * rcp_any(c.Tsb + T2);
-    const double wt = 60.0 * Amu2 * rcp_any(d2 * beta1 * (dw * dw) * c.Re * c.Re);
-    G.v[4] = neg(A.v[4]);
-    G.v[5] = fma(A.v[0] + d2, wt, -A.v[5]);
+    const double d1 = A.v[0];
+    double d2 = G.v[0];
+    double r2 = G.v[1], r3 = G.v[2];
+    double T2 = (G.v[3] - 0.5 * (r2 * r2 + r3 * r3) / d2) / (c.Cv * d2);
+    double Amu2 = (1.0 + c.Tsb) * sqrt(T2 * T2 * T2) / (c.Tsb + T2);
+    double wt = 60.0 * Amu2 / (d2 * beta1 * (dw * dw) * c.Re * c.Re);
+    G.v[4] = -A.v[4];
+    G.v[5] = (d1 + d2) * wt - A.v[5];
   }
   store_cell(L, fidx(b, i2, j2), G);
 }
@@ -84,9 +88,10 @@ __device__ __forceinline__ void bc_symmetry(const Lvl &L, const BlkDev &b, const
   int i1, j1, i2, j2;
   ghost_pair(s.face, i, j, k, i1, j1, i2, j2);
   Cell C = load_cell(L, fidx(b, i1, j1));
-  const double Vn = pow2<1>(fma(C.v[1], nrm.x, C.v[2] * nrm.y));
-  C.v[1] = fma(-Vn, nrm.x, C.v[1]);
-  C.v[2] = fma(-Vn, nrm.y, C.v[2]);
+  const double n1 = nrm.x, n2 = nrm.y;
+  const double Vn = C.v[1] * n1 + C.v[2] * n2;
+  C.v[1] = C.v[1] - 2.0 * Vn * n1;
+  C.v[2] = C.v[2] - 2.0 * Vn * n2;
   store_cell(L, fidx(b, i2, j2), C);
 }
 
@@ -118,7 +123,7 @@ __device__ __forceinline__ double2 edge_normal(const Lvl &L, const BlkDev &b, in
 // formed once and written to all LAP layers.
 __device__ __forceinline__ void bc_farfield(const Lvl &L, const BlkDev &b, const CaseDev &c, const SubDev &s, int i, int j,
                                             double2 nrm) {
-  const double gamma = c.gamma, gm1 = c.gm1;
+  const double gamma = c.gamma, gm1 = gamma - 1.0;
   const double n1 = nrm.x, n2 = nrm.y;
   int i1, j1;
   if (s.face == 1 || s.face == 2) { i1 = i; j1 = j; }
@@ -129,7 +134,7 @@ __device__ __forceinline__ void bc_farfield(const Lvl &L, const BlkDev &b, const
   const double d1 = A.v[0], m1 = A.v[1], m2 = A.v[2], E1 = A.v[3];
   const double rd = rcp(d1);
   const double u1 = m1 * rd, v1 = m2 * rd;
-  const double p1 = (E1 - half(fma(m1, u1, m2 * v1))) * gm1;
+  const double p1 = (E1 - 0.5 * d1 * (u1 * u1 + v1 * v1)) * gm1;
   const double c2 = gamma * p1 * rd;
   const double rc = rsqrt_d(c2);  // 1 / c1
   const double c1 = c2 * rc;
@@ -157,23 +162,23 @@ __device__ __forceinline__ void bc_farfield(const Lvl &L, const BlkDev &b, const
       const double ub = u1 + t * n1, vb = v1 + t * n2;
       const double p2 = 2.0 * pb - p1, d2 = 2.0 * db - d1, u2 = 2.0 * ub - u1, v2 = 2.0 * vb - v1;
       G[0] = d2; G[1] = d2 * u2; G[2] = d2 * v2;
-      G[3] = fma(p2, c.rgm1, half(d2) * fma(u2, u2, v2 * v2));
+      G[3] = p2 * c.rgm1 + 0.5 * d2 * (u2 * u2 + v2 * v2);
     }
   } else {
     const double d_inf = 1.0, u_inf = c.cosA, v_inf = c.sinA, p_inf = c.p00;
     if (c.p_outlet < 0 || at_least(neg(Ma_n), 1.0)) {
       G[0] = d_inf; G[1] = d_inf * u_inf; G[2] = d_inf * v_inf;
-      G[3] = p_inf * c.rgm1 + half(u_inf * u_inf + v_inf * v_inf);
+      G[3] = p_inf / gm1 + 0.5 * d_inf * (u_inf * u_inf + v_inf * v_inf);
     } else {
-      // pb = (p1 + p_inf - X) / 2, so 2 pb - p1 = p_inf - X and pb - p_inf = (p1 - p_inf - X) / 2
-      const double X = (d1 * c1) * fma(u_inf - u1, n1, (v_inf - v1) * n2);
-      const double p2 = p_inf - X, dp = (p1 - p_inf) - X;  // dp: 2 (pb - p_inf)
-      const double d2 = fma(dp, rc * rc, 2.0 * d_inf - d1), t = dp * (rd * rc);
-      const double u2 = fma(t, n1, fma(2.0, u_inf, -u1)), v2 = fma(t, n2, fma(2.0, v_inf, -v1));
+      const double pb = 0.5 * (p1 + p_inf - d1 * c1 * ((u_inf - u1) * n1 + (v_inf - v1) * n2));
+      const double db = d_inf + (pb - p_inf) * (rc * rc);
+      const double t = (p_inf - pb) * (rd * rc);
+      const double ub = u_inf - t * n1, vb = v_inf - t * n2;
+      const double p2 = 2.0 * pb - p1, d2 = 2.0 * db - d1, u2 = 2.0 * ub - u1, v2 = 2.0 * vb - v1;
       G[0] = d2; G[1] = d2 * u2; G[2] = d2 * v2;
-      G[3] = fma(p2, c.rgm1, half(d2) * fma(u2, u2, v2 * v2));
+      G[3] = p2 * c.rgm1 + 0.5 * d2 * (u2 * u2 + v2 * v2);
     }
-    if (L.nvar == 5) G[4] = c.vt_inf * c.rRe;
+    if (L.nvar == 5) G[4] = c.vt_inf / c.Re;
     else if (L.nvar == 6) { G[4] = d_inf * c.Kt_inf; G[5] = d_inf * c.Wt_inf; }
   }
   for (int k = 1; k <= LAP; k++) {
@@ -196,7 +201,7 @@ __device__ __forceinline__ void corner(const Lvl &L, const CaseDev &c, long long
   // lanes past the third repeat it
   const Cell A = load_cell(L, lane == 0 ? i1 : lane == 1 ? i2 : i3);
   const double d = A.v[0], rd = rcp(d), uu = A.v[1] * rd, v = A.v[2] * rd;
-  const double T = (A.v[3] - half(fma(uu, A.v[1], v * A.v[2]))) * (rd * c.rCv);
+  const double T = (A.v[3] - (uu * A.v[1] + v * A.v[2]) * 0.5) * (rd * c.rCv);
   auto across = [](double x) {
     const double x2 = __shfl_sync(0xffffffffu, x, 1), x3 = __shfl_sync(0xffffffffu, x, 2);
     return x + x3 - x2;  // of lane 0
@@ -206,7 +211,7 @@ __device__ __forceinline__ void corner(const Lvl &L, const CaseDev &c, long long
   C.v[0] = d4;
   C.v[1] = d4 * uu4;
   C.v[2] = d4 * v4;
-  C.v[3] = d4 * fma(c.Cv, T4, half(fma(uu4, uu4, v4 * v4)));
+  C.v[3] = d4 * (c.Cv * T4 + (uu4 * uu4 + v4 * v4) * 0.5);
   if (L.nvar > 4) {
     C.v[4] = across(A.v[4]);
     C.v[5] = across(A.v[5]);
@@ -220,8 +225,11 @@ constexpr int BC_SMEM_SUBS = 32;  // subfaces of a block staged in shared memory
 // with a cluster barrier between phases.  On one SM the FP64 instructions of a
 // far-field phase queue up (some 60 per item, one warp instruction per 16 to 19 cycles:
 // twelve warps of a 97 x 97 plate 6 us); on eight SMs a phase costs one item's chain.
-// Measured per call with 512 threads on one SM and as it is: BC_FIGS.  From 152
-// blocks on the blocks fill the chip and a cluster has BC_CTAS_MANY CTAs.
+// Measured per call between events (5 us of them the launch), 512 threads on one SM
+// against eight CTAs: 1025 x 513 54 and 21 us, 16 cases of 385 x 97 22 and 18; 97 x 97
+// 20.4 and 18.5, the chain of a far-field item (some 45 FP64 instructions of 64 cycles)
+// once per phase.  From 152 blocks on the blocks fill the chip and a cluster has
+// BC_CTAS_MANY CTAs.
 constexpr int BC_THREADS = 256, BC_CTAS = 8, BC_CTAS_MANY = 2;
 
 // every global write of the cluster's threads before is seen by them after

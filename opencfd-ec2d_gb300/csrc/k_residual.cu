@@ -13,6 +13,9 @@
 // in its own index range.
 #include "ec2d_dev.cuh"
 #include "ec2d_internal.h"
+#include "ec2d_mixed.cuh"
+
+#include <type_traits>
 
 namespace ec2d {
 
@@ -30,9 +33,40 @@ __device__ __forceinline__ bool tile_ij(const Lvl &L, int &bk, int &i, int &j) {
   return true;
 }
 
+// M (here and below): a context with FP32 parts, whose arithmetic keeps its order of
+// operations (ec2d_mixed.cuh)
+struct Prim { double u, v, T, p, sT; };
+template <bool M>
+__device__ __forceinline__ Prim primitives(const CaseDev &c, double d, double ru, double rv, double E) {
+  Prim w;
+  if constexpr (M) {
+    const double rd = rcp(d);
+    w.u = ru * rd;
+    w.v = rv * rd;
+    w.T = (E - 0.5 * d * (w.u * w.u + w.v * w.v)) * (rd * c.rCv);
+    w.p = c.p00 * d * w.T;
+    w.sT = w.T > 0.0 ? sqrt_p(w.T) : sqrt(w.T);  // the reference's sqrt, NaN for T < 0
+  } else {
+    const double rd = recip(d);
+    w.u = ru * rd;
+    w.v = rv * rd;
+    const double e = E - half(fma(ru, w.u, rv * w.v));
+    w.T = e * (rd * c.rCv);
+    w.p = e * c.gm1;
+    w.sT = root_t(w.T);
+  }
+  return w;
+}
+template <bool M>
+__device__ __forceinline__ double sutherland(const CaseDev &c, const Prim &w) {  // T^1.5 = T sqrt(T)
+  if constexpr (M) return c.rRe * (1.0 + c.Tsb) * (w.T * w.sT) * rcp(c.Tsb + w.T);
+  else return c.mu0 * (w.T * w.sT) * recip(c.Tsb + w.T);
+}
+
 // comput_duvtpckw (sub_Residual.f90:114-152) + get_viscous (:670-689) + Amu_t=0
-// (:172); 21 FP64 instructions per viscous cell instead of 29 (1.05 M cells: 49 us
-// instead of 68)
+// (:172); 21 FP64 instructions per viscous cell of an FP64 context instead of 29 (1.05 M
+// cells: 49 us instead of 68)
+template <bool M>
 __global__ void __launch_bounds__(TILE) k_prim(Lvl L) {
   int bk, i, j;
   if (!tile_ij(L, bk, i, j)) return;
@@ -40,24 +74,20 @@ __global__ void __launch_bounds__(TILE) k_prim(Lvl L) {
   const CaseDev &c = L.cs[b.cas];
   long long id = fidx(b, i, j);
   const long long F = L.F;
-  double d = L.U[id], ru = L.U[F + id], rv = L.U[2 * F + id], E = L.U[3 * F + id];
-  const double rd = rcp(d);
-  const double uu = ru * rd, v = rv * rd;
-  const double e = E - half(fma(ru, uu, rv * v)), T = e * (rd * c.rCv), p = e * c.gm1;
-  const double sT = sqrt_t(T);
+  const double d = L.U[id];
+  const Prim w = primitives<M>(c, d, L.U[F + id], L.U[2 * F + id], L.U[3 * F + id]);
   L.q[Q_D * F + id] = d;
-  L.q[Q_U * F + id] = uu;
-  L.q[Q_V * F + id] = v;
-  L.q[Q_T * F + id] = T;
-  L.q[Q_P * F + id] = p;
+  L.q[Q_U * F + id] = w.u;
+  L.q[Q_V * F + id] = w.v;
+  L.q[Q_T * F + id] = w.T;
+  L.q[Q_P * F + id] = w.p;
   bool interior = (i >= 1 && i <= b.nx - 1 && j >= 1 && j <= b.ny - 1);
   if (interior) {
-    if (!at_least(T, 1.0e-5)) set_status(L.status + 4 * b.cas, 3, bk, i, j);
-    L.q[Q_C * F + id] = sT * c.rMa;
+    if (!at_least(w.T, 1.0e-5)) set_status(L.status + 4 * b.cas, 3, bk, i, j);
+    L.q[Q_C * F + id] = w.sT * c.rMa;
   }
   if (L.visc) {
-    if (i >= 0 && i <= b.nx && j >= 0 && j <= b.ny)
-      L.amu[id] = c.mu0 * (T * sT) * rcp(c.Tsb + T);  // T^1.5 = T sqrt(T)
+    if (i >= 0 && i <= b.nx && j >= 0 && j <= b.ny) L.amu[id] = sutherland<M>(c, w);
     if (!L.keep_amut) L.amut[id] = 0.0;
   }
 }
@@ -66,129 +96,136 @@ __device__ __forceinline__ bool in_fdm_core(const BlkDev &b, int i, int j) {
   return b.fdm && (i >= LFDM + 2 && i <= b.nx - LFDM - 1) && (j >= LFDM + 2 && j <= b.ny - LFDM - 1);
 }
 
-// viscosity and heat conduction of a face times its length s, from the cells cl and
-// cr next to it; a level without a turbulence model or a restricted eddy
-// viscosity has amut = 0
-template <typename T>
-__device__ __forceinline__ void face_viscosity(const Lvl &L, const CaseDev &c, long long cl, long long cr, T s, T &mu, T &k) {
-  const T h = half(s), ml = to<T>(L.amu[cl]) + to<T>(L.amu[cr]);
-  mu = ml * h;
-  k = mu * to<T>(c.kpr);
-  if (L.turb != Turb_NONE || L.keep_amut) {
-    const T mt = (to<T>(L.amut[cl]) + to<T>(L.amut[cr])) * h;
-    k = fma(mt, to<T>(c.kprt), k);
-    mu += mt;
+// reconstruction and inviscid flux of a face, F = -s (flux)
+template <bool M, typename T>
+__device__ __forceinline__ void inviscid(const Lvl &L, const CaseDev &c, int scheme, T S0[4][4], T n1, T n2, T s, T *F) {
+  T UL[4], UR[4];
+  if constexpr (M) {
+    mixed::reconstruct(L.recon, scheme, S0, to<T>(c.gamma), UL, UR);
+    T QL[4] = {UL[0], UL[1] * n1 + UL[2] * n2, -UL[1] * n2 + UL[2] * n1, UL[3]};
+    T QR[4] = {UR[0], UR[1] * n1 + UR[2] * n2, -UR[1] * n2 + UR[2] * n1, UR[3]};
+    T Fl[4];
+    mixed::face_flux(L.flux, QL, QR, Fl, to<T>(c.gamma), to<T>(c.ggm1));
+    F[0] = -Fl[0] * s;
+    F[1] = -(Fl[1] * n1 - Fl[2] * n2) * s;
+    F[2] = -(Fl[1] * n2 + Fl[2] * n1) * s;
+    F[3] = -Fl[3] * s;
+  } else {
+    const Gas G = gas(c);
+    reconstruct(L.recon, scheme, S0, G, UL, UR);
+    face_flux(L.flux, UL, UR, n1, n2, s, F, G);
   }
+}
+// viscous terms of a face, added to F.  across: from the cell before the face to the
+// one after; along: the sum over both cells of the differences between their
+// neighbours beside the face's ends.  g: the face's four metric planes; ml, tl and
+// mr, tr: laminar and eddy viscosity before and after the face (eddy: the latter
+// are not zero by the level's model); lo, hi: a face on the block's first or last
+// line, which takes the interior cell's.
+template <typename T>
+struct FaceDiff { T xu, xv, xT, yu, yv, yT, us, vs; };
+template <bool M, bool IFACE, typename T>
+__device__ __forceinline__ void viscous(const CaseDev &c, const double *g, long long F, const FaceDiff<T> &D, T ml, T mr,
+                                        bool eddy, T tl, T tr, bool lo, bool hi, T n1, T n2, T s, T *Fo) {
+  if constexpr (M) {
+    T Amu1, Amk1;
+    const T Cp = to<T>(c.Cp), rPr = to<T>(c.rPr), rPrT = (T)(1.0 / PrT);
+    if (lo) {
+      Amu1 = mr + tr;
+      Amk1 = Cp * (mr * rPr + tr * rPrT);
+    } else if (hi) {
+      Amu1 = ml + tl;
+      Amk1 = Cp * (ml * rPr + tl * rPrT);
+    } else {
+      // the two families of faces add the viscosities in their own order
+      if (IFACE) Amu1 = (ml + mr + tl + tr) * T(0.5);
+      else Amu1 = (mr + ml + tr + tl) * T(0.5);
+      Amk1 = Cp * ((ml + mr) * rPr + (tl + tr) * rPrT) * T(0.5);
+    }
+    const T yu = D.yu * T(0.25), yv = D.yv * T(0.25), yT = D.yT * T(0.25);
+    mixed::viscous_face_m(to<T>(g[0]), to<T>(g[F]), to<T>(g[2 * F]), to<T>(g[3 * F]), IFACE ? D.xu : yu, IFACE ? D.xv : yv,
+                          IFACE ? D.xT : yT, IFACE ? yu : D.xu, IFACE ? yv : D.xv, IFACE ? yT : D.xT, Amu1, Amk1,
+                          D.us * T(0.5), D.vs * T(0.5), n1, n2, s, Fo[1], Fo[2], Fo[3]);
+  } else {
+    const double h = half(s);
+    double mu = ((lo ? mr : ml) + (hi ? ml : mr)) * h, k = mu * c.kpr;
+    if (eddy) {
+      const double mt = ((lo ? tr : tl) + (hi ? tl : tr)) * h;
+      k = fma(mt, c.kprt, k);
+      mu += mt;
+    }
+    viscous_face_m(g[0], g[F], g[2 * F], g[3 * F], IFACE ? D.xu : D.yu, IFACE ? D.xv : D.yv, IFACE ? D.xT : D.yT,
+                   IFACE ? D.yu : D.xu, IFACE ? D.yv : D.xv, IFACE ? D.yT : D.xT, mu, k, D.us, D.vs, n1, n2, Fo[1],
+                   Fo[2], Fo[3]);
+  }
+}
+// the differences from u(k), v(k), T(k) at cell k; r: the cell after the face, st: to the
+// cell before it, ot: along the face
+template <bool M, typename T, typename Fu, typename Fv, typename FT>
+__device__ __forceinline__ FaceDiff<T> face_diff(long long r, long long st, long long ot, Fu u, Fv v, FT t) {
+  const long long l = r - st, n = r + ot, z = r - ot;
+  auto along = [&](auto &q) -> T {
+    if constexpr (M) return q(n - st) + q(n) - q(z - st) - q(z);
+    else return (q(n - st) - q(z - st)) + (q(n) - q(z));
+  };
+  return {u(r) - u(l), v(r) - v(l), t(r) - t(l), along(u), along(v), along(t), u(r) + u(l), v(r) + v(l)};
 }
 
 // The face kernels are bound by the issue of FP64 instructions (one per 16 to 19
 // cycles and SM; memory traffic is a tenth of the time): a viscous MUSCL3 / AUSM+
-// face takes about 195 of them (reconstruction 96, flux 54, viscous terms 44) where
+// face takes about 190 of them (reconstruction 96, flux 50, viscous terms 44) where
 // the formulas written out with divides, rotations and floating-point
-// selects took 298, and the flux planes of 1.05 M cells take 0.39 ms per direction
-// instead of 0.60 (HLLC with characteristic WENO3 on 131 x 59 cells 22 us instead
-// of 41, most of them the chain of one face).  FP32: the values are
-// converted on the integer pipes (to<float>), not by the FP64 pipe.
-// i-direction face loop of Residual_FVM (sub_Residual.f90:238-346): face (i,j),
-// i=1..nx, j=1..ny-1, between cells (i-1,j) and (i,j).
-template <typename T>
-__global__ void __launch_bounds__(TILE) k_flux_i(Lvl L) {
-  int bk, i, j;
-  if (!core_ij(L, bk, i, j)) return;
-  const BlkDev &b = L.blk[bk];
-  if (i < 1 || i > b.nx || j < 1 || j > b.ny - 1) return;
-  if (in_fdm_core(b, i, j)) return;
-  const CaseDev &c = L.cs[b.cas];
-  const long long F = L.F;
-  long long id = fidx(b, i, j);
-  T si = to<T>(L.geo[G_SI * F + id]), n1 = to<T>(L.geo[G_NI1 * F + id]), n2 = to<T>(L.geo[G_NI2 * F + id]);
-  T S0[4][4], UL[4], UR[4];
-  if (L.recon == Recon_Original) {
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      long long s = id + (k - 2);
-      S0[k][0] = to<T>(L.q[Q_D * F + s]); S0[k][1] = to<T>(L.q[Q_U * F + s]);
-      S0[k][2] = to<T>(L.q[Q_V * F + s]); S0[k][3] = to<T>(L.q[Q_P * F + s]);
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-#pragma unroll
-      for (int m = 0; m < 4; m++) S0[k][m] = to<T>(L.U[m * F + id + (k - 2)]);
-  }
-  const Gas<T> G = gas<T>(c);
-  reconstruct(L.recon, L.scheme, S0, G, UL, UR);
-  T Fl[4];
-  face_flux(L.flux, UL, UR, n1, n2, si, Fl, G);
-  if (L.visc) {
-    const long long w = id - 1, nN = id + b.P, nS = id - b.P;
-    // cells of the viscosity: both sides, or the interior one twice
-    const long long cl = i == 1 ? id : w, cr = i == b.nx ? w : id;
-    T mu, k;
-    face_viscosity<T>(L, c, cl, cr, si, mu, k);
-    const double *uu = L.q + Q_U * F, *vv = L.q + Q_V * F, *TT = L.q + Q_T * F;
-    const double *g = L.geo + id;
-    const T ul = to<T>(uu[w]), ur = to<T>(uu[id]), vl = to<T>(vv[w]), vr = to<T>(vv[id]);
-    const T Dju = (to<T>(uu[nN - 1]) - to<T>(uu[nS - 1])) + (to<T>(uu[nN]) - to<T>(uu[nS]));
-    const T Djv = (to<T>(vv[nN - 1]) - to<T>(vv[nS - 1])) + (to<T>(vv[nN]) - to<T>(vv[nS]));
-    const T DjT = (to<T>(TT[nN - 1]) - to<T>(TT[nS - 1])) + (to<T>(TT[nN]) - to<T>(TT[nS]));
-    viscous_face_m(to<T>(g[G_VIP * F]), to<T>(g[G_VIQ * F]), to<T>(g[G_VIR * F]), to<T>(g[G_VIS * F]), ur - ul, vr - vl,
-                   to<T>(TT[id]) - to<T>(TT[w]), Dju, Djv, DjT, mu, k, ul + ur, vl + vr, n1, n2, Fl[1], Fl[2], Fl[3]);
-  }
-#pragma unroll
-  for (int m = 0; m < 4; m++) L.fi[m * F + id] = to_double(Fl[m]);
-}
-
-// j-direction face loop of Residual_FVM (sub_Residual.f90:352-455): face (i,j),
+// selects take 298 (M, ec2d_mixed.cuh), and the flux planes of 1.05 M cells take
+// 0.39 ms per direction instead of 0.60 (HLLC with characteristic WENO3 on 131 x 59
+// cells 22 us instead of 41, most of them the chain of one face).  In FP32 the
+// values are converted on the integer pipes (to<float>), not by the FP64 pipe.
+// IFACE: face loop in i of Residual_FVM (sub_Residual.f90:238-346), face (i,j),
+// i=1..nx, j=1..ny-1, between cells (i-1,j) and (i,j); else in j (:352-455), face (i,j),
 // i=1..nx-1, j=1..ny, between cells (i,j-1) and (i,j).
-template <typename T>
-__global__ void __launch_bounds__(TILE) k_flux_j(Lvl L) {
+template <bool M, bool IFACE, typename T>
+__global__ void __launch_bounds__(TILE) k_flux(Lvl L) {
   int bk, i, j;
   if (!core_ij(L, bk, i, j)) return;
   const BlkDev &b = L.blk[bk];
-  if (i < 1 || i > b.nx - 1 || j < 1 || j > b.ny) return;
+  if (i < 1 || i > b.nx - !IFACE || j < 1 || j > b.ny - IFACE) return;
   if (in_fdm_core(b, i, j)) return;
   const CaseDev &c = L.cs[b.cas];
-  const long long F = L.F;
-  const long long P = b.P;
-  long long id = fidx(b, i, j);
-  T sj = to<T>(L.geo[G_SJ * F + id]), n1 = to<T>(L.geo[G_NJ1 * F + id]), n2 = to<T>(L.geo[G_NJ2 * F + id]);
-  T S0[4][4], UL[4], UR[4];
+  const long long F = L.F, st = IFACE ? 1 : b.P, id = fidx(b, i, j);
+  const T s = to<T>(L.geo[(IFACE ? G_SI : G_SJ) * F + id]), n1 = to<T>(L.geo[(IFACE ? G_NI1 : G_NJ1) * F + id]),
+          n2 = to<T>(L.geo[(IFACE ? G_NI2 : G_NJ2) * F + id]);
+  T S0[4][4];
   int scheme = L.scheme;
   if (L.recon == Recon_Original) {
-    scheme = L.gscheme;  // the reference passes the global Iflag_Scheme here (sub_Residual.f90:367)
+    if (!IFACE) scheme = L.gscheme;  // the reference passes the global Iflag_Scheme here (sub_Residual.f90:367)
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      long long s = id + (k - 2) * P;
-      S0[k][0] = to<T>(L.q[Q_D * F + s]); S0[k][1] = to<T>(L.q[Q_U * F + s]);
-      S0[k][2] = to<T>(L.q[Q_V * F + s]); S0[k][3] = to<T>(L.q[Q_P * F + s]);
+      const long long q = id + (k - 2) * st;
+      S0[k][0] = to<T>(L.q[Q_D * F + q]); S0[k][1] = to<T>(L.q[Q_U * F + q]);
+      S0[k][2] = to<T>(L.q[Q_V * F + q]); S0[k][3] = to<T>(L.q[Q_P * F + q]);
     }
   } else {
 #pragma unroll
     for (int k = 0; k < 4; k++)
 #pragma unroll
-      for (int m = 0; m < 4; m++) S0[k][m] = to<T>(L.U[m * F + id + (k - 2) * P]);
+      for (int m = 0; m < 4; m++) S0[k][m] = to<T>(L.U[m * F + id + (k - 2) * st]);
   }
-  const Gas<T> G = gas<T>(c);
-  reconstruct(L.recon, scheme, S0, G, UL, UR);
   T Fl[4];
-  face_flux(L.flux, UL, UR, n1, n2, sj, Fl, G);
+  inviscid<M>(L, c, scheme, S0, n1, n2, s, Fl);
   if (L.visc) {
-    const long long s = id - P;
-    const long long cl = j == 1 ? id : s, cr = j == b.ny ? s : id;
-    T mu, k;
-    face_viscosity<T>(L, c, cl, cr, sj, mu, k);
     const double *uu = L.q + Q_U * F, *vv = L.q + Q_V * F, *TT = L.q + Q_T * F;
-    const double *g = L.geo + id;
-    const T ul = to<T>(uu[s]), ur = to<T>(uu[id]), vl = to<T>(vv[s]), vr = to<T>(vv[id]);
-    const T Diu = (to<T>(uu[s + 1]) - to<T>(uu[s - 1])) + (to<T>(uu[id + 1]) - to<T>(uu[id - 1]));
-    const T Div = (to<T>(vv[s + 1]) - to<T>(vv[s - 1])) + (to<T>(vv[id + 1]) - to<T>(vv[id - 1]));
-    const T DiT = (to<T>(TT[s + 1]) - to<T>(TT[s - 1])) + (to<T>(TT[id + 1]) - to<T>(TT[id - 1]));
-    viscous_face_m(to<T>(g[G_VJP * F]), to<T>(g[G_VJQ * F]), to<T>(g[G_VJR * F]), to<T>(g[G_VJS * F]), Diu, Div, DiT,
-                   ur - ul, vr - vl, to<T>(TT[id]) - to<T>(TT[s]), mu, k, ul + ur, vl + vr, n1, n2, Fl[1], Fl[2], Fl[3]);
+    auto u = [=](long long k) { return to<T>(uu[k]); };
+    auto v = [=](long long k) { return to<T>(vv[k]); };
+    auto t = [=](long long k) { return to<T>(TT[k]); };
+    const bool eddy = M || L.turb != Turb_NONE || L.keep_amut;
+    T tl = T(0), tr = T(0);
+    if (eddy) { tl = to<T>(L.amut[id - st]); tr = to<T>(L.amut[id]); }
+    viscous<M, IFACE>(c, L.geo + (IFACE ? G_VIP : G_VJP) * F + id, F, face_diff<M, T>(id, st, IFACE ? b.P : 1, u, v, t),
+                      to<T>(L.amu[id - st]), to<T>(L.amu[id]), eddy, tl, tr, (IFACE ? i : j) == 1,
+                      IFACE ? i == b.nx : j == b.ny, n1, n2, s, Fl);
   }
+  double *out = IFACE ? L.fi : L.fj;
 #pragma unroll
-  for (int m = 0; m < 4; m++) L.fj[m * F + id] = to_double(Fl[m]);
+  for (int m = 0; m < 4; m++) out[m * F + id] = to_double(Fl[m]);
 }
 
 // Norm reductions.  max |Res| is reduced on the bit patterns: for
@@ -315,6 +352,22 @@ __device__ __forceinline__ void final_norm(const Lvl &L, int cs, int m) {
   if (lane == 0) L.norms[cs * 12 + m] = out;
 }
 
+// viscous spectral radii of a cell (comput_Lvc)
+template <bool M>
+__device__ __forceinline__ void viscous_radii(const CaseDev &c, const double *g, long long F, double d, double amu, bool eddy,
+                                              double amut, double &Lvi, double &Lvj) {
+  double m;
+  if constexpr (M) {
+    m = c.gamma * rcp(d) * (amu * c.rPr + amut * (1.0 / PrT));
+  } else {
+    m = amu * c.gpr;
+    if (eddy) m = fma(amut, c.gprt, m);
+    m *= recip(d);
+  }
+  Lvi = m * g[G_VI2 * F];
+  Lvj = m * g[G_VJ2 * F];
+}
+
 // flux differences (sub_Residual.f90:460-468), comput_Lvc (sub_NS_singlegrid.f90:352-388)
 // and comput_dt (sub_NS_singlegrid.f90:324-348) for interior cells
 // NORM: also the tile's partial norms of Res (the work of k_norm_partial,
@@ -324,7 +377,7 @@ __device__ __forceinline__ void final_norm(const Lvl &L, int cs, int m) {
 // post: RES_ADD_FORCE (Res += QF once the norms are taken), RES_FORCE_FN
 // (QF -= Res), RES_SET_UN (Un = U over 0..nx, 0..ny): the multigrid steps
 // that follow a residual evaluation, done in the same pass
-template <bool NORM, bool FINAL>
+template <bool M, bool NORM, bool FINAL>
 __global__ void __launch_bounds__(TILE) k_res(Lvl L, int post) {
   int bk, i, j;
   bool act = core_ij(L, bk, i, j);
@@ -371,11 +424,8 @@ __global__ void __launch_bounds__(TILE) k_res(Lvl L, int post) {
     double Lci = (fabs(uni) + cc) * si, Lcj = (fabs(unj) + cc) * sj;
     double Lvi = 0.0, Lvj = 0.0;
     if (L.visc) {
-      double m = L.amu[id] * c.gpr;
-      if (L.turb != Turb_NONE || L.keep_amut) m = fma(L.amut[id], c.gprt, m);
-      m *= rcp(d);
-      Lvi = m * g[G_VI2 * F];
-      Lvj = m * g[G_VJ2 * F];
+      const bool eddy = L.turb != Turb_NONE || L.keep_amut;
+      viscous_radii<M>(c, g, F, d, L.amu[id], eddy, eddy ? L.amut[id] : 0.0, Lvi, Lvj);
     }
     L.lc[L_CI * F + id] = Lci;
     L.lc[L_CJ * F + id] = Lcj;
@@ -386,7 +436,7 @@ __global__ void __launch_bounds__(TILE) k_res(Lvl L, int post) {
     else {
       double sum = Lci + Lcj;
       if (L.visc) sum += Lvi + Lvj;
-      dt = c.CFL * s0 * rcp(sum);
+      dt = c.CFL * s0 * (M ? rcp(sum) : recip(sum));
       if (above(dt, c.dtmax)) dt = c.dtmax;
       if (below(dt, c.dtmin)) dt = c.dtmin;
     }
@@ -431,7 +481,7 @@ constexpr int RNT = RES_TILE_THREADS;
 // kernel is as long as one thread's chain)
 static_assert((RTX + 1) * RTY + RTX * (RTY + 1) <= RNT && RGN <= RNT && RTX * RTY <= RNT, "a thread per item");
 
-template <bool NORM, bool FINAL>
+template <bool M, bool NORM, bool FINAL>
 __global__ void __launch_bounds__(RNT) k_residual_tile(Lvl L, const int4 *rt, int post) {
   __shared__ double sd[RGN], su[RGN], sv[RGN], sp[RGN], sT[RGN], sc[RGN], smu[RGN];
   __shared__ double sU[4][RGN];
@@ -451,17 +501,14 @@ __global__ void __launch_bounds__(RNT) k_residual_tile(Lvl L, const int4 *rt, in
     if (i < -1 || i > nx + 1 || j < -1 || j > ny + 1) continue;
     const long long id = fidx(b, i, j);
     const double d = L.U[id], ru = L.U[F + id], rv = L.U[2 * F + id], E = L.U[3 * F + id];
-    const double rd = rcp(d);
-    const double uu = ru * rd, v = rv * rd;
-    const double e = E - half(fma(ru, uu, rv * v)), T = e * (rd * c.rCv), pp = e * c.gm1;
-    const double st = sqrt_t(T);
-    sd[t] = d; su[t] = uu; sv[t] = v; sT[t] = T; sp[t] = pp;
-    sc[t] = st * c.rMa;
+    const Prim w = primitives<M>(c, d, ru, rv, E);
+    sd[t] = d; su[t] = w.u; sv[t] = w.v; sT[t] = w.T; sp[t] = w.p;
+    sc[t] = w.sT * c.rMa;
     sU[0][t] = d; sU[1][t] = ru; sU[2][t] = rv; sU[3][t] = E;
     const bool own = i >= i0 && i <= i1 && j >= j0 && j <= j1;
-    if (own && !at_least(T, 1.0e-5)) set_status(L.status + 4 * b.cas, 3, bk, i, j);
+    if (own && !at_least(w.T, 1.0e-5)) set_status(L.status + 4 * b.cas, 3, bk, i, j);
     if (L.visc) {
-      const double mu = c.mu0 * (T * st) * rcp(c.Tsb + T);
+      const double mu = sutherland<M>(c, w);
       smu[t] = mu;
       // Amu over 0..nx x 0..ny as k_prim leaves it: the tile's cells, and the
       // block's ghost lines next to them when the tile is on the block's edge
@@ -482,7 +529,7 @@ __global__ void __launch_bounds__(RNT) k_residual_tile(Lvl L, const int4 *rt, in
     const int r = R(i, j), st = ifc ? 1 : RGX;  // stencil stride in the tile's shared arrays
     const double s = L.geo[(ifc ? G_SI : G_SJ) * F + id];
     const double n1 = L.geo[(ifc ? G_NI1 : G_NJ1) * F + id], n2 = L.geo[(ifc ? G_NI2 : G_NJ2) * F + id];
-    double S0[4][4], UL[4], UR[4];
+    double S0[4][4];
     int scheme = L.scheme;
     if (L.recon == Recon_Original) {
       if (!ifc) scheme = L.gscheme;  // the global Iflag_Scheme in the j direction (sub_Residual.f90:367)
@@ -497,25 +544,16 @@ __global__ void __launch_bounds__(RNT) k_residual_tile(Lvl L, const int4 *rt, in
 #pragma unroll
         for (int m = 0; m < 4; m++) S0[k][m] = sU[m][r + (k - 2) * st];
     }
-    const Gas<double> G = gas<double>(c);
-    reconstruct(L.recon, scheme, S0, G, UL, UR);
     double Fl[4];
-    face_flux(L.flux, UL, UR, n1, n2, s, Fl, G);
+    inviscid<M>(L, c, scheme, S0, n1, n2, s, Fl);
     if (L.visc) {
-      const double *g = L.geo + id;
-      const int up = r - st;  // the upstream cell of the face
-      const bool lo = ifc ? i == 1 : j == 1, hi = ifc ? i == nx : j == ny;
-      const double mu = (smu[lo ? r : up] + smu[hi ? up : r]) * half(s);
-      // differences across the face, and along it from the four cells beside its ends
-      const int ot = ifc ? RGX : 1, a = r + ot, z = r - ot;
-      const double xu = su[r] - su[up], xv = sv[r] - sv[up], xT = sT[r] - sT[up];
-      const double yu = (su[a - st] - su[z - st]) + (su[a] - su[z]);
-      const double yv = (sv[a - st] - sv[z - st]) + (sv[a] - sv[z]);
-      const double yT = (sT[a - st] - sT[z - st]) + (sT[a] - sT[z]);
-      const double *m = g + (ifc ? G_VIP : G_VJP) * F;
-      viscous_face_m(m[0], m[F], m[2 * F], m[3 * F], ifc ? xu : yu, ifc ? xv : yv, ifc ? xT : yT, ifc ? yu : xu,
-                     ifc ? yv : xv, ifc ? yT : xT, mu, mu * c.kpr, su[r] + su[up], sv[r] + sv[up], n1, n2, Fl[1], Fl[2],
-                     Fl[3]);
+      auto u = [&](long long k) { return su[k]; };
+      auto v = [&](long long k) { return sv[k]; };
+      auto t = [&](long long k) { return sT[k]; };
+      const FaceDiff<double> D = face_diff<M, double>(r, st, ifc ? RGX : 1, u, v, t);
+      const double ml = smu[r - st], mr = smu[r], *g = L.geo + id;
+      if (ifc) viscous<M, true>(c, g + G_VIP * F, F, D, ml, mr, false, 0.0, 0.0, i == 1, i == nx, n1, n2, s, Fl);
+      else viscous<M, false>(c, g + G_VJP * F, F, D, ml, mr, false, 0.0, 0.0, j == 1, j == ny, n1, n2, s, Fl);
     }
 #pragma unroll
     for (int m = 0; m < 4; m++) (ifc ? fi[m][j - j0][i - i0] : fj[m][j - j0][i - i0]) = Fl[m];
@@ -562,11 +600,7 @@ __global__ void __launch_bounds__(RNT) k_residual_tile(Lvl L, const int4 *rt, in
     const double uni = uu * ni1 + vv * ni2, unj = uu * nj1 + vv * nj2;
     const double Lci = (fabs(uni) + cc) * si, Lcj = (fabs(unj) + cc) * sj;
     double Lvi = 0.0, Lvj = 0.0;
-    if (L.visc) {
-      const double m = smu[r] * c.gpr * rcp(d);
-      Lvi = m * g[G_VI2 * F];
-      Lvj = m * g[G_VJ2 * F];
-    }
+    if (L.visc) viscous_radii<M>(c, g, F, d, smu[r], false, 0.0, Lvi, Lvj);
     L.lc[L_CI * F + id] = Lci;
     L.lc[L_CJ * F + id] = Lcj;
     L.lc[L_VI * F + id] = Lvi;
@@ -576,7 +610,7 @@ __global__ void __launch_bounds__(RNT) k_residual_tile(Lvl L, const int4 *rt, in
     else {
       double sum = Lci + Lcj;
       if (L.visc) sum += Lvi + Lvj;
-      dt = c.CFL * s0 * rcp(sum);
+      dt = c.CFL * s0 * (M ? rcp(sum) : recip(sum));
       if (above(dt, c.dtmax)) dt = c.dtmax;
       if (below(dt, c.dtmin)) dt = c.dtmin;
     }
@@ -624,7 +658,8 @@ __global__ void __launch_bounds__(384) k_norm_final(Lvl L) {
   final_norm(L, k / 12, k % 12);
 }
 
-// set-up: the viscous metric coefficients (G_VIP..G_VJS) of the i-faces (i = 1..nx, j =
+// set-up, and when a context gets or loses its FP32 parts: the viscous metric
+// coefficients (G_VIP..G_VJS) of the i-faces (i = 1..nx, j =
 // 1..ny-1) and j-faces (i = 1..nx-1, j = 1..ny) from the cell centres, with the
 // stencils of Residual_FVM (sub_Residual.f90:313-330, 419-436), and the cell
 // metric factors of the spectral radii
@@ -635,6 +670,14 @@ __global__ void __launch_bounds__(TILE) k_face_metrics(Lvl L) {
   const long long F = L.F, P = b.P, id = fidx(b, i, j);
   const double *x1 = L.geo + G_X1 * F, *y1 = L.geo + G_Y1 * F;
   double *g = L.geo + id;
+  // fi, fj: the factors of the differences in i and j (1/4 of those along the face)
+  auto put = [&](int to, int nrm, double A, double B, double C, double D, double fi, double fj) {
+    const double n1 = g[nrm * F], n2 = g[(nrm + 1) * F];
+    g[to * F] = L.mixed ? A : fi * (A * n1 - C * n2);
+    g[(to + 1) * F] = L.mixed ? B : fj * (D * n2 - B * n1);
+    g[(to + 2) * F] = L.mixed ? C : fi * (A * n2 + C * n1);
+    g[(to + 3) * F] = L.mixed ? D : fj * (B * n2 + D * n1);
+  };
   if (i >= 1 && i <= b.nx && j >= 1 && j <= b.ny - 1) {
     const long long w = id - 1, nN = id + P, nS = id - P;
     const double Dix = x1[id] - x1[w], Diy = y1[id] - y1[w];
@@ -642,9 +685,7 @@ __global__ void __launch_bounds__(TILE) k_face_metrics(Lvl L) {
     const double Djy = (y1[nN - 1] + y1[nN] - y1[nS - 1] - y1[nS]) * 0.25;
     const double Ds = 1.0 / (Dix * Djy - Djx * Diy);
     const double A = Djy * Ds, B = Diy * Ds, C = Djx * Ds, D = Dix * Ds;
-    const double n1 = g[G_NI1 * F], n2 = g[G_NI2 * F];
-    g[G_VIP * F] = A * n1 - C * n2; g[G_VIQ * F] = 0.25 * (D * n2 - B * n1);
-    g[G_VIR * F] = A * n2 + C * n1; g[G_VIS * F] = 0.25 * (B * n2 + D * n1);
+    put(G_VIP, G_NI1, A, B, C, D, 1.0, 0.25);
   }
   if (i >= 1 && i <= b.nx - 1 && j >= 1 && j <= b.ny) {
     const long long s = id - P;
@@ -653,9 +694,7 @@ __global__ void __launch_bounds__(TILE) k_face_metrics(Lvl L) {
     const double Djx = x1[id] - x1[s], Djy = y1[id] - y1[s];
     const double Ds = 1.0 / (Dix * Djy - Djx * Diy);
     const double A = Djy * Ds, B = Diy * Ds, C = Djx * Ds, D = Dix * Ds;
-    const double n1 = g[G_NJ1 * F], n2 = g[G_NJ2 * F];
-    g[G_VJP * F] = 0.25 * (A * n1 - C * n2); g[G_VJQ * F] = D * n2 - B * n1;
-    g[G_VJR * F] = 0.25 * (A * n2 + C * n1); g[G_VJS * F] = B * n2 + D * n1;
+    put(G_VJP, G_NJ1, A, B, C, D, 0.25, 1.0);
   }
   if (i >= 1 && i <= b.nx - 1 && j >= 1 && j <= b.ny - 1) {
     // comput_Lvc (sub_NS_singlegrid.f90:352-388): face metrics averaged over
@@ -676,28 +715,39 @@ __global__ void __launch_bounds__(TILE) k_face_metrics(Lvl L) {
 }
 void launch_face_metrics(const Lvl &L, cudaStream_t s) { k_face_metrics<<<L.ntiles, TILE, 0, s>>>(L); }
 
-void launch_prim(const Lvl &L, cudaStream_t s) { k_prim<<<L.ntiles, TILE, 0, s>>>(L); }
-void launch_flux_i(const Lvl &L, bool fp32, cudaStream_t s) {
-  if (fp32) k_flux_i<float><<<L.nctiles, TILE, 0, s>>>(L);
-  else k_flux_i<double><<<L.nctiles, TILE, 0, s>>>(L);
+// f(std::integral_constant<bool, M>): with the level's kind of arithmetic
+template <typename Fn>
+static void by_kind(const Lvl &L, Fn f) {
+  if (L.mixed) f(std::true_type());
+  else f(std::false_type());
 }
-void launch_flux_j(const Lvl &L, bool fp32, cudaStream_t s) {
-  if (fp32) k_flux_j<float><<<L.nctiles, TILE, 0, s>>>(L);
-  else k_flux_j<double><<<L.nctiles, TILE, 0, s>>>(L);
+void launch_prim(const Lvl &L, cudaStream_t s) {
+  by_kind(L, [&](auto M) { k_prim<M.value><<<L.ntiles, TILE, 0, s>>>(L); });
 }
+template <bool IFACE>
+static void launch_flux(const Lvl &L, bool fp32, cudaStream_t s) {
+  if (fp32) k_flux<true, IFACE, float><<<L.nctiles, TILE, 0, s>>>(L);
+  else by_kind(L, [&](auto M) { k_flux<M.value, IFACE, double><<<L.nctiles, TILE, 0, s>>>(L); });
+}
+void launch_flux_i(const Lvl &L, bool fp32, cudaStream_t s) { launch_flux<true>(L, fp32, s); }
+void launch_flux_j(const Lvl &L, bool fp32, cudaStream_t s) { launch_flux<false>(L, fp32, s); }
 // with_norms: the tile partials inside k_res; with few cases the last CTA of
 // k_res also forms the per-case norms (norms_fused_final() tells the caller)
 bool norms_fused_final(const Lvl &L) { return L.ncase <= 8; }
 void launch_res(const Lvl &L, bool with_norms, int post, cudaStream_t s) {
-  if (!with_norms) k_res<false, false><<<L.nctiles, TILE, 0, s>>>(L, post);
-  else if (norms_fused_final(L)) k_res<true, true><<<L.nctiles, TILE, 0, s>>>(L, post);
-  else k_res<true, false><<<L.nctiles, TILE, 0, s>>>(L, post);
+  by_kind(L, [&](auto M) {
+    if (!with_norms) k_res<M.value, false, false><<<L.nctiles, TILE, 0, s>>>(L, post);
+    else if (norms_fused_final(L)) k_res<M.value, true, true><<<L.nctiles, TILE, 0, s>>>(L, post);
+    else k_res<M.value, true, false><<<L.nctiles, TILE, 0, s>>>(L, post);
+  });
 }
 // Lr: the level with npart, case_tile0, case_ntile and nctr of the 2-D tile list
 void launch_residual_tile(const Lvl &Lr, const int4 *rt, int ntiles, bool with_norms, int post, cudaStream_t s) {
-  if (!with_norms) k_residual_tile<false, false><<<ntiles, RNT, 0, s>>>(Lr, rt, post);
-  else if (norms_fused_final(Lr)) k_residual_tile<true, true><<<ntiles, RNT, 0, s>>>(Lr, rt, post);
-  else k_residual_tile<true, false><<<ntiles, RNT, 0, s>>>(Lr, rt, post);
+  by_kind(Lr, [&](auto M) {
+    if (!with_norms) k_residual_tile<M.value, false, false><<<ntiles, RNT, 0, s>>>(Lr, rt, post);
+    else if (norms_fused_final(Lr)) k_residual_tile<M.value, true, true><<<ntiles, RNT, 0, s>>>(Lr, rt, post);
+    else k_residual_tile<M.value, true, false><<<ntiles, RNT, 0, s>>>(Lr, rt, post);
+  });
 }
 void launch_norms(const Lvl &L, bool partials, cudaStream_t s) {
   if (partials) k_norm_partial<<<L.nctiles, TILE, 0, s>>>(L);

@@ -1,7 +1,8 @@
 // k_turb.cu -- turbulence-model residual rows (Spalart-Allmaras,
 // sub_turbulence_SA.f90; k-omega SST, sub_turbulence_SST.f90), the ghost
 // eddy viscosity at walls (Amut_boundary), the finite-difference WENO5 patch
-// (sub_Finite_Difference.f90) and the dual-time source term.
+// (sub_Finite_Difference.f90) and the dual-time source term.  Contexts with FP32
+// parts take the face and residual kernels of k_turb_mixed.cu.
 #include "ec2d_dev.cuh"
 #include "ec2d_internal.h"
 
@@ -76,13 +77,13 @@ __global__ void k_sa_faces(Lvl L) {
   const double *vt = L.U + 4 * F, *d = L.q + Q_D * F, *uu = L.q + Q_U * F, *vv = L.q + Q_V * F;
   const double *amu = L.amu;
   const double c0 = 0.5 * (1.0 + sa::Cb2) / sa::sigma;
-  const double nu = amu[id] * rcp(d[id]);
+  const double nu = amu[id] * recip(d[id]);
   if (i >= 1 && i <= b.nx && j >= 1 && j <= b.ny - 1) {
     long long w = id - 1, nN = id + P, nS = id - P;
     double s0 = L.geo[G_SI * F + id], n1 = L.geo[G_NI1 * F + id], n2 = L.geo[G_NI2 * F + id];
     double vn1 = uu[w] * n1 + vv[w] * n2, vn2 = uu[id] * n1 + vv[id] * n2;
     const double vf = fma(pos_part(vn1), vt[w], neg_part(vn2) * vt[id]) * s0;
-    const double v0 = c0 * ((vt[id] + nu) + fma(amu[w], rcp(d[w]), vt[w]));
+    const double v0 = c0 * ((vt[id] + nu) + fma(amu[w], recip(d[w]), vt[w]));
     // the normal derivative by the face's coefficients formed at set-up (k_face_metrics)
     const double *gm = L.geo + id;
     double Div = vt[id] - vt[w];
@@ -96,7 +97,7 @@ __global__ void k_sa_faces(Lvl L) {
     double s0 = L.geo[G_SJ * F + id], n1 = L.geo[G_NJ1 * F + id], n2 = L.geo[G_NJ2 * F + id];
     double vn1 = uu[s] * n1 + vv[s] * n2, vn2 = uu[id] * n1 + vv[id] * n2;
     const double vf = fma(pos_part(vn1), vt[s], neg_part(vn2) * vt[id]) * s0;
-    const double v0 = c0 * ((vt[id] + nu) + fma(amu[s], rcp(d[s]), vt[s]));
+    const double v0 = c0 * ((vt[id] + nu) + fma(amu[s], recip(d[s]), vt[s]));
     const double *gm = L.geo + id;
     double Div = (vt[s + 1] - vt[s - 1]) + (vt[id + 1] - vt[id - 1]);
     double Djv = vt[id] - vt[s];
@@ -111,7 +112,7 @@ __global__ void k_sa_faces(Lvl L) {
 // so the error stays below an ulp; 9 FP64 instructions against about 40 of
 // cbrt(sqrt(a / b)), which serves the rest of the range.
 __device__ __forceinline__ double sixth_root(double a, double ra, double b) {
-  if (!(at_least(b, 64.0) && below(b, 1.0e37))) return cbrt(sqrt(a * rcp(b)));
+  if (!(at_least(b, 64.0) && below(b, 1.0e37))) return cbrt(sqrt(a * recip(b)));
   const double q = b * ra, w = to_double(exp2f(log2f(to<float>(q)) * (-1.0f / 6.0f)));
   const double w2 = w * w, e = fma(-q, w2 * w2 * w2, 1.0);
   return fma(w, e * fma(e, 7.0 / 72.0, 1.0 / 6.0), w);
@@ -130,26 +131,26 @@ __global__ void k_sa_res(Lvl L) {
   long long id = fidx(b, i, j);
   const double *x1 = L.geo + G_X1 * F, *y1 = L.geo + G_Y1 * F, *uu = L.q + Q_U * F, *vv = L.q + Q_V * F;
   double vt = L.U[4 * F + id], d = L.q[Q_D * F + id], amu = L.amu[id];
-  const double ramu = rcp(amu);
-  double v0 = (vt + amu * rcp(d)) * (sa::Cb2 / sa::sigma);
+  const double ramu = recip(amu);
+  double v0 = (vt + amu * recip(d)) * (sa::Cb2 / sa::sigma);
   const double r = (L.fi[4 * F + id + 1] - L.fi[4 * F + id]) + (L.fj[4 * F + id + P] - L.fj[4 * F + id]) -
                    v0 * ((L.fi[5 * F + id + 1] - L.fi[5 * F + id]) + (L.fj[5 * F + id + P] - L.fj[5 * F + id]));
   // the halves of the central differences cancel in the quotients
   const double Dix = x1[id + 1] - x1[id - 1], Diy = y1[id + 1] - y1[id - 1];
   const double Djx = x1[id + P] - x1[id - P], Djy = y1[id + P] - y1[id - P];
-  const double Ds = rcp(Dix * Djy - Djx * Diy);
+  const double Ds = recip(Dix * Djy - Djx * Diy);
   const double Diu = uu[id + 1] - uu[id - 1], Div = vv[id + 1] - vv[id - 1];
   const double Dju = uu[id + P] - uu[id - P], Djv = vv[id + P] - vv[id - P];
   const double S = fabs(((Div * Djy - Djv * Diy) - (Dju * Dix - Diu * Djx)) * Ds);
   double dw = L.geo[G_DW * F + id];
   double X = d * vt * ramu;
   double X3 = X * X * X;
-  double fv1 = X3 * rcp(X3 + sa::Cv1 * sa::Cv1 * sa::Cv1);
-  double fv2 = 1.0 - X * rcp(1.0 + X * fv1);
+  double fv1 = X3 * recip(X3 + sa::Cv1 * sa::Cv1 * sa::Cv1);
+  double fv2 = 1.0 - X * recip(1.0 + X * fv1);
   double kd = sa::kap * dw;
-  const double rkd2 = rcp(kd * kd);  // 1 / (kappa d)^2
+  const double rkd2 = recip(kd * kd);  // 1 / (kappa d)^2
   double S1 = fmax(S + fv2 * vt * rkd2, (double)0.3f * S);  // 0.3 is a single-precision literal
-  double rr = fmin(vt * rcp(S1) * rkd2, 10.0);
+  double rr = fmin(vt * recip(S1) * rkd2, 10.0);
   double r2 = rr * rr, r6 = r2 * r2 * r2;
   double g = rr + sa::Cw2 * (r6 - rr);
   double g2 = g * g, g6 = g2 * g2 * g2;
@@ -158,7 +159,7 @@ __global__ void k_sa_res(Lvl L) {
   // exp(-X^2 / 2) is zero from X^2 = 1492 on, in most of a boundary layer
   const double X2 = X * X, ft2 = at_least(X2, 1492.0) ? 0.0 : sa::Ct3 * exp(-sa::Ct4 * X2);
   const double Cw1 = sa::Cb1 / (sa::kap * sa::kap) + (1.0 + sa::Cb2) / sa::sigma;
-  double q = vt * rcp(dw);
+  double q = vt * recip(dw);
   double Q = sa::Cb1 * (1.0 - ft2) * S1 * vt - (Cw1 * fw - sa::Cb1 * ft2 / (sa::kap * sa::kap)) * (q * q);
   L.res[4 * F + id] = r + Q * L.geo[G_VOL * F + id];
 }
@@ -166,6 +167,7 @@ __global__ void k_sa_res(Lvl L) {
 void launch_sa(const Lvl &L, cudaStream_t s) {
   k_sa_mut<<<L.ntiles, TILE, 0, s>>>(L);
   k_amut_boundary<<<L.nblk, 128, 0, s>>>(L);
+  if (L.mixed) { launch_sa_rows_mixed(L, s); return; }
   k_sa_faces<<<L.ntiles, TILE, 0, s>>>(L);
   k_sa_res<<<L.ntiles, TILE, 0, s>>>(L);
 }
@@ -195,7 +197,7 @@ __global__ void k_sst_cell(Lvl L) {
   long long id = fidx(b, i, j);
   const double *x1 = L.geo + G_X1 * F, *y1 = L.geo + G_Y1 * F, *uu = L.q + Q_U * F, *vv = L.q + Q_V * F;
   const double *d = L.q + Q_D * F, *U5 = L.U + 4 * F, *U6 = L.U + 5 * F;
-  const double dc = d[id], rd = rcp_any(dc), K = U5[id] * rd, W = U6[id] * rd;
+  const double dc = d[id], rd = recip_any(dc), K = U5[id] * rd, W = U6[id] * rd;
   // k and omega of every cell that a face reads
   L.tb[T_K * F + id] = K;
   L.tb[T_W * F + id] = W;
@@ -203,8 +205,8 @@ __global__ void k_sst_cell(Lvl L) {
   // central differences (their halves cancel in the quotients)
   const double Dix = x1[id + 1] - x1[id - 1], Diy = y1[id + 1] - y1[id - 1];
   const double Djx = x1[id + P] - x1[id - P], Djy = y1[id + P] - y1[id - P];
-  const double Ds = rcp(Dix * Djy - Djx * Diy);
-  const double re = rcp_any(d[id + 1]), rw = rcp_any(d[id - 1]), rn = rcp_any(d[id + P]), rs = rcp_any(d[id - P]);
+  const double Ds = recip(Dix * Djy - Djx * Diy);
+  const double re = recip_any(d[id + 1]), rw = recip_any(d[id - 1]), rn = recip_any(d[id + P]), rs = recip_any(d[id - P]);
   const double Diu = uu[id + 1] - uu[id - 1], Div = vv[id + 1] - vv[id - 1];
   const double Dju = uu[id + P] - uu[id - P], Djv = vv[id + P] - vv[id - P];
   const double Dik = U5[id + 1] * re - U5[id - 1] * rw, Diw = U6[id + 1] * re - U6[id - 1] * rw;
@@ -213,18 +215,18 @@ __global__ void k_sst_cell(Lvl L) {
   const double kx = Dik * Djy - Djk * Diy, wx = Diw * Djy - Djw * Diy;
   const double ky = Djk * Dix - Dik * Djx, wy = Djw * Dix - Diw * Djx;
   const double rRe = c.rRe, amu = L.amu[id], amus = amu * Re;
-  const double dw = L.geo[G_DW * F + id], rdw = rcp_any(dw), rW = rcp_any(W);
+  const double dw = L.geo[G_DW * F + id], rdw = recip_any(dw), rW = recip_any(W);
   const double c009 = (double)0.09f;  // single-precision literal (sub_turbulence_SST.f90:87,96)
   const double t2 = 500.0 * amu * rRe * rd * rW * (rdw * rdw);
-  const double kw = sqrt_p(fabs(K)) * rW * rdw * rcp(c009 * Re);
+  const double kw = root(fabs(K)) * rW * rdw * recip(c009 * Re);
   const double arg2 = fmax(pow2<1>(kw), t2);
   const double f2 = tanh(arg2 * arg2);
   const double dK = dc * K;
-  double amuts = fmin(fmin(dK * rW, sst::a1 * dK * Re * rcp_any(f2 * fabs(omega))), 100000.0);
-  const double Kws = (kx * wx + ky * wy) * (Ds * Ds) * dc * (2.0 * sst::sw2) * rcp_any(W + 1.0e-20);
+  double amuts = fmin(fmin(dK * rW, sst::a1 * dK * Re * recip_any(f2 * fabs(omega))), 100000.0);
+  const double Kws = (kx * wx + ky * wy) * (Ds * Ds) * dc * (2.0 * sst::sw2) * recip_any(W + 1.0e-20);
   const double CD = fmax(Kws, 1.0e-20);
   const double arg3 = fmax(kw, t2);
-  const double arg1 = fmin(arg3, 4.0 * sst::sw2 * dK * rcp_any(CD * (dw * dw)));
+  const double arg1 = fmin(arg3, 4.0 * sst::sw2 * dK * recip_any(CD * (dw * dw)));
   double a1s = arg1 * arg1;
   double f1 = tanh(a1s * a1s);
   const double om2 = omega * omega, g1 = 1.0 - f1;
@@ -306,9 +308,13 @@ __global__ void k_sst_res(Lvl L) {
 }
 
 void launch_sst(const Lvl &L, cudaStream_t s) {
-  k_sst_cell<<<L.ntiles, TILE, 0, s>>>(L);
-  k_sst_faces<<<L.ntiles, TILE, 0, s>>>(L);
-  k_sst_res<<<L.ntiles, TILE, 0, s>>>(L);
+  if (L.mixed) {
+    launch_sst_rows_mixed(L, s);
+  } else {
+    k_sst_cell<<<L.ntiles, TILE, 0, s>>>(L);
+    k_sst_faces<<<L.ntiles, TILE, 0, s>>>(L);
+    k_sst_res<<<L.ntiles, TILE, 0, s>>>(L);
+  }
   k_amut_boundary<<<L.nblk, 128, 0, s>>>(L);
 }
 
@@ -322,7 +328,7 @@ enum { D_SPI = 0, D_SPJ = 8, D_FI = 16, D_FJ = 20, D_EV1 = 24, D_EV2 = 27 };
 // and E - E+ are selects.
 __device__ __forceinline__ void split_sw(double d, double u, double v, double cc, double A1, double A2,
                                          const CaseDev &c, double *fp, double *fm) {
-  const double w = fma(A1, A1, A2 * A2), rss = rsqrt_d(w), cs = cc * (w * rss);
+  const double w = fma(A1, A1, A2 * A2), rss = rroot(w), cs = cc * (w * rss);
   const double c1 = cc * (A1 * rss), c2 = cc * (A2 * rss);
   const double t0 = half(d * c.rg), E1 = A1 * u + A2 * v, E2 = E1 - cs, E3 = E1 + cs;
   const double e1 = E1 * (t0 * pow2<1>(c.gm1)), e2 = E2 * t0, e3 = E3 * t0;
@@ -352,7 +358,7 @@ __global__ void k_fdm_split(Lvl L) {
   const long long F = L.F;
   long long id = fidx(b, i, j);
   double d = L.q[Q_D * F + id], u = L.q[Q_U * F + id], v = L.q[Q_V * F + id], cc = L.q[Q_C * F + id];
-  const double rJ = rcp(L.met[M_JAC * F + id]);
+  const double rJ = recip(L.met[M_JAC * F + id]);
   double fp[4], fm[4];
   // blockIdx.y: 0 the i-direction split, 1 the j-direction split (two threads per cell)
   const int dir = blockIdx.y;
@@ -385,7 +391,7 @@ __device__ __forceinline__ double weno5(double a, double b, double c, double d, 
   D2 *= 3.0 * D2;
   const double E0 = pow2<1>(D0), q = D0 * D1, sixth = 1.0 / 6.0;
   const double h = half(d3), p0 = fma(-sixth, s3, h), p1 = fma(-sixth, s2, h), p2 = fma(2.0 * sixth, s1, half(d2));
-  return fma(fma(D2, fma(D1, p0, E0 * p1), q * p2), rcp(fma(D2, D1 + E0, q)), c);
+  return fma(fma(D2, fma(D1, p0, E0 * p1), q * p2), recip(fma(D2, D1 + E0, q)), c);
 }
 
 // WENO5 half-point fluxes (sub_Finite_Difference.f90:37-77) and the central
@@ -426,7 +432,7 @@ __global__ void k_fdm_flux(Lvl L) {
     double ui = half(uu[id + 1] - uu[id - 1]), vi = half(vv[id + 1] - vv[id - 1]), Ti = half(TT[id + 1] - TT[id - 1]);
     double uj = half(uu[id + P] - uu[id - P]), vj = half(vv[id + P] - vv[id - P]), Tj = half(TT[id + P] - TT[id - P]);
     double Akx = L.met[M_KX * F + id], Aky = L.met[M_KY * F + id], Aix = L.met[M_IX * F + id], Aiy = L.met[M_IY * F + id];
-    const double rJ = rcp(L.met[M_JAC * F + id]);
+    const double rJ = recip(L.met[M_JAC * F + id]);
     double ux = ui * Akx + uj * Aix, vx = vi * Akx + vj * Aix, Tx = Ti * Akx + Tj * Aix;
     double uy = ui * Aky + uj * Aiy, vy = vi * Aky + vj * Aiy, Ty = Ti * Aky + Tj * Aiy;
     double t11 = (4.0 / 3.0 * ux - 2.0 / 3.0 * vy) * mu0, t22 = (4.0 / 3.0 * vy - 2.0 / 3.0 * ux) * mu0;
@@ -463,6 +469,7 @@ __global__ void k_fdm_res(Lvl L) {
 }
 
 void launch_fdm(const Lvl &L, cudaStream_t s) {
+  if (L.mixed) { launch_fdm_mixed(L, s); return; }
   k_fdm_split<<<dim3(L.ntiles, 2), TILE, 0, s>>>(L);
   k_fdm_flux<<<dim3(L.ntiles, L.visc ? 3 : 2), TILE, 0, s>>>(L);
   k_fdm_res<<<L.ntiles, TILE, 0, s>>>(L);
