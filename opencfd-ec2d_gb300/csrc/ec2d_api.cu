@@ -613,8 +613,8 @@ void K(ec2d_ctx *ctx, const char *name, int level, int nk, Fn fn) {
 
 // Comput_Residual_one_mesh (sub_Residual.f90:13-107) for all blocks of a level
 // post: RES_ADD_FORCE / RES_FORCE_FN / RES_SET_UN steps that follow the
-// residual in the caller's sequence, done inside k_res when the norms are
-// final there, as separate kernels otherwise
+// residual in the caller's sequence, done inside k_res when it takes the norm
+// partials, as separate kernels otherwise
 // the coarse levels of a turbulent multigrid run keep the eddy viscosity
 // restricted from the finer level instead of zero
 static void apply_mg_amut(ec2d_ctx *ctx) {
@@ -647,20 +647,15 @@ void residual(ec2d_ctx *ctx, int l, int post = 0) {
   const bool dual = ctx->P.Time_Method == Time_Dual && l == 1;
   const bool f32 = ctx->coarse_fp32 && l >= 2;
   if (ctx->tile_residual && lv.n_rtiles > 0 && L.turb == Turb_NONE && !L.fdm && !L.keep_amut && !dual && !f32) {
-    // the whole residual in one kernel over 2-D tiles (norm partials inside;
-    // with few cases the per-case norms and the multigrid post-steps too)
+    // the whole residual in one kernel over 2-D tiles (norm partials and the multigrid
+    // post-steps inside; with few cases of few tiles the per-case norms too)
     Lvl Lr = L;
     Lr.npart = lv.d_rnpart;
     Lr.case_tile0 = lv.d_rcase_tile0;
     Lr.case_ntile = lv.d_rcase_ntile;
     Lr.nctr = lv.d_rnctr;
-    const int inpass = norms_fused_final(L) ? post : 0;
-    K(ctx, "k_residual_tile", l, 1, [&] { launch_residual_tile(Lr, lv.d_rtiles, lv.n_rtiles, true, inpass, s); });
+    K(ctx, "k_residual_tile", l, 1, [&] { launch_residual_tile(Lr, lv.d_rtiles, lv.n_rtiles, true, post, s); });
     if (!norms_fused_final(L)) K(ctx, "norms", l, 1, [&] { launch_norms(Lr, false, s); });
-    const int rest = post & ~inpass;
-    if (rest & RES_ADD_FORCE) K(ctx, "k_add_force", l, 1, [&] { launch_add_force(L, s); });
-    if (rest & RES_FORCE_FN) K(ctx, "k_force_fn", l, 1, [&] { launch_force_fn(L, s); });
-    if (rest & RES_SET_UN) K(ctx, "k_set_un", l, 1, [&] { launch_set_un(L, 4, s); });
     return;
   }
   K(ctx, "k_prim", l, 1, [&] { launch_prim(L, s); });
@@ -687,24 +682,25 @@ void residual(ec2d_ctx *ctx, int l, int post = 0) {
     K(ctx, "k_flux_j", l, 1, [&] { launch_flux_j(L, f32, s); });
   }
   const bool fused = !L.fdm && !dual;  // Res final after k_res: norm partials fused into it
-  // Within a step the norms of an evaluation whose Res stays as k_res
-  // leaves it (no forcing added) go to the norms branch: the kernels that
-  // follow only read Res, and the norms are read after the step.  k_res without
-  // them is about half as long (7 against 14 us per launch on the flat
-  // plate's levels); the partials and the reduction are the same kernels
-  // as for the FDM patch, so the norms are bit-identical either way.
-  if (fused && ctx->norm_branch && ctx->concurrent && !ctx->timing && !(post & RES_ADD_FORCE) &&
-      norms_fused_final(L)) {
-    K(ctx, "k_res", l, 1, [&] { launch_res(L, false, post, s); });
-    ctx->launches += 2;
+  // Within a step the norms of an evaluation go to the norms branch: the
+  // kernels that follow do not need them, and they are read after the step.
+  // Where Res stays as k_res leaves it (no forcing added) and the last CTA would
+  // form the norms, k_res goes without them, about half as long (7 against
+  // 14 us per launch on the flat plate's levels); where k_res only takes the partials,
+  // the reduction alone is on the branch.  The reduction order is the same
+  // either way, so the norms are bit-identical.
+  const bool final_in = norms_fused_final(L);
+  if (fused && ctx->norm_branch && ctx->concurrent && !ctx->timing && !(final_in && (post & RES_ADD_FORCE))) {
+    K(ctx, "k_res", l, 1, [&] { launch_res(L, !final_in, post, s); });
+    ctx->launches += final_in ? 2 : 1;
     cudaEventRecord(ctx->ev_nfork[l], s);
     cudaStreamWaitEvent(ctx->nstream, ctx->ev_nfork[l], 0);
-    launch_norms(L, true, ctx->nstream);
+    launch_norms(L, final_in, ctx->nstream);
     cudaEventRecord(ctx->ev_norm[l], ctx->nstream);
     ctx->norm_open[l] = true;
     return;
   }
-  const int inpass = (fused && norms_fused_final(L)) ? post : 0;
+  const int inpass = fused ? post : 0;  // the partial norms are taken of Res before the forcing
   K(ctx, "k_res", l, 1, [&] { launch_res(L, fused, inpass, s); });
   if (L.fdm) K(ctx, "fdm", l, 3, [&] { launch_fdm(L, s); });
   if (dual) {

@@ -652,10 +652,37 @@ __global__ void __launch_bounds__(TILE) k_norm_partial(Lvl L) {
   tile_partials(L, act, vres);
 }
 
-// per-case reduction of the tile partials (one warp per case and quantity)
-__global__ void __launch_bounds__(384) k_norm_final(Lvl L) {
-  const int k = blockIdx.x * 12 + (threadIdx.x >> 5);
-  final_norm(L, k / 12, k % 12);
+// per-case reduction of the tile partials, one CTA per case and quantity: a thread
+// takes one of the 128 partial results that a warp of final_norm keeps, in the same order
+__global__ void __launch_bounds__(128) k_norm_final(Lvl L) {
+  __shared__ double acc[128];
+  const int cs = blockIdx.x / 12, m = blockIdx.x % 12, nt = L.case_ntile[cs];
+  const double *p = L.npart + (size_t)L.case_tile0[cs] * 12 + m;
+  if (m < 6) {
+    long long a = 0;
+#pragma unroll 8
+    for (int t = threadIdx.x; t < nt; t += 128) a = max(a, __double_as_longlong(p[(size_t)t * 12]));
+    acc[threadIdx.x] = __longlong_as_double(a);
+  } else {
+    double q = 0.0;
+#pragma unroll 8
+    for (int t = threadIdx.x; t < nt; t += 128) q += p[(size_t)t * 12];
+    acc[threadIdx.x] = q;
+  }
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  const double *r = acc + threadIdx.x;
+  double out;
+  if (m < 6) {
+    long long b = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) b = max(b, __double_as_longlong(r[32 * k]));
+    out = __longlong_as_double(warp_max_bits(b));
+  } else {
+    const double s = warp_sum((r[0] + r[32]) + (r[64] + r[96]));
+    out = (m - 6 < L.nvar) ? sqrt(s / (1.0 * L.case_ncell[cs])) : 0.0;
+  }
+  if (threadIdx.x == 0) L.norms[cs * 12 + m] = out;
 }
 
 // set-up, and when a context gets or loses its FP32 parts: the viscous metric
@@ -731,9 +758,12 @@ static void launch_flux(const Lvl &L, bool fp32, cudaStream_t s) {
 }
 void launch_flux_i(const Lvl &L, bool fp32, cudaStream_t s) { launch_flux<true>(L, fp32, s); }
 void launch_flux_j(const Lvl &L, bool fp32, cudaStream_t s) { launch_flux<false>(L, fp32, s); }
-// with_norms: the tile partials inside k_res; with few cases the last CTA of
-// k_res also forms the per-case norms (norms_fused_final() tells the caller)
-bool norms_fused_final(const Lvl &L) { return L.ncase <= 8; }
+// with_norms: the tile partials inside k_res; with few cases of few tiles the last CTA of
+// k_res also forms the per-case norms (norms_fused_final() tells the caller).  A warp of
+// that CTA takes three quantities of a case, a round of loads per 128 tiles each, while the rest
+// of the chip stands idle: 2 us at 144 tiles, 70 us at the 8242 tiles of 1.05 M cells, where
+// a CTA per quantity (k_norm_final) takes 5 us; they cross near 1000 tiles.
+bool norms_fused_final(const Lvl &L) { return L.ncase <= 8 && L.nctiles <= 1024; }
 void launch_res(const Lvl &L, bool with_norms, int post, cudaStream_t s) {
   by_kind(L, [&](auto M) {
     if (!with_norms) k_res<M.value, false, false><<<L.nctiles, TILE, 0, s>>>(L, post);
@@ -751,7 +781,7 @@ void launch_residual_tile(const Lvl &Lr, const int4 *rt, int ntiles, bool with_n
 }
 void launch_norms(const Lvl &L, bool partials, cudaStream_t s) {
   if (partials) k_norm_partial<<<L.nctiles, TILE, 0, s>>>(L);
-  k_norm_final<<<L.ncase, 384, 0, s>>>(L);
+  k_norm_final<<<L.ncase * 12, 128, 0, s>>>(L);
 }
 
 }  // namespace ec2d
