@@ -2256,15 +2256,7 @@ int ec2d_mlp_predict(ec2d_mlp *m, const float *feat, long long n, float *pred) {
   if (!m || !feat || !pred || n < 1) return EC2D_ERR_ARG;
   Net &net = m->net;
   cudaSetDevice(net.device);
-  float *df = nullptr, *dp = nullptr;
-  CK(cudaMalloc(&df, (size_t)n * NIN * sizeof(float)));
-  CK(cudaMalloc(&dp, (size_t)n * NOUT * sizeof(float)));
-  CK(cudaMemcpy(df, feat, (size_t)n * NIN * sizeof(float), cudaMemcpyHostToDevice));
-  int r = net.predict(df, n, dp);
-  cudaStreamSynchronize(net.stream);
-  if (r == 0) cudaMemcpy(pred, dp, (size_t)n * NOUT * sizeof(float), cudaMemcpyDeviceToHost);
-  cudaFree(df);
-  cudaFree(dp);
+  const int r = net.predict_host(feat, n, pred);
   if (r) return EC2D_ERR_CUDA;
   return net.check_err() ? EC2D_ERR_TIMEOUT : EC2D_OK;
 }

@@ -3,6 +3,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <mutex>
 #include <vector>
 
 namespace ec2d {
@@ -88,6 +89,8 @@ struct Layer {
   __nv_bfloat16 *wk = nullptr, *wtk = nullptr;  // packed for the fused kernels (width 256)
 };
 
+constexpr int HOST_SLOTS = 4;  // chunks of a host prediction on the device
+
 struct Net {
   int device = 0, width = 256, nlin = 7;
   unsigned long long seed = 0;
@@ -111,6 +114,13 @@ struct Net {
   int cap_fused = 0, fpart_ks = 0;
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // predictions for host rows: a ring of chunks on the device, kept with the net (at
+  // most HOST_SLOTS chunks, 15 MB); one call at a time uses it
+  std::mutex host_mu;
+  float *host_in = nullptr, *host_out = nullptr;
+  long long host_cap = 0;  // rows of the ring
+  cudaStream_t copy = nullptr;
+  cudaEvent_t ev_in[HOST_SLOTS] = {}, ev_out[HOST_SLOTS] = {};
   // samples (device): features n x NIN, targets n x NOUT
   float *feat = nullptr, *targ = nullptr;
   long long nsamp = 0, cap_samp = 0;
@@ -140,6 +150,7 @@ struct Net {
   int fit_normalization();
   int reserve_samples(long long n);
   int predict(const float *feat, long long n, float *pred);
+  int predict_host(const float *feat, long long n, float *pred);  // rows in host memory
   int check_err();  // 0, or 1 if a tcgen05 wait timed out since the last call
 };
 
