@@ -781,7 +781,7 @@ int Net::predict(const float *f, long long n, float *pred) {
 // host until they are done, so they have a stream of their own; while the first
 // chunks are computed the host touches the pages that the results will go to (for a
 // buffer fresh from the allocator that is most of a copy's time).  300007 rows: 918 us
-// with two allocations and plain copies around one launch, PREDICT_FIGS this way.
+// with two allocations and plain copies around one launch, 637 us this way.
 int Net::predict_host(const float *f, long long n, float *pred) {
   std::lock_guard<std::mutex> lock(host_mu);
   const long long CH = fused() ? 152 * 128 * 4 : 4 * 16384;

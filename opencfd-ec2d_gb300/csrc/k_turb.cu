@@ -370,22 +370,22 @@ __global__ void k_fdm_split(Lvl L) {
 // fp_weno5 at point k from v[k-2..k+2] = a, b, c, d, e; fm_weno5 is the same with the
 // points in reverse (sub_Finite_Difference.f90:207-275).  The reference forms the
 // weights as a_k = C_k / (ep + S_k)^2 and W_k = a_k / sum(a); over the common
-// denominator D_0 D_1 D_2 (D_k = (ep + S_k)^2, here of 12/13 of both) they are
+// denominator D_0 D_1 D_2 (D_k = (ep + S_k)^2) they are
 // W_0 : W_1 : W_2 = 3 D_1 D_2 : 6 D_0 D_2 : D_0 D_1.  Smoothness indicators and
 // candidate values are written in the first and second differences of v,
-//   S_0: s3, s3 - 2 d3;  S_1: s2, d2 + d3;  S_2: s1, s1 + 2 d2,
+//   S_0 = d3^2 + s3 (4/3 s3 - d3),  S_1 = d3^2 + s2 (4/3 s2 - d3),  S_2 = d2^2 + s1 (4/3 s1 + d2),
 //   q_0 - c = d3/2 - s3/6,  q_1 - c = d3/2 - s2/6,  q_2 - c = d2/2 + s1/3,
-// 36 FP64 instructions per value; written out from the five values with an IEEE
+// 32 FP64 instructions per value; written out from the five values with an IEEE
 // divide it took 60, and the 65 k cells of a 513 x 129 block took 203 us with
 // split and residual, three launches (125 us now).  D_k >= 1e-12, so numerator and denominator stay above
 // 1e-36, and they overflow only for smoothness indicators beyond about 1e50, far
 // from any split flux of this solver.
 __device__ __forceinline__ double weno5(double a, double b, double c, double d, double e) {
-  const double ep = 1.0e-6 * 12.0 / 13.0, t = 3.0 / 13.0;
+  const double ep = 1.0e-6, t = 4.0 / 3.0;
   const double d1 = b - a, d2 = c - b, d3 = d - c, d4 = e - d;
   const double s1 = d2 - d1, s2 = d3 - d2, s3 = d4 - d3;
-  const double y0 = fma(-2.0, d3, s3), y1 = d2 + d3, y2 = fma(2.0, d2, s1);
-  double D0 = fma(t * y0, y0, fma(s3, s3, ep)), D1 = fma(t * y1, y1, fma(s2, s2, ep)), D2 = fma(t * y2, y2, fma(s1, s1, ep));
+  const double c3 = fma(d3, d3, ep), c2 = fma(d2, d2, ep);
+  double D0 = fma(s3, fma(t, s3, -d3), c3), D1 = fma(s2, fma(t, s2, -d3), c3), D2 = fma(s1, fma(t, s1, d2), c2);
   D0 *= D0;
   D1 *= D1;
   D2 *= 3.0 * D2;
