@@ -88,20 +88,22 @@ int push_record(int nv) { return (4 * HREC + (nv > 4 ? 2 * TREC : 0) + UREC + 1)
 
 template <int NV>
 __device__ __forceinline__ void face_term(const double *U, double n1, double n2, double cc, double gm1, double *K) {
-  const double r = rcp(U[0]);
+  const double r = recip(U[0]);
   const double un = (U[1] * n1 + U[2] * n2) * r;
-  const double p = gm1 * (U[3] - 0.5 * (U[1] * U[1] + U[2] * U[2]) * r);
+  const double p = gm1 * fma(-half(fma(U[1], U[1], U[2] * U[2])), r, U[3]);
   const double w = un + cc;
-  K[0] -= U[0] * w;
-  K[1] -= fma(U[1], w, p * n1);
-  K[2] -= fma(U[2], w, p * n2);
-  K[3] -= fma(U[3], w, p * un);
+  K[0] = fma(-U[0], w, K[0]);
+  K[1] = fma(-U[1], w, fma(-p, n1, K[1]));
+  K[2] = fma(-U[2], w, fma(-p, n2, K[2]));
+  K[3] = fma(-U[3], w, fma(-p, un, K[3]));
 #pragma unroll
-  for (int m = 4; m < NV; m++) K[m] -= U[m] * un;
+  for (int m = 4; m < NV; m++) K[m] = fma(-U[m], un, K[m]);
 }
 
 // the records of both passes, all cells at once (force: Res + QF in place of
-// Res, see k_lusgs_prep)
+// Res, see k_lusgs_prep).  Bound by FP64 issue on large levels (65 k cells 29 us) and by one
+// cell's chain on small ones: some 95 instructions per cell at NV = 4, 125 with
+// third-order reciprocals, halves by multiplication and sums not folded into FMAs.
 template <int NV, bool update>
 __global__ void __launch_bounds__(TILE) k_push_prep(Lvl L, double alfa1, int force) {
   int bk, i, j;
@@ -111,15 +113,15 @@ __global__ void __launch_bounds__(TILE) k_push_prep(Lvl L, double alfa1, int for
   const CaseDev &c = L.cs[b.cas];
   const long long F = L.F, P = b.P;
   const long long id = fidx(b, i, j);
-  const double gm1 = c.gamma - 1.0, hg = 0.5 * gm1;
+  const double gm1 = c.gm1, hg = half(gm1);
   const double *g = L.geo, *lc = L.lc;
   const bool visc = L.visc != 0;
   const size_t cell = (size_t)b.cell0 + (size_t)(j - 1) * (b.nx - 1) + (i - 1);
   const double vol = g[G_VOL * F + id];
   const double Lv = lc[L_VI * F + id] + lc[L_VJ * F + id];
-  double alfa = vol * rcp(lc[L_DT * F + id]) + 1.0 * (lc[L_CI * F + id] + lc[L_CJ * F + id]) + vol * alfa1;
-  if (visc) alfa += 2.0 * Lv;
-  const double ia = rcp(alfa);
+  double alfa = fma(vol, recip(lc[L_DT * F + id]), fma(vol, alfa1, lc[L_CI * F + id] + lc[L_CJ * F + id]));
+  if (visc) alfa += pow2<1>(Lv);
+  const double ia = recip(alfa);
   const double ni1 = g[G_NI1 * F + id], ni2 = g[G_NI2 * F + id], nj1 = g[G_NJ1 * F + id], nj2 = g[G_NJ2 * F + id];
   double u[NV], res[NV];
 #pragma unroll
@@ -145,13 +147,13 @@ __global__ void __launch_bounds__(TILE) k_push_prep(Lvl L, double alfa1, int for
         double Un[NV];
 #pragma unroll
         for (int m = 0; m < NV; m++) Un[m] = L.U[m * F + nb];
-        cc = 0.5 * lc[(dir == 0 ? L_CI : L_CJ) * F + nb];
+        cc = half(lc[(dir == 0 ? L_CI : L_CJ) * F + nb]);
         if (visc) cc += lc[(dir == 0 ? L_VI : L_VJ) * F + nb];
         cc *= ia;
         // forward: +0.5 s of this cell's face; backward: -0.5 s of the
         // neighbour's face with this cell's normal (the reference pairs the
         // normal of face i with the length of face i+1, sub_LU_SGS.f90:87-88,95-96)
-        const double hh = (fwd ? 0.5 : -0.5) * g[(dir == 0 ? G_SI : G_SJ) * F + (fwd ? id : nb)] * ia;
+        const double h2 = half(g[(dir == 0 ? G_SI : G_SJ) * F + (fwd ? id : nb)]), hh = (fwd ? h2 : -h2) * ia;
         s1 = hh * (dir == 0 ? ni1 : nj1);
         s2 = hh * (dir == 0 ? ni2 : nj2);
         face_term<NV>(Un, s1, s2, cc, gm1, K);
@@ -180,7 +182,7 @@ __global__ void __launch_bounds__(TILE) k_push_prep(Lvl L, double alfa1, int for
       w[T_AT / 2] = make_double2(at(4 < NV ? 4 : 0), at(m5));
       w[T_UT / 2] = make_double2(u[4 < NV ? 4 : 0], u[m5]);
       w[T_DT / 2] = make_double2(0.0, 0.0);
-      w[T_RT / 2] = make_double2(NV == 5 ? alfa * rcp(alfa + Lv) : 0.0, 0.0);
+      w[T_RT / 2] = make_double2(NV == 5 ? alfa * recip(alfa + Lv) : 0.0, 0.0);
     }
   }
   if (!update) {
