@@ -187,10 +187,10 @@ __device__ __forceinline__ float sqrt_p<float>(float x) { return sqrtf(x); }
 // one FP64 warp instruction per 16 to 19 cycles, and each holds its sub-partition
 // for 64, while that sub-partition could issue an integer or FP32 instruction
 // every cycle: whatever needs no FP64 pipe is done beside it.
-//   * reciprocals and reciprocal square roots start from 44-bit values formed in
-//     FP32 and integers (rcp_seed, rsqrt_seed) and need one step, two and three FP64
-//     instructions (a divide takes about nine, the hardware's 20-bit
-//     approximation with a third-order step three and five);
+//   * reciprocals are formed in FP32 and integers altogether, roots and quotients start
+//     from 44-bit values formed there and need three FP64 instructions (a divide
+//     takes about nine, the hardware's 20-bit approximation with a third-order step
+//     three for a reciprocal and five for a root);
 //   * negation, powers of two and comparisons are integer operations.
 // x 2^K, K in -3..1: exact; zeros, infinities and NaNs stay what they are, and so
 // do values below 2^-1019
@@ -244,11 +244,15 @@ __device__ __forceinline__ bool above(double x, double y) {
   return i > __double_as_longlong(y) && i <= 0x7ff0000000000000ll;
 }
 
-// 1/x to about 44 bits: x's mantissa as a float and the float of its remaining
-// bits, the FP32 approximate reciprocal r of the first, and the correction
-// r (e + e^2), e = 1 - x r, added to r's double as an integer.  NaN for zero,
-// subnormal, infinite or NaN x and from 2^1022.
-__device__ __forceinline__ double rcp_seed(double x) {
+// 1/x without the FP64 pipe.  In FP32: x's mantissa as a float and the float of its
+// remaining bits, the approximate reciprocal r of the first, and the correction r
+// (e + e^2), e = 1 - x r, added to r's double as an integer: 44 bits (FULL = false).
+// Then a Newton step in integers: with the mantissas as 53-bit integers X and R the
+// remainder 2^105 - X R is below 2^62, so it is known from the product modulo 2^64, and R
+// times it, shifted, is added: half an ulp and 2^-18 more.  NaN for zero, subnormal,
+// infinite or NaN x and from 2^1022.
+template <bool FULL>
+__device__ __forceinline__ double reciprocal(double x) {
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
   const float xf = __uint_as_float((__funnelshift_l(lo, hi, 3) & 0x7fffffu) | 0x3f800000u);
   const float xl = fmaf(__uint_as_float(((lo >> 6) & 0x7fffffu) | 0x3f800000u), 0x1p-23f, -0x1p-23f);
@@ -258,11 +262,19 @@ __device__ __forceinline__ double rcp_seed(double x) {
   // the correction in units of 2^-52 (the double's are 2^-53 below 1)
   const int q = __float2int_rn(r * 0x1p52f * fmaf(e, e, e));
   const unsigned rb = __float_as_uint(r), ex = hi & 0x7ff00000u;
-  const unsigned long long y = (((unsigned long long)(rb >> 3) << 32) | (rb << 29)) + (unsigned long long)(2ll * q);
+  unsigned long long y = (((unsigned long long)(rb >> 3) << 32) | (rb << 29)) + (unsigned long long)(2ll * q);
+  if (FULL) {
+    const unsigned Rl = (unsigned)y, Rh = (unsigned)(y >> 32) - (125u << 20);  // 2^53 r
+    const unsigned Xh = (hi & 0xfffffu) | 0x100000u;                           // 2^52 x
+    const unsigned ph = __umulhi(lo, Rl) + lo * Rh + Xh * Rl;  // bits 32 to 63 of X R
+    const int c = (__mulhi((int)~ph, (int)__funnelshift_l(Rl, Rh, 9)) + (1 << 17)) >> 18;
+    y += (unsigned long long)(long long)c;
+  }
   const unsigned yh = (unsigned)(y >> 32) + ((1023u - 127u) << 20) + (0x3ff00000u - ex);
   return __hiloint2double(ex - 0x00100000u < 0x7fc00000u ? (int)(yh | (hi & 0x80000000u)) : 0x7ff80000,
                           (int)(unsigned)y);
 }
+__device__ __forceinline__ double rcp_seed(double x) { return reciprocal<false>(x); }
 // 1/sqrt(x) to about 44 bits the same way: the exponent made even, r the FP32
 // approximate reciprocal root, the correction r e (1/2 + 3/8 e), e = 1 - x r^2.
 // NaN for negative, infinite or NaN x; for zero (and subnormal x) NaN or, ZERO, 1,
@@ -288,11 +300,7 @@ __device__ __forceinline__ double rsqrt_seed(double x) {
   return __hiloint2double(hi - 0x00100000u < 0x7fe00000u ? (int)yh : out, (int)(unsigned)y);
 }
 
-// 1/x: the rounded quotient in all of 8e8 samples
-__device__ __forceinline__ double recip(double x) {
-  const double r = rcp_seed(x);
-  return fma(r, fma(-x, r, 1.0), r);
-}
+__device__ __forceinline__ double recip(double x) { return reciprocal<true>(x); }
 // 1/x where x may be zero or infinite: by the divide there
 __device__ __forceinline__ double recip_any(double x) {
   return ((unsigned)__double2hiint(x) & 0x7ff00000u) - 0x00100000u < 0x7fc00000u ? recip(x) : 1.0 / x;

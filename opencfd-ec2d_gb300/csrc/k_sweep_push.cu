@@ -9,7 +9,7 @@
 // one (a shuffle, a select) and back costs about 50 more than that pipe's own
 // latency (measured).  So the FP64 instructions and the crossings per cell
 // set the time, and everything else has to fit in their shadow.  What keeps
-// them few (4 variables: 8 FP64 instructions and 3 crossings; 15 and 5 when a
+// them few (4 variables: 6 FP64 instructions and 3 crossings; 15 and 5 when a
 // cell pulled its neighbours' states):
 //  * the records hold the face normals, dissipation coefficients and constant
 //    terms already multiplied by 1/alfa of the cell that receives the term,
@@ -23,8 +23,8 @@
 //    2 p / (gamma - 1), and its term of variable q is s_q w + p' g_q with g =
 //    (0, n1, n2, u_n) (gamma - 1) / 2: (rho, rho u, rho v, E) w plus the
 //    pressure terms of F_n;
-//  * 1/rho starts from a 44-bit value formed on the integer and FP32 pipes
-//    while the FP64 pipe forms m (rcp_seed), so one Newton step is enough.
+//  * 1/rho is formed on the integer and FP32 pipes while the FP64 pipe forms m
+//    (recip).
 // The first half row (lanes 0-3) serves the next cell of the own row: its
 // accumulator starts from that cell's constant term and stays in the lane.
 // The second half serves the same column of the next row: its four sums move
@@ -476,7 +476,7 @@ __device__ __forceinline__ void push_pass(const Lvl &L, const BlkDev &bd, PWarp 
     const double a1 = is_p ? neg(v1) : cur.n.x, a2 = is_p ? neg(v2) : cur.n.y;
     const double kz = is_p ? twice(v3) : cur.c;
     const double m = fma(v1, a1, v2 * a2);
-    const double r0 = rcp_seed(v0), rd = fma(r0, fma(-v0, r0, 1.0), r0);
+    const double rd = recip(v0);
     // the next step's fields and this step's results, in the shadow of the
     // longest stretch of FP64 instructions
     load(next, t + 1);
