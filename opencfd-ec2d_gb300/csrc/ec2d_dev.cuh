@@ -188,7 +188,7 @@ __device__ __forceinline__ float sqrt_p<float>(float x) { return sqrtf(x); }
 // for 64, while that sub-partition could issue an integer or FP32 instruction
 // every cycle: whatever needs no FP64 pipe is done beside it.
 //   * reciprocals are formed in FP32 and integers altogether, roots and quotients start
-//     from 44-bit values formed there and need three FP64 instructions (a divide
+//     from 43-bit values formed there and need three FP64 instructions (a divide
 //     takes about nine, the hardware's 20-bit approximation with a third-order step
 //     three for a reciprocal and five for a root);
 //   * negation, powers of two and comparisons are integer operations.
@@ -246,10 +246,10 @@ __device__ __forceinline__ bool above(double x, double y) {
 
 // 1/x without the FP64 pipe.  In FP32: x's mantissa as a float and the float of its
 // remaining bits, the approximate reciprocal r of the first, and the correction r
-// (e + e^2), e = 1 - x r, added to r's double as an integer: 44 bits (FULL = false).
+// (e + e^2), e = 1 - x r, added to r's double as an integer: 43 bits (FULL = false).
 // Then a Newton step in integers: with the mantissas as 53-bit integers X and R the
 // remainder 2^105 - X R is below 2^62, so it is known from the product modulo 2^64, and R
-// times it, shifted, is added: half an ulp and 2^-18 more.  NaN for zero, subnormal,
+// times it, shifted, is added: half an ulp and 2^-17 more.  NaN for zero, subnormal,
 // infinite or NaN x and from 2^1022.
 template <bool FULL>
 __device__ __forceinline__ double reciprocal(double x) {
@@ -259,10 +259,12 @@ __device__ __forceinline__ double reciprocal(double x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(xf));  // in (0.5, 1]
   const float e = fmaf(-xl, r, fmaf(-xf, r, 1.0f));
-  // the correction in units of 2^-52 (the double's are 2^-53 below 1)
-  const int q = __float2int_rn(r * 0x1p52f * fmaf(e, e, e));
+  // the correction in units of 2^-43, rounded by the float that has its last bit there
+  const int q = __float_as_int(fmaf(r * 0x1p43f, fmaf(e, e, e), 0x1.8p23f)) - 0x4b400000;
   const unsigned rb = __float_as_uint(r), ex = hi & 0x7ff00000u;
-  unsigned long long y = (((unsigned long long)(rb >> 3) << 32) | (rb << 29)) + (unsigned long long)(2ll * q);
+  // 1/x of the mantissa as a double's bits with the float's exponent bias (units of
+  // 2^-53 below 1, so that the sum is right on both sides of 1)
+  unsigned long long y = (((unsigned long long)(rb >> 3) << 32) | (rb << 29)) + (unsigned long long)((long long)q << 10);
   if (FULL) {
     const unsigned Rl = (unsigned)y, Rh = (unsigned)(y >> 32) - (125u << 20);  // 2^53 r
     const unsigned Xh = (hi & 0xfffffu) | 0x100000u;                           // 2^52 x
@@ -270,12 +272,11 @@ __device__ __forceinline__ double reciprocal(double x) {
     const int c = (__mulhi((int)~ph, (int)__funnelshift_l(Rl, Rh, 9)) + (1 << 17)) >> 18;
     y += (unsigned long long)(long long)c;
   }
-  const unsigned yh = (unsigned)(y >> 32) + ((1023u - 127u) << 20) + (0x3ff00000u - ex);
-  return __hiloint2double(ex - 0x00100000u < 0x7fc00000u ? (int)(yh | (hi & 0x80000000u)) : 0x7ff80000,
-                          (int)(unsigned)y);
+  const unsigned bias = ((1023u - 127u) << 20) + 0x3ff00000u - ex + (hi & 0x80000000u);
+  return __hiloint2double(ex - 0x00100000u < 0x7fc00000u ? (int)((unsigned)(y >> 32) + bias) : 0x7ff80000, (int)(unsigned)y);
 }
 __device__ __forceinline__ double rcp_seed(double x) { return reciprocal<false>(x); }
-// 1/sqrt(x) to about 44 bits the same way: the exponent made even, r the FP32
+// 1/sqrt(x) to about 43 bits the same way: the exponent made even, r the FP32
 // approximate reciprocal root, the correction r e (1/2 + 3/8 e), e = 1 - x r^2.
 // NaN for negative, infinite or NaN x; for zero (and subnormal x) NaN or, ZERO, 1,
 // so that x times the root is zero.
@@ -290,14 +291,14 @@ __device__ __forceinline__ double rsqrt_seed(double x) {
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(xf));  // in (0.5, 1]
   const float r2 = r * r, r2l = fmaf(r, r, -r2);
   const float e = fmaf(-xl, r2, fmaf(-xf, r2l, fmaf(-xf, r2, 1.0f)));
-  const int q = __float2int_rn(r * 0x1p52f * (e * fmaf(0.375f, e, 0.5f)));
+  const int q = __float_as_int(fmaf(r * 0x1p43f, e * fmaf(0.375f, e, 0.5f), 0x1.8p23f)) - 0x4b400000;
   const unsigned rb = __float_as_uint(r);
-  const unsigned long long y = (((unsigned long long)(rb >> 3) << 32) | (rb << 29)) + (unsigned long long)(2ll * q);
+  const unsigned long long y = (((unsigned long long)(rb >> 3) << 32) | (rb << 29)) + (unsigned long long)((long long)q << 10);
   // x = m 4^k with k = (exponent - odd) / 2 of the unbiased exponent
   const int k = ((int)(hi >> 20) - 1023 - (int)odd) >> 1;
-  const unsigned yh = (unsigned)(y >> 32) + ((1023u - 127u) << 20) - ((unsigned)k << 20);
+  const unsigned bias = ((1023u - 127u) << 20) - ((unsigned)k << 20);
   const int out = ZERO && (hi & 0x7ff00000u) == 0 ? 0x3ff00000 : 0x7ff80000;
-  return __hiloint2double(hi - 0x00100000u < 0x7fe00000u ? (int)yh : out, (int)(unsigned)y);
+  return __hiloint2double(hi - 0x00100000u < 0x7fe00000u ? (int)((unsigned)(y >> 32) + bias) : out, (int)(unsigned)y);
 }
 
 __device__ __forceinline__ double recip(double x) { return reciprocal<true>(x); }
