@@ -16,11 +16,13 @@
 //                    double-buffered shared slot, one CTA barrier per plane;
 //                    where the inboxes do not fit shared memory.
 // What bounds the sweep is the chain of about 20 dependent FP32 operations and
-// one reciprocal per cell (some 150 cycles) and what cannot be put beside it.
-// Flat plate, 2 x 96 x 96 cells, with the record builder and the update: 123 us
-// (152 with the barrier per plane); 24 x 24 cells 41 us.  A step is about 130
-// instructions of one warp at four cycles each; records by bulk copy in windows
-// that lag with the rows, and dU stored in the warps' order, measured the same.
+// one reciprocal per cell (some 150 cycles) and what cannot be put beside it: a step
+// is about 90 instructions of one warp at four cycles each.  Flat plate, 2 x 96 x 96
+// cells, with the record builder and the update: 93 us (152 with the barrier per
+// plane, 123 with branches in a step, the inbox read at its end and the records
+// converted by conversion instructions, which occupy the FP64 pipe); 24 x 24 cells 35 us.
+// Records by bulk copy in windows that lag with the rows, and dU stored in the warps'
+// order, measured the same.
 // One difference in arithmetic, not in the operator: the flux difference of comput_DFn
 // (sub_LU_SGS.f90:117-138), F_n(U + dU) - F_n(U), is evaluated in the
 // algebraically identical increment form
@@ -103,30 +105,30 @@ __global__ void __launch_bounds__(TILE) k_lusgs_prep32(Lvl L, double alfa1, int 
   double p = gm1 * (U[3] - 0.5 * (U[1] * u + U[2] * v));
 #pragma unroll
   for (int m = 0; m < NV; m++) {
-    rf[RC::A + m] = (float)((force && m < 4) ? L.res[m * F + id] + L.qf[m * F + id] : L.res[m * F + id]);
+    rf[RC::A + m] = to<float>((force && m < 4) ? L.res[m * F + id] + L.qf[m * F + id] : L.res[m * F + id]);
     rb[RC::A + m] = 0.0f;
   }
   float *rr[2] = {rf, rb};
 #pragma unroll
   for (int pass = 0; pass < 2; pass++) {
     float *q = rr[pass];
-    q[RC::B + 0] = (float)U[0];
-    q[RC::B + 1] = (float)U[1];
-    q[RC::B + 2] = (float)U[2];
-    q[RC::B + 3] = (float)(U[3] + p);
+    q[RC::B + 0] = to<float>(U[0]);
+    q[RC::B + 1] = to<float>(U[1]);
+    q[RC::B + 2] = to<float>(U[2]);
+    q[RC::B + 3] = to<float>(U[3] + p);
 #pragma unroll
-    for (int m = 4; m < NV; m++) q[RC::B + m] = (float)U[m];
-    q[RC::BU] = (float)u;
-    q[RC::BV] = (float)v;
-    q[RC::IA] = (float)ia;
-    q[RC::IA5] = (float)ia5;
+    for (int m = 4; m < NV; m++) q[RC::B + m] = to<float>(U[m]);
+    q[RC::BU] = to<float>(u);
+    q[RC::BV] = to<float>(v);
+    q[RC::IA] = to<float>(ia);
+    q[RC::IA5] = to<float>(ia5);
 #pragma unroll
     for (int dir = 0; dir < 2; dir++) {  // 0: i-neighbour, 1: j-neighbour
       const bool fwd = pass == 0;
       const long long step = dir == 0 ? 1 : P;
       // the cell that takes the term, the one that gives it
       const bool up = fwd != PUSH;  // the other cell has the smaller index
-      const long long other = up ? id - step : id + step, to = PUSH ? other : id, nb = PUSH ? id : other;
+      const long long other = up ? id - step : id + step, taker = PUSH ? other : id, nb = PUSH ? id : other;
       const bool has = dir == 0 ? (up ? i > 1 : i < b.nx - 1) : (up ? j > 1 : j < b.ny - 1);
       double cc = 0.0, hh = 0.0, n1 = 0.0, n2 = 0.0;
       if (has) {
@@ -134,14 +136,14 @@ __global__ void __launch_bounds__(TILE) k_lusgs_prep32(Lvl L, double alfa1, int 
         if (visc) cc += lc[(dir == 0 ? L_VI : L_VJ) * F + nb];
         // forward: +0.5 s of the taking cell's face; backward: -0.5 s of the
         // giving cell's face with the taking cell's normal (sub_LU_SGS.f90:87-88,95-96)
-        hh = 0.5 * g[(dir == 0 ? G_SI : G_SJ) * F + (fwd ? to : nb)];
+        hh = 0.5 * g[(dir == 0 ? G_SI : G_SJ) * F + (fwd ? taker : nb)];
         if (!fwd) hh = -hh;
-        n1 = g[(dir == 0 ? G_NI1 : G_NJ1) * F + to];
-        n2 = g[(dir == 0 ? G_NI2 : G_NJ2) * F + to];
+        n1 = g[(dir == 0 ? G_NI1 : G_NJ1) * F + taker];
+        n2 = g[(dir == 0 ? G_NI2 : G_NJ2) * F + taker];
       }
-      q[dir == 0 ? RC::CI : RC::CJ] = (float)cc;
-      q[dir == 0 ? RC::N1I : RC::N1J] = (float)(hh * n1);
-      q[dir == 0 ? RC::N2I : RC::N2J] = (float)(hh * n2);
+      q[dir == 0 ? RC::CI : RC::CJ] = to<float>(cc);
+      q[dir == 0 ? RC::N1I : RC::N1J] = to<float>(hh * n1);
+      q[dir == 0 ? RC::N2I : RC::N2J] = to<float>(hh * n2);
     }
   }
   char *base = reinterpret_cast<char *>(L.rec);
@@ -340,8 +342,24 @@ __device__ __forceinline__ float4 box_read4(unsigned a) {
   asm volatile("ld.volatile.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
   return v;
 }
-__device__ __forceinline__ void box_write4(unsigned a, float x, float y, float z, float w) {
-  asm volatile("st.volatile.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+__device__ __forceinline__ void box_write4_if(bool p, unsigned a, float x, float y, float z, float w) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t@p st.volatile.shared.v4.f32 [%0], {%1, %2, %3, %4};\n\t}" ::"r"(a),
+               "f"(x), "f"(y), "f"(z), "f"(w), "r"((int)p)
+               : "memory");
+}
+__device__ __forceinline__ void stg4_if(bool p, float *a, float x, float y, float z, float w) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t@p st.global.v4.f32 [%0], {%1, %2, %3, %4};\n\t}" ::"l"(a), "f"(x),
+               "f"(y), "f"(z), "f"(w), "r"((int)p)
+               : "memory");
+}
+__device__ __forceinline__ void stg_if(bool p, float *a, float x) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t@p st.global.f32 [%0], %1;\n\t}" ::"l"(a), "f"(x), "r"((int)p)
+               : "memory");
+}
+__device__ __forceinline__ void cp16_if(bool p, unsigned d, const char *src) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t@p cp.async.cg.shared.global [%0], [%1], 16;\n\t}" ::"r"(d), "l"(src),
+               "r"((int)p)
+               : "memory");
 }
 constexpr int PUSH32_THREADS = 352;  // the rings of as many rows fill the shared memory
 template <int NV>
@@ -362,9 +380,15 @@ __device__ __forceinline__ void push32_pass(const Lvl &L, const BlkDev &bd, int 
   const bool has_box = FWD ? j0 > 1 : j0 + 32 <= rows, has_out = FWD ? j0 + 32 <= rows : j0 > 1;
   const bool first = lane == (FWD ? 0 : last), sends = has_out && !L.silent_band_edge && lane == (FWD ? last : 0);
   const int from = FWD ? (lane + 31) & 31 : (lane + 1) & 31;
-  auto src = [&](int k) { return src_row + (size_t)(FWD ? k : ni - 1 - k) * RC::BYTES; };
-  auto fetch = [&](int k) {
-    if (row_ok && k < ni) fetch32<NV>(rec + (k & (PRING32 - 1)) * RC::BYTES, src(k));
+  auto src = [&](int k) { return src_row + (ptrdiff_t)(FWD ? k : ni - 1 - k) * RC::BYTES; };
+  const unsigned ring = (unsigned)__cvta_generic_to_shared(rec);
+  // (k below PRING32 - 2: requested before the first step)
+  auto fetch = [&](int k, int from_k = PRING32 - 2) {
+    const bool go = row_ok && k >= from_k && k < ni;
+    const unsigned d = ring + (unsigned)(k & (PRING32 - 1)) * RC::BYTES;
+    const char *p = src(k);
+#pragma unroll
+    for (int b = 0; b < RC::BYTES; b += 16) cp16_if(go, d + b, p + b);
     cp_commit();
   };
   auto read = [&](float (&c)[RC::NF], int k) {
@@ -376,26 +400,31 @@ __device__ __forceinline__ void push32_pass(const Lvl &L, const BlkDev &bd, int 
     }
   };
   int gave_up = -1;
-  // the inbox entry of step t; polled in the middle of the step before
+  // the inbox entry of step t: read in the middle of the step before (peek), and
+  // again at its end while a word of it is empty (poll)
   float in[NV];
 #pragma unroll
   for (int m = 0; m < NV; m++) in[m] = 0.0f;
+  auto peek = [&](int t) {
+    if (!has_box) return;
+    const unsigned p = box + 4u * SB * (unsigned)min(t, ni - 1);
+    const float4 v = box_read4(p);
+    in[0] = v.x; in[1] = v.y; in[2] = v.z; in[3] = v.w;
+    if (NV > 4) {
+      const float4 w = box_read4(p + 16u);
+      in[4 < NV ? 4 : 0] = w.x;
+      if (NV > 5) in[NV - 1] = w.y;
+    }
+  };
   auto poll = [&](int t) {
     if (!has_box || t >= ni || gave_up >= 0) return;
-    const unsigned p = box + 4u * SB * (unsigned)t;
     for (int n = 0;; n++) {
-      const float4 v = box_read4(p);
-      in[0] = v.x; in[1] = v.y; in[2] = v.z; in[3] = v.w;
-      if (NV > 4) {
-        const float4 w = box_read4(p + 16u);
-        in[4 < NV ? 4 : 0] = w.x;
-        if (NV > 5) in[NV - 1] = w.y;
-      }
       bool empty = false;
 #pragma unroll
       for (int m = 0; m < NV; m++) empty |= __float_as_uint(in[m]) == EMPTY32;
-      if (!__any_sync(FULL, empty)) break;
+      if (!empty) break;  // (one word for the whole warp: every lane finds the same)
       if (n == WAIT32) { gave_up = t; break; }
+      peek(t);
     }
   };
   float st[SL::S], own[NV], down[NV];  // the cell's state; the terms for the next cell and the next row
@@ -407,22 +436,25 @@ __device__ __forceinline__ void push32_pass(const Lvl &L, const BlkDev &bd, int 
   // records of the row's first visits; visit k + PRING32 - 2 is requested in visit
   // k, one group a step, so that the record of visit k + 1 has landed at the
   // end of visit k
-  for (int k = 0; k < PRING32 - 2; k++) fetch(k);
+  for (int k = 0; k < PRING32 - 2; k++) fetch(k, 0);
   cp_wait_push();
   read(c0, 0);
+  peek(0);
   poll(0);
+  // no branch but the poll: what a lane may not keep or store is selected or
+  // predicated, so that the loads of the next step are issued among the arithmetic
   auto step = [&](int t, float (&cur)[RC::NF], float (&next)[RC::NF]) {
     const int k = t - lag;
     const bool act = row_ok && (unsigned)k < (unsigned)ni;
     float nb[NV];
 #pragma unroll
     for (int m = 0; m < NV; m++) nb[m] = __shfl_sync(FULL, down[m], from);
-    if (first)
 #pragma unroll
-      for (int m = 0; m < NV; m++) nb[m] = has_box ? in[m] : 0.0f;
-    if (k >= 0) fetch(k + PRING32 - 2);
-    else cp_commit();
+    for (int m = 0; m < NV; m++) nb[m] = first ? in[m] : nb[m];
+    fetch(k + PRING32 - 2);
     cp_wait_push();
+    read(next, max(k + 1, 0));
+    peek(t + 1);
     const float ia = cur[RC::IA], ia5 = cur[RC::IA5];
     float dn[NV];
 #pragma unroll
@@ -433,25 +465,27 @@ __device__ __forceinline__ void push32_pass(const Lvl &L, const BlkDev &bd, int 
       const float inv = (NV == 5 && m == 4) ? ia5 : ia;
       dn[m] = FWD ? acc * inv : cur[RC::A + m] + acc * inv;
     }
-    if (act) {
+    float x[NV], y[NV];
 #pragma unroll
-      for (int m = 0; m < NV; m++) st[SL::D + m] = dn[m];
-      shipped_state<NV>(st, cur, gm1);
-      dterm<NV>(st, cur[RC::N1J], cur[RC::N2J], cur[RC::CJ], down);
-      dterm<NV>(st, cur[RC::N1I], cur[RC::N2I], cur[RC::CI], own);
-      if (sends) {
-        const unsigned o = out + 4u * SB * (unsigned)k;
-        box_write4(o, down[0], down[1], down[2], down[3]);
-        if (NV > 4) box_write4(o + 16u, down[4 < NV ? 4 : 0], down[NV - 1], 0.0f, 0.0f);
-      }
-      // forward: the A field of the backward record; backward: the final dU
-      // replaces it there (k_apply32 widens it afterwards)
-      float *w = reinterpret_cast<float *>(dst_row + (size_t)(FWD ? k : ni - 1 - k) * RC::BYTES);
-      *reinterpret_cast<float4 *>(w) = make_float4(dn[0], dn[1], dn[2], dn[3]);
+    for (int m = 0; m < NV; m++) st[SL::D + m] = dn[m];
+    shipped_state<NV>(st, cur, gm1);
+    dterm<NV>(st, cur[RC::N1J], cur[RC::N2J], cur[RC::CJ], y);
+    dterm<NV>(st, cur[RC::N1I], cur[RC::N2I], cur[RC::CI], x);
 #pragma unroll
-      for (int m = 4; m < NV; m++) w[m] = dn[m];
+    for (int m = 0; m < NV; m++) {
+      down[m] = act ? y[m] : down[m];
+      own[m] = act ? x[m] : own[m];
     }
-    read(next, max(k + 1, 0));
+    const bool send = sends && act;
+    const unsigned o = out + 4u * SB * (unsigned)k;
+    box_write4_if(send, o, down[0], down[1], down[2], down[3]);
+    if (NV > 4) box_write4_if(send, o + 16u, down[4 < NV ? 4 : 0], down[NV - 1], 0.0f, 0.0f);
+    // forward: the A field of the backward record; backward: the final dU
+    // replaces it there (k_apply32 widens it afterwards)
+    float *w = reinterpret_cast<float *>(dst_row + (ptrdiff_t)(FWD ? k : ni - 1 - k) * RC::BYTES);
+    stg4_if(act, w, dn[0], dn[1], dn[2], dn[3]);
+#pragma unroll
+    for (int m = 4; m < NV; m++) stg_if(act, w + m, dn[m]);
     poll(t + 1);
   };
   const int steps = ni + last;
@@ -512,7 +546,7 @@ __global__ void __launch_bounds__(TILE) k_apply32(Lvl L, int update) {
   // only inside du_LU_SGS_2D and the update after it)
 #pragma unroll
   for (int m = 0; m < NV; m++) {
-    double d = (double)rb[RC::A + m];
+    const double d = to_double(rb[RC::A + m]);
     if (update) L.U[m * F + id] += d;
     else L.du[m * F + id] = d;
   }
