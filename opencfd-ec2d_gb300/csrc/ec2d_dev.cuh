@@ -338,6 +338,18 @@ __device__ __forceinline__ double root_ratio(double a, double b) {
   return fma(half(y), fma(-(g * fabs(b)), g, fabs(a)), g);
 }
 
+// the rounded quotient and root in three FP64 instructions where the operands are of
+// ordinary size (2^-400 to 2^400), by the divide and the square root function elsewhere
+__device__ __forceinline__ bool ordinary(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7fffffffu) - ((1023u - 400u) << 20) < (800u << 20);
+}
+__device__ __forceinline__ double div_r(double a, double b) {
+  return ordinary(a) && ordinary(b) ? quot(a, b, rcp_seed(b)) : a / b;
+}
+__device__ __forceinline__ double sqrt_r(double x) { return ordinary(x) && sign_clear(x) ? root(x) : sqrt(x); }
+// tanh(x), x >= 0: 1 from 22 on, as the function gives it
+__device__ __forceinline__ double tanh_pos(double x) { return at_least(x, 22.0) ? 1.0 : tanh(x); }
+
 // the gas constants of a case in the arithmetic of a face
 struct Gas {
   double g, gm1, ggm1, rgm1, rg;  // gamma, gamma - 1, gamma / (gamma - 1), 1 / (gamma - 1), 1 / gamma

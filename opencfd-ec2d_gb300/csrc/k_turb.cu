@@ -220,7 +220,7 @@ __global__ void k_sst_cell(Lvl L) {
   const double t2 = 500.0 * amu * rRe * rd * rW * (rdw * rdw);
   const double kw = root(fabs(K)) * rW * rdw * recip(c009 * Re);
   const double arg2 = fmax(pow2<1>(kw), t2);
-  const double f2 = tanh(arg2 * arg2);
+  const double f2 = tanh_pos(arg2 * arg2);
   const double dK = dc * K;
   double amuts = fmin(fmin(dK * rW, sst::a1 * dK * Re * recip_any(f2 * fabs(omega))), 100000.0);
   const double Kws = (kx * wx + ky * wy) * (Ds * Ds) * dc * (2.0 * sst::sw2) * recip_any(W + 1.0e-20);
@@ -228,7 +228,7 @@ __global__ void k_sst_cell(Lvl L) {
   const double arg3 = fmax(kw, t2);
   const double arg1 = fmin(arg3, 4.0 * sst::sw2 * dK * recip_any(CD * (dw * dw)));
   double a1s = arg1 * arg1;
-  double f1 = tanh(a1s * a1s);
+  double f1 = tanh_pos(a1s * a1s);
   const double om2 = omega * omega, g1 = 1.0 - f1;
   double Pk = amuts * om2;
   double Pk0 = fmin(Pk, 20.0 * sst::betas * K * W * (Re * Re));

@@ -1,7 +1,8 @@
 // k_turb_mixed.cu -- the turbulence rows and the finite-difference patch of contexts
 // with FP32 parts: the kernels of k_turb.cu with the order of operations of the
 // formulas written out, so that the FP32 roundings that follow see the same FP64 values
-// bit for bit (ec2d_mixed.cuh has the reason and the figures).
+// bit for bit (ec2d_mixed.cuh has the reason and the figures).  Divides and square roots
+// are div_r and sqrt_r, which round as the divide and the function do.
 #include "ec2d_dev.cuh"
 #include "ec2d_internal.h"
 
@@ -86,7 +87,7 @@ __global__ void k_sa_res(Lvl L) {
   r = r + L.fj[4 * F + id + P] - L.fj[4 * F + id] - v0 * (L.fj[5 * F + id + P] - L.fj[5 * F + id]);
   double Dix = (x1[id + 1] - x1[id - 1]) * 0.5, Diy = (y1[id + 1] - y1[id - 1]) * 0.5;
   double Djx = (x1[id + P] - x1[id - P]) * 0.5, Djy = (y1[id + P] - y1[id - P]) * 0.5;
-  double Ds = 1.0 / (Dix * Djy - Djx * Diy);
+  double Ds = div_r(1.0, Dix * Djy - Djx * Diy);
   double Diu = (uu[id + 1] - uu[id - 1]) * 0.5, Div = (vv[id + 1] - vv[id - 1]) * 0.5;
   double Dju = (uu[id + P] - uu[id - P]) * 0.5, Djv = (vv[id + P] - vv[id - P]) * 0.5;
   double vx = (Div * Djy - Djv * Diy) * Ds;
@@ -106,8 +107,10 @@ __global__ void k_sa_res(Lvl L) {
   double g2 = g * g, g6 = g2 * g2 * g2;
   const double c36 = sa::Cw3 * sa::Cw3 * sa::Cw3 * sa::Cw3 * sa::Cw3 * sa::Cw3;
   // x^(1/6) as cbrt(sqrt(x)): both within an ulp, cheaper than pow
-  double fw = g * cbrt(sqrt((1.0 + c36) * rcp(g6 + c36)));
-  double ft2 = sa::Ct3 * exp(-sa::Ct4 * X * X);
+  double fw = g * cbrt(sqrt_r((1.0 + c36) * rcp(g6 + c36)));
+  const double ax = -sa::Ct4 * X * X;
+  // exp is zero below -746, in most of a boundary layer
+  double ft2 = sa::Ct3 * (at_least(-ax, 746.0) ? 0.0 : exp(ax));
   const double Cw1 = sa::Cb1 / (sa::kap * sa::kap) + (1.0 + sa::Cb2) / sa::sigma;
   double q = vt * rcp(dw);
   double Q = sa::Cb1 * (1.0 - ft2) * S1 * vt - (Cw1 * fw - sa::Cb1 * ft2 / (sa::kap * sa::kap)) * (q * q);
@@ -137,11 +140,11 @@ __global__ void k_sst_cell(Lvl L) {
   long long id = fidx(b, i, j);
   const double *x1 = L.geo + G_X1 * F, *y1 = L.geo + G_Y1 * F, *uu = L.q + Q_U * F, *vv = L.q + Q_V * F;
   const double *d = L.q + Q_D * F, *U5 = L.U + 4 * F, *U6 = L.U + 5 * F;
-  auto Kt = [&](long long k) { return U5[k] / d[k]; };
-  auto Wt = [&](long long k) { return U6[k] / d[k]; };
+  auto Kt = [&](long long k) { return div_r(U5[k], d[k]); };
+  auto Wt = [&](long long k) { return div_r(U6[k], d[k]); };
   double Dix = (x1[id + 1] - x1[id - 1]) * 0.5, Diy = (y1[id + 1] - y1[id - 1]) * 0.5;
   double Djx = (x1[id + P] - x1[id - P]) * 0.5, Djy = (y1[id + P] - y1[id - P]) * 0.5;
-  double Ds = 1.0 / (Dix * Djy - Djx * Diy);
+  double Ds = div_r(1.0, Dix * Djy - Djx * Diy);
   double Diu = (uu[id + 1] - uu[id - 1]) * 0.5, Div = (vv[id + 1] - vv[id - 1]) * 0.5;
   double Dik = (Kt(id + 1) - Kt(id - 1)) * 0.5, Diw = (Wt(id + 1) - Wt(id - 1)) * 0.5;
   double Dju = (uu[id + P] - uu[id - P]) * 0.5, Djv = (vv[id + P] - vv[id - P]) * 0.5;
@@ -154,22 +157,22 @@ __global__ void k_sst_cell(Lvl L) {
   double omega = vx - uy;
   double dc = d[id], K = Kt(id), W = Wt(id), dw = L.geo[G_DW * F + id];
   const double c009 = (double)0.09f;  // single-precision literal (sub_turbulence_SST.f90:87,96)
-  double t2 = 500.0 * amus / (dc * W * (dw * dw) * (Re * Re));
-  double arg2 = fmax(2.0 * sqrt(fabs(K)) / (c009 * W * dw * Re), t2);
-  double f2 = tanh(arg2 * arg2);
-  double amuts = fmin(fmin(dc * K / W, sst::a1 * dc * K * Re / (f2 * fabs(omega))), 100000.0);
-  double Kws = 2.0 * (kx * wx + ky * wy) * dc * sst::sw2 / (W + 1.0e-20);
+  double t2 = div_r(500.0 * amus, dc * W * (dw * dw) * (Re * Re));
+  double arg2 = fmax(div_r(2.0 * sqrt_r(fabs(K)), c009 * W * dw * Re), t2);
+  double f2 = tanh_pos(arg2 * arg2);
+  double amuts = fmin(fmin(div_r(dc * K, W), div_r(sst::a1 * dc * K * Re, f2 * fabs(omega))), 100000.0);
+  double Kws = div_r(2.0 * (kx * wx + ky * wy) * dc * sst::sw2, W + 1.0e-20);
   double CD = fmax(Kws, 1.0e-20);
-  double arg3 = fmax(sqrt(fabs(K)) / (c009 * W * dw * Re), t2);
-  double arg1 = fmin(arg3, 4.0 * dc * sst::sw2 * K / (CD * (dw * dw)));
+  double arg3 = fmax(div_r(sqrt_r(fabs(K)), c009 * W * dw * Re), t2);
+  double arg1 = fmin(arg3, div_r(4.0 * dc * sst::sw2 * K, CD * (dw * dw)));
   double a1s = arg1 * arg1;
-  double f1 = tanh(a1s * a1s);
+  double f1 = tanh_pos(a1s * a1s);
   double Pk = amuts * omega * omega;
   double Pk0 = fmin(Pk, 20.0 * sst::betas * K * W * (Re * Re));
-  double Qk = Pk0 / Re - sst::betas * dc * W * K * Re;
+  double Qk = div_r(Pk0, Re) - sst::betas * dc * W * K * Re;
   double Cw = f1 * sst::Cw1 + (1.0 - f1) * sst::Cw2;
   double beta = f1 * sst::beta1 + (1.0 - f1) * sst::beta2;
-  double Qw = Cw * dc * omega * omega / Re - beta * dc * (W * W) * Re + (1.0 - f1) * Kws / Re;
+  double Qw = div_r(Cw * dc * omega * omega, Re) - beta * dc * (W * W) * Re + div_r((1.0 - f1) * Kws, Re);
   L.tb[T_AMUS * F + id] = amus;
   L.tb[T_AMUTS * F + id] = amuts;
   L.tb[T_F1 * F + id] = f1;
@@ -190,8 +193,8 @@ __global__ void k_sst_faces(Lvl L) {
   const double *x1 = L.geo + G_X1 * F, *y1 = L.geo + G_Y1 * F, *uu = L.q + Q_U * F, *vv = L.q + Q_V * F;
   const double *d = L.q + Q_D * F, *U5 = L.U + 4 * F, *U6 = L.U + 5 * F;
   const double *amus = L.tb + T_AMUS * F, *amuts = L.tb + T_AMUTS * F;
-  auto Kt = [&](long long k) { return U5[k] / d[k]; };
-  auto Wt = [&](long long k) { return U6[k] / d[k]; };
+  auto Kt = [&](long long k) { return div_r(U5[k], d[k]); };
+  auto Wt = [&](long long k) { return div_r(U6[k], d[k]); };
   double f1 = L.tb[T_F1 * F + id];
   double sk = f1 * sst::sk1 + (1.0 - f1) * sst::sk2;
   double sw = f1 * sst::sw1 + (1.0 - f1) * sst::sw2;
@@ -209,14 +212,14 @@ __global__ void k_sst_faces(Lvl L) {
     double Dix = x1[id] - x1[w], Diy = y1[id] - y1[w];
     double Djx = (x1[nN - 1] + x1[nN] - x1[nS - 1] - x1[nS]) * 0.25;
     double Djy = (y1[nN - 1] + y1[nN] - y1[nS - 1] - y1[nS]) * 0.25;
-    double Ds = 1.0 / (Dix * Djy - Djx * Diy);
+    double Ds = div_r(1.0, Dix * Djy - Djx * Diy);
     double Dik = Kt(id) - Kt(w), Diw = Wt(id) - Wt(w);
     double Djk = (Kt(nN - 1) + Kt(nN) - Kt(nS - 1) - Kt(nS)) * 0.25;
     double Djw = (Wt(nN - 1) + Wt(nN) - Wt(nS - 1) - Wt(nS)) * 0.25;
     double Kx = (Dik * Djy - Djk * Diy) * Ds, Wx = (Diw * Djy - Djw * Diy) * Ds;
     double Ky = (-Dik * Djx + Djk * Dix) * Ds, Wy = (-Diw * Djx + Djw * Dix) * Ds;
-    L.fi[4 * F + id] = Fk + A1 * (Kx * n1 + Ky * n2) * si / Re;
-    L.fi[5 * F + id] = Fw + A2 * (Wx * n1 + Wy * n2) * si / Re;
+    L.fi[4 * F + id] = Fk + div_r(A1 * (Kx * n1 + Ky * n2) * si, Re);
+    L.fi[5 * F + id] = Fw + div_r(A2 * (Wx * n1 + Wy * n2) * si, Re);
   }
   if (i >= 1 && i <= b.nx - 1 && j >= 1 && j <= b.ny) {
     long long s = id - P;
@@ -232,14 +235,14 @@ __global__ void k_sst_faces(Lvl L) {
     double Dix = (x1[s + 1] + x1[id + 1] - x1[s - 1] - x1[id - 1]) * 0.25;
     double Diy = (y1[s + 1] + y1[id + 1] - y1[s - 1] - y1[id - 1]) * 0.25;
     double Djx = x1[id] - x1[s], Djy = y1[id] - y1[s];
-    double Ds = 1.0 / (Dix * Djy - Djx * Diy);
+    double Ds = div_r(1.0, Dix * Djy - Djx * Diy);
     double Dik = (Kt(s + 1) + Kt(id + 1) - Kt(s - 1) - Kt(id - 1)) * 0.25;
     double Diw = (Wt(s + 1) + Wt(id + 1) - Wt(s - 1) - Wt(id - 1)) * 0.25;
     double Djk = Kt(id) - Kt(s), Djw = Wt(id) - Wt(s);
     double Kx = (Dik * Djy - Djk * Diy) * Ds, Wx = (Diw * Djy - Djw * Diy) * Ds;
     double Ky = (-Dik * Djx + Djk * Dix) * Ds, Wy = (-Diw * Djx + Djw * Dix) * Ds;
-    L.fj[4 * F + id] = Fk + A1 * (Kx * n1 + Ky * n2) * sj / Re;
-    L.fj[5 * F + id] = Fw + A2 * (Wx * n1 + Wy * n2) * sj / Re;
+    L.fj[4 * F + id] = Fk + div_r(A1 * (Kx * n1 + Ky * n2) * sj, Re);
+    L.fj[5 * F + id] = Fw + div_r(A2 * (Wx * n1 + Wy * n2) * sj, Re);
   }
 }
 
@@ -259,8 +262,8 @@ __global__ void k_sst_res(Lvl L) {
   r6 = r6 + L.fj[5 * F + id + P] - L.fj[5 * F + id] + L.tb[T_QW * F + id] * vol;
   L.res[4 * F + id] = r5;
   L.res[5 * F + id] = r6;
-  L.amu[id] = L.tb[T_AMUS * F + id] / c.Re;
-  L.amut[id] = L.tb[T_AMUTS * F + id] / c.Re;
+  L.amu[id] = div_r(L.tb[T_AMUS * F + id], c.Re);
+  L.amut[id] = div_r(L.tb[T_AMUTS * F + id], c.Re);
 }
 
 // ---- finite-difference patch (sub_Finite_Difference.f90:4-275) --------------
@@ -271,14 +274,14 @@ enum { D_SPI = 0, D_SPJ = 8, D_FI = 16, D_FJ = 20, D_EV1 = 24, D_EV2 = 27 };
 // split_Steger_Warming, sub_Finite_Difference.f90:154-202
 __device__ __forceinline__ void split_sw(double d, double u, double v, double cc, double A1, double A2,
                                          double gamma, double *fp, double *fm) {
-  double tmp1 = 2.0 * (gamma - 1.0), tmp3 = (3.0 - gamma) / (2.0 * (gamma - 1.0));
-  double vs = A1 * u + A2 * v, ss = sqrt(A1 * A1 + A2 * A2);
-  const double rss = 1.0 / ss;
+  double tmp1 = 2.0 * (gamma - 1.0), tmp3 = div_r(3.0 - gamma, 2.0 * (gamma - 1.0));
+  double vs = A1 * u + A2 * v, ss = sqrt_r(A1 * A1 + A2 * A2);
+  const double rss = div_r(1.0, ss);
   double ak1 = A1 * rss, ak2 = A2 * rss;
   double E1 = vs, E2 = vs - cc * ss, E3 = vs + cc * ss;
   double E1P = (E1 + fabs(E1)) * 0.5, E2P = (E2 + fabs(E2)) * 0.5, E3P = (E3 + fabs(E3)) * 0.5;
   double E1M = E1 - E1P, E2M = E2 - E2P, E3M = E3 - E3P;
-  double tmp0 = d / (2.0 * gamma);
+  double tmp0 = div_r(d, 2.0 * gamma);
   double uc1 = u - cc * ak1, uc2 = u + cc * ak1, vc1 = v - cc * ak2, vc2 = v + cc * ak2;
   double vvc1 = (uc1 * uc1 + vc1 * vc1) / 2.0, vvc2 = (uc2 * uc2 + vc2 * vc2) / 2.0;
   double vv = (gamma - 1.0) * (u * u + v * v), W2 = tmp3 * cc * cc;
@@ -302,7 +305,7 @@ __global__ void k_fdm_split(Lvl L) {
   const long long F = L.F;
   long long id = fidx(b, i, j);
   double d = L.q[Q_D * F + id], u = L.q[Q_U * F + id], v = L.q[Q_V * F + id], cc = L.q[Q_C * F + id];
-  const double rJ = 1.0 / L.met[M_JAC * F + id];  // one divide for the metric quotients
+  const double rJ = div_r(1.0, L.met[M_JAC * F + id]);  // one divide for the metric quotients
   double fp[4], fm[4];
   // blockIdx.y: 0 the i-direction split, 1 the j-direction split (two threads per cell)
   const int dir = blockIdx.y;
@@ -325,7 +328,7 @@ __device__ __forceinline__ double weno5_mix(double S0, double S1, double S2, dou
   const double ep = 1.0e-6, C03 = 3.0 / 10.0, C13 = 3.0 / 5.0, C23 = 1.0 / 10.0;
   const double D0 = (ep + S0) * (ep + S0), D1 = (ep + S1) * (ep + S1), D2 = (ep + S2) * (ep + S2);
   const double n0 = C03 * (D1 * D2), n1 = C13 * (D0 * D2), n2 = C23 * (D0 * D1);
-  return (n0 * q03 + n1 * q13 + n2 * q23) / (n0 + n1 + n2);
+  return div_r(n0 * q03 + n1 * q13 + n2 * q23, n0 + n1 + n2);
 }
 __device__ __forceinline__ double weno5_p(double vm2, double vm1, double v0, double vp1, double vp2) {
   double t0 = v0 - 2.0 * vp1 + vp2, t1 = 3.0 * v0 - 4.0 * vp1 + vp2;
@@ -386,11 +389,11 @@ __global__ void k_fdm_flux(Lvl L) {
   if (part == 2 && L.visc && i >= 2 && i <= nxF - 1 && j >= 2 && j <= nyF - 1) {
     const double *uu = L.q + Q_U * F, *vv = L.q + Q_V * F, *TT = L.q + Q_T * F;
     double mu0 = L.amu[id] + L.amut[id];
-    double Ak0 = c.Cp * (L.amu[id] / c.Pr + L.amut[id] / PrT);
+    double Ak0 = c.Cp * (div_r(L.amu[id], c.Pr) + div_r(L.amut[id], PrT));
     double ui = 0.5 * (uu[id + 1] - uu[id - 1]), vi = 0.5 * (vv[id + 1] - vv[id - 1]), Ti = 0.5 * (TT[id + 1] - TT[id - 1]);
     double uj = 0.5 * (uu[id + P] - uu[id - P]), vj = 0.5 * (vv[id + P] - vv[id - P]), Tj = 0.5 * (TT[id + P] - TT[id - P]);
     double Akx = L.met[M_KX * F + id], Aky = L.met[M_KY * F + id], Aix = L.met[M_IX * F + id], Aiy = L.met[M_IY * F + id];
-    const double rJ = 1.0 / L.met[M_JAC * F + id];
+    const double rJ = div_r(1.0, L.met[M_JAC * F + id]);
     double ux = ui * Akx + uj * Aix, vx = vi * Akx + vj * Aix, Tx = Ti * Akx + Tj * Aix;
     double uy = ui * Aky + uj * Aiy, vy = vi * Aky + vj * Aiy, Ty = Ti * Aky + Tj * Aiy;
     double t11 = (4.0 / 3.0 * ux - 2.0 / 3.0 * vy) * mu0, t22 = (4.0 / 3.0 * vy - 2.0 / 3.0 * ux) * mu0;
