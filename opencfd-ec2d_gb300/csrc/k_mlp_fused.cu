@@ -52,8 +52,7 @@ namespace ec2d {
 namespace fused {
 
 constexpr int W = 256, TILE_B = 128 * W * 2, SMALL_B = 128 * 16 * 2;  // bytes of a 128-row block, of a 16-column one
-constexpr int STAGE_B = W * 32 * 2, NSTAGE = 5;                       // a weight chunk: 256 rows x 32 of K
-constexpr int EW = 16, ECOL = 64 / (EW / 4);  // epilogue warps; columns of each 64 a warp takes
+constexpr int STAGE_B = W * 32 * 2;  // a weight chunk: 256 rows x 32 of K
 constexpr int WAIT_LIMIT = 1 << 22;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -161,19 +160,39 @@ __device__ __forceinline__ void sts16(uint32_t a, uint32_t x, uint32_t y, uint32
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * EW) : "memory"); }
 
-constexpr int S_A = 0, S_E = S_A + TILE_B, S_X = S_E + TILE_B, S_O = S_X + SMALL_B, S_W = S_O + SMALL_B,
-              S_END = S_W + NSTAGE * STAGE_B;
+// The three forms of the tile kernel.
+//   FORM_TRAIN   forward, loss gradient and backward of tile blockIdx.x
+//   FORM_ONE     forward of tiles blockIdx.x, + gridDim.x, ... with predictions out, a
+//                CTA per SM: sixteen epilogue warps on one tile, the MMAs of a
+//                layer 64 columns behind the epilogue of the last (with eight warps alone
+//                a layer took 8,000 cycles)
+//   FORM_TWO     the same with two CTAs per SM of eight epilogue warps, one accumulator
+//                and a short weight ring each: one CTA's MMAs run under the other's
+//                epilogue.  A tile took 53,900 cycles in FORM_ONE, with the special-function
+//                unit 46 % and the issue slots 49 % busy.  For more tiles than
+//                SMs; up to that a tile alone is faster in FORM_ONE.
+enum { FORM_TRAIN, FORM_ONE, FORM_TWO };
+template <int FORM>
+struct Form {
+  static constexpr bool TRAIN = FORM == FORM_TRAIN, TWO = FORM == FORM_TWO;
+  static constexpr int EW = TWO ? 8 : 16, ECOL = 64 / (EW / 4);  // epilogue warps; columns of each 64 a warp takes
+  static constexpr int NSTAGE = TWO ? 2 : 5, COLS = TWO ? W : 2 * W;  // weight ring; TMEM columns
+  static constexpr int THREADS = 32 * (EW + 2);
+  static constexpr int S_A = 0, S_E = S_A + TILE_B, S_X = S_E + (TRAIN ? TILE_B : 0), S_O = S_X + SMALL_B,
+                       S_W = S_O + (TRAIN ? SMALL_B : 0), S_END = S_W + NSTAGE * STAGE_B;
+};
 
-// TRAIN: forward, loss gradient and backward of tile blockIdx.x; else forward
-// of tiles blockIdx.x, + gridDim.x, ... with predictions out.  Warps 0 to EW -
-// 1: inputs and epilogues (warp w: rows 32 (w % 4) .. of the tile, columns ECOL
-// (w / 4) .. of each 64); then one warp for the bulk copies and one for MMAs and
-// TMEM.  Sixteen epilogue warps keep the special-function unit fed; with eight
-// a layer took 8,000 cycles.
-template <bool TRAIN>
-__global__ void __launch_bounds__(32 * (EW + 2), 1) k_mlp_tile(const __grid_constant__ FusedArgs a) {
+// Warps 0 to EW - 1: inputs and epilogues (warp w: rows 32 (w % 4) .. of the tile,
+// columns ECOL (w / 4) .. of each 64); then one warp for the bulk copies and one for
+// MMAs and TMEM.
+template <int FORM>
+__global__ void __launch_bounds__(Form<FORM>::THREADS, Form<FORM>::TWO ? 2 : 1)
+    k_mlp_tile(const __grid_constant__ FusedArgs a) {
+  using C = Form<FORM>;
+  constexpr bool TRAIN = C::TRAIN;
+  constexpr int EW = C::EW, ECOL = C::ECOL, NSTAGE = C::NSTAGE, S_A = C::S_A, S_E = C::S_E, S_X = C::S_X, S_O = C::S_O,
+                S_W = C::S_W, NACC = C::COLS / W;  // accumulators
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) uint64_t bars[2 * NSTAGE + 4 + 4];
   __shared__ uint32_t tmem_sh;
@@ -187,7 +206,8 @@ __global__ void __launch_bounds__(32 * (EW + 2), 1) k_mlp_tile(const __grid_cons
   const uint32_t accfull = b0 + 8u * (2 * NSTAGE + 4), hfull = accfull + 8, hdone = accfull + 16, efree = accfull + 24;
   const int nl = a.nlin;
   if (warp == EW + 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_sh)) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_sh)), "n"(C::COLS)
+                 : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
@@ -271,10 +291,13 @@ __global__ void __launch_bounds__(32 * (EW + 2), 1) k_mlp_tile(const __grid_cons
       };
       for (int t = blockIdx.x; t < a.ntiles && !*dead; t += step_tiles) {
         for (int l = 0; l < nl; l++, gen++) {
-          product(s0 + (l == 0 ? S_X : S_A), l == 0, l < nl - 1 ? W : 16, (l & 1) * W,
-                  [&](int c) { return wait(afull(c), gen & 1u, dead, a.err); });
+          // (one accumulator: only once the epilogue has read all of it)
+          if (C::TWO)
+            for (int c = 0; c < 4; c++) wait(afull(c), gen & 1u, dead, a.err);
+          product(s0 + (l == 0 ? S_X : S_A), l == 0, l < nl - 1 ? W : 16, (l % NACC) * W,
+                  [&](int c) { return C::TWO ? !*dead : wait(afull(c), gen & 1u, dead, a.err); });
           // the chunks of A that a one-chunk product did not wait for
-          if (l == 0)
+          if (!C::TWO && l == 0)
             for (int c = 1; c < 4; c++) wait(afull(c), gen & 1u, dead, a.err);
           commit(accfull);
         }
@@ -306,6 +329,7 @@ __global__ void __launch_bounds__(32 * (EW + 2), 1) k_mlp_tile(const __grid_cons
       __syncwarp();
       if (lane == 0) mbar_arrive(afull(c));
     };
+    auto epi_barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(32 * EW) : "memory"); };
     auto stores_read = [&] {  // the last bulk store has read its shared memory
       if (TRAIN) {
         if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -352,7 +376,8 @@ __global__ void __launch_bounds__(32 * (EW + 2), 1) k_mlp_tile(const __grid_cons
         for (int c = 0; c < 4; c++) {
           const int col = c * 64 + h * ECOL;
           uint32_t v[ECOL];
-          tmem_ld16(v, lane_base + (l & 1) * W + col);
+          if constexpr (ECOL == 32) tmem_ld32(v, lane_base + (l % NACC) * W + col);
+          else tmem_ld16(v, lane_base + (l % NACC) * W + col);
           ld_wait();
 #pragma unroll
           for (int p = 0; p < ECOL / 8; p++) {
@@ -376,7 +401,7 @@ __global__ void __launch_bounds__(32 * (EW + 2), 1) k_mlp_tile(const __grid_cons
       fence_after();
       if (h == 0) {
         uint32_t v[16];
-        tmem_ld16(v, lane_base + ((nl - 1) & 1) * W);
+        tmem_ld16(v, lane_base + ((nl - 1) % NACC) * W);
         ld_wait();
         if (!TRAIN) {
           if (row < a.n)
@@ -419,7 +444,7 @@ __global__ void __launch_bounds__(32 * (EW + 2), 1) k_mlp_tile(const __grid_cons
 #pragma unroll 1
           for (int c = 0; c < 4; c++) {
             const int col = c * 64 + h * ECOL;
-            uint32_t v[ECOL], z[ECOL];
+            uint32_t v[16], z[16];  // (ECOL)
             tmem_ld16(v, lane_base + col);
             tmem_ld16(z, lane_base + W + col);
             ld_wait();
@@ -449,7 +474,7 @@ __global__ void __launch_bounds__(32 * (EW + 2), 1) k_mlp_tile(const __grid_cons
   __syncthreads();
   if (*dead)  // copies and MMAs in flight end before the shared memory is given up
     for (int k = 0; k < 1000; k++) __nanosleep(1000);
-  if (warp == EW + 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+  if (warp == EW + 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(C::COLS) : "memory");
 }
 
 // ---- weight gradients -------------------------------------------------------
@@ -721,15 +746,18 @@ int fused_tiles_per_wave() {
   }();
   return n;
 }
+template <int FORM>
+static void launch_tile(const FusedArgs &a, int grid, cudaStream_t s) {
+  using C = fused::Form<FORM>;
+  cudaFuncSetAttribute(fused::k_mlp_tile<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::S_END);
+  fused::k_mlp_tile<FORM><<<grid, C::THREADS, C::S_END, s>>>(a);
+}
 void launch_mlp_forward(const FusedArgs &a, cudaStream_t s) {
-  cudaFuncSetAttribute(fused::k_mlp_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, fused::S_END);
-  const int grid = a.ntiles < fused_tiles_per_wave() ? a.ntiles : fused_tiles_per_wave();
-  fused::k_mlp_tile<false><<<grid, 32 * (fused::EW + 2), fused::S_END, s>>>(a);
+  const int sms = fused_tiles_per_wave();
+  if (a.ntiles <= sms) launch_tile<fused::FORM_ONE>(a, a.ntiles, s);
+  else launch_tile<fused::FORM_TWO>(a, a.ntiles < 2 * sms ? a.ntiles : 2 * sms, s);
 }
-void launch_mlp_train_tile(const FusedArgs &a, cudaStream_t s) {
-  cudaFuncSetAttribute(fused::k_mlp_tile<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, fused::S_END);
-  fused::k_mlp_tile<true><<<a.ntiles, 32 * (fused::EW + 2), fused::S_END, s>>>(a);
-}
+void launch_mlp_train_tile(const FusedArgs &a, cudaStream_t s) { launch_tile<fused::FORM_TRAIN>(a, a.ntiles, s); }
 void launch_mlp_dw(const FusedArgs &a, float *part, long long unit_stride, int ks, int rows, cudaStream_t s) {
   const int sm = fused::DW_NS * fused::DW_STAGE;
   cudaFuncSetAttribute(fused::k_mlp_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
