@@ -453,6 +453,9 @@ int build_level(ec2d_ctx *ctx, int l) {
   L.tb = (L.turb == Turb_SST) ? dalloc<double>(lv, SST_PLANES * F) : (L.turb == Turb_BL) ? dalloc<double>(lv, F) : nullptr;
   bool anyfdm = false;
   for (auto &B : lv.hb) anyfdm |= B.fdm;
+  long long ncells = 0;
+  for (const auto &B : lv.hb) ncells += (long long)(B.nx - 1) * (B.ny - 1);
+  if (slope_level(L, ncells) && !(L.slope = dalloc<double>(lv, 16 * F))) return EC2D_ERR_NOMEM;
   L.met = anyfdm ? dalloc<double>(lv, 5 * F) : nullptr;
   L.fdm = anyfdm ? dalloc<double>(lv, 30 * F) : nullptr;
   for (auto &B : lv.hb) lv.max_rows = std::max(lv.max_rows, B.ny - 1);
@@ -664,6 +667,7 @@ void residual(ec2d_ctx *ctx, int l, int post = 0) {
     else if (L.turb == Turb_SST) K(ctx, "sst", l, 4, [&] { launch_sst(L, s); });
     else if (L.turb == Turb_BL) K(ctx, "bl", l, 2, [&] { launch_bl(L, s); });
   }
+  if (L.slope && !L.mixed) K(ctx, "k_slopes", l, 1, [&] { launch_slopes(L, s); });
   // the i- and j-face kernels read the same primitives and write separate
   // planes: they run concurrently on two streams (graph branches); with
   // kernel timing on they run one after the other

@@ -96,6 +96,7 @@ struct Lvl {
   double *U, *q, *amu, *amut, *res, *lc, *du, *geo, *un, *deltu, *qf, *un1;
   double *fi, *fj;          // face-flux scratch, 6 planes each
   double *tb;               // turbulence scratch planes
+  double *slope;            // limited MUSCL3 slopes, 16 planes (large FP64 levels; else null)
   double *met;              // FDM metrics Akx,Aky,Aix,Aiy,Ajac
   double *fdm;              // FDM scratch planes
   double *lu;               // LU-SGS pre-pass planes (4 NV + 10)
@@ -427,6 +428,17 @@ __device__ __forceinline__ void scheme_pair(double u1, double u2, double u3, dou
     }
   }
   l = r = 0.0;
+}
+
+// The same MUSCL3 states from one cell: van Albada's s and both corrections depend on the
+// cell's differences dm and dp alone.  a: to its upper face (left state u + a), b: to its
+// lower face (right state u - b).
+__device__ __forceinline__ void muscl3_slopes(double dm, double dp, double &a, double &b) {
+  const double ep = 1.0e-6;
+  const double s = fma(pow2<1>(dp), dm, ep) * recip(fma(dm, dm, fma(dp, dp, ep)));
+  const double ks = (1.0 / 3.0) * s, sum = dm + dp, w = dp - dm;
+  a = pow2<-2>(s) * fma(ks, w, sum);
+  b = fma(half(s), sum, -a);  // s/4 (sum - ks w)
 }
 
 // conservative (rho, rho u, rho v, E) -> primitive (rho, u, v, p), as at the

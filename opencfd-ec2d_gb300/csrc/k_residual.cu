@@ -96,6 +96,34 @@ __device__ __forceinline__ bool in_fdm_core(const BlkDev &b, int i, int j) {
   return b.fdm && (i >= LFDM + 2 && i <= b.nx - LFDM - 1) && (j >= LFDM + 2 && j <= b.ny - LFDM - 1);
 }
 
+// Limited slopes of a large level's cells in both directions (Lvl::slope, planes 8 dir +
+// 2 variable: to the upper face, + 1: to the lower).  The limiter belongs to the cell, so
+// the two faces of a direction share it: 96 FP64 instructions per cell here and 8 per face
+// for the states, against 2 x 80 where each face forms both of its sides.
+// The planes' traffic (256 bytes per cell) hides behind the FP64 pipe, but the launch
+// and the planes pay only on large levels (slope_level).
+__global__ void __launch_bounds__(TILE) k_slopes(Lvl L) {
+  int bk, i, j;
+  if (!core_ij(L, bk, i, j)) return;
+  const BlkDev &b = L.blk[bk];
+  const long long F = L.F, id = fidx(b, i, j);
+#pragma unroll
+  for (int dir = 0; dir < 2; dir++) {
+    if (dir == 0 ? j < 1 || j > b.ny - 1 || i < 0 || i > b.nx : i < 1 || i > b.nx - 1 || j < 0 || j > b.ny) continue;
+    const long long st = dir == 0 ? 1 : b.P;
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      const int pl = m == 0 ? Q_D : m == 1 ? Q_U : m == 2 ? Q_V : Q_P;
+      const double *q = L.q + pl * F + id;
+      const double u = q[0];
+      double a, c;
+      muscl3_slopes(u - q[-st], q[st] - u, a, c);
+      L.slope[(8 * dir + 2 * m) * F + id] = a;
+      L.slope[(8 * dir + 2 * m + 1) * F + id] = c;
+    }
+  }
+}
+
 // reconstruction and inviscid flux of a face, F = -s (flux)
 template <bool M, typename T>
 __device__ __forceinline__ void inviscid(const Lvl &L, const CaseDev &c, int scheme, T S0[4][4], T n1, T n2, T s, T *F) {
@@ -182,7 +210,8 @@ __device__ __forceinline__ FaceDiff<T> face_diff(long long r, long long st, long
 // IFACE: face loop in i of Residual_FVM (sub_Residual.f90:238-346), face (i,j),
 // i=1..nx, j=1..ny-1, between cells (i-1,j) and (i,j); else in j (:352-455), face (i,j),
 // i=1..nx-1, j=1..ny, between cells (i,j-1) and (i,j).
-template <bool M, bool IFACE, typename T>
+// SLOPES: from the cells' limited slopes (k_slopes).
+template <bool M, bool IFACE, bool SLOPES, typename T>
 __global__ void __launch_bounds__(TILE) k_flux(Lvl L) {
   int bk, i, j;
   if (!core_ij(L, bk, i, j)) return;
@@ -193,24 +222,36 @@ __global__ void __launch_bounds__(TILE) k_flux(Lvl L) {
   const long long F = L.F, st = IFACE ? 1 : b.P, id = fidx(b, i, j);
   const T s = to<T>(L.geo[(IFACE ? G_SI : G_SJ) * F + id]), n1 = to<T>(L.geo[(IFACE ? G_NI1 : G_NJ1) * F + id]),
           n2 = to<T>(L.geo[(IFACE ? G_NI2 : G_NJ2) * F + id]);
-  T S0[4][4];
-  int scheme = L.scheme;
-  if (L.recon == Recon_Original) {
-    if (!IFACE) scheme = L.gscheme;  // the reference passes the global Iflag_Scheme here (sub_Residual.f90:367)
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const long long q = id + (k - 2) * st;
-      S0[k][0] = to<T>(L.q[Q_D * F + q]); S0[k][1] = to<T>(L.q[Q_U * F + q]);
-      S0[k][2] = to<T>(L.q[Q_V * F + q]); S0[k][3] = to<T>(L.q[Q_P * F + q]);
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-#pragma unroll
-      for (int m = 0; m < 4; m++) S0[k][m] = to<T>(L.U[m * F + id + (k - 2) * st]);
-  }
   T Fl[4];
-  inviscid<M>(L, c, scheme, S0, n1, n2, s, Fl);
+  if constexpr (SLOPES) {
+    double UL[4], UR[4];
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      const int pl = m == 0 ? Q_D : m == 1 ? Q_U : m == 2 ? Q_V : Q_P;
+      const double *sp = L.slope + ((IFACE ? 0 : 8) + 2 * m) * F + id;
+      UL[m] = L.q[pl * F + id - st] + sp[-st];
+      UR[m] = L.q[pl * F + id] - sp[F];
+    }
+    face_flux(L.flux, UL, UR, n1, n2, s, Fl, gas(c));
+  } else {
+    T S0[4][4];
+    int scheme = L.scheme;
+    if (L.recon == Recon_Original) {
+      if (!IFACE) scheme = L.gscheme;  // the reference passes the global Iflag_Scheme here (sub_Residual.f90:367)
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const long long q = id + (k - 2) * st;
+        S0[k][0] = to<T>(L.q[Q_D * F + q]); S0[k][1] = to<T>(L.q[Q_U * F + q]);
+        S0[k][2] = to<T>(L.q[Q_V * F + q]); S0[k][3] = to<T>(L.q[Q_P * F + q]);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+#pragma unroll
+        for (int m = 0; m < 4; m++) S0[k][m] = to<T>(L.U[m * F + id + (k - 2) * st]);
+    }
+    inviscid<M>(L, c, scheme, S0, n1, n2, s, Fl);
+  }
   if (L.visc) {
     const double *uu = L.q + Q_U * F, *vv = L.q + Q_V * F, *TT = L.q + Q_T * F;
     auto u = [=](long long k) { return to<T>(uu[k]); };
@@ -751,10 +792,20 @@ static void by_kind(const Lvl &L, Fn f) {
 void launch_prim(const Lvl &L, cudaStream_t s) {
   by_kind(L, [&](auto M) { k_prim<M.value><<<L.ntiles, TILE, 0, s>>>(L); });
 }
+// A level takes the slopes pass if it has planes for it (slope_level, at set-up) and is FP64
+// throughout.  2 x 1024 x 512 cells: slopes 195 us, faces 2 x 217, the RK3 step 2.26 ->
+// 2.07 ms.  With the pass everywhere a RANS step of 66 k cells is 1 % slower, a V-cycle of
+// 18 k cells 0.7 %, 16 k cells of an airfoil 0.9 %.
+static bool slopes(const Lvl &L) { return L.slope != nullptr && !L.mixed; }
+bool slope_level(const Lvl &L, long long cells) {
+  return cells >= SLOPE_CELLS && L.recon == Recon_Original && L.scheme == Scheme_MUSCL3 && L.gscheme == Scheme_MUSCL3;
+}
+void launch_slopes(const Lvl &L, cudaStream_t s) { k_slopes<<<L.nctiles, TILE, 0, s>>>(L); }
 template <bool IFACE>
 static void launch_flux(const Lvl &L, bool fp32, cudaStream_t s) {
-  if (fp32) k_flux<true, IFACE, float><<<L.nctiles, TILE, 0, s>>>(L);
-  else by_kind(L, [&](auto M) { k_flux<M.value, IFACE, double><<<L.nctiles, TILE, 0, s>>>(L); });
+  if (fp32) k_flux<true, IFACE, false, float><<<L.nctiles, TILE, 0, s>>>(L);
+  else if (slopes(L)) k_flux<false, IFACE, true, double><<<L.nctiles, TILE, 0, s>>>(L);
+  else by_kind(L, [&](auto M) { k_flux<M.value, IFACE, false, double><<<L.nctiles, TILE, 0, s>>>(L); });
 }
 void launch_flux_i(const Lvl &L, bool fp32, cudaStream_t s) { launch_flux<true>(L, fp32, s); }
 void launch_flux_j(const Lvl &L, bool fp32, cudaStream_t s) { launch_flux<false>(L, fp32, s); }
