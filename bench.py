@@ -48,11 +48,13 @@ FALLBACK_HBM = 6800.0
 #   k_lusgs   read Res(4), U(4), dt, vol, Lci, Lcj, Lvi, Lvj, si, sj,
 #             ni1, ni2, nj1, nj2; dU written, re-read and rewritten (12) = 32 w
 #   k_add_du  read U(4), dU(4), write U(4)                            = 12 w
+#   k_slopes  read d,u,v,p; write two corrections per variable and
+#             direction (16)                                          = 20 w
 #   k_residual_tile  the residual stage in one kernel: read U(4), 7 metrics,
 #             x1, y1 (viscous inverse Jacobians counted as the metrics);
 #             write Res(4), Lci, Lcj, Lvi, Lvj, dt                    = 22 w
 BYTES_PER_UNIT = {"k_prim": 96, "k_flux_i": 128, "k_flux_j": 128, "k_res": 240, "k_lusgs": 256, "k_add_du": 96,
-                  "k_residual_tile": 176}
+                  "k_residual_tile": 176, "k_slopes": 160}
 
 
 def peaks():
@@ -277,17 +279,17 @@ def time_to_drop(g, cells, cap_s=60.0, target=1e-8, check=25):
 
 
 # DRAM bytes per launch of the dominant kernel on this workload, from one
-# ncu capture of the default wavefront (k_lusgs_sweep_quad<1, 8>) on the fine
+# ncu capture of the default wavefront (k_push_sweep<4, true>) on the fine
 # level (dram__bytes_read.sum + dram__bytes_write.sum, caches flushed before
 # the launch; the run is in the profiling summaries of the repo)
-PROFILED_TRAFFIC = {("k_lusgs", 1): 7426816.0}
+PROFILED_TRAFFIC = {("k_lusgs", 1): 5948672.0}
 # FP64 work per fine cell of one laminar residual evaluation (k_prim,
-# k_flux_i, k_flux_j, k_res; AUSM+, MUSCL van Albada, primitive
-# reconstruction) on the 4.19 M-cell grid, from one ncu capture of those
+# k_slopes, k_flux i and j, k_res; AUSM+, MUSCL van Albada, primitive
+# reconstruction) on 1.05 M cells, from one ncu capture of those
 # kernels (thread instructions executed / cells): FLOPs = dadd + dmul +
 # 2 dfma, instructions = dadd + dmul + dfma.  Every FP64 instruction takes
 # one issue slot of the FP64 pipe, whose rate is half the FMA FLOP rate.
-FP64_PER_CELL_RESIDUAL = {"chain": (966.1, 689.9), "tile": (None, None)}
+FP64_PER_CELL_RESIDUAL = {"chain": (467.1, 361.9), "tile": (None, None)}
 SWEEP_PLANES = lambda blocks, lev: 2 * max((b.nx - 1) // 2 ** (lev - 1) + (b.ny - 1) // 2 ** (lev - 1) - 1
                                          for b in blocks)
 
@@ -776,7 +778,7 @@ def run_gb300(args, rank, world):
         kind = "one-lane" if cs != 0 else ("eight-lane bands" if lanes == 8 else "four-lane bands")
         return {"lusgs_kernel": kind, "lusgs_ctas": cs, "rows": rpw, "lanes": lanes if cs == 0 else 1,
                 "concurrent_faces": cc, "ms": ms,
-                "residual": "one kernel over shared-memory tiles" if g.tile_residual() else "four-kernel chain"}
+                "residual": "one kernel over shared-memory tiles" if g.tile_residual() else "kernel chain"}
 
     tuned = {"fp64": shape(tune())}
 
@@ -829,10 +831,10 @@ def run_gb300(args, rank, world):
         planes = SWEEP_PLANES(blocks, klev)
         s_calls, s_ms = sweep_ms.get(klev, (kcalls, kms))
         cpp = s_ms / s_calls * 1e-3 * mhz * 1e6 / planes
-        # the FP64 chain of one plane: 15 operations per cell and lane with
+        # the FP64 chain of one plane: 6 operations per cell and lane with
         # eight lanes per row, 18 with four, 31 per cell with one, 64 cycles each
         kind = tuned["fp64"]["lusgs_kernel"]
-        floor = {"eight-lane bands": 15, "four-lane bands": 18}.get(kind, 31) * 64
+        floor = {"eight-lane bands": 6, "four-lane bands": 18}.get(kind, 31) * 64
         roofline["bound"] = "latency"
         roofline["hbm_frac"] = roofline["frac"]
         roofline["sweep_avg_launch_us"] = s_ms / s_calls * 1e3
