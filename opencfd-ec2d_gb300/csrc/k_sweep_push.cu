@@ -39,12 +39,14 @@
 // copies of 16 cells (loads into registers three cells ahead cost 150 cycles
 // per cell), and what has to be stored goes out behind the shuffles.
 //
-// Measured (GB300, 2,070 MHz, events, with the launch): 2 x 96 x 96 cells
-// 339 -> 200 us (1,840 -> 1,080 cycles per plane), 256 x 64 one block 564 ->
-// 311 us, 64 x 16 147 -> 82 us; 4 x 128 x 128 with the SA row 622 -> 390 us,
-// with the SST rows 749 -> 373 us.  A warp alone takes about 960 cycles per
-// cell, of them 8 x 64 FP64 and 3 x 75 the crossings; a row of warps adds half
-// a cell per warp at its start.  Bands of 8 to 16 rows per CTA measure the same.
+// Measured (GB300, 2,070 MHz, events, with the launch; the pull form before it in
+// brackets): 2 x 96 x 96 cells 174 us (339), 940 cycles per plane (1,840), 256 x 64 one
+// block 266 us (564), 64 x 16 72 us (147); 4 x 128 x 128 with the SA row 348 us
+// (622), with the SST rows 337 us (749).  Of a plane 6 x 64 cycles are FP64 and 3 x 75
+// crossings; the reciprocal's chain is as long as the two instructions of m, and a row of
+// warps adds half a cell per warp at its start.  With two FP64 Newton instructions for
+// the reciprocal 2 x 96 x 96 took 200 us.  Bands of 8 to 16 rows per CTA measure
+// the same.
 #include <algorithm>
 
 #include "ec2d_dev.cuh"
