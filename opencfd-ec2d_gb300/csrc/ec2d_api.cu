@@ -453,9 +453,6 @@ int build_level(ec2d_ctx *ctx, int l) {
   L.tb = (L.turb == Turb_SST) ? dalloc<double>(lv, SST_PLANES * F) : (L.turb == Turb_BL) ? dalloc<double>(lv, F) : nullptr;
   bool anyfdm = false;
   for (auto &B : lv.hb) anyfdm |= B.fdm;
-  long long ncells = 0;
-  for (const auto &B : lv.hb) ncells += (long long)(B.nx - 1) * (B.ny - 1);
-  if (slope_level(L, ncells) && !(L.slope = dalloc<double>(lv, 16 * F))) return EC2D_ERR_NOMEM;
   L.met = anyfdm ? dalloc<double>(lv, 5 * F) : nullptr;
   L.fdm = anyfdm ? dalloc<double>(lv, 30 * F) : nullptr;
   for (auto &B : lv.hb) lv.max_rows = std::max(lv.max_rows, B.ny - 1);
@@ -1239,6 +1236,14 @@ int ec2d_setup(ec2d_ctx *ctx) {
     for (auto &b : ctx->lv[l].blk) mx = std::max(mx, (size_t)(b.nx + 3) * (b.ny + 3) * 6);
   CK(cudaMalloc(&ctx->d_stage, mx * sizeof(double)));
   ctx->stage_n = mx;
+  // slope planes of large levels, after everything that a context cannot do without: where
+  // the memory does not hold them, the faces form their own limiters
+  for (int l = 1; l <= ctx->num_mesh; l++) {
+    Level &lv = ctx->lv[l];
+    long long ncells = 0;
+    for (const auto &B : lv.hb) ncells += (long long)(B.nx - 1) * (B.ny - 1);
+    if (slope_level(lv.L, ncells) && !(lv.L.slope = dalloc<double>(lv, 16 * lv.L.F))) cudaGetLastError();
+  }
   CK(cudaDeviceSynchronize());
   ctx->setup_done = true;
   apply_mg_amut(ctx);
