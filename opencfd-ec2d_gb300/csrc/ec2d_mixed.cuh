@@ -8,7 +8,7 @@
 // mixed-precision runs stay what they were, bit for bit, these contexts keep the order of
 // operations of the formulas written out, and FP64 contexts use the
 // shorter one of ec2d_dev.cuh.  Both are compared with the oracle to the same
-// bounds.  A face takes 298 FP64 instructions against 190 there.
+// bounds.  A face takes 298 FP64 instructions against 172 there.
 #pragma once
 #include "ec2d_dev.cuh"
 

@@ -64,8 +64,8 @@ __device__ __forceinline__ double sutherland(const CaseDev &c, const Prim &w) { 
 }
 
 // comput_duvtpckw (sub_Residual.f90:114-152) + get_viscous (:670-689) + Amu_t=0
-// (:172); 21 FP64 instructions per viscous cell of an FP64 context instead of 29 (1.05 M
-// cells: 49 us instead of 68)
+// (:172); 16 FP64 instructions per viscous cell of an FP64 context instead of 29 (1.05 M
+// cells: 39 us instead of 68)
 template <bool M>
 __global__ void __launch_bounds__(TILE) k_prim(Lvl L) {
   int bk, i, j;
@@ -201,11 +201,12 @@ __device__ __forceinline__ FaceDiff<T> face_diff(long long r, long long st, long
 
 // The face kernels are bound by the issue of FP64 instructions (one per 16 to 19
 // cycles and SM; memory traffic is a tenth of the time): a viscous MUSCL3 / AUSM+
-// face takes about 190 of them (reconstruction 96, flux 50, viscous terms 44) where
-// the formulas written out with divides, rotations and floating-point
-// selects take 298 (M, ec2d_mixed.cuh), and the flux planes of 1.05 M cells take
-// 0.39 ms per direction instead of 0.60 (HLLC with characteristic WENO3 on 131 x 59
-// cells 22 us instead of 41, most of them the chain of one face).  In FP32 the
+// face takes about 172 of them (reconstruction 80, flux 50, viscous terms 42; 103 from
+// the cells' slopes) where the formulas written out with divides, rotations and
+// floating-point selects take 298 (M, ec2d_mixed.cuh).  65 k cells take 27 us per
+// direction between events instead of 39, 1.05 M cells with the slopes 217 (and 195 for
+// both directions' slopes) instead of 600, HLLC with characteristic WENO3 on 131 x
+// 59 cells 22 instead of 41, most of them the chain of one face.  In FP32 the
 // values are converted on the integer pipes (to<float>), not by the FP64 pipe.
 // IFACE: face loop in i of Residual_FVM (sub_Residual.f90:238-346), face (i,j),
 // i=1..nx, j=1..ny-1, between cells (i-1,j) and (i,j); else in j (:352-455), face (i,j),

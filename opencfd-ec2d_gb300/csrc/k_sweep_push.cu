@@ -104,8 +104,8 @@ __device__ __forceinline__ void face_term(const double *U, double n1, double n2,
 
 // the records of both passes, all cells at once (force: Res + QF in place of
 // Res, see k_lusgs_prep).  Bound by FP64 issue on large levels (65 k cells 29 us) and by one
-// cell's chain on small ones: some 95 instructions per cell at NV = 4, 125 with
-// third-order reciprocals, halves by multiplication and sums not folded into FMAs.
+// cell's chain on small ones: 100 instructions per cell at NV = 4 (ncu), with reciprocals
+// and halves off the FP64 pipe and every term folded into an FMA.
 template <int NV, bool update>
 __global__ void __launch_bounds__(TILE) k_push_prep(Lvl L, double alfa1, int force) {
   int bk, i, j;

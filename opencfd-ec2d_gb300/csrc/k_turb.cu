@@ -246,7 +246,7 @@ __global__ void k_sst_cell(Lvl L) {
 // k and omega come from planes that k_sst_cell fills once per cell, and the normal
 // derivatives from the set-up coefficients, where each face divided twelve times by the
 // density and formed its Jacobian: the four kernels of the model on 65 k cells take
-// 58 us instead of 125.
+// 54 us instead of 125.
 // k and omega face fluxes, i faces (sub_turbulence_SST.f90:129-182) and j
 // faces (:198-248); planes 4/5 of fi and fj
 __global__ void k_sst_faces(Lvl L) {
@@ -375,9 +375,9 @@ __global__ void k_fdm_split(Lvl L) {
 // candidate values are written in the first and second differences of v,
 //   S_0 = d3^2 + s3 (4/3 s3 - d3),  S_1 = d3^2 + s2 (4/3 s2 - d3),  S_2 = d2^2 + s1 (4/3 s1 + d2),
 //   q_0 - c = d3/2 - s3/6,  q_1 - c = d3/2 - s2/6,  q_2 - c = d2/2 + s1/3,
-// 32 FP64 instructions per value; written out from the five values with an IEEE
+// 30 FP64 instructions per value; written out from the five values with an IEEE
 // divide it took 60, and the 65 k cells of a 513 x 129 block took 203 us with
-// split and residual, three launches (125 us now).  D_k >= 1e-12, so numerator and denominator stay above
+// split and residual, three launches (110 us now).  D_k >= 1e-12, so numerator and denominator stay above
 // 1e-36, and they overflow only for smoothness indicators beyond about 1e50, far
 // from any split flux of this solver.
 __device__ __forceinline__ double weno5(double a, double b, double c, double d, double e) {
