@@ -188,10 +188,9 @@ __device__ __forceinline__ float sqrt_p<float>(float x) { return sqrtf(x); }
 // one FP64 warp instruction per 16 to 19 cycles, and each holds its sub-partition
 // for 64, while that sub-partition could issue an integer or FP32 instruction
 // every cycle: whatever needs no FP64 pipe is done beside it.
-//   * reciprocals are formed in FP32 and integers altogether, roots and quotients start
-//     from 43-bit values formed there and need three FP64 instructions (a divide
-//     takes about nine, the hardware's 20-bit approximation with a third-order step
-//     three for a reciprocal and five for a root);
+//   * reciprocals and reciprocal roots are formed in FP32 and integers altogether (a
+//     divide takes about nine FP64 instructions, the hardware's 20-bit approximation with
+//     a third-order step three for a reciprocal and five for a root);
 //   * negation, powers of two and comparisons are integer operations.
 // x 2^K, K in -3..1: exact; zeros, infinities and NaNs stay what they are, and so
 // do values below 2^-1019
@@ -277,12 +276,15 @@ __device__ __forceinline__ double reciprocal(double x) {
   return __hiloint2double(ex - 0x00100000u < 0x7fc00000u ? (int)((unsigned)(y >> 32) + bias) : 0x7ff80000, (int)(unsigned)y);
 }
 __device__ __forceinline__ double rcp_seed(double x) { return reciprocal<false>(x); }
-// 1/sqrt(x) to about 43 bits the same way: the exponent made even, r the FP32
-// approximate reciprocal root, the correction r e (1/2 + 3/8 e), e = 1 - x r^2.
+// 1/sqrt(x) the same way: the exponent made even, r the FP32 approximate reciprocal root
+// of the mantissa m in [1, 4), e = 1 - m r^2, and r (1 + e/2 + 3/8 e^2).  FULL = false: e in
+// FP32, 43 bits.  FULL: with A = 2^24 r and X the 53-bit mantissa, e is -X A^2 modulo 2^96 (known
+// to 2^-67 from four 32-bit products), r e/2 is A times it, shifted; only the term
+// in e^2 is FP32: half an ulp and 2^-8 more.
 // NaN for negative, infinite or NaN x; for zero (and subnormal x) NaN or, ZERO, 1,
 // so that x times the root is zero.
-template <bool ZERO>
-__device__ __forceinline__ double rsqrt_seed(double x) {
+template <bool ZERO, bool FULL>
+__device__ __forceinline__ double rsqrt_x(double x) {
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
   const unsigned odd = (hi & 0x00100000u) ? 0u : 1u;  // biased exponent even: mantissa in [2, 4)
   const float xf = __uint_as_float((__funnelshift_l(lo, hi, 3) & 0x7fffffu) | (odd ? 0x40000000u : 0x3f800000u));
@@ -292,9 +294,24 @@ __device__ __forceinline__ double rsqrt_seed(double x) {
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(xf));  // in (0.5, 1]
   const float r2 = r * r, r2l = fmaf(r, r, -r2);
   const float e = fmaf(-xl, r2, fmaf(-xf, r2l, fmaf(-xf, r2, 1.0f)));
-  const int q = __float_as_int(fmaf(r * 0x1p43f, e * fmaf(0.375f, e, 0.5f), 0x1.8p23f)) - 0x4b400000;
   const unsigned rb = __float_as_uint(r);
-  const unsigned long long y = (((unsigned long long)(rb >> 3) << 32) | (rb << 29)) + (unsigned long long)((long long)q << 10);
+  unsigned long long y = ((unsigned long long)(rb >> 3) << 32) | (rb << 29);  // 2^53 r
+  if (FULL) {
+    const unsigned A = rb - (125u << 23), Xh = (hi & 0xfffffu) | 0x100000u;
+    const unsigned long long S = (unsigned long long)A * A;
+    const unsigned Sl = (unsigned)S, Sh = (unsigned)(S >> 32);
+    // bits 32 to 95 of X A^2: 2^(68 - odd) (1 - e) modulo 2^64
+    const unsigned long long M = (unsigned long long)Xh * Sl + (unsigned long long)lo * Sh + __umulhi(lo, Sl) +
+                                 ((unsigned long long)(Xh * Sh) << 32);
+    const long long E = -(long long)M;
+    const long long c = (long long)(int)A * (int)(E >> 32) + (long long)__umulhi(A, (unsigned)E);  // 2^(8 - odd) r e/2
+    const int q = __float_as_int(fmaf(r * (odd ? 0x1.8p58f : 0x1.8p59f), e * e, 0x1.8p23f)) - 0x4b400000;  // r 3/8 e^2
+    const int sh = 8 - (int)odd;
+    y += (unsigned long long)((c + q + (1 << (sh - 1))) >> sh);
+  } else {
+    const int q = __float_as_int(fmaf(r * 0x1p43f, e * fmaf(0.375f, e, 0.5f), 0x1.8p23f)) - 0x4b400000;
+    y += (unsigned long long)((long long)q << 10);
+  }
   // x = m 4^k with k = (exponent - odd) / 2 of the unbiased exponent
   const int k = ((int)(hi >> 20) - 1023 - (int)odd) >> 1;
   const unsigned bias = ((1023u - 127u) << 20) - ((unsigned)k << 20);
@@ -318,26 +335,16 @@ __device__ __forceinline__ double quot(double a, double b, double y) {
 __device__ __forceinline__ double pos_part(double x) { return __double2hiint(x) >= 0 ? x : 0.0; }
 __device__ __forceinline__ double neg_part(double x) { return __double2hiint(x) < 0 ? x : 0.0; }
 
-// 1/sqrt(x), x > 0, to two ulps
-__device__ __forceinline__ double rroot(double x) {
-  const double y = rsqrt_seed<false>(x), e = fma(-x, y * y, 1.0);
-  return fma(half(y), e, y);
-}
-// sqrt(x): from g = x y the remainder x - g^2, exact by an fma, gives the root's last bits
-// (the rounded root in all of 8e8 samples)
-__device__ __forceinline__ double root(double x) {
-  const double y = rsqrt_seed<true>(x), g = x * y;
-  return fma(half(y), fma(-g, g, x), g);
-}
+// 1/sqrt(x), x > 0
+__device__ __forceinline__ double rroot(double x) { return rsqrt_x<false, true>(x); }
+// sqrt(x) = x / sqrt(x), within an ulp of the rounded root
+__device__ __forceinline__ double root(double x) { return x * rsqrt_x<true, true>(x); }
 // the square root function where x is not a positive normal number (T < 0: NaN)
 __device__ __forceinline__ double root_t(double x) {
   return (unsigned)__double2hiint(x) - 0x00100000u < 0x7fe00000u ? root(x) : sqrt(x);
 }
-// sqrt(a / b) = |a| / sqrt(a b): no reciprocal; the same remainder, a - g^2 b; to two ulps
-__device__ __forceinline__ double root_ratio(double a, double b) {
-  const double w = a * b, y = rsqrt_seed<true>(w), g = fabs(a) * y;
-  return fma(half(y), fma(-(g * fabs(b)), g, fabs(a)), g);
-}
+// sqrt(a / b) = |a| / sqrt(a b): no reciprocal; to two ulps
+__device__ __forceinline__ double root_ratio(double a, double b) { return fabs(a) * rsqrt_x<true, true>(a * b); }
 
 // the rounded quotient and root in three FP64 instructions where the operands are of
 // ordinary size (2^-400 to 2^400), by the divide and the square root function elsewhere
@@ -347,7 +354,12 @@ __device__ __forceinline__ bool ordinary(double x) {
 __device__ __forceinline__ double div_r(double a, double b) {
   return ordinary(a) && ordinary(b) ? quot(a, b, rcp_seed(b)) : a / b;
 }
-__device__ __forceinline__ double sqrt_r(double x) { return ordinary(x) && sign_clear(x) ? root(x) : sqrt(x); }
+// (from g = x y, y to 43 bits, the remainder x - g^2, exact by an fma, gives the last bits)
+__device__ __forceinline__ double sqrt_r(double x) {
+  if (!(ordinary(x) && sign_clear(x))) return sqrt(x);
+  const double y = rsqrt_x<false, false>(x), g = x * y;
+  return fma(half(y), fma(-g, g, x), g);
+}
 // tanh(x), x >= 0: 1 from 22 on, as the function gives it
 __device__ __forceinline__ double tanh_pos(double x) { return at_least(x, 22.0) ? 1.0 : tanh(x); }
 
