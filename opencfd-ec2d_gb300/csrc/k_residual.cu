@@ -156,24 +156,25 @@ template <bool M, bool IFACE, typename T>
 __device__ __forceinline__ void viscous(const CaseDev &c, const double *g, long long F, const FaceDiff<T> &D, T ml, T mr,
                                         bool eddy, T tl, T tr, bool lo, bool hi, T n1, T n2, T s, T *Fo) {
   if constexpr (M) {
+    // (the laminar product fused, the eddy one rounded: the order is part of the results)
     T Amu1, Amk1;
     const T Cp = to<T>(c.Cp), rPr = to<T>(c.rPr), rPrT = (T)(1.0 / PrT);
     if (lo) {
       Amu1 = mr + tr;
-      Amk1 = Cp * (mr * rPr + tr * rPrT);
+      Amk1 = Cp * fma(mr, rPr, tr * rPrT);
     } else if (hi) {
       Amu1 = ml + tl;
-      Amk1 = Cp * (ml * rPr + tl * rPrT);
+      Amk1 = Cp * fma(ml, rPr, tl * rPrT);
     } else {
       // the two families of faces add the viscosities in their own order
-      if (IFACE) Amu1 = (ml + mr + tl + tr) * T(0.5);
-      else Amu1 = (mr + ml + tr + tl) * T(0.5);
-      Amk1 = Cp * ((ml + mr) * rPr + (tl + tr) * rPrT) * T(0.5);
+      if (IFACE) Amu1 = mixed::scaled<-1>(ml + mr + tl + tr);
+      else Amu1 = mixed::scaled<-1>(mr + ml + tr + tl);
+      Amk1 = mixed::scaled<-1>(Cp * fma(ml + mr, rPr, (tl + tr) * rPrT));
     }
-    const T yu = D.yu * T(0.25), yv = D.yv * T(0.25), yT = D.yT * T(0.25);
+    const T yu = mixed::scaled<-2>(D.yu), yv = mixed::scaled<-2>(D.yv), yT = mixed::scaled<-2>(D.yT);
     mixed::viscous_face_m(to<T>(g[0]), to<T>(g[F]), to<T>(g[2 * F]), to<T>(g[3 * F]), IFACE ? D.xu : yu, IFACE ? D.xv : yv,
                           IFACE ? D.xT : yT, IFACE ? yu : D.xu, IFACE ? yv : D.xv, IFACE ? yT : D.xT, Amu1, Amk1,
-                          D.us * T(0.5), D.vs * T(0.5), n1, n2, s, Fo[1], Fo[2], Fo[3]);
+                          mixed::scaled<-1>(D.us), mixed::scaled<-1>(D.vs), n1, n2, s, Fo[1], Fo[2], Fo[3]);
   } else {
     const double h = half(s);
     double mu = ((lo ? mr : ml) + (hi ? ml : mr)) * h, k = mu * c.kpr;
