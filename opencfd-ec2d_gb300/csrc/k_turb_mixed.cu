@@ -180,7 +180,8 @@ __global__ void k_sst_cell(Lvl L) {
   L.tb[T_QW * F + id] = Qw;
 }
 
-// k and omega face fluxes, i faces (sub_turbulence_SST.f90:129-182) and j
+// k and omega face fluxes (the sum of both sides with the first product fused: the order is
+// part of the results where the cells flow together), i faces (sub_turbulence_SST.f90:129-182) and j
 // faces (:198-248); planes 4/5 of fi and fj
 __global__ void k_sst_faces(Lvl L) {
   int bk, i, j;
@@ -202,8 +203,8 @@ __global__ void k_sst_faces(Lvl L) {
     long long w = id - 1, nN = id + P, nS = id - P;
     double si = L.geo[G_SI * F + id], n1 = L.geo[G_NI1 * F + id], n2 = L.geo[G_NI2 * F + id];
     double un1 = uu[w] * n1 + vv[w] * n2, un2 = uu[id] * n1 + vv[id] * n2;
-    double Fk = -0.5 * ((un1 + fabs(un1)) * Kt(w) + (un2 - fabs(un2)) * Kt(id)) * si;
-    double Fw = -0.5 * ((un1 + fabs(un1)) * Wt(w) + (un2 - fabs(un2)) * Wt(id)) * si;
+    double Fk = -0.5 * fma(un1 + fabs(un1), Kt(w), (un2 - fabs(un2)) * Kt(id)) * si;
+    double Fw = -0.5 * fma(un1 + fabs(un1), Wt(w), (un2 - fabs(un2)) * Wt(id)) * si;
     double A1, A2;
     if (i == 1) { A1 = amus[id] + sk * amuts[id]; A2 = amus[id] + sw * amuts[id]; }
     else if (i == b.nx) { A1 = amus[w] + sk * amuts[w]; A2 = amus[w] + sw * amuts[w]; }
@@ -225,8 +226,8 @@ __global__ void k_sst_faces(Lvl L) {
     long long s = id - P;
     double sj = L.geo[G_SJ * F + id], n1 = L.geo[G_NJ1 * F + id], n2 = L.geo[G_NJ2 * F + id];
     double un1 = uu[s] * n1 + vv[s] * n2, un2 = uu[id] * n1 + vv[id] * n2;
-    double Fk = -0.5 * ((un1 + fabs(un1)) * Kt(s) + (un2 - fabs(un2)) * Kt(id)) * sj;
-    double Fw = -0.5 * ((un1 + fabs(un1)) * Wt(s) + (un2 - fabs(un2)) * Wt(id)) * sj;
+    double Fk = -0.5 * fma(un1 + fabs(un1), Kt(s), (un2 - fabs(un2)) * Kt(id)) * sj;
+    double Fw = -0.5 * fma(un1 + fabs(un1), Wt(s), (un2 - fabs(un2)) * Wt(id)) * sj;
     double A1, A2;
     if (j == 1) { A1 = amus[id] + sk * amuts[id]; A2 = amus[id] + sw * amuts[id]; }
     else if (j == b.ny) { A1 = amus[s] + sk * amuts[s]; A2 = amus[s] + sw * amuts[s]; }
