@@ -289,7 +289,7 @@ PROFILED_TRAFFIC = {("k_lusgs", 1): 5948672.0}
 # kernels (thread instructions executed / cells): FLOPs = dadd + dmul +
 # 2 dfma, instructions = dadd + dmul + dfma.  Every FP64 instruction takes
 # one issue slot of the FP64 pipe, whose rate is half the FMA FLOP rate.
-FP64_PER_CELL_RESIDUAL = {"chain": (467.1, 361.9), "tile": (None, None)}
+FP64_PER_CELL_RESIDUAL = {"chain": (443.0, 347.9), "tile": (None, None)}
 SWEEP_PLANES = lambda blocks, lev: 2 * max((b.nx - 1) // 2 ** (lev - 1) + (b.ny - 1) // 2 ** (lev - 1) - 1
                                          for b in blocks)
 

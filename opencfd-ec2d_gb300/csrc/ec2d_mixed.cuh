@@ -8,8 +8,8 @@
 // mixed-precision runs stay what they were, bit for bit, these contexts keep the order of
 // operations of the formulas written out, and FP64 contexts use the
 // shorter one of ec2d_dev.cuh.  Both are compared with the oracle to the same
-// bounds.  A face takes 298 FP64 instructions (some
-// 270 without the powers of two and comparisons) against 166 there.
+// bounds.  A viscous AUSM+ face takes 273 FP64 instructions (298 with every power of two
+// on the FP64 pipe; 343 -> 322 us per direction of a batched polar) against 166 there.
 #pragma once
 #include "ec2d_dev.cuh"
 

@@ -64,8 +64,8 @@ __device__ __forceinline__ double sutherland(const CaseDev &c, const Prim &w) { 
 }
 
 // comput_duvtpckw (sub_Residual.f90:114-152) + get_viscous (:670-689) + Amu_t=0
-// (:172); 16 FP64 instructions per viscous cell of an FP64 context instead of 29 (1.05 M
-// cells: 39 us instead of 68)
+// (:172); 14 FP64 instructions per viscous cell of an FP64 context instead of 29 (1.05 M
+// cells: 36 us instead of 68)
 template <bool M>
 __global__ void __launch_bounds__(TILE) k_prim(Lvl L) {
   int bk, i, j;
@@ -202,10 +202,10 @@ __device__ __forceinline__ FaceDiff<T> face_diff(long long r, long long st, long
 
 // The face kernels are bound by the issue of FP64 instructions (one per 16 to 19
 // cycles and SM; memory traffic is a tenth of the time): a viscous MUSCL3 / AUSM+
-// face takes about 172 of them (reconstruction 80, flux 50, viscous terms 42; 103 from
+// face takes about 166 of them (reconstruction 80, flux 44, viscous terms 42; 97 from
 // the cells' slopes) where the formulas written out with divides, rotations and
-// floating-point selects take 298 (M, ec2d_mixed.cuh).  65 k cells take 27 us per
-// direction between events instead of 39, 1.05 M cells with the slopes 217 (and 195 for
+// floating-point selects take 273 (M, ec2d_mixed.cuh).  65 k cells take 27 us per
+// direction between events instead of 39, 1.05 M cells with the slopes 205 (and 195 for
 // both directions' slopes) instead of 600, HLLC with characteristic WENO3 on 131 x
 // 59 cells 22 instead of 41, most of them the chain of one face.  In FP32 the
 // values are converted on the integer pipes (to<float>), not by the FP64 pipe.
@@ -795,7 +795,7 @@ void launch_prim(const Lvl &L, cudaStream_t s) {
   by_kind(L, [&](auto M) { k_prim<M.value><<<L.ntiles, TILE, 0, s>>>(L); });
 }
 // A level takes the slopes pass if it has planes for it (slope_level, at set-up) and is FP64
-// throughout.  2 x 1024 x 512 cells: slopes 195 us, faces 2 x 217, the RK3 step 2.26 ->
+// throughout.  2 x 1024 x 512 cells: slopes 195 us, faces 2 x 217 (205 since), the RK3 step 2.26 ->
 // 2.07 ms.  With the pass everywhere a RANS step of 66 k cells is 1 % slower, a V-cycle of
 // 18 k cells 0.7 %, 16 k cells of an airfoil 0.9 %.
 static bool slopes(const Lvl &L) { return L.slope != nullptr && !L.mixed; }
