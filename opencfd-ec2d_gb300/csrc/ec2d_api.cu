@@ -664,7 +664,7 @@ void residual(ec2d_ctx *ctx, int l, int post = 0) {
     else if (L.turb == Turb_SST) K(ctx, "sst", l, 4, [&] { launch_sst(L, s); });
     else if (L.turb == Turb_BL) K(ctx, "bl", l, 2, [&] { launch_bl(L, s); });
   }
-  if (L.slope && !L.mixed) K(ctx, "k_slopes", l, 1, [&] { launch_slopes(L, s); });
+  if (L.slope && !f32) K(ctx, "k_slopes", l, 1, [&] { launch_slopes(L, s); });
   // the i- and j-face kernels read the same primitives and write separate
   // planes: they run concurrently on two streams (graph branches); with
   // kernel timing on they run one after the other

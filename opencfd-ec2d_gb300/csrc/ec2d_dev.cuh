@@ -96,7 +96,7 @@ struct Lvl {
   double *U, *q, *amu, *amut, *res, *lc, *du, *geo, *un, *deltu, *qf, *un1;
   double *fi, *fj;          // face-flux scratch, 6 planes each
   double *tb;               // turbulence scratch planes
-  double *slope;            // limited MUSCL3 slopes, 16 planes (large FP64 levels; else null)
+  double *slope;            // limited MUSCL3 slopes or states, 16 planes (large levels; else null)
   double *met;              // FDM metrics Akx,Aky,Aix,Aiy,Ajac
   double *fdm;              // FDM scratch planes
   double *lu;               // LU-SGS pre-pass planes (4 NV + 10)

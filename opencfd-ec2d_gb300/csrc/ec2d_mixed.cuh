@@ -110,6 +110,17 @@ __device__ __forceinline__ T scheme_fm(T u1, T u2, T u3, T u4, int flag) {
   return T(0.0);
 }
 
+// MUSCL3 states of cell u2 towards its upper and its lower face, the bits of scheme_fp and
+// scheme_fm there: the fused products are written out as the compiler chooses them in those
+__device__ __forceinline__ void muscl3_states(double u1, double u2, double u3, double &hi, double &lo) {
+  const double ep = 1.0e-6, k3 = 1.0 / 3.0;
+  const double up = u3 - u2, um = u2 - u1;
+  const double s = fma(scaled<1>(up), um, ep) * rcp(fma(um, um, up * up) + ep);
+  const double q = scaled<-2>(s), a = fma(-k3, s, 1.0), b = fma(k3, s, 1.0);
+  hi = fma(q, fma(a, um, b * up), u2);
+  lo = fma(-q, fma(a, up, b * um), u2);
+}
+
 // conservative (rho, rho u, rho v, E) -> primitive (rho, u, v, p), as at the
 // end of Reconstuction_conservative/Characteristic (sub_Residual.f90:526-527)
 template <typename T>

@@ -99,9 +99,12 @@ __device__ __forceinline__ bool in_fdm_core(const BlkDev &b, int i, int j) {
 // Limited slopes of a large level's cells in both directions (Lvl::slope, planes 8 dir +
 // 2 variable: to the upper face, + 1: to the lower).  The limiter belongs to the cell, so
 // the two faces of a direction share it: 96 FP64 instructions per cell here and 8 per face
-// for the states, against 2 x 80 where each face forms both of its sides.
+// for the states, against 2 x 80 where each face forms both of its sides.  M: the planes
+// hold the states themselves, with the bits that the faces form (batch of 16 airfoils,
+// 0.6 M cells on the finest level: 3.49 -> 3.32 ms per V-cycle).
 // The planes' traffic (256 bytes per cell) hides behind the FP64 pipe, but the launch
 // and the planes pay only on large levels (slope_level).
+template <bool M>
 __global__ void __launch_bounds__(TILE) k_slopes(Lvl L) {
   int bk, i, j;
   if (!core_ij(L, bk, i, j)) return;
@@ -117,19 +120,18 @@ __global__ void __launch_bounds__(TILE) k_slopes(Lvl L) {
       const double *q = L.q + pl * F + id;
       const double u = q[0];
       double a, c;
-      muscl3_slopes(u - q[-st], q[st] - u, a, c);
+      if constexpr (M) mixed::muscl3_states(q[-st], u, q[st], a, c);
+      else muscl3_slopes(u - q[-st], q[st] - u, a, c);
       L.slope[(8 * dir + 2 * m) * F + id] = a;
       L.slope[(8 * dir + 2 * m + 1) * F + id] = c;
     }
   }
 }
 
-// reconstruction and inviscid flux of a face, F = -s (flux)
+// inviscid flux of a face from the states before and after it, F = -s (flux)
 template <bool M, typename T>
-__device__ __forceinline__ void inviscid(const Lvl &L, const CaseDev &c, int scheme, T S0[4][4], T n1, T n2, T s, T *F) {
-  T UL[4], UR[4];
+__device__ __forceinline__ void inviscid_states(const Lvl &L, const CaseDev &c, const T *UL, const T *UR, T n1, T n2, T s, T *F) {
   if constexpr (M) {
-    mixed::reconstruct(L.recon, scheme, S0, to<T>(c.gamma), UL, UR);
     T QL[4] = {UL[0], UL[1] * n1 + UL[2] * n2, -UL[1] * n2 + UL[2] * n1, UL[3]};
     T QR[4] = {UR[0], UR[1] * n1 + UR[2] * n2, -UR[1] * n2 + UR[2] * n1, UR[3]};
     T Fl[4];
@@ -139,10 +141,16 @@ __device__ __forceinline__ void inviscid(const Lvl &L, const CaseDev &c, int sch
     F[2] = -(Fl[1] * n2 + Fl[2] * n1) * s;
     F[3] = -Fl[3] * s;
   } else {
-    const Gas G = gas(c);
-    reconstruct(L.recon, scheme, S0, G, UL, UR);
-    face_flux(L.flux, UL, UR, n1, n2, s, F, G);
+    face_flux(L.flux, UL, UR, n1, n2, s, F, gas(c));
   }
+}
+// the same with the reconstruction
+template <bool M, typename T>
+__device__ __forceinline__ void inviscid(const Lvl &L, const CaseDev &c, int scheme, T S0[4][4], T n1, T n2, T s, T *F) {
+  T UL[4], UR[4];
+  if constexpr (M) mixed::reconstruct(L.recon, scheme, S0, to<T>(c.gamma), UL, UR);
+  else reconstruct(L.recon, scheme, S0, gas(c), UL, UR);
+  inviscid_states<M>(L, c, UL, UR, n1, n2, s, F);
 }
 // viscous terms of a face, added to F.  across: from the cell before the face to the
 // one after; along: the sum over both cells of the differences between their
@@ -231,10 +239,10 @@ __global__ void __launch_bounds__(TILE) k_flux(Lvl L) {
     for (int m = 0; m < 4; m++) {
       const int pl = m == 0 ? Q_D : m == 1 ? Q_U : m == 2 ? Q_V : Q_P;
       const double *sp = L.slope + ((IFACE ? 0 : 8) + 2 * m) * F + id;
-      UL[m] = L.q[pl * F + id - st] + sp[-st];
-      UR[m] = L.q[pl * F + id] - sp[F];
+      UL[m] = M ? sp[-st] : L.q[pl * F + id - st] + sp[-st];
+      UR[m] = M ? sp[F] : L.q[pl * F + id] - sp[F];
     }
-    face_flux(L.flux, UL, UR, n1, n2, s, Fl, gas(c));
+    inviscid_states<M>(L, c, UL, UR, n1, n2, s, Fl);
   } else {
     T S0[4][4];
     int scheme = L.scheme;
@@ -794,19 +802,20 @@ static void by_kind(const Lvl &L, Fn f) {
 void launch_prim(const Lvl &L, cudaStream_t s) {
   by_kind(L, [&](auto M) { k_prim<M.value><<<L.ntiles, TILE, 0, s>>>(L); });
 }
-// A level takes the slopes pass if it has planes for it (slope_level, at set-up) and is FP64
-// throughout.  2 x 1024 x 512 cells: slopes 195 us, faces 2 x 217 (205 since), the RK3 step 2.26 ->
+// A level takes the slopes pass if it has planes for it (slope_level, at set-up) and its
+// faces are FP64.  2 x 1024 x 512 cells: slopes 195 us, faces 2 x 217 (205 since), the RK3 step 2.26 ->
 // 2.07 ms.  With the pass everywhere a RANS step of 66 k cells is 1 % slower, a V-cycle of
 // 18 k cells 0.7 %, 16 k cells of an airfoil 0.9 %.
-static bool slopes(const Lvl &L) { return L.slope != nullptr && !L.mixed; }
 bool slope_level(const Lvl &L, long long cells) {
   return cells >= SLOPE_CELLS && L.recon == Recon_Original && L.scheme == Scheme_MUSCL3 && L.gscheme == Scheme_MUSCL3;
 }
-void launch_slopes(const Lvl &L, cudaStream_t s) { k_slopes<<<L.nctiles, TILE, 0, s>>>(L); }
+void launch_slopes(const Lvl &L, cudaStream_t s) {
+  by_kind(L, [&](auto M) { k_slopes<M.value><<<L.nctiles, TILE, 0, s>>>(L); });
+}
 template <bool IFACE>
 static void launch_flux(const Lvl &L, bool fp32, cudaStream_t s) {
   if (fp32) k_flux<true, IFACE, false, float><<<L.nctiles, TILE, 0, s>>>(L);
-  else if (slopes(L)) k_flux<false, IFACE, true, double><<<L.nctiles, TILE, 0, s>>>(L);
+  else if (L.slope) by_kind(L, [&](auto M) { k_flux<M.value, IFACE, true, double><<<L.nctiles, TILE, 0, s>>>(L); });
   else by_kind(L, [&](auto M) { k_flux<M.value, IFACE, false, double><<<L.nctiles, TILE, 0, s>>>(L); });
 }
 void launch_flux_i(const Lvl &L, bool fp32, cudaStream_t s) { launch_flux<true>(L, fp32, s); }
