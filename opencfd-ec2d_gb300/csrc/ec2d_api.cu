@@ -664,7 +664,7 @@ void residual(ec2d_ctx *ctx, int l, int post = 0) {
     else if (L.turb == Turb_SST) K(ctx, "sst", l, 4, [&] { launch_sst(L, s); });
     else if (L.turb == Turb_BL) K(ctx, "bl", l, 2, [&] { launch_bl(L, s); });
   }
-  if (L.slope && !f32) K(ctx, "k_slopes", l, 1, [&] { launch_slopes(L, s); });
+  if (takes_slopes(L) && !f32) K(ctx, "k_slopes", l, 1, [&] { launch_slopes(L, s); });
   // the i- and j-face kernels read the same primitives and write separate
   // planes: they run concurrently on two streams (graph branches); with
   // kernel timing on they run one after the other
@@ -1242,6 +1242,7 @@ int ec2d_setup(ec2d_ctx *ctx) {
     Level &lv = ctx->lv[l];
     long long ncells = 0;
     for (const auto &B : lv.hb) ncells += (long long)(B.nx - 1) * (B.ny - 1);
+    lv.L.slope_fp64 = ncells >= SLOPE_CELLS;
     if (slope_level(lv.L, ncells) && !(lv.L.slope = dalloc<double>(lv, 16 * lv.L.F))) cudaGetLastError();
   }
   CK(cudaDeviceSynchronize());

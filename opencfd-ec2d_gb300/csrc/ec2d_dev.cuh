@@ -97,6 +97,7 @@ struct Lvl {
   double *fi, *fj;          // face-flux scratch, 6 planes each
   double *tb;               // turbulence scratch planes
   double *slope;            // limited MUSCL3 slopes or states, 16 planes (large levels; else null)
+  int slope_fp64;           // the pass also where the context has no FP32 parts
   double *met;              // FDM metrics Akx,Aky,Aix,Aiy,Ajac
   double *fdm;              // FDM scratch planes
   double *lu;               // LU-SGS pre-pass planes (4 NV + 10)

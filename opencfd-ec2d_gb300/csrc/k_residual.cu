@@ -803,19 +803,23 @@ void launch_prim(const Lvl &L, cudaStream_t s) {
   by_kind(L, [&](auto M) { k_prim<M.value><<<L.ntiles, TILE, 0, s>>>(L); });
 }
 // A level takes the slopes pass if it has planes for it (slope_level, at set-up) and its
-// faces are FP64.  2 x 1024 x 512 cells: slopes 195 us, faces 2 x 217 (205 since), the RK3 step 2.26 ->
-// 2.07 ms.  With the pass everywhere a RANS step of 66 k cells is 1 % slower, a V-cycle of
-// 18 k cells 0.7 %, 16 k cells of an airfoil 0.9 %.
+// faces are FP64: from 262,144 cells, in contexts with FP32 parts from 65,536, whose faces
+// save twice as much.  2 x 1024 x 512 cells in FP64: slopes 195 us, faces 2 x 217 (205
+// since), the RK3 step 2.26 -> 2.07 ms; with the pass everywhere a RANS step of 66 k cells
+// is 1 % slower, a V-cycle of 18 k cells 0.7 %, 16 k cells of an airfoil 0.9 %.  With FP32 sweeps
+// an SA residual of 131 k cells 271 -> 254 us, of 66 k 162 -> 158, of 33 k 105 -> 103, of
+// 16 k 74.2 -> 74.9; a V-cycle of 18 k cells 0.4 % slower.
 bool slope_level(const Lvl &L, long long cells) {
-  return cells >= SLOPE_CELLS && L.recon == Recon_Original && L.scheme == Scheme_MUSCL3 && L.gscheme == Scheme_MUSCL3;
+  return cells >= SLOPE_CELLS_MIXED && L.recon == Recon_Original && L.scheme == Scheme_MUSCL3 && L.gscheme == Scheme_MUSCL3;
 }
+bool takes_slopes(const Lvl &L) { return L.slope && (L.mixed || L.slope_fp64); }
 void launch_slopes(const Lvl &L, cudaStream_t s) {
   by_kind(L, [&](auto M) { k_slopes<M.value><<<L.nctiles, TILE, 0, s>>>(L); });
 }
 template <bool IFACE>
 static void launch_flux(const Lvl &L, bool fp32, cudaStream_t s) {
   if (fp32) k_flux<true, IFACE, false, float><<<L.nctiles, TILE, 0, s>>>(L);
-  else if (L.slope) by_kind(L, [&](auto M) { k_flux<M.value, IFACE, true, double><<<L.nctiles, TILE, 0, s>>>(L); });
+  else if (takes_slopes(L)) by_kind(L, [&](auto M) { k_flux<M.value, IFACE, true, double><<<L.nctiles, TILE, 0, s>>>(L); });
   else by_kind(L, [&](auto M) { k_flux<M.value, IFACE, false, double><<<L.nctiles, TILE, 0, s>>>(L); });
 }
 void launch_flux_i(const Lvl &L, bool fp32, cudaStream_t s) { launch_flux<true>(L, fp32, s); }

@@ -1,7 +1,7 @@
 """Residuals of levels at and just below the size from which the limited slopes are
 formed per cell (262144 cells, k_slopes) against the CPU oracle, within the bound of
 the other residual tests; above it also for a scheme that has no slopes, and after
-a switch to FP32 sweeps, which does without them."""
+a switch to FP32 sweeps."""
 import pytest
 
 from ec2d import grids

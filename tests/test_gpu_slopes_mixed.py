@@ -1,5 +1,5 @@
-"""Contexts with FP32 sweeps: a level with the slopes pass (k_slopes, from 262144 cells)
-gives the bits of one without.  Two cases of 131072 cells in one context take the
+"""Contexts with FP32 sweeps: a level with the slopes pass (k_slopes, from 65536 cells)
+gives the bits of one without.  Two cases of 32768 cells in one context take the
 pass, each alone does not; their residuals are the same."""
 import numpy as np
 import pytest
@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 def test_slopes_same_bits(gpu_lib, flux, turb):
     p = Params(Ma=0.6, Re=1e5, If_viscous=int(turb >= 0), Iflag_turbulence_model=max(turb, 0), Iflag_flux=flux,
                Iflag_Scheme=5, CFL=1.0, Time_Method=0, P_outlet=1.0 / (1.4 * 0.36))
-    bl = grids.flat_plate(513, 129, first=2e-3, ratio=1.02)
+    bl = grids.flat_plate(257, 65, first=2e-3, ratio=1.02)
     orc = make_oracle(p, bl)
     orc.init_flow()
     perturb_state(orc, amp=0.02, seed=flux)
