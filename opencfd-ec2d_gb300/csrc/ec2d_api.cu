@@ -2258,7 +2258,14 @@ int ec2d_mlp_loss_grad(ec2d_mlp *m, const float *x, const float *y, int B, doubl
 
 int ec2d_mlp_set_gemm(ec2d_mlp *m, int kind) {
   if (!m || (kind != 0 && kind != 1)) return EC2D_ERR_ARG;
-  m->net.gemm_kind = kind;
+  Net &net = m->net;
+  if (kind == net.gemm_kind) return EC2D_OK;
+  net.gemm_kind = kind;
+  // the copies of the weights that the path reads: training on the mma.sync path
+  // leaves the packed ones of the fused kernels as they were
+  CK(cudaSetDevice(net.device));
+  net.refresh_bf16();
+  CK(cudaGetLastError());
   return EC2D_OK;
 }
 
