@@ -2067,6 +2067,7 @@ int ec2d_mlp_add_samples(ec2d_mlp *m, ec2d_ctx *ctx) {
   if (net.device != ctx->device) return EC2D_ERR_ARG;
   cudaSetDevice(ctx->device);
   const Lvl &L = ctx->lv[1].L;
+  net.drop_graph();  // it holds the samples' place and number
   long long n0 = net.nsamp, n = L.ncell;
   if (net.reserve_samples(n0 + n)) return EC2D_ERR_NOMEM;
   CK(cudaStreamSynchronize(net.stream));
@@ -2084,6 +2085,8 @@ int ec2d_mlp_num_samples(ec2d_mlp *m, long long *n) {
 
 int ec2d_mlp_clear_samples(ec2d_mlp *m) {
   if (!m) return EC2D_ERR_ARG;
+  cudaSetDevice(m->net.device);
+  m->net.drop_graph();
   m->net.nsamp = 0;
   return EC2D_OK;
 }
@@ -2100,10 +2103,10 @@ int ec2d_mlp_train(ec2d_mlp *m, int steps, int batch, double lr, double *loss_ou
   cudaSetDevice(net.device);
   if (net.fused() ? net.ensure_fused(batch) : net.ensure_batch(batch)) return EC2D_ERR_NOMEM;
   // one training step as a CUDA graph (its minibatch seed and Adam step count
-  // live in device memory), re-recorded when batch, rate or GEMM path change
+  // live in device memory), re-recorded when batch, rate or GEMM path change, and
+  // after the samples have (drop_graph)
   if (!net.train_graph || net.graph_batch != batch || net.graph_lr != (float)lr || net.graph_kind != net.gemm_kind) {
-    if (net.train_graph) cudaGraphExecDestroy(net.train_graph);
-    net.train_graph = nullptr;
+    net.drop_graph();
     CK(cudaStreamSynchronize(net.stream));
     CK(cudaStreamBeginCapture(net.stream, cudaStreamCaptureModeThreadLocal));
     net.train_step(batch, (float)lr);

@@ -147,6 +147,7 @@ struct Net {
   void adam(float lr);
   void gather(int B);
   void train_step(int B, float lr);  // minibatch, forward, backward, Adam
+  void drop_graph();
   int fit_normalization();
   int reserve_samples(long long n);
   int predict(const float *feat, long long n, float *pred);

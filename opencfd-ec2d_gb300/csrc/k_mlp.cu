@@ -708,6 +708,15 @@ void Net::train_step(int B, float lr) {
   adam(lr);
 }
 
+// the recorded training step, which holds the addresses of the batch buffers and the
+// samples
+void Net::drop_graph() {
+  if (!train_graph) return;
+  cudaStreamSynchronize(stream);
+  cudaGraphExecDestroy(train_graph);
+  train_graph = nullptr;
+}
+
 int Net::fit_normalization() {
   if (nsamp < 2) return 1;
   cudaMemsetAsync(d_moments, 0, 2 * (NIN + NOUT) * sizeof(double), stream);
