@@ -684,7 +684,8 @@ void residual(ec2d_ctx *ctx, int l, int post = 0) {
   }
   const bool fused = !L.fdm && !dual;  // Res final after k_res: norm partials fused into it
   // Within a step the norms of an evaluation go to the norms branch: the
-  // kernels that follow do not need them, and they are read after the step.
+  // kernels that follow do not need them, and they are read after the step;
+  // whatever writes Res again waits for them (join_norms).
   // Where Res stays as k_res leaves it (no forcing added) and the last CTA would
   // form the norms, k_res goes without them, about half as long (7 against
   // 14 us per launch on the flat plate's levels); where k_res only takes the partials,
@@ -733,6 +734,7 @@ void advance_counters(ec2d_ctx *ctx, int l) {
 // same result.
 void step_euler(ec2d_ctx *ctx, int l, bool fresh = false) {
   if (!fresh) residual(ctx, l);
+  if (l != 1) join_norms(ctx, l);  // the update leaves Res + QF in Res
   K(ctx, "k_euler", l, 1, [&] { launch_euler(ctx->lv[l].L, l != 1, ctx->stream); });
   bc_all(ctx, l);
   advance_counters(ctx, l);
@@ -743,6 +745,7 @@ void step_rk3(ec2d_ctx *ctx, int l) {
   K(ctx, "k_set_un", l, 1, [&] { launch_set_un(L, L.nvar, ctx->stream); });
   for (int k = 0; k < 3; k++) {
     residual(ctx, l);
+    if (l != 1) join_norms(ctx, l);  // the update leaves Res + QF in Res
     K(ctx, "k_rk3", l, 1, [&] { launch_rk3(L, k, l != 1, ctx->stream); });
     bc_all(ctx, l);
   }
@@ -771,7 +774,10 @@ void lusgs_update(ec2d_ctx *ctx, int l, double alfa1, bool force = false) {
       K(ctx, "k_lusgs", l, 2, [&] { go(0); });
     }
   } else {
-    if (force) K(ctx, "k_add_force", l, 1, [&] { launch_add_force(L, ctx->stream); });
+    if (force) {
+      join_norms(ctx, l);
+      K(ctx, "k_add_force", l, 1, [&] { launch_add_force(L, ctx->stream); });
+    }
     K(ctx, "k_lusgs_generic", l, 1, [&] { launch_lusgs(L, alfa1, ctx->stream); });
     K(ctx, "k_add_du", l, 1, [&] { launch_add_du(L, ctx->stream); });
   }
