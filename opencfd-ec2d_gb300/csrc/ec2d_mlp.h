@@ -91,7 +91,20 @@ struct Layer {
 
 constexpr int HOST_SLOTS = 4;  // chunks of a host prediction on the device
 
-struct Net {
+// Buffers of the GEMM path for batches of up to cap_batch rows, and of the fused
+// training pass (width 256; up to cap_fused rows): activations and dZ in 128-row blocks,
+// partial weight gradients of every layer.  Each set is replaced as a whole.
+struct BatchBuf {
+  __nv_bfloat16 *X = nullptr, *H[MAX_HIDDEN] = {}, *dOut = nullptr, *dA = nullptr, *dB = nullptr, *T1 = nullptr,
+                *T2 = nullptr;
+  float *Y = nullptr, *Z[MAX_HIDDEN] = {}, *out = nullptr, *part = nullptr, *cpart = nullptr, *lpart = nullptr;
+};
+struct FusedBuf {
+  __nv_bfloat16 *Xt = nullptr, *Ht[MAX_HIDDEN] = {}, *dZt[MAX_HIDDEN] = {}, *dOt = nullptr;
+  float *fpart = nullptr, *fcpart = nullptr, *lrow = nullptr;
+};
+
+struct Net : BatchBuf, FusedBuf {
   int device = 0, width = 256, nlin = 7;
   unsigned long long seed = 0;
   cudaStream_t stream = nullptr;
@@ -102,16 +115,9 @@ struct Net {
   int gemm_kind = 1;      // 1: tcgen05 GEMMs (default), 0: mma.sync GEMMs
   float *d_loss = nullptr;
   double *d_moments = nullptr;
-  // batch buffers
-  int cap_batch = 0;
-  __nv_bfloat16 *X = nullptr, *H[MAX_HIDDEN] = {}, *dOut = nullptr, *dA = nullptr, *dB = nullptr, *T1 = nullptr,
-                *T2 = nullptr;
-  float *Y = nullptr, *Z[MAX_HIDDEN] = {}, *out = nullptr, *part = nullptr, *cpart = nullptr, *lpart = nullptr;
-  // fused kernels (width 256): activations and dZ in 128-row blocks, partial
-  // weight gradients of every layer, and a second stream for the biases
-  __nv_bfloat16 *Xt = nullptr, *Ht[MAX_HIDDEN] = {}, *dZt[MAX_HIDDEN] = {}, *dOt = nullptr;
-  float *fpart = nullptr, *fcpart = nullptr, *lrow = nullptr;
-  int cap_fused = 0, fpart_ks = 0;
+  int cap_batch = 0, cap_fused = 0;
+  std::vector<void *> batch_mem, fused_mem;  // the memory of the two sets
+  // a second stream for the biases of the fused pass
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // predictions for host rows: a ring of chunks on the device, kept with the net (at

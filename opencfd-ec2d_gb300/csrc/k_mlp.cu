@@ -538,26 +538,65 @@ void Net::refresh_bf16() {
   }
 }
 
+// Buffers of a batch, allocated as a whole: a set that does not fit is given back and
+// leaves the net as it was.  take() puts it in the place of the set in `old`; the
+// stream has come to its end then (drop_graph and the synchronisation before).
+struct Buffers {
+  cudaStream_t stream;
+  std::vector<void *> mem;
+  bool ok = true;
+  template <class T>
+  void get(T *&p, size_t n) {
+    p = nullptr;
+    void *q = nullptr;
+    if (!ok) return;
+    if (cudaMalloc(&q, n * sizeof(T) + 16) != cudaSuccess) {
+      cudaGetLastError();  // the caller reports it
+      ok = false;
+      return;
+    }
+    mem.push_back(q);
+    cudaMemsetAsync(q, 0, n * sizeof(T) + 16, stream);
+    p = (T *)q;
+  }
+  void take(std::vector<void *> &old) {
+    for (void *q : old) cudaFree(q);
+    old.swap(mem);
+    mem.clear();
+  }
+  ~Buffers() {
+    if (!mem.empty()) cudaStreamSynchronize(stream);
+    for (void *q : mem) cudaFree(q);
+  }
+};
+
 int Net::ensure_batch(int B) {
   if (B <= cap_batch) return 0;
-  cap_batch = B;
-  const int W = width;
-  X = dev_alloc<__nv_bfloat16>(owned, (size_t)B * NIN_PAD);
-  Y = dev_alloc<float>(owned, (size_t)B * NOUT);
+  const size_t W = width, n = B;
+  BatchBuf b;
+  Buffers f{stream};
+  f.get(b.X, n * NIN_PAD);
+  f.get(b.Y, n * NOUT);
   for (int l = 0; l < nlin - 1; l++) {
-    H[l] = dev_alloc<__nv_bfloat16>(owned, (size_t)B * W);
-    Z[l] = dev_alloc<float>(owned, (size_t)B * W);
+    f.get(b.H[l], n * W);
+    f.get(b.Z[l], n * W);
   }
-  out = dev_alloc<float>(owned, (size_t)B * NOUT_PAD);
-  dOut = dev_alloc<__nv_bfloat16>(owned, (size_t)B * NOUT_PAD);
-  dA = dev_alloc<__nv_bfloat16>(owned, (size_t)B * W);
-  dB = dev_alloc<__nv_bfloat16>(owned, (size_t)B * W);
-  T1 = dev_alloc<__nv_bfloat16>(owned, (size_t)B * (W > NIN_PAD ? W : NIN_PAD));
-  T2 = dev_alloc<__nv_bfloat16>(owned, (size_t)B * W);
-  part = dev_alloc<float>(owned, (size_t)KSPLIT * W * W);
-  cpart = dev_alloc<float>(owned, (size_t)(B / 256 + 1) * W);
-  lpart = dev_alloc<float>(owned, (size_t)(B / 256 + 1));
-  return part ? 0 : 1;
+  f.get(b.out, n * NOUT_PAD);
+  f.get(b.dOut, n * NOUT_PAD);
+  f.get(b.dA, n * W);
+  f.get(b.dB, n * W);
+  f.get(b.T1, n * (W > NIN_PAD ? W : NIN_PAD));
+  f.get(b.T2, n * W);
+  f.get(b.part, KSPLIT * W * W);
+  f.get(b.cpart, (n / 256 + 1) * W);
+  f.get(b.lpart, n / 256 + 1);
+  if (!f.ok) return 1;
+  drop_graph();
+  cudaStreamSynchronize(stream);
+  f.take(batch_mem);
+  static_cast<BatchBuf &>(*this) = b;
+  cap_batch = B;
+  return 0;
 }
 
 PackArgs Net::pack_args() const {
@@ -587,28 +626,34 @@ static int weight_splits(int B) {
   return ks;
 }
 
-// buffers of the fused training pass; grown, never shrunk, freed with the net
+// buffers of the fused training pass; grown as a whole, never shrunk, freed with the net
 int Net::ensure_fused(int B) {
-  if (!side) {
-    if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming) != cudaSuccess)
-      return 1;
+  if ((!side && cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) ||
+      (!ev_fork && cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming) != cudaSuccess) ||
+      (!ev_join && cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming) != cudaSuccess)) {
+    cudaGetLastError();
+    return 1;
   }
   if (B > cap_fused) {
-    Xt = dev_alloc<__nv_bfloat16>(owned, (size_t)B * 16);
-    dOt = dev_alloc<__nv_bfloat16>(owned, (size_t)B * 16);
+    const size_t n = B;
+    FusedBuf b;
+    Buffers f{stream};
+    f.get(b.Xt, n * 16);
+    f.get(b.dOt, n * 16);
     for (int l = 0; l < nlin - 1; l++) {
-      Ht[l] = dev_alloc<__nv_bfloat16>(owned, (size_t)B * width);
-      dZt[l] = dev_alloc<__nv_bfloat16>(owned, (size_t)B * width);
-      if (!Ht[l] || !dZt[l]) return 1;
+      f.get(b.Ht[l], n * width);
+      f.get(b.dZt[l], n * width);
     }
-    fcpart = dev_alloc<float>(owned, (size_t)(B / 256) * width * nlin);
-    lrow = dev_alloc<float>(owned, B);
-    if (!Xt || !dOt || !fcpart || !lrow) return 1;
+    f.get(b.fcpart, n / 256 * width * nlin);
+    f.get(b.lrow, n);
+    f.get(b.fpart, (size_t)2 * nlin * KSPLIT * 128 * width);
+    if (!f.ok) return 1;
+    drop_graph();
+    cudaStreamSynchronize(stream);
+    f.take(fused_mem);
+    static_cast<FusedBuf &>(*this) = b;
     cap_fused = B;
   }
-  if (!fpart && !(fpart = dev_alloc<float>(owned, (size_t)2 * nlin * KSPLIT * 128 * width))) return 1;
   return 0;
 }
 
@@ -745,8 +790,12 @@ int Net::reserve_samples(long long n) {
   long long cap = cap_samp ? cap_samp : 1 << 20;
   while (cap < n) cap *= 2;
   float *f = nullptr, *t = nullptr;
-  if (cudaMalloc(&f, (size_t)cap * NIN * sizeof(float)) != cudaSuccess) return 1;
-  if (cudaMalloc(&t, (size_t)cap * NOUT * sizeof(float)) != cudaSuccess) { cudaFree(f); return 1; }
+  if (cudaMalloc(&f, (size_t)cap * NIN * sizeof(float)) != cudaSuccess ||
+      cudaMalloc(&t, (size_t)cap * NOUT * sizeof(float)) != cudaSuccess) {
+    cudaGetLastError();  // the caller reports it
+    cudaFree(f);
+    return 1;
+  }
   if (nsamp) {
     cudaMemcpyAsync(f, feat, (size_t)nsamp * NIN * sizeof(float), cudaMemcpyDeviceToDevice, stream);
     cudaMemcpyAsync(t, targ, (size_t)nsamp * NOUT * sizeof(float), cudaMemcpyDeviceToDevice, stream);
@@ -862,8 +911,10 @@ void Net::destroy() {
   cudaSetDevice(device);
   if (stream) cudaStreamSynchronize(stream);
   if (train_graph) cudaGraphExecDestroy(train_graph);
-  for (void *p : owned) cudaFree(p);
-  owned.clear();
+  for (auto *set : {&owned, &batch_mem, &fused_mem}) {
+    for (void *p : *set) cudaFree(p);
+    set->clear();
+  }
   if (feat) cudaFree(feat);
   if (targ) cudaFree(targ);
   if (side) cudaStreamDestroy(side);
