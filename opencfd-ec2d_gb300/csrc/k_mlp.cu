@@ -26,6 +26,9 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <functional>
+#include <memory>
+#include <new>
 #include <vector>
 
 #include "ec2d_dev.cuh"
@@ -842,6 +845,14 @@ int Net::predict(const float *f, long long n, float *pred) {
 // with two allocations and plain copies around one launch, 637 us this way.
 int Net::predict_host(const float *f, long long n, float *pred) {
   std::lock_guard<std::mutex> lock(host_mu);
+  // results that lie on the features of later chunks: from a copy of the features
+  std::unique_ptr<float[]> own;
+  if (std::less<>()(f, (const float *)pred + n * NOUT) && std::less<>()((const float *)pred, f + n * NIN)) {
+    own.reset(new (std::nothrow) float[(size_t)n * NIN]);
+    if (!own) return 1;
+    memcpy(own.get(), f, (size_t)n * NIN * sizeof(float));
+    f = own.get();
+  }
   const long long CH = fused() ? 152 * 128 * 4 : 4 * 16384;
   const long long nch = (n + CH - 1) / CH;
   const int slots = (int)(nch < HOST_SLOTS ? nch : HOST_SLOTS);
