@@ -332,6 +332,11 @@ __device__ __forceinline__ double quot(double a, double b, double y) {
   const double q = a * y;
   return fma(fma(-b, q, a), y, q);
 }
+// the same with infinities (of a, or of the quotient), picked by an integer compare
+__device__ __forceinline__ double quot_any(double a, double b, double y) {
+  const double q = a * y, r = fma(fma(-b, q, a), y, q);
+  return ((unsigned)__double2hiint(q) & 0x7ff00000u) == 0x7ff00000u ? q : r;
+}
 // max(x, 0) and min(x, 0) by the sign (a NaN goes to one of them)
 __device__ __forceinline__ double pos_part(double x) { return __double2hiint(x) >= 0 ? x : 0.0; }
 __device__ __forceinline__ double neg_part(double x) { return __double2hiint(x) < 0 ? x : 0.0; }

@@ -129,7 +129,7 @@ __global__ void k_euler(Lvl L, int force) {
     double r = L.res[m * F + id];
     const double U = L.U[m * F + id];
     if (force && m < 4) { r = r + L.qf[m * F + id]; L.res[m * F + id] = r; }
-    const double du = quot(r, vol, y);
+    const double du = quot_any(r, vol, y);
     L.U[m * F + id] = U + dt * du;
   }
 }
@@ -149,7 +149,7 @@ __global__ void k_rk3(Lvl L, int stage, int force) {
     if (m >= L.nvar) break;
     double r = L.res[m * F + id];
     if (force && m < 4) { r = r + L.qf[m * F + id]; L.res[m * F + id] = r; }
-    const double du = quot(r, vol, y);
+    const double du = quot_any(r, vol, y);
     L.U[m * F + id] = Ra[stage] * L.un[m * F + id] + Rg[stage] * L.U[m * F + id] + dt * Rb[stage] * du;
   }
 }
