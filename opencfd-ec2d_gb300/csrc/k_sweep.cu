@@ -1,6 +1,6 @@
 // k_sweep.cu -- the LU-SGS operator (du_LU_SGS_2D, sub_LU_SGS.f90:4-108) as a
-// latency-optimised wavefront, with one or four lanes per row, and the choice
-// of the wavefront's shape; the eight-lane form is in k_sweep_push.cu.
+// latency-optimised wavefront, with one, four or eight lanes per row in pull form, and the
+// choice of the wavefront's shape; the push form, eight lanes, is in k_sweep_push.cu.
 //
 // The Gauss-Seidel order of the reference is kept exactly: the forward sweep
 // visits hyperplanes p = i+j = 2..nx+ny-2, the backward sweep p = nx+ny-2..2,
@@ -55,7 +55,7 @@ constexpr int TILE = EC2D_TILE;
 //       normal flux is linear in n, so F_n(W, s) = 0.5 s F_n(W, n) and the
 //       constant half F_n(U_nb) of the difference moves into the record
 //  G1I..GCJ  (gamma - 1) times n1, n2 and cc of face i and j,
-//       the pressure coefficients of the four-lane sweep, which ships
+//       the pressure coefficients of the multi-lane sweeps, which ship
 //       p / (gamma - 1)
 template <int NV>
 struct Rec {
@@ -794,32 +794,286 @@ __global__ void __launch_bounds__(QL * QROWS, 1) k_lusgs_sweep_quad(Lvl L, int R
   if (CS > 1) cluster_barrier();  // no CTA leaves while a neighbour may still write into it
 }
 
-// the four-lane kernel serves NV = 4 levels whose blocks have at most 16 bands
-// of rows and QCOLS cells per row, when every CTA of the launch gets an SM of
-// its own (with fewer SMs, one lane per row needs fewer FP64 instructions) and
-// the device can hold one of its clusters
+// ---- eight lanes per row in pull form ------------------------------------------
+//
+// What the push form of k_sweep_push.cu, about 2.4 times as fast, has no room for in
+// shared memory: long rows in tall bands with turbulence variables (192 rows of 1024
+// cells with k and omega: 3.85 ms, 7.2 with one lane per row), and with four variables
+// the sweep without the update.  As the four-lane kernel, but lanes 0-3 add the row's
+// own previous cell and lanes 4-7 the neighbouring row, on operands selected per lane
+// (one FP64 instruction stream for both halves), and a shuffle-add joins them: 15
+// operations per cell and lane.  A CTA holds at most 16 rows.  With NV = 5, 6 every lane
+// also carries the turbulence rows, the upstream neighbour of its half adding F_n(X_2) +
+// (0.5 Lc + Lv) dX as the one-lane sweep does; lane q = 0 of the leading half stores them.
+constexpr int OROWS = 16;  // rows per CTA
+// doubles per row of a slot and per inbox entry: those of the four-lane kernel, then
+// U + dU and dU of each turbulence variable (NV = 5: nu~; 6: k, omega)
+template <int NV>
+constexpr int oslot() { return QS + 2 * (NV - 4); }
+struct ORec {
+  double a, u, c0, k, c, ia;    // k, c: the raw pressure coefficient and 0.5 Lc + Lv of the half's face
+  double2 n;                    // its scaled normal
+  double at[2], ut[2], c0t[2];  // the turbulence rows' A, U and C0
+  double ia5;                   // NV = 5: 1/(alfa + Lv) of the SA row
+};
+// own: lanes 0-3, face i; else face j
+template <int NV>
+struct OLane {
+  using RC = Rec<NV>;
+  int offk, offn, offc;
+  bool own;
+  QLane sel;
+  __device__ __forceinline__ OLane(int q, bool first) : own(first), sel(qlane(q)) {
+    offk = own ? (q == 1 ? RC::G1I : q == 2 ? RC::G2I : RC::GCI) : (q == 1 ? RC::G1J : q == 2 ? RC::G2J : RC::GCJ);
+    offn = own ? RC::N1I : RC::N1J;
+    offc = own ? RC::CI : RC::CJ;
+  }
+};
+template <bool FWD, bool update, int NV>
+__device__ __forceinline__ void oload(ORec &r, const double *rec, int q, const OLane<NV> &l) {
+  using RC = Rec<NV>;
+  if (!FWD || l.own) r.a = __ldcg(rec + RC::A + q);
+  if (FWD || !update) r.u = __ldcg(rec + RC::U + q);
+  if (!FWD && l.own) r.c0 = __ldcg(rec + RC::C0 + q);
+  r.k = __ldcg(rec + l.offk);
+  if (NV == 5) {
+    // the normals sit at odd offsets of a 5-variable record: two 8-byte loads
+    r.n.x = __ldcg(rec + l.offn);
+    r.n.y = __ldcg(rec + l.offn + 1);
+    r.ia5 = __ldcg(rec + RC::IA5);
+  } else {
+    r.n = __ldcg(reinterpret_cast<const double2 *>(rec + l.offn));
+  }
+#pragma unroll
+  for (int t = 0; t < NV - 4; t++) {
+    r.at[t] = __ldcg(rec + RC::A + 4 + t);
+    r.ut[t] = __ldcg(rec + RC::U + 4 + t);
+    if (!FWD) r.c0t[t] = __ldcg(rec + RC::C0 + 4 + t);
+  }
+  r.c = __ldcg(rec + l.offc);
+  r.ia = __ldcg(rec + RC::IA);
+}
+
+// one pass of a band (qpass)
+template <bool update, bool FWD, int NV>
+__device__ __forceinline__ void opass(const Lvl &L, const BlkDev &bd, const QBand &B, double *slot, double *inbox,
+                                      unsigned long long *mbar, unsigned rbox, unsigned rmbar, const double *rsrc,
+                                      double *recBw, double gm1) {
+  using RC = Rec<NV>;
+  constexpr int S = oslot<NV>(), NT = NV - 4;  // turbulence rows
+  const int R = B.R, rl = B.rl, q = B.q, j = B.j, rows = B.rows, ni = B.ni;
+  const long long F = L.F;
+  const OLane<NV> ln(q, !((threadIdx.x >> 2) & 1));
+  const bool own = ln.own;  // the leading half also stores and sends
+  const bool from_box = B.row_ok && (FWD ? (rl == 0 && B.rank > 0) : (rl == R - 1 && (int)B.rank + 1 < B.CS && j < rows));
+  const bool to_box = B.row_ok && !L.silent_band_edge &&
+                      (FWD ? (rl == R - 1 && (int)B.rank + 1 < B.CS && j < rows) : (rl == 0 && B.rank > 0));
+  auto src = [&](int k) { return rsrc + (size_t)(FWD ? k : ni - 1 - k) * RC::N; };
+  const int j0 = (int)B.rank * R + 1, j1 = min((int)B.rank * R + R, rows);
+  const int plo = j0 + 1, phi = j1 + ni;  // planes holding a cell of this band
+  auto pos = [&](int p) { return FWD ? p - plo : phi - p; };
+  ORec r0, r1, r2, r3;
+  if (B.row_ok) {
+    const int m0 = pos(FWD ? j + 1 : ni + j) % 4;  // set of the row's first cell
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      if (c >= ni) break;
+      const int m = (m0 + c) & 3;
+      if (m == 0) oload<FWD, update, NV>(r0, src(c), q, ln);
+      else if (m == 1) oload<FWD, update, NV>(r1, src(c), q, ln);
+      else if (m == 2) oload<FWD, update, NV>(r2, src(c), q, ln);
+      else oload<FWD, update, NV>(r3, src(c), q, ln);
+    }
+  }
+  double wx = 0.0, wu = 0.0, wv = 0.0, wp = 0.0;  // the row's previous cell
+  double wt[2] = {0.0, 0.0}, wd[2] = {0.0, 0.0};   // and its turbulence X + dX, dX
+  int gave_up = 0;                                 // first column whose inbox wait gave up
+  const int gl = (threadIdx.x & 31) & ~7;          // the row's first lane
+  auto plane = [&](int p, const ORec &cur, ORec &ahead) {
+    const int i = p - j, buf = p & 1;
+    const bool act = B.row_ok && i >= 1 && i <= ni;
+    const int k = FWD ? i - 1 : ni - i;
+    if (act && k + 3 < ni) oload<FWD, update, NV>(ahead, src(k + 3), q, ln);
+    double acc = 0.0, acct[2] = {0.0, 0.0};
+    if (act) {
+      // both halves run the same FP64 instructions on their own operands
+      const double *s = slot + ((size_t)(buf ^ 1) * R + min(max(FWD ? rl - 1 : rl + 1, 0), R - 1)) * S;
+      if (!own && from_box) {
+        if (!gave_up && !qwait(mbar + i - 1)) gave_up = i;
+        s = inbox + (size_t)(i - 1) * S;
+      }
+      const double2 uv = *reinterpret_cast<const double2 *>(s + 4);
+      const double sp = s[6], sx = s[q];
+      const bool has = own ? (FWD ? (i > 1) : (i < ni)) : (FWD ? (j > 1) : (j < rows));
+      const double X = own ? wx : sx, Uu = own ? wu : uv.x, Vv = own ? wv : uv.y, P = own ? wp : sp;
+      acc = own ? (FWD ? cur.a : cur.c0) : 0.0;
+#pragma unroll
+      for (int t = 0; t < NT; t++) acct[t] = own ? (FWD ? cur.at[t] : cur.c0t[t]) : 0.0;
+      if (has) {
+        const double w = fma(Uu, cur.n.x, fma(Vv, cur.n.y, cur.c));
+        acc = fma(X, w, fma(P, qcoef(cur.k, ln.sel), acc));
+        if (NT > 0) {
+          // F_n(X_2) + (0.5 Lc + Lv) dX: the dissipation on the increment
+          const double un = fma(Uu, cur.n.x, Vv * cur.n.y);
+#pragma unroll
+          for (int t = 0; t < NT; t++) {
+            const double T2 = own ? wt[t] : s[8 + 2 * t], D2 = own ? wd[t] : s[9 + 2 * t];
+            acct[t] = fma(cur.c, D2, fma(T2, un, acct[t]));
+          }
+        }
+      }
+    }
+    // the two halves of the row add their neighbours' terms
+    const double other = __shfl_xor_sync(0xffffffffu, acc, 4);
+    double othert[2] = {0.0, 0.0};
+#pragma unroll
+    for (int t = 0; t < NT; t++) othert[t] = __shfl_xor_sync(0xffffffffu, acct[t], 4);
+    double st = 0.0, dn = 0.0, stt[2] = {0.0, 0.0}, dnt[2] = {0.0, 0.0};
+    if (act) {
+      acc = acc + other;
+#pragma unroll
+      for (int t = 0; t < NT; t++) {
+        // the turbulence rows never take the fused U update (only the mean
+        // flow is carried as U + dU); the SA row has its own 1/alfa
+        const double inv = NV == 5 ? cur.ia5 : cur.ia;
+        const double a = acct[t] + othert[t];
+        dnt[t] = FWD ? a * inv : fma(a, inv, cur.at[t]);
+        stt[t] = cur.ut[t] + dnt[t];
+      }
+      if (update) {
+        st = fma(acc, cur.ia, FWD ? cur.u : cur.a);
+      } else {
+        dn = FWD ? acc * cur.ia : fma(acc, cur.ia, cur.a);
+        st = cur.u + dn;
+      }
+    }
+    const double s0 = __shfl_sync(0xffffffffu, st, gl), s1 = __shfl_sync(0xffffffffu, st, gl + 1);
+    const double s2 = __shfl_sync(0xffffffffu, st, gl + 2), s3 = __shfl_sync(0xffffffffu, st, gl + 3);
+    if (act) {
+      const double rd = rcp(s0);
+      const double u = s1 * rd, v = s2 * rd;
+      const double pr = fma(-0.5, fma(s2, v, s1 * u), s3);  // p / (gamma - 1)
+      const double H = fma(gm1, pr, s3);
+      const double x = q == 3 ? H : st;
+      if (to_box && own && q == 0) {
+        const unsigned a = rbox + 8u * S * (unsigned)(i - 1), m = rmbar + 8u * (unsigned)(i - 1);
+        qsend2(a, s0, s1, m);
+        qsend2(a + 16u, s2, H, m);
+        qsend2(a + 32u, u, v, m);
+        qsend2(a + 48u, pr, 0.0, m);
+#pragma unroll
+        for (int t = 0; t < NT; t++) qsend2(a + 64u + 16u * t, stt[t], dnt[t], m);
+      }
+      double *o = slot + ((size_t)buf * R + rl) * S;
+      if (own) o[q] = x;
+      if (own && q == 0) *reinterpret_cast<double2 *>(o + 4) = make_double2(u, v);
+      if (own && q == 1) o[6] = pr;
+#pragma unroll
+      for (int t = 0; t < NT; t++) {
+        if (own && q == 2 + t) *reinterpret_cast<double2 *>(o + 8 + 2 * t) = make_double2(stt[t], dnt[t]);
+        wt[t] = stt[t];
+        wd[t] = dnt[t];
+      }
+      wx = x; wu = u; wv = v; wp = pr;
+      if (own && FWD) {
+        recBw[(size_t)(i - 1) * RC::N + RC::A + q] = update ? st : dn;
+#pragma unroll
+        for (int t = 0; t < NT; t++)
+          if (q == 0) recBw[(size_t)(i - 1) * RC::N + RC::A + 4 + t] = dnt[t];
+      } else if (own) {
+        const long long id = bd.off + (long long)(j + 2) * bd.P + (i + 2);
+        if (update) L.U[q * F + id] = st;
+        else L.du[q * F + id] = dn;
+#pragma unroll
+        for (int t = 0; t < NT; t++)
+          if (q == 0) {
+            if (update) L.U[(4 + t) * F + id] = stt[t];
+            else L.du[(4 + t) * F + id] = dnt[t];
+          }
+      }
+    }
+    __syncthreads();
+  };
+  const int np = phi - plo + 1;  // planes of the pass; positions past np - 1 hold no cell
+  for (int t = 0; t < np; t += 4) {
+    plane(FWD ? plo + t : phi - t, r0, r3);
+    plane(FWD ? plo + t + 1 : phi - t - 1, r1, r0);
+    plane(FWD ? plo + t + 2 : phi - t - 2, r2, r1);
+    plane(FWD ? plo + t + 3 : phi - t - 3, r3, r2);
+  }
+  if (gave_up) set_status(L.status + 4 * bd.cas, 4, B.bk, gave_up, j);
+}
+
+template <bool update, int NV>
+__global__ void __launch_bounds__(8 * OROWS, 1) k_lusgs_sweep_oct(Lvl L, int R, int CS) {
+  // [2][R][S] slots | inbox F [ni][S] | inbox B | mbarriers F [ni] | B
+  extern __shared__ __align__(16) double sh[];
+  constexpr int S = oslot<NV>();
+  QBand B;
+  B.rank = CS > 1 ? cluster_rank() : 0u;
+  B.bk = blockIdx.x / CS;
+  const BlkDev bd = L.blk[B.bk];  // by value: no re-reads after global stores
+  B.R = R; B.CS = CS;
+  B.rows = bd.ny - 1;
+  B.ni = bd.nx - 1;
+  B.rl = threadIdx.x / 8;
+  B.q = threadIdx.x & 3;
+  B.j = (int)B.rank * R + B.rl + 1;
+  B.row_ok = B.rl < R && B.j <= B.rows;
+  const int ni = B.ni;
+  const double gm1 = L.cs[bd.cas].gamma - 1.0;
+  double *slot = sh;
+  double *inF = sh + (size_t)2 * R * S, *inB = inF + (size_t)ni * S;
+  unsigned long long *mbF = reinterpret_cast<unsigned long long *>(inB + (size_t)ni * S), *mbB = mbF + ni;
+  unsigned rboxF = 0, rmbF = 0, rboxB = 0, rmbB = 0;
+  if (CS > 1) {
+    for (int t = threadIdx.x; t < 2 * ni; t += blockDim.x) qarm(mbF + t, 8u * S);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if ((int)B.rank + 1 < CS) { rboxF = remote_smem(inF, B.rank + 1); rmbF = remote_smem(mbF, B.rank + 1); }
+    if (B.rank > 0) { rboxB = remote_smem(inB, B.rank - 1); rmbB = remote_smem(mbB, B.rank - 1); }
+    cluster_barrier();  // every inbox armed before any CTA writes into one
+  }
+  const int jr = B.row_ok ? B.j : 1;  // record pointers of idle rows stay in the array
+  const double *recF = L.rec + ((size_t)bd.cell0 + (size_t)(jr - 1) * ni) * Rec<NV>::N;
+  const double *recB = recF + (size_t)L.ncell * Rec<NV>::N;
+  double *recBw = L.rec + ((size_t)L.ncell + bd.cell0 + (size_t)(jr - 1) * ni) * Rec<NV>::N;
+  opass<update, true, NV>(L, bd, B, slot, inF, mbF, rboxF, rmbF, recF, recBw, gm1);
+  opass<update, false, NV>(L, bd, B, slot, inB, mbB, rboxB, rmbB, recB, recBw, gm1);
+  if (CS > 1) cluster_barrier();  // no CTA leaves while a neighbour may still write into it
+}
+
+// These kernels serve levels whose blocks have at most 16 bands of rows and QCOLS cells
+// per row, when every CTA of the launch gets an SM of its own (with fewer SMs, one lane
+// per row needs fewer FP64 instructions) and the device can hold one of its clusters:
+// four lanes with NV = 4 and bands of up to 32 rows; eight with up to 16, and with
+// NV = 4 only without the update, whose push form has room wherever this one has.
 // rmax: most rows per CTA (4..32).  Clusters of more than 8 CTAs are
 // non-portable sizes, asked for explicitly.
 struct QuadShape {
   int CS, R, th;
   size_t smem;
 };
-static QuadShape quad_shape(int max_rows, int max_cols, int rmax) {
+static QuadShape quad_shape(int max_rows, int max_cols, int rmax, int lpr, int nv) {
   QuadShape q;
   rmax = std::max(4, std::min(rmax, QROWS));
   q.CS = (max_rows + rmax - 1) / rmax;
   q.R = (max_rows + q.CS - 1) / q.CS;
-  q.th = (QL * q.R + 31) / 32 * 32;
-  q.smem = (size_t)2 * q.R * QS * sizeof(double) + (q.CS > 1 ? (size_t)max_cols * 2 * (QS * sizeof(double) + 8) : 0);
+  q.th = (lpr * q.R + 31) / 32 * 32;
+  const size_t S = (QS + 2 * (nv - 4)) * sizeof(double);
+  q.smem = 2 * q.R * S + (q.CS > 1 ? (size_t)max_cols * 2 * (S + 8) : 0);
   return q;
+}
+static void (*quad_kernel(int lpr, int update, int nv))(Lvl, int, int) {
+  if (nv == 5) return update ? k_lusgs_sweep_oct<true, 5> : k_lusgs_sweep_oct<false, 5>;
+  if (nv == 6) return update ? k_lusgs_sweep_oct<true, 6> : k_lusgs_sweep_oct<false, 6>;
+  if (lpr == 8) return k_lusgs_sweep_oct<false, 4>;
+  return update ? k_lusgs_sweep_quad<true> : k_lusgs_sweep_quad<false>;
 }
 // the kernel's attributes for a launch of this shape (dynamic shared memory
 // beyond 48 KiB, cluster sizes beyond 8)
-static void quad_attributes(const QuadShape &q) {
-  for (auto kern : {k_lusgs_sweep_quad<true>, k_lusgs_sweep_quad<false>}) {
-    if (q.smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)q.smem);
-    if (q.CS > 8) cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  }
+static void quad_attributes(const QuadShape &q, void (*kern)(Lvl, int, int)) {
+  if (q.smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)q.smem);
+  if (q.CS > 8) cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
 static cudaLaunchConfig_t quad_config(const Lvl &L, const QuadShape &q, cudaLaunchAttribute *attr, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
@@ -835,33 +1089,34 @@ static cudaLaunchConfig_t quad_config(const Lvl &L, const QuadShape &q, cudaLaun
   cfg.numAttrs = 1;
   return cfg;
 }
-static bool quad_fits(const Lvl &L, int max_rows, int max_cols, int rmax) {
+static bool quad_fits(const Lvl &L, int update, int max_rows, int max_cols, int rmax, int lpr) {
   static const int nsm = [] {
     int dev = 0, n = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
     return n;
   }();
-  const QuadShape q = quad_shape(max_rows, max_cols, rmax);
-  if (!(L.nvar == 4 && max_rows >= 1 && q.CS <= 16 && max_cols <= QCOLS && L.nblk * q.CS <= nsm)) return false;
+  if (lpr == 8 ? rmax > OROWS || (L.nvar == 4 && update) : L.nvar != 4) return false;
+  const QuadShape q = quad_shape(max_rows, max_cols, rmax, lpr, L.nvar);
+  if (!(max_rows >= 1 && q.CS <= 16 && max_cols <= QCOLS && L.nblk * q.CS <= nsm)) return false;
   if (q.CS <= 8) return true;
   // a non-portable cluster size: launchable only if the device can place one
-  quad_attributes(q);
+  const auto kern = quad_kernel(lpr, update, L.nvar);
+  quad_attributes(q, kern);
   cudaLaunchAttribute attr[1];
   const cudaLaunchConfig_t cfg = quad_config(L, q, attr, nullptr);
   int nclusters = 0;
-  const bool ok = cudaOccupancyMaxActiveClusters(&nclusters, k_lusgs_sweep_quad<true>, &cfg) == cudaSuccess &&
-                  nclusters >= 1;
+  const bool ok = cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg) == cudaSuccess && nclusters >= 1;
   cudaGetLastError();  // a refused query leaves no error behind
   return ok;
 }
-static void launch_quad(const Lvl &L, int update, int max_rows, int max_cols, int rmax, cudaStream_t s) {
-  const QuadShape q = quad_shape(max_rows, max_cols, rmax);
-  quad_attributes(q);
+static void launch_quad(const Lvl &L, int update, int max_rows, int max_cols, int rmax, int lpr, cudaStream_t s) {
+  const QuadShape q = quad_shape(max_rows, max_cols, rmax, lpr, L.nvar);
+  const auto kern = quad_kernel(lpr, update, L.nvar);
+  quad_attributes(q, kern);
   cudaLaunchAttribute attr[1];
   const cudaLaunchConfig_t cfg = quad_config(L, q, attr, s);
-  if (update) cudaLaunchKernelEx(&cfg, k_lusgs_sweep_quad<true>, L, q.R, q.CS);
-  else cudaLaunchKernelEx(&cfg, k_lusgs_sweep_quad<false>, L, q.R, q.CS);
+  cudaLaunchKernelEx(&cfg, kern, L, q.R, q.CS);
 }
 // lanes per row of a band of at most rmax rows (lanes 0: eight up to 16 rows)
 static int quad_lanes(int rmax, int lanes) { return lanes == 4 || lanes == 8 ? lanes : (rmax <= 16 ? 8 : 4); }
@@ -908,9 +1163,9 @@ void sweep_nv(const Lvl &L, double alfa1, int mode, int max_rows, int max_cols, 
   const int update = mode & LUSGS_UPDATE, force = mode & LUSGS_FORCE;
   const bool prep = !(mode & LUSGS_SWEEP_ONLY), sweep = !(mode & LUSGS_PREP_ONLY);
   if (cs == 0) {
-    // the requested band height and lanes, else other heights: eight lanes
-    // where the shared memory holds the records and inboxes of its warps, four
-    // where it does not (long rows in tall bands)
+    // the requested band height and lanes, else other heights: eight lanes in push form
+    // where the shared memory holds the records and inboxes of its warps; where it does
+    // not (long rows in tall bands), eight in pull form at the requested height, or four
     const bool eight = quad_lanes(rpw, NV > 4 ? 8 : lanes) == 8;
     for (int r : {rpw, 8, 16, 24, 32}) {
       if (!eight || !push_fits(L, update, max_rows, max_cols, r)) continue;
@@ -918,12 +1173,13 @@ void sweep_nv(const Lvl &L, double alfa1, int mode, int max_rows, int max_cols, 
       if (sweep) launch_push(L, update, max_rows, max_cols, r, s);
       return;
     }
-    for (int r : {eight ? 24 : rpw, 24, 32}) {
-      if (!quad_fits(L, max_rows, max_cols, r)) continue;
+    auto quad = [&](int r, int lpr) {
+      if (!quad_fits(L, update, max_rows, max_cols, r, lpr)) return false;
       if (prep) k_lusgs_prep<NV><<<L.nctiles, TILE, 0, s>>>(L, alfa1, force);
-      if (sweep) launch_quad(L, update, max_rows, max_cols, r, s);
-      return;
-    }
+      if (sweep) launch_quad(L, update, max_rows, max_cols, r, lpr, s);
+      return true;
+    };
+    if (quad(rpw, eight ? 8 : 4) || quad(24, 4) || quad(32, 4)) return;
     cs = 1;  // one CTA per block, full warps
     rpw = 32;
   }
