@@ -50,11 +50,12 @@ FALLBACK_HBM = 6800.0
 #   k_add_du  read U(4), dU(4), write U(4)                            = 12 w
 #   k_slopes  read d,u,v,p; write two corrections per variable and
 #             direction (16)                                          = 20 w
+#   k_slopes_i, k_slopes_j  the same for one direction                = 12 w
 #   k_residual_tile  the residual stage in one kernel: read U(4), 7 metrics,
 #             x1, y1 (viscous inverse Jacobians counted as the metrics);
 #             write Res(4), Lci, Lcj, Lvi, Lvj, dt                    = 22 w
 BYTES_PER_UNIT = {"k_prim": 96, "k_flux_i": 128, "k_flux_j": 128, "k_res": 240, "k_lusgs": 256, "k_add_du": 96,
-                  "k_residual_tile": 176, "k_slopes": 160}
+                  "k_residual_tile": 176, "k_slopes": 160, "k_slopes_i": 96, "k_slopes_j": 96}
 
 
 def peaks():

@@ -425,6 +425,7 @@ int build_level(ec2d_ctx *ctx, int l) {
   L.visc = P.If_viscous;
   L.turb = (l == 1) ? P.Iflag_turbulence_model : Turb_NONE;
   L.time_method = P.Time_Method;
+  L.slopes = slope_level(L, L.ncell);
   int nv = L.nvar;
   BlkDev *dblk = dalloc<BlkDev>(lv, lv.blk.size());
   SubDev *dsub = dalloc<SubDev>(lv, lv.sub.size());
@@ -461,7 +462,11 @@ int build_level(ec2d_ctx *ctx, int l) {
   const size_t smem_max = 227 * 1024;
   lv.fast64 = lv.max_rows <= 1024 && lusgs_smem(nv, lv.max_rows) <= smem_max;
   lv.fast32 = lv.max_rows <= 1024 && lusgs32_smem(nv, lv.max_rows) <= smem_max;
-  L.rec = (lv.fast64 || lv.fast32) ? dalloc<double>(lv, (size_t)2 * L.ncell * lusgs_planes(nv)) : nullptr;
+  const size_t nrec = (size_t)2 * L.ncell * lusgs_planes(nv);
+  L.rec = (lv.fast64 || lv.fast32) ? dalloc<double>(lv, nrec) : nullptr;
+  // the sweep records live from their builder to the end of the sweep: between the
+  // primitives and the fluxes their array is free
+  L.slope = (size_t)16 * F <= nrec ? L.rec : nullptr;
   {
     size_t nbcn = 0;
     for (auto &sd : lv.sub)
@@ -664,13 +669,20 @@ void residual(ec2d_ctx *ctx, int l, int post = 0) {
     else if (L.turb == Turb_SST) K(ctx, "sst", l, 4, [&] { launch_sst(L, s); });
     else if (L.turb == Turb_BL) K(ctx, "bl", l, 2, [&] { launch_bl(L, s); });
   }
-  if (takes_slopes(L) && !f32) K(ctx, "k_slopes", l, 1, [&] { launch_slopes(L, s); });
   // the i- and j-face kernels read the same primitives and write separate
   // planes: they run concurrently on two streams (graph branches); with
   // kernel timing on they run one after the other
   // face fluxes of a coarse level in FP32 when selected (the coarse levels
   // only smooth the fine-level correction)
-  if (!ctx->timing && ctx->concurrent) {
+  const bool slopes = takes_slopes(L) && !f32, in_turn = slopes && !L.slope;
+  if (slopes && !in_turn) K(ctx, "k_slopes", l, 1, [&] { launch_slopes(L, SLOPES_I | SLOPES_J, s); });
+  if (in_turn) {
+    // one direction after the other: their slopes take turns in the same planes
+    K(ctx, "k_slopes_i", l, 1, [&] { launch_slopes(L, SLOPES_I, s); });
+    K(ctx, "k_flux_i", l, 1, [&] { launch_flux_i(L, f32, s); });
+    K(ctx, "k_slopes_j", l, 1, [&] { launch_slopes(L, SLOPES_J, s); });
+    K(ctx, "k_flux_j", l, 1, [&] { launch_flux_j(L, f32, s); });
+  } else if (!ctx->timing && ctx->concurrent) {
     ctx->launches += 2;
     cudaEventRecord(ctx->ev_fork, s);
     cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0);
@@ -1242,15 +1254,6 @@ int ec2d_setup(ec2d_ctx *ctx) {
     for (auto &b : ctx->lv[l].blk) mx = std::max(mx, (size_t)(b.nx + 3) * (b.ny + 3) * 6);
   CK(cudaMalloc(&ctx->d_stage, mx * sizeof(double)));
   ctx->stage_n = mx;
-  // slope planes of large levels, after everything that a context cannot do without: where
-  // the memory does not hold them, the faces form their own limiters
-  for (int l = 1; l <= ctx->num_mesh; l++) {
-    Level &lv = ctx->lv[l];
-    long long ncells = 0;
-    for (const auto &B : lv.hb) ncells += (long long)(B.nx - 1) * (B.ny - 1);
-    lv.L.slope_fp64 = ncells >= SLOPE_CELLS;
-    if (slope_level(lv.L, ncells) && !(lv.L.slope = dalloc<double>(lv, 16 * lv.L.F))) cudaGetLastError();
-  }
   CK(cudaDeviceSynchronize());
   ctx->setup_done = true;
   apply_mg_amut(ctx);

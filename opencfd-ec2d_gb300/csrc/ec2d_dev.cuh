@@ -19,7 +19,7 @@ namespace ec2d {
 constexpr int LAP = 2;
 constexpr int LFDM = 4;
 constexpr double PrT = 0.9;
-constexpr int SST_PLANES = 7;  // scratch planes of the SST model
+constexpr int SST_PLANES = 5;  // scratch planes of the SST model
 
 enum { Scheme_UD1 = 0, Scheme_NND2 = 1, Scheme_UD3 = 2, Scheme_WENO3 = 3,
        Scheme_MUSCL2 = 4, Scheme_MUSCL3 = 5, Scheme_OMUSCL2 = 6 };
@@ -94,10 +94,10 @@ struct Lvl {
   const int2 *ctiles;       // the same over the core window (core_ij)
   int nctiles;
   double *U, *q, *amu, *amut, *res, *lc, *du, *geo, *un, *deltu, *qf, *un1;
-  double *fi, *fj;          // face-flux scratch, 6 planes each
+  double *fi, *fj;          // face-flux scratch, 6 planes each (before the fluxes also slopes, k and omega)
   double *tb;               // turbulence scratch planes
-  double *slope;            // limited MUSCL3 slopes or states, 16 planes (large levels; else null)
-  int slope_fp64;           // the pass also where the context has no FP32 parts
+  int slopes;               // MUSCL3 slopes once per cell (k_slopes): 0 no, 1 where the context has FP32 parts, 2 always
+  double *slope;            // their 16 planes, in rec; null: 8 planes of fi, fj and res for a direction at a time
   double *met;              // FDM metrics Akx,Aky,Aix,Aiy,Ajac
   double *fdm;              // FDM scratch planes
   double *lu;               // LU-SGS pre-pass planes (4 NV + 10)

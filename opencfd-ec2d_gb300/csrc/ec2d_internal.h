@@ -24,9 +24,10 @@ void launch_norms(const Lvl &L, bool partials, cudaStream_t s);
 void launch_residual_tile(const Lvl &Lr, const int4 *rt, int ntiles, bool with_norms, int post, cudaStream_t s);
 bool norms_fused_final(const Lvl &L);
 constexpr long long SLOPE_CELLS = 262144, SLOPE_CELLS_MIXED = 65536;  // cells from which a level takes the slopes pass
-bool slope_level(const Lvl &L, long long cells);
+int slope_level(const Lvl &L, long long cells);
 bool takes_slopes(const Lvl &L);
-void launch_slopes(const Lvl &L, cudaStream_t s);
+enum { SLOPES_I = 1, SLOPES_J = 2 };
+void launch_slopes(const Lvl &L, int dirs, cudaStream_t s);
 // k_turb.cu
 void launch_sa(const Lvl &L, cudaStream_t s);
 void launch_sst(const Lvl &L, cudaStream_t s);

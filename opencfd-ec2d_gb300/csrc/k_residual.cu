@@ -96,22 +96,33 @@ __device__ __forceinline__ bool in_fdm_core(const BlkDev &b, int i, int j) {
   return b.fdm && (i >= LFDM + 2 && i <= b.nx - LFDM - 1) && (j >= LFDM + 2 && j <= b.ny - LFDM - 1);
 }
 
-// Limited slopes of a large level's cells in both directions (Lvl::slope, planes 8 dir +
-// 2 variable: to the upper face, + 1: to the lower).  The limiter belongs to the cell, so
-// the two faces of a direction share it: 96 FP64 instructions per cell here and 8 per face
-// for the states, against 2 x 80 where each face forms both of its sides.  M: the planes
+// Limited slopes of a large level's cells, two planes per direction and variable (to the
+// upper face, to the lower).  The limiter belongs to the cell, so the two faces of a
+// direction share it: 96 FP64 instructions per cell here and 8 per face for the states,
+// against 2 x 80 where each face forms both of its sides.  M: the planes
 // hold the states themselves, with the bits that the faces form (batch of 16 airfoils,
 // 0.6 M cells on the finest level: 3.49 -> 3.32 ms per V-cycle).
 // The planes' traffic (256 bytes per cell) hides behind the FP64 pipe, but the launch
-// and the planes pay only on large levels (slope_level).
+// pays only on large levels (slope_level).
+// The planes are memory that holds nothing between the primitives and the fluxes: the
+// array of the sweep records, or, where a level has none (more rows than a CTA's sweep
+// takes) or a smaller one, eight planes for one direction at a time: the turbulence rows
+// of the face fluxes, and the mean-flow rows of Res, which k_res and the FDM patch
+// fill over every interior cell.  Taking turns costs 2 x 1024 x 512 cells 0.8 % of an
+// RK3 step and 0.3 M cells 2 % of a residual against planes of their own.
+__device__ __forceinline__ double *slope_planes(const Lvl &L, bool iface, int m) {
+  if (L.slope) return L.slope + ((iface ? 0 : 8) + 2 * m) * L.F;
+  return m == 0 ? L.fi + 4 * L.F : m == 1 ? L.fj + 4 * L.F : L.res + (2 * m - 4) * L.F;
+}
 template <bool M>
-__global__ void __launch_bounds__(TILE) k_slopes(Lvl L) {
+__global__ void __launch_bounds__(TILE) k_slopes(Lvl L, int dirs) {
   int bk, i, j;
   if (!core_ij(L, bk, i, j)) return;
   const BlkDev &b = L.blk[bk];
   const long long F = L.F, id = fidx(b, i, j);
 #pragma unroll
   for (int dir = 0; dir < 2; dir++) {
+    if (!(dirs & (dir == 0 ? SLOPES_I : SLOPES_J))) continue;
     if (dir == 0 ? j < 1 || j > b.ny - 1 || i < 0 || i > b.nx : i < 1 || i > b.nx - 1 || j < 0 || j > b.ny) continue;
     const long long st = dir == 0 ? 1 : b.P;
 #pragma unroll
@@ -122,8 +133,9 @@ __global__ void __launch_bounds__(TILE) k_slopes(Lvl L) {
       double a, c;
       if constexpr (M) mixed::muscl3_states(q[-st], u, q[st], a, c);
       else muscl3_slopes(u - q[-st], q[st] - u, a, c);
-      L.slope[(8 * dir + 2 * m) * F + id] = a;
-      L.slope[(8 * dir + 2 * m + 1) * F + id] = c;
+      double *sp = slope_planes(L, dir == 0, m) + id;
+      sp[0] = a;
+      sp[F] = c;
     }
   }
 }
@@ -238,7 +250,7 @@ __global__ void __launch_bounds__(TILE) k_flux(Lvl L) {
 #pragma unroll
     for (int m = 0; m < 4; m++) {
       const int pl = m == 0 ? Q_D : m == 1 ? Q_U : m == 2 ? Q_V : Q_P;
-      const double *sp = L.slope + ((IFACE ? 0 : 8) + 2 * m) * F + id;
+      const double *sp = slope_planes(L, IFACE, m) + id;
       UL[m] = M ? sp[-st] : L.q[pl * F + id - st] + sp[-st];
       UR[m] = M ? sp[F] : L.q[pl * F + id] - sp[F];
     }
@@ -802,19 +814,19 @@ static void by_kind(const Lvl &L, Fn f) {
 void launch_prim(const Lvl &L, cudaStream_t s) {
   by_kind(L, [&](auto M) { k_prim<M.value><<<L.ntiles, TILE, 0, s>>>(L); });
 }
-// A level takes the slopes pass if it has planes for it (slope_level, at set-up) and its
-// faces are FP64: from 262,144 cells, in contexts with FP32 parts from 65,536, whose faces
-// save twice as much.  2 x 1024 x 512 cells in FP64: slopes 195 us, faces 2 x 217 (205
+// A level takes the slopes pass if its faces are MUSCL3 on the primitives and in FP64: from
+// 262,144 cells, in contexts with FP32 parts from 65,536, whose faces save twice as much.  2 x 1024 x 512 cells in FP64: slopes 195 us, faces 2 x 217 (205
 // since), the RK3 step 2.26 -> 2.07 ms; with the pass everywhere a RANS step of 66 k cells
 // is 1 % slower, a V-cycle of 18 k cells 0.7 %, 16 k cells of an airfoil 0.9 %.  With FP32 sweeps
 // an SA residual of 131 k cells 271 -> 254 us, of 66 k 162 -> 158, of 33 k 105 -> 103, of
 // 16 k 74.2 -> 74.9; a V-cycle of 18 k cells 0.4 % slower.
-bool slope_level(const Lvl &L, long long cells) {
-  return cells >= SLOPE_CELLS_MIXED && L.recon == Recon_Original && L.scheme == Scheme_MUSCL3 && L.gscheme == Scheme_MUSCL3;
+int slope_level(const Lvl &L, long long cells) {
+  if (L.recon != Recon_Original || L.scheme != Scheme_MUSCL3 || L.gscheme != Scheme_MUSCL3) return 0;
+  return cells >= SLOPE_CELLS ? 2 : cells >= SLOPE_CELLS_MIXED ? 1 : 0;
 }
-bool takes_slopes(const Lvl &L) { return L.slope && (L.mixed || L.slope_fp64); }
-void launch_slopes(const Lvl &L, cudaStream_t s) {
-  by_kind(L, [&](auto M) { k_slopes<M.value><<<L.nctiles, TILE, 0, s>>>(L); });
+bool takes_slopes(const Lvl &L) { return L.slopes == 2 || (L.slopes == 1 && L.mixed); }
+void launch_slopes(const Lvl &L, int dirs, cudaStream_t s) {
+  by_kind(L, [&](auto M) { k_slopes<M.value><<<L.nctiles, TILE, 0, s>>>(L, dirs); });
 }
 template <bool IFACE>
 static void launch_flux(const Lvl &L, bool fp32, cudaStream_t s) {

@@ -180,8 +180,10 @@ constexpr double sk2 = 1.0, sw2 = 0.856, beta2 = 0.0828, Cw2 = 0.440;
 constexpr double a1 = 0.31, betas = 0.09;
 }
 // scratch planes in L.tb
-enum { T_AMUS = 0, T_AMUTS = 1, T_F1 = 2, T_QK = 3, T_QW = 4, T_K = 5, T_W = 6 };
-static_assert(T_W + 1 == SST_PLANES, "planes of the SST scratch");
+enum { T_AMUS = 0, T_AMUTS = 1, T_F1 = 2, T_QK = 3, T_QW = 4 };
+static_assert(T_QW + 1 == SST_PLANES, "planes of the SST scratch");
+// k and omega, in two of the planes that the mean-flow fluxes fill after the model
+enum { FI_K = 0, FI_W = 1 };
 
 // cell pass (sub_turbulence_SST.f90:53-121): eddy viscosity, blending f1 and
 // the k/omega sources; Amu is scaled by Re for the model and scaled back
@@ -199,8 +201,8 @@ __global__ void k_sst_cell(Lvl L) {
   const double *d = L.q + Q_D * F, *U5 = L.U + 4 * F, *U6 = L.U + 5 * F;
   const double dc = d[id], rd = recip_any(dc), K = U5[id] * rd, W = U6[id] * rd;
   // k and omega of every cell that a face reads
-  L.tb[T_K * F + id] = K;
-  L.tb[T_W * F + id] = W;
+  L.fi[FI_K * F + id] = K;
+  L.fi[FI_W * F + id] = W;
   if (i < 1 || i > b.nx - 1 || j < 1 || j > b.ny - 1) return;
   // central differences (their halves cancel in the quotients)
   const double Dix = x1[id + 1] - x1[id - 1], Diy = y1[id + 1] - y1[id - 1];
@@ -256,7 +258,7 @@ __global__ void k_sst_faces(Lvl L) {
   const CaseDev &c = L.cs[b.cas];
   const long long F = L.F, P = b.P;
   long long id = fidx(b, i, j);
-  const double *uu = L.q + Q_U * F, *vv = L.q + Q_V * F, *K = L.tb + T_K * F, *W = L.tb + T_W * F;
+  const double *uu = L.q + Q_U * F, *vv = L.q + Q_V * F, *K = L.fi + FI_K * F, *W = L.fi + FI_W * F;
   const double *amus = L.tb + T_AMUS * F, *amuts = L.tb + T_AMUTS * F, *g = L.geo + id;
   const double f1 = L.tb[T_F1 * F + id];
   const double sk = f1 * sst::sk1 + (1.0 - f1) * sst::sk2;

@@ -1,6 +1,8 @@
 """A batch whose buffers the device does not hold is refused as out of memory, gives
 back what it had taken, and leaves the network as it was: gradients and training
 steps of an earlier batch are those of a network that never asked."""
+import gc
+
 import numpy as np
 import pytest
 import torch
@@ -33,11 +35,12 @@ def test_refused_batch(gpu_lib, kind):
         net.fit_normalization()
         net.train(3, batch=512, lr=1e-3)
         if ask:
+            gc.collect()  # (contexts and nets of other tests)
             free = torch.cuda.mem_get_info()[0]
             with pytest.raises(gpu.EC2DError) as e:
                 net.train(1, batch=TOO_LARGE, lr=1e-3)
             assert e.value.code == EC2D_ERR_NOMEM
-            assert torch.cuda.mem_get_info()[0] == free
+            assert torch.cuda.mem_get_info()[0] >= free
         loss = net.loss_grad(x, y)
         grads = [a for l in range(net.nlin) for a in net.get_grads(l)]
         net.train(3, batch=512, lr=2e-3)  # a step recorded after the refusal
