@@ -109,8 +109,8 @@ __global__ void k_sa_faces(Lvl L) {
 
 // (a / b)^(1/6), b >= 64: w = (b / a)^(-1/6) to about 2^-19 in FP32, then one step of
 // Householder's third-order iteration for w^-6 = b / a.  The float w has exact squares,
-// so the error stays below an ulp; 9 FP64 instructions against about 40 of
-// cbrt(sqrt(a / b)), which serves the rest of the range.
+// so the relative error stays below 0.84 eps (0.73 in 4e6 samples; 0.78 of cbrt(sqrt(a / b)));
+// 9 FP64 instructions against about 40 of those functions, which serve the rest of the range.
 __device__ __forceinline__ double sixth_root(double a, double ra, double b) {
   if (!(at_least(b, 64.0) && below(b, 1.0e37))) return cbrt(sqrt(a * recip(b)));
   const double q = b * ra, w = to_double(exp2f(log2f(to<float>(q)) * (-1.0f / 6.0f)));
