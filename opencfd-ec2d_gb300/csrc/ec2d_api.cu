@@ -2248,7 +2248,7 @@ int ec2d_mlp_loss_grad(ec2d_mlp *m, const float *x, const float *y, int B, doubl
   if (!m || !x || !y || B < 256 || B % 256) return EC2D_ERR_ARG;
   Net &net = m->net;
   cudaSetDevice(net.device);
-  if (net.ensure_batch(B) || (net.fused() && net.ensure_fused(B))) return EC2D_ERR_NOMEM;
+  if (net.fused() ? net.ensure_fused(B) || net.ensure_stage(B) : net.ensure_batch(B)) return EC2D_ERR_NOMEM;
   std::vector<__nv_bfloat16> xb((size_t)B * NIN_PAD, __float2bfloat16(0.0f));
   for (int r = 0; r < B; r++)
     for (int c = 0; c < NIN; c++) xb[(size_t)r * NIN_PAD + c] = __float2bfloat16(x[(size_t)r * NIN + c]);

@@ -91,20 +91,24 @@ struct Layer {
 
 constexpr int HOST_SLOTS = 4;  // chunks of a host prediction on the device
 
-// Buffers of the GEMM path for batches of up to cap_batch rows, and of the fused
+// Standardised rows that a host or the GEMM path's gather hands over (up to cap_stage
+// rows); buffers of the GEMM path for batches of up to cap_batch rows; and of the fused
 // training pass (width 256; up to cap_fused rows): activations and dZ in 128-row blocks,
 // partial weight gradients of every layer.  Each set is replaced as a whole.
+struct StageBuf {
+  __nv_bfloat16 *X = nullptr;
+  float *Y = nullptr;
+};
 struct BatchBuf {
-  __nv_bfloat16 *X = nullptr, *H[MAX_HIDDEN] = {}, *dOut = nullptr, *dA = nullptr, *dB = nullptr, *T1 = nullptr,
-                *T2 = nullptr;
-  float *Y = nullptr, *Z[MAX_HIDDEN] = {}, *out = nullptr, *part = nullptr, *cpart = nullptr, *lpart = nullptr;
+  __nv_bfloat16 *H[MAX_HIDDEN] = {}, *dOut = nullptr, *dA = nullptr, *dB = nullptr, *T1 = nullptr, *T2 = nullptr;
+  float *Z[MAX_HIDDEN] = {}, *out = nullptr, *part = nullptr, *cpart = nullptr, *lpart = nullptr;
 };
 struct FusedBuf {
   __nv_bfloat16 *Xt = nullptr, *Ht[MAX_HIDDEN] = {}, *dZt[MAX_HIDDEN] = {}, *dOt = nullptr;
   float *fpart = nullptr, *fcpart = nullptr, *lrow = nullptr;
 };
 
-struct Net : BatchBuf, FusedBuf {
+struct Net : StageBuf, BatchBuf, FusedBuf {
   int device = 0, width = 256, nlin = 7;
   unsigned long long seed = 0;
   cudaStream_t stream = nullptr;
@@ -115,8 +119,8 @@ struct Net : BatchBuf, FusedBuf {
   int gemm_kind = 1;      // 1: tcgen05 GEMMs (default), 0: mma.sync GEMMs
   float *d_loss = nullptr;
   double *d_moments = nullptr;
-  int cap_batch = 0, cap_fused = 0;
-  std::vector<void *> batch_mem, fused_mem;  // the memory of the two sets
+  int cap_stage = 0, cap_batch = 0, cap_fused = 0;
+  std::vector<void *> stage_mem, batch_mem, fused_mem;  // the memory of the sets
   // a second stream for the biases of the fused pass
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -142,6 +146,7 @@ struct Net : BatchBuf, FusedBuf {
   void refresh_bf16();
   void gemm(const __nv_bfloat16 *A, int lda, const __nv_bfloat16 *B, int ldb, int M, int N, int K, int ksplit,
             const Epi &e);
+  int ensure_stage(int B);
   int ensure_batch(int B);
   bool fused() const { return width == 256 && gemm_kind == 1; }
   int ensure_fused(int B);

@@ -573,13 +573,26 @@ struct Buffers {
   }
 };
 
+int Net::ensure_stage(int B) {
+  if (B <= cap_stage) return 0;
+  StageBuf b;
+  Buffers f{stream};
+  f.get(b.X, (size_t)B * NIN_PAD);
+  f.get(b.Y, (size_t)B * NOUT);
+  if (!f.ok) return 1;
+  drop_graph();
+  cudaStreamSynchronize(stream);
+  f.take(stage_mem);
+  static_cast<StageBuf &>(*this) = b;
+  cap_stage = B;
+  return 0;
+}
+
 int Net::ensure_batch(int B) {
   if (B <= cap_batch) return 0;
   const size_t W = width, n = B;
   BatchBuf b;
   Buffers f{stream};
-  f.get(b.X, n * NIN_PAD);
-  f.get(b.Y, n * NOUT);
   for (int l = 0; l < nlin - 1; l++) {
     f.get(b.H[l], n * W);
     f.get(b.Z[l], n * W);
@@ -593,7 +606,7 @@ int Net::ensure_batch(int B) {
   f.get(b.part, KSPLIT * W * W);
   f.get(b.cpart, (n / 256 + 1) * W);
   f.get(b.lpart, n / 256 + 1);
-  if (!f.ok) return 1;
+  if (!f.ok || ensure_stage(B)) return 1;
   drop_graph();
   cudaStreamSynchronize(stream);
   f.take(batch_mem);
@@ -922,7 +935,7 @@ void Net::destroy() {
   cudaSetDevice(device);
   if (stream) cudaStreamSynchronize(stream);
   if (train_graph) cudaGraphExecDestroy(train_graph);
-  for (auto *set : {&owned, &batch_mem, &fused_mem}) {
+  for (auto *set : {&owned, &stage_mem, &batch_mem, &fused_mem}) {
     for (void *p : *set) cudaFree(p);
     set->clear();
   }

@@ -50,3 +50,21 @@ def test_refused_batch(gpu_lib, kind):
     for a, b in zip(*outs):
         np.testing.assert_array_equal(a, b)
     s.close()
+
+
+def _taken(kind, call):
+    net = gpu.WarmStartNet(hidden=6, width=256, seed=3)
+    net.set_gemm(kind)
+    gc.collect()
+    free = torch.cuda.mem_get_info()[0]
+    call(net)
+    n = free - torch.cuda.mem_get_info()[0]
+    net.close()
+    return n
+
+
+def test_gradients_of_large_batches(gpu_lib):
+    """the fused kernels take no more than the separate ones, whose buffers they do without"""
+    x, y = np.zeros((65536, mo.NIN), np.float32), np.zeros((65536, mo.NOUT), np.float32)
+    _taken(1, lambda net: net.loss_grad(x[:256], y[:256]))
+    assert _taken(1, lambda net: net.loss_grad(x, y)) <= _taken(0, lambda net: net.loss_grad(x, y))
