@@ -362,8 +362,9 @@ int ec2d_mlp_predict(ec2d_mlp *m, const float *feat, long long n, float *pred);
  * every candidate launch configuration on the context's own cases and keeps
  * the fastest: the shape of the FP64 LU-SGS wavefront (lusgs_cs = 0: row
  * bands of at most rows_per_warp rows on the CTAs of a cluster, eight lanes
- * per row for bands of up to 16 rows and four for taller ones, where the
- * level has 4 variables, at most 8 bands and 1024 cells per row, else as 1;
+ * per row for bands of up to 16 rows and, with 4 variables, four for taller
+ * ones, where a block has at most 16 bands, every band gets an SM and its
+ * rows fit shared memory, else as 1;
  * 1: one CTA per block with rows_per_warp (32, 24 or 16) rows per warp; 2, 4,
  * 8: a thread-block cluster of that many CTAs with a barrier per plane) and
  * whether independent kernels run concurrently on two stream pairs (the i-

@@ -101,7 +101,7 @@ struct Lvl {
   double *met;              // FDM metrics Akx,Aky,Aix,Aiy,Ajac
   double *fdm;              // FDM scratch planes
   double *lu;               // LU-SGS pre-pass planes (4 NV + 10)
-  double *rec;              // LU-SGS per-cell sweep records: [2 passes][ncell][4 NV + 10]
+  double *rec;              // LU-SGS per-cell sweep records, [2 passes][ncell][lusgs_planes(NV)] (null: rows too many)
   double2 *bcn;             // unit normals of the far-field and symmetry boundary nodes
   int ncell;                // interior cells of the level (all blocks of all cases)
   double *npart;            // norm partials: per tile 2*6 doubles
@@ -109,7 +109,7 @@ struct Lvl {
   const int *case_tile0, *case_ntile, *case_ncell;  // per case: first tile, tiles, interior cells
   unsigned *nctr;           // tiles of k_res done (the last one reduces the partials)
   int *status;              // per case: code, block, i, j
-  int silent_band_edge;     // test hook: band edges of the four-lane wavefront send nothing
+  int silent_band_edge;     // test hook: band edges of the banded wavefronts send nothing
   int mixed;                // a context with FP32 parts: arithmetic of ec2d_mixed.cuh
   int keep_amut;            // coarse level: amut is restricted from the finer level, not zeroed
 };

@@ -21,14 +21,15 @@
 // needed both operands transposed.
 //
 // Measured (GB300, 6 hidden layers): a training step of 16,384 rows 742 -> 168
-// us (tile kernel 86 us, weight gradients 25, reduce 13; ncu), 46 -> 194 TFLOP/s;
+// us (tile kernel 88 us, weight gradients 27, reduce 17, and beside those two the column
+// sums 24 and the bias update 13; each alone, ncu), 46 -> 194 TFLOP/s;
 // predictions of 300,007 rows 2.9 -> 0.43 ms in the kernel.  The training tile
 // kernel is bound by the weights its 128 CTAs each read from L2 (310 MB a step).
 //
 // Arithmetic is that of the separate kernels (k_gemm_tc.cu, k_mlp.cu): BF16
 // operands, FP32 accumulation over K in steps of 16 in the same order, the
 // same splits of the batch summed in the same order, so a training run gives
-// the same weights.
+// the same weights (below z = -87 SiLU is about -1e-36 here and rounds to -0 there).
 //
 // Layout.  Activations (and dZ) of 128 rows x 256 columns are a block of 8 x 8
 // core matrices of 128 contiguous bytes (8 rows of 16 bytes): row group r / 8

@@ -248,7 +248,7 @@ __global__ void k_sst_cell(Lvl L) {
 // k and omega come from planes that k_sst_cell fills once per cell, and the normal
 // derivatives from the set-up coefficients, where each face divided twelve times by the
 // density and formed its Jacobian: the four kernels of the model on 65 k cells take
-// 54 us instead of 125.
+// 55 us instead of 125.
 // k and omega face fluxes, i faces (sub_turbulence_SST.f90:129-182) and j
 // faces (:198-248); planes 4/5 of fi and fj
 __global__ void k_sst_faces(Lvl L) {
